@@ -8,7 +8,7 @@ kinds of contraction tree.  ``run`` resets the state where the pass starts from
 
 The outputs are what does not depend on the gauge of the singular vectors: the
 state vector, amplitudes, expectation values, gradients, shots, and the bonds
-and split paths as whole numbers.
+as whole numbers.
 """
 from __future__ import annotations
 
@@ -156,9 +156,10 @@ def _random_mps(n, chi, seed):
 
 
 def _padded_mps(n, chi, rank, seed):
-    """A random state of bond rank `rank` carried at bond `chi` on every inner bond."""
+    """A random state of bond rank `rank` carried at bond `chi` on every inner
+    bond, its norm brought down as truncation does (no split renormalises)."""
     rng = np.random.default_rng(seed)
-    core = _random_mps(n, rank, seed)
+    core = [0.03 * t for t in _random_mps(n, rank, seed)]
     frames = [np.ones((1, 1))]
     for q in range(n - 1):
         r = core[q].shape[2]
@@ -268,9 +269,8 @@ def run(state):
         for q, t in enumerate(state["sites"]):
             m.set_site(q, t)
         m.apply_gates(state["gates"])
-        rec = m.split_records()
-        return {"state": m.contract_to_statevector(), "bonds": m.bond_dims(), "kept": rec["chi"].copy(),
-                "path": rec["path"].copy()}
+        return {"state": m.contract_to_statevector(), "bonds": m.bond_dims(),
+                "kept": m.split_records()["chi"].copy()}
     if kind == "batch":
         b = state["batch"]
         b.reset()
@@ -567,7 +567,7 @@ def exact(case, seed):
     if kind == "loaded":
         n = case["n"]
         m = _Mps(n, case["chi"], _padded_mps(n, case["chi"], case["rank"], seed)).apply(_step(n))
-        return {"state": m.dense(), "bonds": None, "kept": None, "path": None}
+        return {"state": m.dense(), "bonds": None, "kept": None}
     if kind == "batch":
         return {"amplitudes": np.array([_Mps(n, chi).apply(g).zero()
                                         for n, chi, g in _slices(case, seed)]), "bonds": None}
