@@ -162,18 +162,19 @@ struct Op {
 
 // Launch shape of one Jacobi phase for a group of jobs.
 struct PhaseCfg {
-    int C = 0;            // cluster size
+    int C = 0;            // cluster size (the largest of the group's tasks)
     size_t smem = 0;
-    int threads = 0;      // one warp per column pair of a block, at most kJacobiThreads
+    int threads = 0;      // one warp per column of a block
     bool staged = false;  // jacobi_staged_kernel with blocks of b columns
-    bool reg = false;     // cluster Jacobi variant with register-resident top columns
+    int kr = 0;           // row groups of the cluster Jacobi's instance
     int b = 0;
+    int idx_off = 0;      // task list
 };
 
 // Jobs of one wave whose SVDs share launch shapes: one phase in the plain
 // form; the complex64 first phase and the FP64 finish in the precision form.
 struct Group {
-    int mode, idx_off, count;
+    int mode, count;
     int nph = 1;
     PhaseCfg ph[2];
 };
@@ -362,8 +363,10 @@ std::once_flag g_attr_once;
 cudaError_t g_attr_err = cudaSuccess;
 
 void set_kernel_attributes() {
-    for (const void* f : {jacobi_kernel(false, false), jacobi_kernel(true, false), jacobi_kernel(false, true),
-                          jacobi_kernel(true, true), jacobi_staged(false), jacobi_staged(true)}) {
+    std::vector<const void*> jacobi = jacobi_ring_kernels();
+    jacobi.push_back(jacobi_staged(false));
+    jacobi.push_back(jacobi_staged(true));
+    for (const void* f : jacobi) {
         if (g_attr_err == cudaSuccess)
             g_attr_err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemLimit));
         if (g_attr_err == cudaSuccess)
@@ -379,62 +382,68 @@ void set_kernel_attributes() {
         g_attr_err = cudaFuncSetAttribute(amplitude_zero_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
 }
 
-int round_up(int x, int q) { return ((x + q - 1) / q) * q; }
+// Launch shape of a cluster Jacobi task: C CTAs (a power of two), blocks of b
+// columns, kr row groups.
+struct RingShape {
+    int C = 0, b = 0, kr = 0, warps = 0;
+    size_t smem = 0;
+};
 
-// Cluster size for a Jacobi SVD of an M x N working matrix.  Every sweep has
-// N'-1 steps (N' = N padded to a multiple of 4C) whatever C is; a larger C
-// gives each CTA fewer column pairs per step (b = N'/2C) but adds 2C-1 block
-// exchanges per sweep.  The model below (FP64 work per step and CTA, a floor
-// for one pair's latency, a fixed cost per exchange plus its DSMEM traffic)
-// picks the fastest sweep when the wave's splits cannot fill the GPU, and the
-// least SM-time per split when they can.
-// Cluster size of a Jacobi group, from clock64 measurements of the kernel.
-// A single state is latency-bound (a few splits per level): a round costs
-// its shared-memory traffic at 64 B/clk (at least ~0.3 us) and a block
-// exchange ~2 us plus its DSMEM stores; blocks wider than the register
-// variant's 12 warps are not considered for columns it can hold, and once
-// the wave's clusters would fill the GPU the cost counts SM time.  A batch
-// is throughput-bound (its waves fill the GPU), so SM time (sweep time x C)
-// decides for every wave, with the round cost of the variant that runs it:
-// the dependent rotation chain (~1900 cycles with the top column in
-// registers, ~1300 without) or 3 or 6 passes of the partner columns at
-// 128 B/clk, whichever is larger, and ~4600 cycles per exchange.  That
-// choice depends on the shape alone, so a slice's results do not depend on
-// the other slices of its batch.
-bool jacobi_reg_variant(int M, int b) { return M <= kJacobiRegMaxRows && b <= kJacobiRegThreads / 32; }
+// The shape of an M x N working matrix (with vrows rows of V under it) on C
+// CTAs; false when it does not fit.  A block of odd width takes one warp more,
+// for the pairs inside the blocks.
+bool ring_shape(int M, int N, int vrows, size_t elem, int C, RingShape* out) {
+    const bool fp32 = elem == sizeof(float2);
+    RingShape s;
+    s.C = C;
+    s.b = (N + 2 * C - 1) / (2 * C);
+    s.kr = jacobi_ring_kr(fp32, M, vrows);
+    if (s.kr == 0) return false;
+    s.warps = s.b + (s.b & 1);
+    s.smem = jacobi_ring_smem(s.b, s.kr, elem);
+    if (s.warps > jacobi_ring_warps(s.kr, int(elem)) || s.smem > kSmemLimit) return false;
+    *out = s;
+    return true;
+}
 
-// len: rows stored per column (M, or M + N when the precision form's first
-// phase carries V).
+// Cluster size of a Jacobi task.  A sweep is (2C - 1) b + b rounds of rotation
+// (about N whatever C is) and 2C - 1 block moves with a cluster barrier.  A
+// round costs its dependent chain and the part of its FP64 work (20
+// instructions per row group and column) that the chain does not hide; the
+// constants are cycles measured on single SVDs of 8 to 384 columns.  A single
+// state is latency-bound (a few splits per level) and takes the shortest
+// sweep, until the wave's clusters would fill the GPU, from where SM time
+// counts.  A batch fills the GPU, so SM time decides, with as many CTAs on an
+// SM as fit it, but never less than the FP64 work; that choice depends on the
+// shape alone, so a slice's results do not depend on the other slices of its
+// batch.  0: no cluster size fits.
 int choose_cluster(const wqc_cuda_ctx* ctx, int M, int N, int max_c, int njobs, int sm_count, size_t elem,
-                   bool throughput, int len = 0) {
-    if (len <= 0) len = M;
+                   bool throughput, int vrows = 0) {
+    RingShape s;
     if (ctx) {
-        auto fits = [&](int Cc) { return Cc >= 1 && Cc <= max_c && jacobi_smem_bytes(len, N, Cc, elem) <= kSmemLimit; };
+        auto fits = [&](int Cc) { return Cc >= 1 && Cc <= max_c && !(Cc & (Cc - 1)) && ring_shape(M, N, vrows, elem, Cc, &s); };
         if (ctx->force_C > 0 && fits(ctx->force_C)) return ctx->force_C;
         for (const auto& t : ctx->tuned)
-            if (t.M == M && t.N == N && t.len == len && t.elem == int(elem) && t.throughput == int(throughput) &&
-                fits(t.C))
+            if (t.M == M && t.N == N && t.len == M + vrows && t.elem == int(elem) &&
+                t.throughput == int(throughput) && fits(t.C))
                 return t.C;
     }
-    int best = -1;
+    int best = 0;
     double best_cost = 1e300;
-    for (int Cc = 1; Cc <= max_c; ++Cc) {
-        if (jacobi_smem_bytes(len, N, Cc, elem) > kSmemLimit) continue;
-        const int Np = round_up(N, 4 * Cc), b = Np / (2 * Cc);
-        const int max_b = throughput ? kJacobiThreads / 32 : jacobi_max_warps(M);
-        if (b > max_b && Cc < max_c) continue;  // more pairs than warps
-        double cost;
+    for (int Cc = 1; Cc <= std::min(max_c, kJacobiRingMaxCluster); Cc *= 2) {
+        if (!ring_shape(M, N, vrows, elem, Cc, &s)) continue;
+        const double work = 10.0 * s.kr * s.b * double(elem) / sizeof(double2);  // FP64 pipe cycles of a round
+        const double round = 620.0 + 20.0 * s.kr + 0.6 * work;
+        const double rounds = 2.0 * Cc * s.b;
+        const double moves = Cc > 1 ? (2 * Cc - 1) * 700.0 + 2500.0 : 200.0;
+        double cost = rounds * round + moves;
         if (throughput) {
-            const bool reg = jacobi_reg_variant(M, b);
-            const double traffic = (reg ? 3.0 : 6.0) * double(elem) * b * len / 128.0;
-            const double round = std::max(reg ? 1900.0 : 1300.0, traffic);
-            const double cycles = Np * round + (Cc > 1 ? (2 * Cc - 1) * 4600.0 : 0.0);
-            cost = cycles / 1900.0 * Cc;  // SM-microseconds at ~1.9 GHz
-        } else {
-            const double step = std::max(0.3, b * (8.0 * M + 12.0 * len) / 64.0 / 1900.0);
-            const double exch = Cc > 1 ? 2.0 + 2.0 * b * len * 16.0 / 1.0e5 : 0.0;
-            cost = (Np - 1) * step + (2 * Cc - 1) * exch;
-            if (double(njobs) * Cc >= 1.5 * sm_count) cost *= Cc;
+            const int by_threads = 2048 / (32 * s.warps), by_smem = int(kSmemLimit / s.smem);
+            const int by_regs = 65536 / (32 * s.warps * std::min(255, 2 * s.kr * int(elem) / 4 + 48));
+            const int ctas = std::max(1, std::min(std::min(by_threads, by_smem), by_regs));
+            cost = Cc * std::max(cost / ctas, rounds * work);
+        } else if (double(njobs) * Cc >= 1.5 * sm_count) {
+            cost *= Cc;
         }
         if (cost < best_cost) {
             best_cost = cost;
@@ -694,20 +703,26 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                 w.oq_count = int(lb.oq.size());
                 first = false;
             }
-            // Jacobi groups: key (mode, shape of phase 1, shape of phase 2);
-            // a shape is a cluster size, or -b for the staged kernel with
-            // blocks of b columns.
+            // Jacobi groups: the tasks of a mode that run in one launch (one
+            // per phase).  Launches of a stream follow one another, so a
+            // latency-bound wave puts all of a mode's cluster tasks into one
+            // launch, whatever their shapes: it lasts as long as its longest
+            // task.  A batch keeps tasks of unlike column length apart, whose
+            // registers and shared memory would be those of the longest.
             struct GKey {
                 int mode, k1, k2;
             };
-            std::vector<std::pair<GKey, std::vector<int>>> groups;
-            auto add = [&](int mode, int k1, int k2, int local) {
+            struct Task {
+                int local, c1, c2;  // job of the wave, cluster size per phase
+            };
+            std::vector<std::pair<GKey, std::vector<Task>>> groups;
+            auto add = [&](int mode, int k1, int k2, const Task& t) {
                 for (auto& g : groups)
                     if (g.first.mode == mode && g.first.k1 == k1 && g.first.k2 == k2) {
-                        g.second.push_back(local);
+                        g.second.push_back(t);
                         return;
                     }
-                groups.push_back({{mode, k1, k2}, {local}});
+                groups.push_back({{mode, k1, k2}, {t}});
             };
             auto shape = [&](size_t k, int& rows, int& cols, int& ell) {
                 rows = 2 * lb.bounds[k].first;
@@ -738,21 +753,23 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                 remaining -= sel.size();
             }
             const int nj_wave = int(sel.size());
-            // A shape beyond every cluster's shared memory goes to the staged
-            // kernel (0: no kernel takes it).
-            auto cluster_or_staged = [&](int M, int N, size_t elem, int len) {
-                const int c =
-                    choose_cluster(m->ctx, M, N, m->ctx->max_cluster, nj_wave, m->ctx->sm_count, elem, m->batch, len);
-                return c >= 1 ? c : -jacobi_staged_b(len, N, elem, kSmemLimit, nullptr);
+            // A shape beyond every cluster goes to the staged kernel: its key
+            // is -b, the width of its blocks (0: no kernel takes it).
+            auto key_of = [&](int M, int N, size_t elem, int vrows, int& c) {
+                c = choose_cluster(m->ctx, M, N, m->ctx->max_cluster, nj_wave, m->ctx->sm_count, elem, m->batch, vrows);
+                if (c < 1) return -jacobi_staged_b(M + vrows, N, elem, kSmemLimit, nullptr);
+                return m->batch ? jacobi_ring_kr(elem == sizeof(float2), M, vrows) : 1;
             };
-            auto keys = [&](int M, int N, int& k1, int& k2) {
+            auto add_task = [&](int mode, int M, int N, int local) {
+                Task t{local, 0, 0};
+                int k1, k2 = 0;
                 if (m->fp32) {
-                    k1 = cluster_or_staged(M, N, sizeof(float2), M + N);
-                    k2 = cluster_or_staged(M, N, sizeof(double2), M);
+                    k1 = key_of(M, N, sizeof(float2), N, t.c1);
+                    k2 = key_of(M, N, sizeof(double2), 0, t.c2);
                 } else {
-                    k1 = cluster_or_staged(M, N, sizeof(double2), M);
-                    k2 = 0;
+                    k1 = key_of(M, N, sizeof(double2), 0, t.c1);
                 }
+                add(mode, k1, k2, t);
             };
             w.jobs_off = int(plan.jobs.size());
             w.njobs = nj_wave;
@@ -772,62 +789,63 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                 w.max_rows = std::max(w.max_rows, rows);
                 w.max_cols = std::max(w.max_cols, cols);
                 w.max_ell = std::max(w.max_ell, ell);
-                int M, N, k1, k2;
+                int M, N;
                 dims(k, kJacobiExact, M, N);
-                keys(M, N, k1, k2);
-                add(kJacobiExact, k1, k2, local);
+                add_task(kJacobiExact, M, N, local);
                 if (rs) {
                     w.any_rsvd = true;
-                    add(kJacobiFallback, k1, k2, local);
+                    add_task(kJacobiFallback, M, N, local);
                     dims(k, kJacobiRsvd, M, N);
-                    keys(M, N, k1, k2);
-                    add(kJacobiRsvd, k1, k2, local);
+                    add_task(kJacobiRsvd, M, N, local);
                 }
             }
-            // Launch shape of one phase for the jobs of a group.
-            auto fill = [&](PhaseCfg& pc, int key, int mode, const std::vector<int>& locals, size_t elem, bool with_v) {
-                size_t sm = 0;
-                int bmax = 1, mmax = 1;
-                if (key < 0) {
+            // Launch shape of one phase for the tasks of a group.
+            auto fill = [&](PhaseCfg& pc, int key, bool first, int mode, const std::vector<Task>& tasks, size_t elem,
+                            bool with_v) {
+                pc.idx_off = int(plan.idx.size());
+                if (key <= 0) {
                     pc.staged = true;
                     pc.b = -key;
                     pc.C = m->ctx->max_cluster;
-                    for (int local : locals) {
+                    for (const Task& t : tasks) {
                         int M, N;
-                        dims(sel[local], mode, M, N);
-                        sm = std::max(sm, size_t(2) * pc.b * size_t(with_v ? M + N : M) * elem);
+                        dims(sel[t.local], mode, M, N);
+                        pc.smem = std::max(pc.smem, size_t(2) * pc.b * size_t(with_v ? M + N : M) * elem);
+                        plan.idx.push_back(jacobi_entry(t.local, 0));
                     }
-                    pc.smem = sm;
                     pc.threads = 32 * std::min(kJacobiStagedThreads / 32, std::max(4, pc.b));
                     return;
                 }
-                pc.C = key;
-                for (int local : locals) {
+                int warps = 1, b = 1;
+                for (const Task& t : tasks) {
                     int M, N;
-                    dims(sel[local], mode, M, N);
-                    sm = std::max(sm, jacobi_smem_bytes(with_v ? M + N : M, N, std::max(pc.C, 1), elem));
-                    bmax = std::max(bmax, round_up(N, 4 * std::max(pc.C, 1)) / (2 * std::max(pc.C, 1)));
-                    mmax = std::max(mmax, M);
+                    dims(sel[t.local], mode, M, N);
+                    RingShape s;
+                    const int c = first ? t.c1 : t.c2;
+                    ring_shape(M, N, with_v ? N : 0, elem, c, &s);
+                    pc.C = std::max(pc.C, c);
+                    pc.kr = std::max(pc.kr, s.kr);
+                    warps = std::max(warps, s.warps);
+                    b = std::max(b, s.b);
+                    int log2_c = 0;
+                    while ((1 << log2_c) < c) ++log2_c;
+                    plan.idx.push_back(jacobi_entry(t.local, log2_c));
                 }
-                pc.smem = sm;
-                // Register-resident variant when every job of the group fits it.
-                pc.reg = jacobi_reg_variant(mmax, bmax);
-                pc.threads = 32 * std::min((pc.reg ? kJacobiRegThreads : kJacobiThreads) / 32, std::max(2, bmax));
+                pc.threads = 32 * warps;
+                pc.smem = jacobi_ring_smem(b, pc.kr, elem);
             };
             for (auto& g : groups) {
                 Group gr;
                 gr.mode = g.first.mode;
-                gr.idx_off = int(plan.idx.size());
                 gr.count = int(g.second.size());
                 if (m->fp32) {
                     gr.nph = 2;
-                    fill(gr.ph[0], g.first.k1, gr.mode, g.second, sizeof(float2), true);
-                    fill(gr.ph[1], g.first.k2, gr.mode, g.second, sizeof(double2), false);
+                    fill(gr.ph[0], g.first.k1, true, gr.mode, g.second, sizeof(float2), true);
+                    fill(gr.ph[1], g.first.k2, false, gr.mode, g.second, sizeof(double2), false);
                 } else {
                     gr.nph = 1;
-                    fill(gr.ph[0], g.first.k1, gr.mode, g.second, sizeof(double2), false);
+                    fill(gr.ph[0], g.first.k1, true, gr.mode, g.second, sizeof(double2), false);
                 }
-                for (int local : g.second) plan.idx.push_back(local);
                 w.groups.push_back(gr);
             }
             plan.waves.push_back(std::move(w));
@@ -962,7 +980,7 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
         }
         auto launch_phase = [&](const Group& gr, const PhaseCfg& pc, int mode, int phase, bool fp32,
                                 cudaStream_t on) -> wqc_status {
-            if (pc.C < 1) return fail(WQC_ERR_INVALID, "two-site matrix too large for the cluster-resident Jacobi SVD");
+            if (pc.C < 1 || (pc.staged && pc.b < 1)) return fail(WQC_ERR_INVALID, "two-site matrix too large for the cluster-resident Jacobi SVD");
             Timed t(m, 0, on);
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(gr.count * pc.C);
@@ -977,10 +995,10 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
             cfg.attrs = attr;
             cfg.numAttrs = 1;
             if (pc.staged)
-                CUDA_TRY(launch_jacobi_staged(fp32, cfg, d_jobs, m->d_state, m->d_slots, d_idx + gr.idx_off, mode, phase,
+                CUDA_TRY(launch_jacobi_staged(fp32, cfg, d_jobs, m->d_state, m->d_slots, d_idx + pc.idx_off, mode, phase,
                                               kMaxSweeps, pc.b, m->d_status, m->d_counters));
             else
-                CUDA_TRY(launch_jacobi(fp32, pc.reg, cfg, d_jobs, m->d_state, m->d_slots, d_idx + gr.idx_off, mode,
+                CUDA_TRY(launch_jacobi(fp32, pc.kr, cfg, d_jobs, m->d_state, m->d_slots, d_idx + pc.idx_off, mode,
                                        phase, kMaxSweeps, m->d_status, m->d_counters));
             count_launch(m, 0);
             return WQC_OK;
@@ -1246,7 +1264,7 @@ wqc_status wqc_cuda_open(int device, wqc_cuda_ctx** out) {
     {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(16);
-        cfg.blockDim = dim3(kJacobiThreads);
+        cfg.blockDim = dim3(512);
         cfg.dynamicSmemBytes = 200 * 1024;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1256,7 +1274,7 @@ wqc_status wqc_cuda_open(int device, wqc_cuda_ctx** out) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, jacobi_kernel(false, false), &cfg) == cudaSuccess && clusters > 0)
+        if (cudaOccupancyMaxActiveClusters(&clusters, jacobi_staged(false), &cfg) == cudaSuccess && clusters > 0)
             ctx->max_cluster = 16;
         cudaGetLastError();
     }
@@ -1347,7 +1365,7 @@ static wqc_status create_state(wqc_cuda_ctx* ctx, const std::vector<int>& ns, co
     auto no_cluster = [&](int M, int N) {
         return choose_cluster(nullptr, M, N, ctx->max_cluster, 1, ctx->sm_count, sizeof(double2), false) < 1 ||
                (fp32 &&
-                choose_cluster(nullptr, M, N, ctx->max_cluster, 1, ctx->sm_count, sizeof(float2), false, M + N) < 1);
+                choose_cluster(nullptr, M, N, ctx->max_cluster, 1, ctx->sm_count, sizeof(float2), false, N) < 1);
     };
     std::vector<size_t> bucket_bytes, bucket_gs;
     {
@@ -2690,7 +2708,7 @@ void wqc_adjoint_destroy(wqc_adjoint* a) {
 // ===========================================================================
 namespace {
 
-constexpr int kTuneVersion = 1;
+constexpr int kTuneVersion = 2;
 
 std::string tune_fingerprint(const wqc_cuda_ctx* ctx) {
     cudaDeviceProp prop{};
@@ -2846,10 +2864,9 @@ wqc_status wqc_cuda_autotune(wqc_cuda_ctx* ctx, const char* cache_path, double b
                 const int len = precision == WQC_PRECISION_FP32 ? M + N : M;
                 int best_c = 0;
                 double best_ms = 0.0;
-                for (int c = 1; c <= ctx->max_cluster; ++c) {
-                    if (jacobi_smem_bytes(len, N, c, elem) > kSmemLimit) continue;
-                    const int b = round_up(N, 4 * c) / (2 * c);
-                    if (b > kJacobiThreads / 32) continue;  // more column pairs than warps
+                for (int c = 1; c <= std::min(ctx->max_cluster, kJacobiRingMaxCluster); c *= 2) {
+                    RingShape shape;
+                    if (!ring_shape(M, N, len - M, elem, c, &shape)) continue;
                     ctx->force_C = c;
                     const double ms = tune_measure(ctx, chi, precision, throughput ? 32 : 1, 3);
                     ctx->force_C = 0;

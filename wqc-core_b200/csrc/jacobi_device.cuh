@@ -1,0 +1,206 @@
+// Device code shared by the one-sided Jacobi SVD kernels: the pair rotation,
+// the tasks' operands and the factorisation check's constants.
+#pragma once
+
+#include "common.cuh"
+#include "split_kernels.cuh"
+
+namespace wqc {
+
+struct JacobiCtl {
+    int rot;                         // rotations of this sweep
+    int coarse;                      // a pair entered this sweep less orthogonal than the stop bound
+    unsigned long long relmax_bits;  // last allowed sweep: largest squared |gamma|^2 / (alpha beta) (double bits)
+    double fro_part;
+    double chk_in, chk_out;  // this CTA's share of ||X||_F^2 (after dust zeroing) and of sum sigma^2
+};
+
+// The Frobenius part of the reference's factorisation check (svd_reproduces,
+// svd_guard.rs:234-255): sum sigma^2 must equal ||X||_F^2 of the dust-zeroed
+// matrix to SVD_CHECK_TOL = 1e-9 relative (plus 1e-28).  The precision form's
+// complex64 columns carry ~1e-6 of rounding, so it is held to 1e-4.  The
+// probe-vector part needs V, which this Jacobi does not accumulate.
+constexpr double kSvdCheckTol = 1e-9;
+constexpr double kSvdCheckTolFp32 = 1e-4;
+
+// Pairs count as orthogonal at |gamma| <= tol sqrt(alpha beta), just above
+// the rounding of an M <= 512 dot product (sqrt(M) eps: 5e-15 in FP64, 3e-6
+// in FP32), so the sweeps stop and the singular values are exact to second
+// order.  A sweep that every pair entered orthogonal to the stop bound (1e-8;
+// 2e-3) ends the iteration: one-sided Jacobi converges quadratically, so that
+// sweep leaves them at about its square, below tol.  All squared.
+constexpr double kJacobiTol2 = 1e-28, kJacobiTol2Fp32 = 1.6e-11;
+constexpr double kJacobiStop2 = 1e-16, kJacobiStop2Fp32 = 4e-6;
+
+__device__ __forceinline__ double block_total(double v, double* red) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if (lane == 0) red[wid] = v;
+    __syncthreads();
+    double t = 0;
+    for (int w = 0; w < int(blockDim.x >> 5); ++w) t += red[w];
+    return t;
+}
+
+__device__ __forceinline__ int circle_at(int pos, int step, int b) {
+    if (pos == 0) return 0;
+    const int m = b - 1;
+    int v = (pos - 1 - step) % m;
+    if (v < 0) v += m;
+    return v + 1;
+}
+
+// Rotates columns xp, xq (each W then Z, `len` entries, W part `M`).  All
+// lanes compute bitwise-identical reductions (xor butterfly), so the branch is
+// warp-uniform.
+//
+// Two guards keep every applied rotation unitary and the sweep finite:
+// |gamma| is taken with hypot when |gamma|^2 nears the subnormal range, so
+// the phase stays of unit modulus; and a pair whose smaller column has
+// alpha <= floor = (1e-15 ||W||_F)^2 (FP32 columns: (1e-6 ||W||_F)^2) is left
+// alone.  Such a column is at the storage's rounding level: its direction is
+// noise, rotating it against another column changes nothing above
+// floor * ||W||_F^2, and rotating it anyway lets exactly parallel columns (a
+// rank-deficient theta) be re-rotated every sweep until their products go
+// subnormal, and pairs of noise columns keep |gamma|/sqrt(alpha beta) near
+// 1e-8 forever (seen on a 256 x 144 range-finder matrix of the 50-qubit
+// circuit, which then never met the stop test).
+//
+// The columns are complex128 (double2) in the plain form and complex64
+// (float2) in the precision form.  The precision form accumulates the dot
+// products and applies the rotation in FP32; the rotation parameters, the
+// tests against tol and the noise floor, and the convergence measure are
+// FP64 in both.
+template <typename T>
+struct JacobiReal;
+template <>
+struct JacobiReal<double2> {
+    using R = double;
+};
+template <>
+struct JacobiReal<float2> {
+    using R = float;
+};
+
+// Warp sums of four values, every lane receiving the same four totals (so
+// branches on them stay warp-uniform).  Instead of four butterflies (20
+// shuffles) the first two levels split the values between the lane halves
+// (lanes with bit 4 clear keep a, b and pass g, h; then bit 3 picks one of
+// the two), three more levels finish one value per quarter of the warp, and
+// four broadcasts from lanes 0, 8, 16, 24 hand out the totals: 10 shuffles,
+// on the dependent chain of every rotation round.
+template <typename R>
+__device__ __forceinline__ void warp_sum4(R& a, R& b, R& g, R& h, int lane) {
+    const bool hi = lane & 16;
+    R k0 = hi ? g : a, k1 = hi ? h : b;
+    k0 += __shfl_xor_sync(0xffffffffu, hi ? a : g, 16);
+    k1 += __shfl_xor_sync(0xffffffffu, hi ? b : h, 16);
+    const bool b3 = lane & 8;
+    R v = b3 ? k1 : k0;
+    v += __shfl_xor_sync(0xffffffffu, b3 ? k0 : k1, 8);
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    a = __shfl_sync(0xffffffffu, v, 0);
+    b = __shfl_sync(0xffffffffu, v, 8);
+    g = __shfl_sync(0xffffffffu, v, 16);
+    h = __shfl_sync(0xffffffffu, v, 24);
+}
+
+// What a sweep learns from its pairs.  The convergence test needs only
+// whether some pair entered above the stop bound; the ratio itself (an FP64
+// division on every rotation's chain) is taken on the last allowed sweep,
+// where the error message reports it.
+struct JacobiSweep {
+    int rot = 0;
+    bool coarse = false;
+    double relmax = 0.0;
+};
+
+// A warp's findings into its CTA's control block.
+__device__ __forceinline__ void jacobi_report(JacobiCtl& ctl, const JacobiSweep& sw, int lane) {
+    if (lane != 0) return;
+    if (sw.rot) atomicAdd(&ctl.rot, sw.rot);
+    if (sw.coarse) atomicOr(&ctl.coarse, 1);
+    if (sw.relmax > 0.0) atomicMax(&ctl.relmax_bits, (unsigned long long)__double_as_longlong(sw.relmax));
+}
+
+// Rotation parameters from alpha = |p|^2, beta = |q|^2, gamma = <p, q>:
+// returns false when the pair is left alone (noise-level column, or already
+// orthogonal to tol), else c and w = s * phase of the rephased rotation
+// (svd_guard.rs:189-197) xp' = c xp - conj(w) xq, xq' = w xp + c xq.
+//
+// With d = (beta - alpha) / 2 and r = sqrt(d^2 + |gamma|^2) the half-angle
+// form is c^2 = (1 + |d| / r) / 2 and w = sign(d) gamma / (2 r c): two
+// dependent reciprocal square roots (85 cycles each on B200) and no
+// division, where the tangent form took three and its phase a fourth.
+__device__ __forceinline__ bool jacobi_params(double a, double bb, double gr, double gi, double tol2, double stop_rel2,
+                                              double noise_floor, bool want_ratio, JacobiSweep& sw, double& c,
+                                              double& wr, double& wi) {
+    const double g2 = fma(gr, gr, gi * gi);
+    const double ab = a * bb;
+    if (fmin(a, bb) <= noise_floor) return false;  // the smaller column is at the storage's rounding level
+    sw.coarse |= g2 > stop_rel2 * ab;
+    if (want_ratio) sw.relmax = fmax(sw.relmax, g2 / ab);
+    if (g2 == 0.0 || g2 <= tol2 * ab) return false;
+    const double d = 0.5 * (bb - a);
+    const double r2 = fma(d, d, g2);
+    if (g2 > 1e-290) {
+        const double ir = rsqrt(r2);
+        const double c2 = fma(0.5 * fabs(d), ir, 0.5);
+        const double ic = rsqrt(c2);
+        c = c2 * ic;
+        const double f = copysign(0.5 * ir * ic, d);
+        wr = gr * f;
+        wi = gi * f;
+    } else {  // |gamma|^2 near the subnormal range: hypot keeps the rotation unitary
+        const double r = hypot(d, hypot(gr, gi));
+        c = sqrt(0.5 + 0.5 * (fabs(d) / r));
+        const double f = copysign(0.5 / c, d);
+        wr = (gr / r) * f;
+        wi = (gi / r) * f;
+    }
+    ++sw.rot;
+    return true;
+}
+
+__device__ __forceinline__ void jacobi_task(const SplitJob& J, const SplitState& S, const SlotBuffers& B, int mode,
+                                            const double2*& src, int& sr, int& sc, int& ld, int& rows_of_src) {
+    if (mode == kJacobiRsvd) {  // W = B^H, B is ell x cols row-major
+        src = B.b;
+        sr = S.ell;
+        sc = S.cols;
+        ld = S.cols;
+        rows_of_src = 1;
+    } else {  // exact: W = theta (rows >= cols) or theta^H
+        src = B.theta;
+        sr = S.rows;
+        sc = S.cols;
+        ld = S.cols;
+        rows_of_src = S.w_rows_of_src;
+    }
+}
+
+__device__ __forceinline__ bool jacobi_active(const SplitState& S, int mode) {
+    if (mode == kJacobiRsvd) return S.use_rsvd != 0;
+    // The exact path's two modes never overlap: prepare sets path EXACT, and a
+    // fallback changes a range-finder split's path to RSVD_FALLBACK only.
+    if (mode == kJacobiExact) return S.need_exact != 0 && S.path == WQC_SPLIT_EXACT;
+    return S.need_exact != 0 && S.path == WQC_SPLIT_RSVD_FALLBACK;
+}
+
+template <typename T>
+__device__ __forceinline__ T to_store(double2 x);
+template <>
+__device__ __forceinline__ double2 to_store<double2>(double2 x) {
+    return x;
+}
+template <>
+__device__ __forceinline__ float2 to_store<float2>(double2 x) {
+    return make_float2(float(x.x), float(x.y));
+}
+__device__ __forceinline__ double2 to_f64(double2 x) { return x; }
+__device__ __forceinline__ double2 to_f64(float2 x) { return make_double2(x.x, x.y); }
+
+}  // namespace wqc

@@ -12,6 +12,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "jacobi_device.cuh"
 #include "split_kernels.cuh"
 
 namespace cg = cooperative_groups;
@@ -520,155 +521,10 @@ __global__ void __launch_bounds__(kQrClusterThreads, 1) qr_cluster_kernel(const 
     cluster.sync();  // no CTA leaves while another may still read its shared memory
 }
 
-// ---------------------------------------------------------------------------
-// One-sided Hestenes Jacobi SVD on a thread-block cluster.
-//
-// The tall working matrix W (M x N, padded to N' = 2*C*b columns) is held
-// column by column in the shared memory of the C CTAs of one cluster: CTA r
-// holds block r ("top") and block 2C-1-r ("bottom"), b columns each.  The
-// right rotations are not accumulated: at convergence W = X V = U Sigma, and
-// the cut recovers the other side from W and X (absorb_kernel), which keeps
-// the step's shared-memory traffic (its bound) to W's M rows.  A sweep orthogonalises the pairs inside each block, then
-// runs 2C-1 block steps of the b*b cross pairs, rotating the blocks between
-// CTAs by the circle method through distributed shared memory.  Each pair
-// rotation is the reference's rephase-then-real-rotation (svd_guard.rs:
-// 174-199), with column dot products reduced by warp shuffles.
-// ---------------------------------------------------------------------------
-struct JacobiCtl {
-    int rot;
-    unsigned long long relmax_bits;  // largest |gamma|/sqrt(alpha beta) seen this sweep (non-negative double bits)
-    double fro_part;
-    double chk_in, chk_out;  // this CTA's share of ||X||_F^2 (after dust zeroing) and of sum sigma^2
-};
-
-// The Frobenius part of the reference's factorisation check (svd_reproduces,
-// svd_guard.rs:234-255): sum sigma^2 must equal ||X||_F^2 of the dust-zeroed
-// matrix to SVD_CHECK_TOL = 1e-9 relative (plus 1e-28).  The precision form's
-// complex64 columns carry ~1e-6 of rounding, so it is held to 1e-4.  The
-// probe-vector part needs V, which this Jacobi does not accumulate.
-constexpr double kSvdCheckTol = 1e-9;
-constexpr double kSvdCheckTolFp32 = 1e-4;
-
-__device__ __forceinline__ double block_total(double v, double* red) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if (lane == 0) red[wid] = v;
-    __syncthreads();
-    double t = 0;
-    for (int w = 0; w < int(blockDim.x >> 5); ++w) t += red[w];
-    return t;
-}
-
-__device__ __forceinline__ int circle_at(int pos, int step, int b) {
-    if (pos == 0) return 0;
-    const int m = b - 1;
-    int v = (pos - 1 - step) % m;
-    if (v < 0) v += m;
-    return v + 1;
-}
-
-// Rotates columns xp, xq (each W then Z, `len` entries, W part `M`).  All
-// lanes compute bitwise-identical reductions (xor butterfly), so the branch is
-// warp-uniform.  Returns 1 when a rotation was applied.
-//
-// Two guards keep every applied rotation unitary and the sweep finite:
-// |gamma| is taken with hypot when |gamma|^2 nears the subnormal range, so
-// the phase stays of unit modulus; and a pair whose smaller column has
-// alpha <= floor = (1e-15 ||W||_F)^2 (FP32 columns: (1e-6 ||W||_F)^2) is left
-// alone.  Such a column is at the storage's rounding level: its direction is
-// noise, rotating it against another column changes nothing above
-// floor * ||W||_F^2, and rotating it anyway lets exactly parallel columns (a
-// rank-deficient theta) be re-rotated every sweep until their products go
-// subnormal, and pairs of noise columns keep |gamma|/sqrt(alpha beta) near
-// 1e-8 forever (seen on a 256 x 144 range-finder matrix of the 50-qubit
-// circuit, which then never met the stop test).
-//
-// The columns are complex128 (double2) in the plain form and complex64
-// (float2) in the precision form.  The precision form accumulates the dot
-// products and applies the rotation in FP32; the rotation parameters, the
-// tests against tol and the noise floor, and the convergence measure are
-// FP64 in both.
 template <typename T>
-struct JacobiReal;
-template <>
-struct JacobiReal<double2> {
-    using R = double;
-};
-template <>
-struct JacobiReal<float2> {
-    using R = float;
-};
-
-// Warp sums of four values, every lane receiving the same four totals (so
-// branches on them stay warp-uniform).  Instead of four butterflies (20
-// shuffles) the first two levels split the values between the lane halves
-// (lanes with bit 4 clear keep a, b and pass g, h; then bit 3 picks one of
-// the two), three more levels finish one value per quarter of the warp, and
-// four broadcasts from lanes 0, 8, 16, 24 hand out the totals: 10 shuffles,
-// on the dependent chain of every rotation round.
-template <typename R>
-__device__ __forceinline__ void warp_sum4(R& a, R& b, R& g, R& h, int lane) {
-    const bool hi = lane & 16;
-    R k0 = hi ? g : a, k1 = hi ? h : b;
-    k0 += __shfl_xor_sync(0xffffffffu, hi ? a : g, 16);
-    k1 += __shfl_xor_sync(0xffffffffu, hi ? b : h, 16);
-    const bool b3 = lane & 8;
-    R v = b3 ? k1 : k0;
-    v += __shfl_xor_sync(0xffffffffu, b3 ? k0 : k1, 8);
-    v += __shfl_xor_sync(0xffffffffu, v, 4);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    a = __shfl_sync(0xffffffffu, v, 0);
-    b = __shfl_sync(0xffffffffu, v, 8);
-    g = __shfl_sync(0xffffffffu, v, 16);
-    h = __shfl_sync(0xffffffffu, v, 24);
-}
-
-// Rotation parameters from alpha = |p|^2, beta = |q|^2, gamma = <p, q>:
-// returns false when the pair is left alone (noise-level column, or already
-// orthogonal to tol), else c and w = s * phase.
-__device__ __forceinline__ bool jacobi_params(double a, double bb, double gr, double gi, double tol, double noise_floor,
-                                              double& relmax, double& c, double& wr, double& wi) {
-    // Squared forms keep the dependent chain short: |gamma|^2 against
-    // tol^2 alpha beta, one reciprocal square root for the phase.
-    const double g2 = fma(gr, gr, gi * gi);
-    const double ab = a * bb;
-    if (fmin(a, bb) <= noise_floor) return false;  // the smaller column is at the storage's rounding level
-    relmax = fmax(relmax, g2 / ab);  // squared ratio; the caller compares with squared bounds
-    if (g2 == 0.0 || g2 <= tol * tol * ab) return false;
-    double pr, pi, zeta;
-    if (g2 > 1e-290) {
-        const double inv_g = rsqrt(g2);
-        pr = gr * inv_g;
-        pi = gi * inv_g;
-        zeta = 0.5 * (bb - a) * inv_g;
-    } else {  // |gamma|^2 near the subnormal range: hypot keeps the phase of unit modulus
-        const double g = hypot(gr, gi);
-        pr = gr / g;
-        pi = gi / g;
-        zeta = (bb - a) / (2.0 * g);
-    }
-    // tan = sign(zeta) / (|zeta| + u) with u = sqrt(1 + zeta^2) gives
-    // c^2 = (u + |zeta|) / (2u) and s^2 = 1 / (2u (u + |zeta|)): after one
-    // reciprocal square root, c and s are two independent ones, no division.
-    const double az = fabs(zeta);
-    const double q = fma(zeta, zeta, 1.0);
-    const double ru = rsqrt(q);
-    const double u = q * ru;
-    const double c2 = fma(0.5 * az, ru, 0.5);
-    c = c2 * rsqrt(c2);
-    const double s = copysign(rsqrt(2.0 * u * (u + az)), zeta);
-    // With w = s * phase the rephased rotation (svd_guard.rs:189-197) is
-    // xp' = c xp - conj(w) xq,  xq' = w xp + c xq   (|phase| = 1).
-    wr = s * pr;
-    wi = s * pi;
-    return true;
-}
-
-template <typename T>
-__device__ __forceinline__ int jacobi_rotate(T* __restrict__ xp, T* __restrict__ xq, int M, int len, double tol,
-                                             double noise_floor, int lane, double& relmax) {
+__device__ __forceinline__ void jacobi_rotate(T* __restrict__ xp, T* __restrict__ xq, int M, int len, double tol2,
+                                              double stop_rel2, double noise_floor, bool want_ratio, int lane,
+                                              JacobiSweep& sw) {
     using R = typename JacobiReal<T>::R;
     // Two rows per lane per iteration into two accumulator sets: the loads
     // of the second row overlap the first's FMAs and the dependent chains
@@ -699,7 +555,7 @@ __device__ __forceinline__ int jacobi_rotate(T* __restrict__ xp, T* __restrict__
     gi_ += gi1;
     warp_sum4(a_, b_, gr_, gi_, lane);
     double c64, wr64, wi64;
-    if (!jacobi_params(a_, b_, gr_, gi_, tol, noise_floor, relmax, c64, wr64, wi64)) return 0;
+    if (!jacobi_params(a_, b_, gr_, gi_, tol2, stop_rel2, noise_floor, want_ratio, sw, c64, wr64, wi64)) return;
     const R wr = R(wr64), wi = R(wi64), cr = R(c64);
     auto rot = [&](const T u, const T v, T& p, T& q) {
         p.x = fma(cr, u.x, -fma(wr, v.x, wi * v.y));
@@ -730,445 +586,6 @@ __device__ __forceinline__ int jacobi_rotate(T* __restrict__ xp, T* __restrict__
         xp[r] = p;
         xq[r] = q;
     }
-    return 1;
-}
-
-// The same rotation with p held in registers (rows lane + 32 k, M <= 32 *
-// kJacobiRegRows): in a block step warp i keeps its top column for all b
-// rounds, so only the partner q moves through shared memory (the step is
-// bound by shared-memory bandwidth).
-constexpr int kJacobiRegRows = 8;
-
-template <typename T>
-__device__ __forceinline__ int jacobi_rotate_reg(T (&u)[kJacobiRegRows], T* __restrict__ xq, int M, int len,
-                                                 T* __restrict__ xp_tail, double tol, double noise_floor, int lane,
-                                                 double& relmax) {
-    using R = typename JacobiReal<T>::R;
-    T v[kJacobiRegRows];
-#pragma unroll
-    for (int k = 0; k < kJacobiRegRows; ++k) {
-        const int r = lane + 32 * k;
-        if (r < M) {
-            v[k] = xq[r];
-        } else {
-            v[k].x = v[k].y = R(0);
-        }
-    }
-    R a_ = 0, b_ = 0, gr_ = 0, gi_ = 0, a1 = 0, b1 = 0, gr1 = 0, gi1 = 0;
-#pragma unroll
-    for (int k = 0; k < kJacobiRegRows; k += 2) {
-        a_ = fma(u[k].x, u[k].x, fma(u[k].y, u[k].y, a_));
-        b_ = fma(v[k].x, v[k].x, fma(v[k].y, v[k].y, b_));
-        gr_ = fma(u[k].x, v[k].x, fma(u[k].y, v[k].y, gr_));
-        gi_ = fma(u[k].x, v[k].y, fma(-u[k].y, v[k].x, gi_));
-        a1 = fma(u[k + 1].x, u[k + 1].x, fma(u[k + 1].y, u[k + 1].y, a1));
-        b1 = fma(v[k + 1].x, v[k + 1].x, fma(v[k + 1].y, v[k + 1].y, b1));
-        gr1 = fma(u[k + 1].x, v[k + 1].x, fma(u[k + 1].y, v[k + 1].y, gr1));
-        gi1 = fma(u[k + 1].x, v[k + 1].y, fma(-u[k + 1].y, v[k + 1].x, gi1));
-    }
-    a_ += a1;
-    b_ += b1;
-    gr_ += gr1;
-    gi_ += gi1;
-    warp_sum4(a_, b_, gr_, gi_, lane);
-    double c64, wr64, wi64;
-    if (!jacobi_params(a_, b_, gr_, gi_, tol, noise_floor, relmax, c64, wr64, wi64)) return 0;
-    const R wr = R(wr64), wi = R(wi64), cr = R(c64);
-#pragma unroll
-    for (int k = 0; k < kJacobiRegRows; ++k) {
-        const int r = lane + 32 * k;
-        if (r < M) {
-            T p, q;
-            p.x = fma(cr, u[k].x, -fma(wr, v[k].x, wi * v[k].y));
-            p.y = fma(cr, u[k].y, -fma(wr, v[k].y, -wi * v[k].x));
-            q.x = fma(wr, u[k].x, fma(-wi, u[k].y, cr * v[k].x));
-            q.y = fma(wr, u[k].y, fma(wi, u[k].x, cr * v[k].y));
-            u[k] = p;
-            xq[r] = q;
-        }
-    }
-    // Rows M .. len-1 (the right rotations accumulated in the precision
-    // form's first phase) stay in shared memory for both columns.
-    for (int r = M + lane; r < len; r += 32) {
-        const T x = xp_tail[r], y = xq[r];
-        T p, q;
-        p.x = fma(cr, x.x, -fma(wr, y.x, wi * y.y));
-        p.y = fma(cr, x.y, -fma(wr, y.y, -wi * y.x));
-        q.x = fma(wr, x.x, fma(-wi, x.y, cr * y.x));
-        q.y = fma(wr, x.y, fma(wi, x.x, cr * y.y));
-        xp_tail[r] = p;
-        xq[r] = q;
-    }
-    return 1;
-}
-
-// Block copy into another CTA's shared memory: eight local loads, then eight
-// remote stores (which do not stall the thread).
-template <typename T>
-__device__ __forceinline__ void dsmem_push(T* __restrict__ dst, const T* __restrict__ src, size_t n, int tid,
-                                           int nthreads) {
-    size_t e = tid;
-    const size_t st = nthreads;
-    for (; e + 7 * st < n; e += 8 * st) {
-        T v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = src[e + u * st];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) dst[e + u * st] = v[u];
-    }
-    for (; e < n; e += st) dst[e] = src[e];
-}
-
-__device__ __forceinline__ void jacobi_task(const SplitJob& J, const SplitState& S, const SlotBuffers& B, int mode,
-                                            const double2*& src, int& sr, int& sc, int& ld, int& rows_of_src) {
-    if (mode == kJacobiRsvd) {  // W = B^H, B is ell x cols row-major
-        src = B.b;
-        sr = S.ell;
-        sc = S.cols;
-        ld = S.cols;
-        rows_of_src = 1;
-    } else {  // exact: W = theta (rows >= cols) or theta^H
-        src = B.theta;
-        sr = S.rows;
-        sc = S.cols;
-        ld = S.cols;
-        rows_of_src = S.w_rows_of_src;
-    }
-}
-
-__device__ __forceinline__ bool jacobi_active(const SplitState& S, int mode) {
-    if (mode == kJacobiRsvd) return S.use_rsvd != 0;
-    // The exact path's two modes never overlap: prepare sets path EXACT, and a
-    // fallback changes a range-finder split's path to RSVD_FALLBACK only.
-    if (mode == kJacobiExact) return S.need_exact != 0 && S.path == WQC_SPLIT_EXACT;
-    return S.need_exact != 0 && S.path == WQC_SPLIT_RSVD_FALLBACK;
-}
-
-template <typename T>
-__device__ __forceinline__ T to_store(double2 x);
-template <>
-__device__ __forceinline__ double2 to_store<double2>(double2 x) {
-    return x;
-}
-template <>
-__device__ __forceinline__ float2 to_store<float2>(double2 x) {
-    return make_float2(float(x.x), float(x.y));
-}
-__device__ __forceinline__ double2 to_f64(double2 x) { return x; }
-__device__ __forceinline__ double2 to_f64(float2 x) { return make_double2(x.x, x.y); }
-
-template <typename T, bool kReg>
-__global__ void __launch_bounds__(kReg ? kJacobiRegThreads : kJacobiThreads) jacobi_cluster_kernel(
-    const SplitJob* jobs, SplitState* st, const SlotBuffers* slots, const int* idx, int mode, int phase,
-    int max_sweeps, int* status, unsigned long long* counters) {
-    constexpr bool kF64 = sizeof(T) == sizeof(double2);
-    cg::cluster_group cluster = cg::this_cluster();
-    const int C = int(cluster.num_blocks());
-    const int rank = int(cluster.block_rank());
-    const int j = idx[blockIdx.x / C];
-    const SplitState S = st[j];
-    if (!jacobi_active(S, mode)) return;  // uniform over the cluster
-    const SplitJob& J = jobs[j];
-    const SlotBuffers Bf = slots[J.slot];
-    const double2* src;
-    int sr, sc, ld, rows_of_src;
-    jacobi_task(J, S, Bf, mode, src, sr, sc, ld, rows_of_src);
-    const int M = rows_of_src ? sc : sr;
-    const int N = rows_of_src ? sr : sc;
-    const int quantum = 4 * C;
-    const int Np = ((N + quantum - 1) / quantum) * quantum;
-    const int b = Np / (2 * C);
-    // W only, the other side's vectors are recovered from W after the SVD;
-    // the precision form's first phase also carries V (N rows under W).
-    const int vrows = phase == kPhaseFp32V ? N : 0;
-    const int len = M + vrows;
-    const bool colmajor = rows_of_src || phase == kPhaseFinish;
-
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* smem = reinterpret_cast<T*>(smem_raw);
-    __shared__ JacobiCtl ctl;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int nthreads = blockDim.x;  // a multiple of 32, at most kJacobiThreads
-    const int nwarps = nthreads / 32;
-    auto buf = [&](int k) { return smem + size_t(k) * b * len; };
-    __shared__ double red[kJacobiThreads / 32];
-
-    if (tid == 0) ctl.rot = 0;
-    // Buffer roles and block ids after xk block exchanges, the same on every
-    // CTA without reading a neighbour's state: CTA 0 keeps its top block
-    // (position 0) in buffer 0 and receives into buffer 1; every other CTA
-    // turns its (top, bottom, spare) buffers one place per exchange; the
-    // blocks at positions 1 .. 2C-1 move one position on per exchange, so
-    // position p holds block circle_at(p, xk, 2C).
-    int xk = 0;
-    auto top_buf_of = [&](int r, int k) { return r == 0 ? 0 : (3 - k % 3) % 3; };
-    auto bot_buf_of = [&](int r, int k) { return r == 0 ? 1 : (4 - k % 3) % 3; };
-    auto spare_buf_of = [&](int k) { return (5 - k % 3) % 3; };
-    // Frobenius norm over the columns this CTA loads, then over the cluster.
-    // The precision form's finishing phase starts from X V (column-major in
-    // the slot's W buffer), formed from the dust-zeroed X.
-    const double2* wsrc = Bf.w;
-    auto src_at = [&](int i, int col) -> double2 {
-        if (phase == kPhaseFinish) return wsrc[size_t(col) * M + i];
-        return rows_of_src ? cconj(src[size_t(col) * ld + i]) : src[size_t(i) * ld + col];
-    };
-    double part = 0;
-    for (int half = 0; half < 2; ++half) {
-        const int id = half == 0 ? rank : 2 * C - 1 - rank;
-        for (int e = tid; e < b * M; e += nthreads) {
-            int c, i;
-            if (colmajor) { c = e / M; i = e % M; } else { i = e / b; c = e % b; }
-            const int col = id * b + c;
-            if (col < N) part += cnorm2(src_at(i, col));
-        }
-    }
-    {
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        if (lane == 0) red[wid] = part;
-        __syncthreads();
-        if (tid == 0) {
-            double t = 0;
-            for (int w = 0; w < nwarps; ++w) t += red[w];
-            ctl.fro_part = t;
-        }
-    }
-    cluster.sync();
-    double fro2 = 0;
-    for (int r = 0; r < C; ++r) fro2 += cluster.map_shared_rank(&ctl, r)->fro_part;
-    const double dust = sqrt(fro2) * kDustRel;
-    const double dust2 = dust * dust;
-    double chk_in = 0, chk_out = 0;
-    // Load W (dust-zeroed; padding columns zero).
-    for (int half = 0; half < 2; ++half) {
-        const int id = half == 0 ? rank : 2 * C - 1 - rank;
-        T* base = buf(half);
-        for (int e = tid; e < b * M; e += nthreads) {
-            int c, i;
-            if (colmajor) { c = e / M; i = e % M; } else { i = e / b; c = e % b; }
-            const int col = id * b + c;
-            double2 x = col < N ? src_at(i, col) : cmake(0, 0);
-            if (phase != kPhaseFinish && cnorm2(x) < dust2) x = cmake(0, 0);
-            chk_in += cnorm2(x);
-            base[size_t(c) * len + i] = to_store<T>(x);
-        }
-        for (int e = tid; e < b * vrows; e += nthreads) {  // V = I (padding columns: zero)
-            const int c = e / vrows, i = e % vrows;
-            base[size_t(c) * len + M + i] = to_store<T>(cmake(id * b + c == i ? 1.0 : 0.0, 0.0));
-        }
-    }
-    __syncthreads();
-    // Pairs count as orthogonal at |gamma| <= tol sqrt(alpha beta), just
-    // above the rounding of an M <= 512 dot product (sqrt(M) eps: 5e-15 in
-    // FP64, 3e-6 in FP32), so the sweeps stop and the singular values are
-    // exact to second order.  A sweep that every pair entered orthogonal to
-    // stop_rel ends the iteration: one-sided Jacobi converges quadratically,
-    // so that sweep leaves them at about stop_rel^2 <= tol.  Columns at the
-    // storage's rounding level against ||W||_F are left alone (noise floor).
-    const double tol = kF64 ? 1e-14 : 4e-6;
-    const double stop_rel2 = kF64 ? 1e-16 : 4e-6;  // squared: 1e-8 and 2e-3
-    const double noise_floor = (kF64 ? 1e-30 : 1e-12) * fro2;  // squared column norm: 1e-15 (1e-6) of ||W||_F
-    int sweep = 0;
-    bool converged = false;
-    int ctl_rot_last = 0;
-    unsigned long long ctl_relmax_bits_last = 0ull;
-    for (; sweep < max_sweeps; ++sweep) {
-        if (tid == 0) {
-            ctl.rot = 0;
-            ctl.relmax_bits = 0ull;
-        }
-        __syncthreads();
-        int my_rot = 0;
-        double my_rel = 0.0;
-        // Pairs inside each block (circle method on b columns).
-        for (int step = 0; step < b - 1; ++step) {
-            for (int pq = wid; pq < b; pq += nwarps) {
-                const bool top = pq < b / 2;
-                const int i = top ? pq : pq - b / 2;
-                T* base = buf(top ? top_buf_of(rank, xk) : bot_buf_of(rank, xk));
-                const int e1 = circle_at(i, step, b), e2 = circle_at(b - 1 - i, step, b);
-                my_rot += jacobi_rotate(base + size_t(e1) * len, base + size_t(e2) * len, M, len, tol, noise_floor, lane, my_rel);
-            }
-            __syncthreads();
-        }
-        // Cross pairs between the two blocks, 2C-1 block steps.  Warp i pairs
-        // its top column i with bottom column (i + k) % b in round k; when
-        // every warp owns one top column and it fits, the column stays in
-        // registers for the b rounds.
-        const bool reg_path = kReg && M <= 32 * kJacobiRegRows && nwarps >= b;
-        for (int bs = 0; bs < 2 * C - 1; ++bs) {
-            T* tb = buf(top_buf_of(rank, xk));
-            T* bb = buf(bot_buf_of(rank, xk));
-            if (reg_path) {
-                T u[kJacobiRegRows];
-                T* col = tb + size_t(wid) * len;
-                if (wid < b) {
-#pragma unroll
-                    for (int kk = 0; kk < kJacobiRegRows; ++kk) {
-                        const int r = lane + 32 * kk;
-                        if (r < M) {
-                            u[kk] = col[r];
-                        } else {
-                            u[kk].x = u[kk].y = 0;
-                        }
-                    }
-                }
-                for (int k = 0; k < b; ++k) {
-                    if (wid < b)
-                        my_rot += jacobi_rotate_reg(u, bb + size_t((wid + k) % b) * len, M, len, col, tol,
-                                                    noise_floor, lane, my_rel);
-                    __syncthreads();
-                }
-                if (wid < b) {
-#pragma unroll
-                    for (int kk = 0; kk < kJacobiRegRows; ++kk) {
-                        const int r = lane + 32 * kk;
-                        if (r < M) col[r] = u[kk];
-                    }
-                }
-                __syncthreads();
-            } else {
-                for (int k = 0; k < b; ++k) {
-                    for (int i = wid; i < b; i += nwarps) {
-                        const int e2 = (i + k) % b;
-                        my_rot += jacobi_rotate(tb + size_t(i) * len, bb + size_t(e2) * len, M, len, tol, noise_floor,
-                                                lane, my_rel);
-                    }
-                    __syncthreads();
-                }
-            }
-            if (C == 1) continue;
-            // Circle rotation of blocks between CTAs (push protocol, one spare
-            // buffer, two cluster barriers).  Phase 1: as soon as its own
-            // rotations are done, CTA r <= C-2 stores the block that moves to
-            // CTA r+1's top position (CTA 0: its bottom block, the others:
-            // their top) into CTA r+1's spare buffer, which CTA r+1 does not
-            // touch while it rotates.  After the barrier, when every CTA has
-            // finished rotating and sending, phase 2: CTA r >= 1 stores its
-            // bottom block over CTA r-1's old top (CTA 0: its old bottom),
-            // both already sent.  The second barrier makes the received
-            // blocks visible.  Remote stores do not wait for DSMEM latency
-            // as remote loads do (measured: ~2700 cycles per pulled block of
-            // 66 KB).  Roles and block ids follow from the exchange count.
-            const size_t blk = size_t(b) * len;
-            if (rank <= C - 2) {
-                const int src = rank == 0 ? bot_buf_of(0, xk) : top_buf_of(rank, xk);
-                dsmem_push(cluster.map_shared_rank(smem, rank + 1) + size_t(spare_buf_of(xk)) * blk, buf(src), blk,
-                           tid, nthreads);
-            }
-            cluster.sync();
-            if (rank >= 1) {
-                const int dst = rank - 1;
-                const int dbuf = dst == 0 ? bot_buf_of(0, xk) : top_buf_of(dst, xk);
-                dsmem_push(cluster.map_shared_rank(smem, dst) + size_t(dbuf) * blk, buf(bot_buf_of(rank, xk)), blk,
-                           tid, nthreads);
-            }
-            ++xk;
-            cluster.sync();
-        }
-        // Cluster-wide rotation count decides convergence.
-        if (lane == 0 && my_rot) atomicAdd(&ctl.rot, my_rot);
-        if (lane == 0 && my_rel > 0.0) atomicMax(&ctl.relmax_bits, (unsigned long long)__double_as_longlong(my_rel));
-        __syncthreads();
-        int total = 0;
-        double relmax = 0.0;
-        if (C == 1) {
-            total = ctl.rot;
-            relmax = __longlong_as_double((long long)ctl.relmax_bits);
-            __syncthreads();
-        } else {
-            cluster.sync();
-            for (int r = 0; r < C; ++r) {
-                const JacobiCtl* rc = cluster.map_shared_rank(&ctl, r);
-                total += rc->rot;
-                relmax = fmax(relmax, __longlong_as_double((long long)rc->relmax_bits));
-            }
-            cluster.sync();
-        }
-        // Converged when nothing rotated, or when every pair entered this
-        // sweep orthogonal to stop_rel (FP64: 1e-8, leaving them at about
-        // 1e-16, below the rotation tolerance, so a verification sweep would
-        // rotate nothing).
-        ctl_rot_last = total;
-        ctl_relmax_bits_last = (unsigned long long)__double_as_longlong(relmax);
-        if (total == 0 || relmax < stop_rel2) {  // relmax holds squared ratios
-            converged = true;
-            break;
-        }
-    }
-    if (tid == 0 && rank == 0) {
-        if (!converged) {
-            atomicOr(status, kStatusJacobiNoConvergence);
-            // The first such split, its last sweep's rotation count and largest
-            // squared |gamma| / sqrt(alpha beta), for the error message.
-            if (atomicCAS(status + 1, 0, J.seq + 1) == 0) {
-                const unsigned long long bits = ctl_relmax_bits_last;
-                status[2] = ctl_rot_last;
-                status[3] = int(bits >> 32);
-                status[4] = int(bits & 0xffffffffull);
-            }
-        }
-        if (phase != kPhaseFp32V) atomicAdd(counters + 0, 1ull);
-        atomicAdd(counters + (phase == kPhaseFp32V ? 2 : 1), (unsigned long long)(converged ? sweep + 1 : sweep));
-    }
-    if (phase == kPhaseFp32V) {
-        // The accumulated V (FP64) for the finishing phase, and ||X||_F^2
-        // for its dust zeroing of X.
-        for (int half = 0; half < 2; ++half) {
-            const int id = circle_at(half == 0 ? rank : 2 * C - 1 - rank, xk, 2 * C);
-            const T* base = buf(half == 0 ? top_buf_of(rank, xk) : bot_buf_of(rank, xk));
-            for (int c = wid; c < b; c += nwarps) {
-                const int col = id * b + c;
-                if (col >= N) continue;
-                for (int r = lane; r < N; r += 32) Bf.z[size_t(col) * N + r] = to_f64(base[size_t(c) * len + M + r]);
-            }
-        }
-        if (rank == 0 && tid == 0) st[j].fro2 = fro2;
-        cluster.sync();  // no CTA leaves while another may still read its shared memory
-        return;
-    }
-    // Write back: W columns and column norms.
-    for (int half = 0; half < 2; ++half) {
-        const int id = circle_at(half == 0 ? rank : 2 * C - 1 - rank, xk, 2 * C);
-        const T* base = buf(half == 0 ? top_buf_of(rank, xk) : bot_buf_of(rank, xk));
-        for (int c = wid; c < b; c += nwarps) {
-            const int col = id * b + c;
-            if (col >= N) continue;
-            const T* x = base + size_t(c) * len;
-            double s2 = 0;  // column norms in FP64 in both forms
-            for (int r = lane; r < M; r += 32) {
-                const double2 v = to_f64(x[r]);
-                s2 = fma(v.x, v.x, fma(v.y, v.y, s2));
-                Bf.w[size_t(col) * M + r] = v;
-            }
-            for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-            if (lane == 0) {
-                Bf.sigma[col] = sqrt(s2);
-                chk_out += s2;
-            }
-        }
-    }
-    // Factorisation check over the cluster (every CTA reaches it: the loop
-    // above ends on a cluster-uniform decision).
-    {
-        const double in_cta = block_total(chk_in, red);
-        const double out_cta = block_total(chk_out, red);
-        if (tid == 0) {
-            ctl.chk_in = in_cta;
-            ctl.chk_out = out_cta;
-        }
-        cluster.sync();
-        if (rank == 0 && tid == 0) {
-            double tin = 0, tout = 0;
-            for (int r = 0; r < C; ++r) {
-                const JacobiCtl* rc = cluster.map_shared_rank(&ctl, r);
-                tin += rc->chk_in;
-                tout += rc->chk_out;
-            }
-            const double tol = kF64 ? kSvdCheckTol : kSvdCheckTolFp32;
-            if (fabs(tout - tin) > tol * tin + 1e-28) atomicOr(status, kStatusSvdCheck);
-        }
-        cluster.sync();  // no CTA leaves while rank 0 reads its shared memory
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1184,7 +601,7 @@ __global__ void __launch_bounds__(kReg ? kJacobiRegThreads : kJacobiThreads) jac
 // and stores them back.  One cluster barrier separates the steps: every
 // block is held by one pair per step, so a block's store and its next load
 // are ordered by that barrier.  Rotation rule, tolerances, stop test and
-// outputs are those of jacobi_cluster_kernel.
+// outputs are those of jacobi_ring_kernel.
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(const SplitJob* jobs, SplitState* st,
@@ -1195,7 +612,7 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
     cg::cluster_group cluster = cg::this_cluster();
     const int C = int(cluster.num_blocks());
     const int rank = int(cluster.block_rank());
-    const int j = idx[blockIdx.x / C];
+    const int j = jacobi_entry_job(idx[blockIdx.x / C]);
     const SplitState S = st[j];
     if (!jacobi_active(S, mode)) return;  // uniform over the cluster
     const SplitJob& J = jobs[j];
@@ -1208,7 +625,7 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
     const int K = (N + 2 * b - 1) / (2 * b);
     const int nblk = 2 * K;
     const int Np = nblk * b;
-    const int vrows = phase == kPhaseFp32V ? N : 0;  // as in jacobi_cluster_kernel
+    const int vrows = phase == kPhaseFp32V ? N : 0;  // as in jacobi_ring_kernel
     const int len = M + vrows;
     const size_t blk = size_t(b) * len;
     T* G = reinterpret_cast<T*>(Bf.gs);
@@ -1230,7 +647,6 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
         if (phase == kPhaseFinish) return wsrc[size_t(col) * M + i];
         return rows_of_src ? cconj(src[size_t(col) * ld + i]) : src[size_t(i) * ld + col];
     };
-    if (tid == 0) ctl.rot = 0;
     // Frobenius norm: CTA r reads columns r, r+C, ...
     double part = 0;
     for (int col = rank; col < N; col += C)
@@ -1262,8 +678,8 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
     }
     __threadfence();
     cluster.sync();
-    const double tol = kF64 ? 1e-14 : 4e-6;
-    const double stop_rel2 = kF64 ? 1e-16 : 4e-6;
+    const double tol2 = kF64 ? kJacobiTol2 : kJacobiTol2Fp32;
+    const double stop_rel2 = kF64 ? kJacobiStop2 : kJacobiStop2Fp32;
     const double noise_floor = (kF64 ? 1e-30 : 1e-12) * fro2;  // squared column norm: 1e-15 (1e-6) of ||W||_F
     int sweep = 0;
     bool converged = false;
@@ -1272,11 +688,12 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
     for (; sweep < max_sweeps; ++sweep) {
         if (tid == 0) {
             ctl.rot = 0;
+            ctl.coarse = 0;
             ctl.relmax_bits = 0ull;
         }
         __syncthreads();
-        int my_rot = 0;
-        double my_rel = 0.0;
+        JacobiSweep my;
+        const bool want_ratio = sweep == max_sweeps - 1;
         for (int step = 0; step < nblk - 1; ++step) {
             for (int ps = rank; ps < K; ps += C) {
                 const int ida = circle_at(ps, step, nblk), idb = circle_at(nblk - 1 - ps, step, nblk);
@@ -1299,8 +716,8 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
                             T* base = top ? sA : sB;
                             const int e1 = circle_at(i, s2, bb), e2 = circle_at(bb - 1 - i, s2, bb);
                             if (e1 < b && e2 < b)
-                                my_rot += jacobi_rotate(base + size_t(e1) * len, base + size_t(e2) * len, M, len,
-                                                        tol, noise_floor, lane, my_rel);
+                                jacobi_rotate(base + size_t(e1) * len, base + size_t(e2) * len, M, len, tol2,
+                                              stop_rel2, noise_floor, want_ratio, lane, my);
                         }
                         __syncthreads();
                     }
@@ -1308,8 +725,8 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
                 for (int k = 0; k < b; ++k) {
                     for (int i = wid; i < b; i += nwarps) {
                         const int e2 = (i + k) % b;
-                        my_rot += jacobi_rotate(sA + size_t(i) * len, sB + size_t(e2) * len, M, len, tol,
-                                                noise_floor, lane, my_rel);
+                        jacobi_rotate(sA + size_t(i) * len, sB + size_t(e2) * len, M, len, tol2, stop_rel2,
+                                      noise_floor, want_ratio, lane, my);
                     }
                     __syncthreads();
                 }
@@ -1324,21 +741,21 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
             __threadfence();
             cluster.sync();
         }
-        if (lane == 0 && my_rot) atomicAdd(&ctl.rot, my_rot);
-        if (lane == 0 && my_rel > 0.0) atomicMax(&ctl.relmax_bits, (unsigned long long)__double_as_longlong(my_rel));
+        jacobi_report(ctl, my, lane);
         __syncthreads();
-        int total = 0;
-        double relmax = 0.0;
+        int total = 0, coarse = 0;
+        unsigned long long relmax_bits = 0;
         cluster.sync();
         for (int r = 0; r < C; ++r) {
             const JacobiCtl* rc = cluster.map_shared_rank(&ctl, r);
             total += rc->rot;
-            relmax = fmax(relmax, __longlong_as_double((long long)rc->relmax_bits));
+            coarse |= rc->coarse;
+            relmax_bits = max(relmax_bits, rc->relmax_bits);
         }
         cluster.sync();
         ctl_rot_last = total;
-        ctl_relmax_bits_last = (unsigned long long)__double_as_longlong(relmax);
-        if (total == 0 || relmax < stop_rel2) {
+        ctl_relmax_bits_last = relmax_bits;
+        if (total == 0 || !coarse) {
             converged = true;
             break;
         }
@@ -1381,7 +798,7 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
             chk_out += s2;
         }
     }
-    // Factorisation check over the cluster, as in jacobi_cluster_kernel.
+    // Factorisation check over the cluster, as in jacobi_ring_kernel.
     {
         const double in_cta = block_total(chk_in, red);
         const double out_cta = block_total(chk_out, red);
@@ -1804,14 +1221,6 @@ __global__ void __launch_bounds__(256) absorb_kernel(const SplitJob* jobs, const
 }  // namespace wqc
 
 namespace wqc {
-const void* jacobi_kernel(bool fp32, bool reg) {
-    if (reg)
-        return fp32 ? reinterpret_cast<const void*>(jacobi_cluster_kernel<float2, true>)
-                    : reinterpret_cast<const void*>(jacobi_cluster_kernel<double2, true>);
-    return fp32 ? reinterpret_cast<const void*>(jacobi_cluster_kernel<float2, false>)
-                : reinterpret_cast<const void*>(jacobi_cluster_kernel<double2, false>);
-}
-
 const void* qr_cluster(bool global_cols) {
     return global_cols ? reinterpret_cast<const void*>(qr_cluster_kernel<true>)
                        : reinterpret_cast<const void*>(qr_cluster_kernel<false>);
@@ -1836,21 +1245,5 @@ cudaError_t launch_jacobi_staged(bool fp32, const cudaLaunchConfig_t& cfg, const
                                   status, counters);
     return cudaLaunchKernelEx(&cfg, jacobi_staged_kernel<double2>, jobs, st, slots, idx, mode, phase, max_sweeps, b,
                               status, counters);
-}
-
-cudaError_t launch_jacobi(bool fp32, bool reg, const cudaLaunchConfig_t& cfg, const SplitJob* jobs, SplitState* st,
-                          const SlotBuffers* slots, const int* idx, int mode, int phase, int max_sweeps, int* status,
-                          unsigned long long* counters) {
-    if (fp32 && reg)
-        return cudaLaunchKernelEx(&cfg, jacobi_cluster_kernel<float2, true>, jobs, st, slots, idx, mode, phase,
-                                  max_sweeps, status, counters);
-    if (fp32)
-        return cudaLaunchKernelEx(&cfg, jacobi_cluster_kernel<float2, false>, jobs, st, slots, idx, mode, phase,
-                                  max_sweeps, status, counters);
-    if (reg)
-        return cudaLaunchKernelEx(&cfg, jacobi_cluster_kernel<double2, true>, jobs, st, slots, idx, mode, phase,
-                                  max_sweeps, status, counters);
-    return cudaLaunchKernelEx(&cfg, jacobi_cluster_kernel<double2, false>, jobs, st, slots, idx, mode, phase,
-                              max_sweeps, status, counters);
 }
 }  // namespace wqc

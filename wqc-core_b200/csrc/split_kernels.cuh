@@ -1,6 +1,8 @@
 // Kernel entry points of the two-site split pipeline and the site kernels.
 #pragma once
 
+#include <vector>
+
 #include "common.cuh"
 
 namespace wqc {
@@ -9,16 +11,29 @@ enum { kStageY0 = 0, kStageZ = 1, kStageY = 2, kStageB = 3 };
 // Jacobi / finalize modes: the range finder's B^H; theta of a split that takes
 // the exact path from the start; theta of a range-finder split that fell back.
 enum { kJacobiRsvd = 0, kJacobiExact = 1, kJacobiFallback = 2 };
-// Threads of the cluster Jacobi: one warp per column pair of a block per step.
-// The variant for columns of at most kJacobiRegMaxRows rows keeps each
-// warp's top column in registers through a block step and is limited to 12
-// warps (170 registers per thread); the other variant, like the staged
-// Jacobi, takes up to 16 warps.
-constexpr int kJacobiThreads = 512;
-constexpr int kJacobiRegThreads = 384;
-constexpr int kJacobiRegMaxRows = 256;
+// The cluster Jacobi (jacobi_ring.cu) stores a column as `kr` groups of 32
+// rows, one row of each group per lane, and is compiled for these counts: the
+// columns of W in the plain form, W's rows and under them V's (each from a
+// whole group on) in the precision form's first phase.  0: no instance.
+constexpr int jacobi_ring_kr(bool fp32, int M, int vrows) {
+    const int need = (M + 31) / 32 + (vrows + 31) / 32;
+    if (fp32) return need <= 2 ? 2 : need <= 4 ? 4 : need <= 8 ? 8 : need <= 16 ? 16 : need <= 24 ? 24 : 0;
+    return need <= 4 ? (need < 1 ? 1 : need) : need <= 6 ? 6 : need <= 8 ? 8 : need <= 12 ? 12 : 0;
+}
+// Warps of its largest CTA, one per column of a block: what 64 Ki registers
+// hold of two columns' rows per lane and about 60 registers besides.
+constexpr int jacobi_ring_warps(int kr, int elem) {
+    const int regs = 2 * kr * elem / 4 + 62;
+    return regs <= 80 ? 24 : regs <= 128 ? 16 : 12;
+}
+constexpr int kJacobiRingMaxCluster = 16;
+// Entry of a launch's task list: the job in the wave and log2 of the number
+// of CTAs it runs on.
+constexpr int kJacobiEntryShift = 24;
+__host__ __device__ inline int jacobi_entry(int job, int log2_c) { return job | (log2_c << kJacobiEntryShift); }
+__host__ __device__ inline int jacobi_entry_job(int e) { return e & ((1 << kJacobiEntryShift) - 1); }
+__host__ __device__ inline int jacobi_entry_cluster(int e) { return 1 << (e >> kJacobiEntryShift); }
 constexpr int kJacobiStagedThreads = 512;
-inline int jacobi_max_warps(int M) { return (M <= kJacobiRegMaxRows ? kJacobiRegThreads : kJacobiThreads) / 32; }
 
 __global__ void prepare_kernel(const SplitJob* jobs, SplitState* st, int njobs, DeviceMps mps);
 __global__ void merge_gate_kernel(const SplitJob* jobs, const SplitState* st, const SlotBuffers* slots,
@@ -38,16 +53,15 @@ inline size_t qr_cluster_smem_bytes(int m, int n, int C, bool global_cols = fals
     const int cpc = (n + C - 1) / C;
     return ((global_cols ? size_t(0) : size_t(2) * cpc * m) + size_t(3) * m + cpc) * sizeof(double2);
 }
-// The cluster Jacobi SVD kernel (a template over the column type: complex128
-// in the plain form, complex64 in the precision form), reached from other
-// files through these host functions.
-const void* jacobi_kernel(bool fp32, bool reg);
 // Phases of a Jacobi SVD: the plain one; the precision form's first phase
 // (complex64 columns carrying W = X V and the accumulated V, written out as
 // FP64 for the finish); and its finishing phase (FP64 sweeps that start from
 // X V, formed in FP64 by precond_gemm_kernel).
 enum { kPhasePlain = 0, kPhaseFp32V = 1, kPhaseFinish = 2 };
-cudaError_t launch_jacobi(bool fp32, bool reg, const cudaLaunchConfig_t& cfg, const SplitJob* jobs, SplitState* st,
+// The cluster Jacobi: every instance (for the kernel attributes) and a launch
+// of the one for kr row groups, on clusters of the largest size in the list.
+std::vector<const void*> jacobi_ring_kernels();
+cudaError_t launch_jacobi(bool fp32, int kr, const cudaLaunchConfig_t& cfg, const SplitJob* jobs, SplitState* st,
                           const SlotBuffers* slots, const int* idx, int mode, int phase, int max_sweeps, int* status,
                           unsigned long long* counters);
 // The staged variant for working matrices beyond a cluster's shared memory:
@@ -164,14 +178,7 @@ __global__ void adj_split_gemm_kernel(AdjSplit A, int stage);
 __global__ void adj_split_assemble_kernel(AdjSplit A);
 __global__ void adj_split_gate_kernel(AdjSplit A);
 
-// Jacobi shared-memory footprint for a working matrix of M rows and N columns
-// on a cluster of C CTAs, `elem` bytes per complex entry.
-inline size_t jacobi_smem_bytes(int M, int N, int C, size_t elem = sizeof(double2)) {
-    const int quantum = 4 * C;
-    const int Np = ((N + quantum - 1) / quantum) * quantum;
-    const int b = Np / (2 * C);
-    const int nbuf = C == 1 ? 2 : 3;
-    return size_t(nbuf) * b * M * elem;  // W columns only (plus padding columns)
-}
+// Shared memory of a CTA of the cluster Jacobi: two blocks of b columns.
+inline size_t jacobi_ring_smem(int b, int kr, size_t elem) { return size_t(2) * b * 32 * kr * elem; }
 
 }  // namespace wqc
