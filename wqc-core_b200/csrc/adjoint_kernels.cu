@@ -219,7 +219,8 @@ __device__ __forceinline__ int adj_active(const AdjSplit& A, int i, double smax)
 // R_bar^H sqrt(s) over the kept columns (zero elsewhere).
 __global__ void __launch_bounds__(256) adj_split_prep_kernel(AdjSplit A) {
     const SplitState S = *A.st;
-    const int m = S.rows, n = S.cols, N = min(m, n), M = max(m, n), k = S.chi, R = A.R;
+    const int m = S.rows, n = S.cols, N = min(m, n), k = S.chi, R = A.R;
+    const int M = S.w_rows_of_src ? n : m;  // entries of a column of W
     const double smax = N > 0 ? A.sigma[A.perm[0]] : 0.0;
     double2* Wside = S.w_rows_of_src ? A.V : A.U;
     const long stride = long(gridDim.x) * blockDim.x;

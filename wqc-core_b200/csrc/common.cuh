@@ -73,6 +73,7 @@ struct SplitJob {
     int reject;       // reject_truncation (time-split halves)
     int exact_only;   // split rule: exact SVD on every split, no range finder
     int chi_max;      // max bond dimension of the state (or batch slice) the split belongs to
+    int pre;          // bit 0: the exact Jacobi runs on R^H of a QR, bit 1: the range finder's does
     double2 u[16];    // effective 4x4 on theta: u[(so*2+to)*4 + si*2+ti]
 };
 
@@ -84,10 +85,13 @@ struct SplitState {
     int path;            // enum wqc_split_path
     int chi;             // kept bond
     int final_kind;      // 0: exact on theta, 1: rsvd accepted
-    int w_rows_of_src;   // exact Jacobi: 1 when W = theta^H (rows < cols)
+    int w_rows_of_src;   // exact Jacobi: 1 when W's columns are right vectors of theta (cols entries), 0 left
+    int pre_exact;       // the exact Jacobi runs on R^H of a QR (jacobi_qr_kernel)
+    int pre_rsvd;        // the range finder's Jacobi does
     int skip;            // cancelled before this wave: nothing is computed or written
     double discarded;
     double fro2;         // ||X||_F^2 seen by the precision form's first Jacobi phase
+    double pre_fro2;     // ||X||_F^2 of the dust-zeroed X that jacobi_qr_kernel factored
 };
 
 // Per-slot workspace pointers (device memory carved from one arena).

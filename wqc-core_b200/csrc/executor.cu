@@ -176,6 +176,7 @@ struct PhaseCfg {
 struct Group {
     int mode, count;
     int nph = 1;
+    int qr_kr = 0, qr_C = 0;  // QR before the first phase (0: none of the tasks takes one)
     PhaseCfg ph[2];
 };
 
@@ -214,6 +215,12 @@ struct wqc_mps {
     int n = 0, chi = 0;
     bool reject = false;
     bool exact_only = false;  // WQC_SPLIT_RULE_EXACT
+    // No QR before the Jacobi (set while an adjoint runs): the derivative
+    // divides by differences of squared singular values, and on a graded theta
+    // the vectors of the small ones are more exact from a Jacobi on theta
+    // itself (gradient of the 32-qubit ansatz against 64-bit autograd: 3.7e-7
+    // with the QR where 4.7e-8 without).
+    bool direct_svd = false;
     bool fp32 = false;        // WQC_PRECISION_FP32 or _TF32X3: complex64 Jacobi columns
     // WQC_PRECISION_TF32X3: merges on the tensor cores (tc_gemm.cu), their
     // operands staged per wave job as TF32 hi/lo planes under two tensor maps
@@ -372,6 +379,7 @@ void set_kernel_attributes() {
         if (g_attr_err == cudaSuccess)
             g_attr_err = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     }
+    if (g_attr_err == cudaSuccess) g_attr_err = jacobi_qr_attributes();
     for (const void* f : {qr_cluster(false), qr_cluster(true)}) {
         if (g_attr_err == cudaSuccess)
             g_attr_err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemLimit));
@@ -408,9 +416,11 @@ bool ring_shape(int M, int N, int vrows, size_t elem, int C, RingShape* out) {
 
 // Cluster size of a Jacobi task.  A sweep is (2C - 1) b + b rounds of rotation
 // (about N whatever C is) and 2C - 1 block moves with a cluster barrier.  A
-// round costs its dependent chain and the part of its FP64 work (20
-// instructions per row group and column) that the chain does not hide; the
-// constants are cycles measured on single SVDs of 8 to 384 columns.  A single
+// round costs its dependent chain (850 cycles) and, as the block's warps go
+// through it in step, the FP64 pipe's time for all of them (50 instructions a
+// column and 20 per row group) and their shared-memory traffic; constants
+// fitted to single SVDs of 8 to 384 columns on every cluster size (64
+// columns: 1080 cycles a round at b = 4, 1222 at 8, 1620 at 16).  A single
 // state is latency-bound (a few splits per level) and takes the shortest
 // sweep, until the wave's clusters would fill the GPU, from where SM time
 // counts.  A batch fills the GPU, so SM time decides, with as many CTAs on an
@@ -432,10 +442,11 @@ int choose_cluster(const wqc_cuda_ctx* ctx, int M, int N, int max_c, int njobs, 
     double best_cost = 1e300;
     for (int Cc = 1; Cc <= std::min(max_c, kJacobiRingMaxCluster); Cc *= 2) {
         if (!ring_shape(M, N, vrows, elem, Cc, &s)) continue;
-        const double work = 10.0 * s.kr * s.b * double(elem) / sizeof(double2);  // FP64 pipe cycles of a round
-        const double round = 620.0 + 20.0 * s.kr + 0.6 * work;
+        const double kr = s.kr * double(elem) / sizeof(double2);
+        const double work = s.b * (25.0 + 10.0 * kr);  // FP64 pipe cycles of a round
+        const double round = 850.0 + work + 0.6 * kr * kr * s.b;
         const double rounds = 2.0 * Cc * s.b;
-        const double moves = Cc > 1 ? (2 * Cc - 1) * 700.0 + 2500.0 : 200.0;
+        const double moves = Cc > 1 ? (2 * Cc - 1) * 700.0 + 2500.0 : 0.0;
         double cost = rounds * round + moves;
         if (throughput) {
             const int by_threads = 2048 / (32 * s.warps), by_smem = int(kSmemLimit / s.smem);
@@ -729,12 +740,24 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                 cols = 2 * lb.bounds[k].second;
                 ell = std::min(std::min(lb.jobs[k].chi_max + kRsvdOversample, rows), cols);
             };
-            // Working matrix of a job in a mode: M x N, M >= N.
+            // Working matrix of a job in a mode: M x N, M >= N; and the matrix
+            // its Jacobi runs on, R^H where a QR comes first.  Both are upper
+            // bounds, and the choice of a QR is made from them alone, so the
+            // device takes it from the job.
             auto dims = [&](size_t k, int mode, int& M, int& N) {
                 int rows, cols, ell;
                 shape(k, rows, cols, ell);
                 M = mode != kJacobiRsvd ? std::max(rows, cols) : cols;
                 N = mode != kJacobiRsvd ? std::min(rows, cols) : ell;
+            };
+            auto takes_qr = [&](size_t k, int mode) {
+                int M, N;
+                dims(k, mode, M, N);
+                return !m->direct_svd && jacobi_qr_takes(M, N);
+            };
+            auto jacobi_dims = [&](size_t k, int mode, int& M, int& N) {
+                dims(k, mode, M, N);
+                if (takes_qr(k, mode)) M = N;
             };
             // The wave takes the level's next jobs while their bucket has a
             // free slot (every job of a level is independent of the others).
@@ -777,6 +800,7 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                 const size_t k = sel[local];
                 SplitJob J = lb.jobs[k];
                 J.slot = sel_slot[local];
+                J.pre = (takes_qr(k, kJacobiExact) ? 1 : 0) | (takes_qr(k, kJacobiRsvd) ? 2 : 0);
                 plan.jobs.push_back(J);
                 plan.slice_last_wave[lb.job_slice[k]] = std::max(plan.slice_last_wave[lb.job_slice[k]], wave_index);
                 int rows, cols, ell;
@@ -790,12 +814,12 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                 w.max_cols = std::max(w.max_cols, cols);
                 w.max_ell = std::max(w.max_ell, ell);
                 int M, N;
-                dims(k, kJacobiExact, M, N);
+                jacobi_dims(k, kJacobiExact, M, N);
                 add_task(kJacobiExact, M, N, local);
                 if (rs) {
                     w.any_rsvd = true;
                     add_task(kJacobiFallback, M, N, local);
-                    dims(k, kJacobiRsvd, M, N);
+                    jacobi_dims(k, kJacobiRsvd, M, N);
                     add_task(kJacobiRsvd, M, N, local);
                 }
             }
@@ -809,7 +833,7 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                     pc.C = m->ctx->max_cluster;
                     for (const Task& t : tasks) {
                         int M, N;
-                        dims(sel[t.local], mode, M, N);
+                        jacobi_dims(sel[t.local], mode, M, N);
                         pc.smem = std::max(pc.smem, size_t(2) * pc.b * size_t(with_v ? M + N : M) * elem);
                         plan.idx.push_back(jacobi_entry(t.local, 0));
                     }
@@ -819,7 +843,7 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                 int warps = 1, b = 1;
                 for (const Task& t : tasks) {
                     int M, N;
-                    dims(sel[t.local], mode, M, N);
+                    jacobi_dims(sel[t.local], mode, M, N);
                     RingShape s;
                     const int c = first ? t.c1 : t.c2;
                     ring_shape(M, N, with_v ? N : 0, elem, c, &s);
@@ -838,6 +862,13 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                 Group gr;
                 gr.mode = g.first.mode;
                 gr.count = int(g.second.size());
+                for (const Task& t : g.second) {
+                    if (!takes_qr(sel[t.local], gr.mode)) continue;
+                    int M, N;
+                    dims(sel[t.local], gr.mode, M, N);
+                    gr.qr_kr = std::max(gr.qr_kr, jacobi_qr_kr(M));
+                    gr.qr_C = std::max(gr.qr_C, std::min(m->ctx->max_cluster, (N + kJacobiQrPerCta - 1) / kJacobiQrPerCta));
+                }
                 if (m->fp32) {
                     gr.nph = 2;
                     fill(gr.ph[0], g.first.k1, true, gr.mode, g.second, sizeof(float2), true);
@@ -1008,6 +1039,12 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
             for (const Group& gr : w.groups) {
                 if (gr.mode != mode) continue;
                 any = true;
+                if (gr.qr_kr) {
+                    Timed t(m, 0, on);
+                    CUDA_TRY(launch_jacobi_qr(gr.qr_kr, gr.qr_C, gr.count, on, d_jobs, m->d_state, m->d_slots,
+                                              d_idx + gr.ph[0].idx_off, mode, m->d_status));
+                    count_launch(m, 0);
+                }
                 if (gr.nph == 1) {
                     if (wqc_status s = launch_phase(gr, gr.ph[0], mode, kPhasePlain, false, on)) return s;
                 } else if (wqc_status s = launch_phase(gr, gr.ph[0], mode, kPhaseFp32V, true, on)) {
@@ -1030,7 +1067,7 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
                     if (wqc_status s = launch_phase(gr, gr.ph[1], mode, kPhaseFinish, false, on)) return s;
             {
                 Timed t(m, 4, on);
-                svd_probe_kernel<<<dim3(nj, 2), 256, 0, on>>>(d_jobs, m->d_state, m->d_slots, mode, 0, m->d_status);
+                svd_probe_kernel<<<dim3(nj, 2), kProbeThreads, 0, on>>>(d_jobs, m->d_state, m->d_slots, mode, 0, m->d_status);
                 count_launch(m, 4);
             }
             return WQC_OK;
@@ -1118,7 +1155,8 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
             const int kmax = std::min(m->chi, std::min(w.max_rows, w.max_cols));
             auto tiles = [](int x) { return (x + 31) / 32; };
             if (w.any_rsvd) {
-                recover_gemm_kernel<<<dim3(tiles(kmax), tiles(w.max_ell), nj), 256, 0, m->stream>>>(
+                recover_gemm_kernel<<<dim3(tiles(std::max(w.max_cols, kmax)), tiles(std::max(w.max_ell, kmax)), nj), 256, 0,
+                                      m->stream>>>(
                     d_jobs, m->d_state, m->d_slots, m->dev, kRecoverBW);
                 recover_gemm_kernel<<<dim3(tiles(kmax), tiles(w.max_rows), nj), 256, 0, m->stream>>>(
                     d_jobs, m->d_state, m->d_slots, m->dev, kRecoverQT);
@@ -2416,6 +2454,7 @@ wqc_status wqc_adjoint_forward(wqc_mps* m, const wqc_gate* gates, uint32_t count
     a->cp_ub.resize(a->starts.size() + 1);
     const bool rule = m->exact_only;
     m->exact_only = true;
+    m->direct_svd = true;
     wqc_status st = wqc_mps_reset(m);
     for (size_t sgi = 0; sgi < a->starts.size() && st == WQC_OK; ++sgi) {
         if (sgi > 0) st = adj_save(a, sgi);
@@ -2429,6 +2468,7 @@ wqc_status wqc_adjoint_forward(wqc_mps* m, const wqc_gate* gates, uint32_t count
     if (st == WQC_OK) st = adj_save(a, a->starts.size());
     if (st == WQC_OK) st = sync_status(m);
     m->exact_only = rule;
+    m->direct_svd = false;
     a->end_records = m->rec_count;
     if (st != WQC_OK) {
         wqc_adjoint_destroy(a);
@@ -2454,10 +2494,14 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
     CUDA_TRY(cudaSetDevice(m->ctx->device));
     const bool rule = m->exact_only;
     m->exact_only = true;
+    m->direct_svd = true;
     struct RuleGuard {
         wqc_mps* m;
         bool rule;
-        ~RuleGuard() { m->exact_only = rule; }
+        ~RuleGuard() {
+            m->exact_only = rule;
+            m->direct_svd = false;
+        }
     } guard{m, rule};
     AdjBuffers buf(m);
     const size_t site_cap = size_t(chi) * 2 * chi;
@@ -2708,7 +2752,7 @@ void wqc_adjoint_destroy(wqc_adjoint* a) {
 // ===========================================================================
 namespace {
 
-constexpr int kTuneVersion = 2;
+constexpr int kTuneVersion = 1;
 
 std::string tune_fingerprint(const wqc_cuda_ctx* ctx) {
     cudaDeviceProp prop{};
@@ -2722,7 +2766,7 @@ std::string tune_fingerprint(const wqc_cuda_ctx* ctx) {
     return "wqc-jacobi-clusters v" + std::to_string(kTuneVersion) + "|" + name + "|sm=" +
            std::to_string(prop.multiProcessorCount) + "|cc=" + std::to_string(prop.major) + "." +
            std::to_string(prop.minor) + "|driver=" + std::to_string(drv) + "|runtime=" + std::to_string(rt) +
-           "|max_cluster=" + std::to_string(ctx->max_cluster);
+           "|max_cluster=" + std::to_string(ctx->max_cluster) + "|jacobi=ring,qr";
 }
 
 std::string tune_cache_path(const char* path) {

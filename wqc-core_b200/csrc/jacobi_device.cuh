@@ -32,6 +32,17 @@ constexpr double kSvdCheckTolFp32 = 1e-4;
 constexpr double kJacobiTol2 = 1e-28, kJacobiTol2Fp32 = 1.6e-11;
 constexpr double kJacobiStop2 = 1e-16, kJacobiStop2Fp32 = 4e-6;
 
+// Singular values of an exact SVD at or below 18 eps ||X||_F are reported as
+// zero: rounding leaves such values where X has none, their W columns are not
+// orthogonal to the others, and one that a state of large norm lifts over the
+// absolute cutoff of 1e-12 would enter the cut as a vector (a rank 20 theta of
+// norm 1600 kept 250 vectors and a product off by ten times its norm).  At
+// norm 1 the bound is 4e-15 and decides nothing.  Squared.
+constexpr double kJacobiZero2 = 1.6e-29;
+__device__ __forceinline__ double jacobi_sigma(double s2, double fro2, int mode) {
+    return mode != kJacobiRsvd && s2 <= kJacobiZero2 * fro2 ? 0.0 : sqrt(s2);
+}
+
 __device__ __forceinline__ double block_total(double v, double* red) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -165,6 +176,8 @@ __device__ __forceinline__ bool jacobi_params(double a, double bb, double gr, do
     return true;
 }
 
+// The original working matrix X of a task: column j of X (M x N, M >= N) is
+// column j of src, or with rows_of_src the conjugate of src's row j.
 __device__ __forceinline__ void jacobi_task(const SplitJob& J, const SplitState& S, const SlotBuffers& B, int mode,
                                             const double2*& src, int& sr, int& sc, int& ld, int& rows_of_src) {
     if (mode == kJacobiRsvd) {  // W = B^H, B is ell x cols row-major
@@ -173,12 +186,12 @@ __device__ __forceinline__ void jacobi_task(const SplitJob& J, const SplitState&
         sc = S.cols;
         ld = S.cols;
         rows_of_src = 1;
-    } else {  // exact: W = theta (rows >= cols) or theta^H
+    } else {  // exact: theta (rows >= cols) or theta^H
         src = B.theta;
         sr = S.rows;
         sc = S.cols;
         ld = S.cols;
-        rows_of_src = S.w_rows_of_src;
+        rows_of_src = S.rows < S.cols ? 1 : 0;
     }
 }
 
@@ -188,6 +201,46 @@ __device__ __forceinline__ bool jacobi_active(const SplitState& S, int mode) {
     // fallback changes a range-finder split's path to RSVD_FALLBACK only.
     if (mode == kJacobiExact) return S.need_exact != 0 && S.path == WQC_SPLIT_EXACT;
     return S.need_exact != 0 && S.path == WQC_SPLIT_RSVD_FALLBACK;
+}
+
+// Whether the task's Jacobi runs on A = P R^H (jacobi_qr.cu), N x N and
+// column-major in a buffer that nothing else of the split uses by then: Y
+// once Q is formed; the range finder's Q and B for the splits that are not
+// its own (2 R E >= R^2 entries).  W then holds X's right vectors.
+__device__ __forceinline__ bool jacobi_preconditioned(const SplitState& S, int mode) {
+    return mode == kJacobiRsvd ? S.pre_rsvd != 0 : S.pre_exact != 0;
+}
+__device__ __forceinline__ double2* jacobi_pre_matrix(const SlotBuffers& B, int mode) {
+    return mode == kJacobiRsvd ? B.y : B.q;
+}
+
+// The matrix whose columns a Jacobi task orthogonalises.
+struct JacobiMatrix {
+    const double2* p;
+    int M, N, ld;
+    int by_rows;  // column j is the conjugate of row j
+    int by_cols;  // column-major
+    __device__ __forceinline__ double2 at(int i, int col) const {
+        if (by_cols) return p[size_t(col) * ld + i];
+        return by_rows ? cconj(p[size_t(col) * ld + i]) : p[size_t(i) * ld + col];
+    }
+    __device__ __forceinline__ bool contiguous() const { return by_cols || by_rows; }
+};
+__device__ __forceinline__ JacobiMatrix jacobi_matrix(const SplitJob& J, const SplitState& S, const SlotBuffers& B,
+                                                      int mode) {
+    JacobiMatrix x;
+    int sr, sc;
+    jacobi_task(J, S, B, mode, x.p, sr, sc, x.ld, x.by_rows);
+    x.M = x.by_rows ? sc : sr;
+    x.N = x.by_rows ? sr : sc;
+    x.by_cols = 0;
+    if (jacobi_preconditioned(S, mode)) {
+        x.p = jacobi_pre_matrix(B, mode);
+        x.M = x.ld = x.N;
+        x.by_rows = 0;
+        x.by_cols = 1;
+    }
+    return x;
 }
 
 template <typename T>

@@ -104,11 +104,15 @@ __global__ void __launch_bounds__(jacobi_ring_warps(KR, sizeof(T)) * 32) jacobi_
     if (!jacobi_active(S, mode)) return;  // uniform over the task's CTAs
     const SplitJob& J = jobs[j];
     const SlotBuffers Bf = slots[J.slot];
-    const double2* src;
-    int sr, sc, ld, rows_of_src;
-    jacobi_task(J, S, Bf, mode, src, sr, sc, ld, rows_of_src);
-    const int M = rows_of_src ? sc : sr;
-    const int N = rows_of_src ? sr : sc;
+    JacobiMatrix X = jacobi_matrix(J, S, Bf, mode);
+    const bool pre = jacobi_preconditioned(S, mode);
+    if (phase == kPhaseFinish) {  // from X V, in the slot's W buffer
+        X.p = Bf.w;
+        X.ld = X.M;
+        X.by_rows = 0;
+        X.by_cols = 1;
+    }
+    const int M = X.M, N = X.N;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int nthreads = blockDim.x, nwarps = nthreads >> 5;
     const int b = (N + 2 * C - 1) / (2 * C);
@@ -118,7 +122,8 @@ __global__ void __launch_bounds__(jacobi_ring_warps(KR, sizeof(T)) * 32) jacobi_
         if (tid == 0 && rank == 0) atomicOr(status, kStatusBadShape);
         return;
     }
-    const bool colmajor = rows_of_src || phase == kPhaseFinish;
+    const bool colmajor = X.contiguous();
+    const bool dusted = pre || phase == kPhaseFinish;  // entries already dust-zeroed
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* smem = reinterpret_cast<T*>(smem_raw);
@@ -128,14 +133,7 @@ __global__ void __launch_bounds__(jacobi_ring_warps(KR, sizeof(T)) * 32) jacobi_
     __shared__ int ids[2];  // block held by each buffer
     auto column = [&](int buffer, int c) { return smem + size_t(buffer) * blk + size_t(c) * LD; };
 
-    const double2* wsrc = Bf.w;
-    auto src_at = [&](int i, int col) -> double2 {
-        if (phase == kPhaseFinish) return wsrc[size_t(col) * M + i];
-        return rows_of_src ? cconj(src[size_t(col) * ld + i]) : src[size_t(i) * ld + col];
-    };
     // Frobenius norm over the columns this CTA loads, then over the cluster.
-    // The precision form's finishing phase starts from X V (column-major in
-    // the slot's W buffer), formed from the dust-zeroed X.
     double part = 0;
     for (int half = 0; half < 2; ++half) {
         const int id = half * C + rank;
@@ -143,7 +141,7 @@ __global__ void __launch_bounds__(jacobi_ring_warps(KR, sizeof(T)) * 32) jacobi_
             int c, i;
             if (colmajor) { c = e / M; i = e % M; } else { i = e / b; c = e % b; }
             const int col = id * b + c;
-            if (col < N) part += cnorm2(src_at(i, col));
+            if (col < N) part += cnorm2(X.at(i, col));
         }
     }
     const double cta_part = block_total(part, red);
@@ -169,8 +167,8 @@ __global__ void __launch_bounds__(jacobi_ring_warps(KR, sizeof(T)) * 32) jacobi_
             int c, i;
             if (colmajor) { c = e / M; i = e % M; } else { i = e / b; c = e % b; }
             const int col = id * b + c;
-            double2 x = col < N ? src_at(i, col) : cmake(0, 0);
-            if (phase != kPhaseFinish && cnorm2(x) < dust2) x = cmake(0, 0);
+            double2 x = col < N ? X.at(i, col) : cmake(0, 0);
+            if (!dusted && cnorm2(x) < dust2) x = cmake(0, 0);
             chk_in += cnorm2(x);
             column(half, c)[i] = to_store<T>(x);
         }
@@ -356,7 +354,7 @@ __global__ void __launch_bounds__(jacobi_ring_warps(KR, sizeof(T)) * 32) jacobi_
             }
             for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
             if (lane == 0) {
-                Bf.sigma[col] = sqrt(s2);
+                Bf.sigma[col] = jacobi_sigma(s2, fro2, mode);
                 chk_out += s2;
             }
         }
@@ -375,6 +373,7 @@ __global__ void __launch_bounds__(jacobi_ring_warps(KR, sizeof(T)) * 32) jacobi_
                 tin += rc->chk_in;
                 tout += rc->chk_out;
             }
+            if (pre) tin = S.pre_fro2;  // the matrix before its QR
             const double tol = kF64 ? kSvdCheckTol : kSvdCheckTolFp32;
             if (fabs(tout - tin) > tol * tin + 1e-28) atomicOr(status, kStatusSvdCheck);
         }

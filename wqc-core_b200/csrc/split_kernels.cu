@@ -45,7 +45,11 @@ __global__ void prepare_kernel(const SplitJob* jobs, SplitState* st, int njobs, 
     s.use_rsvd = (!J.reject && !J.exact_only && s.ell > 0 && s.ell < min(s.rows, s.cols) && worth) ? 1 : 0;
     s.need_exact = s.use_rsvd ? 0 : 1;
     s.path = s.use_rsvd ? WQC_SPLIT_RSVD : WQC_SPLIT_EXACT;
-    s.w_rows_of_src = s.rows < s.cols ? 1 : 0;
+    s.pre_exact = J.pre & 1;
+    s.pre_rsvd = (J.pre >> 1) & 1;
+    // W of X = theta (rows >= cols) holds left vectors, of theta^H right ones;
+    // a Jacobi on R^H gives the other side.
+    s.w_rows_of_src = (s.rows < s.cols) != (s.pre_exact != 0) ? 1 : 0;
     st[j] = s;
 }
 
@@ -617,11 +621,16 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
     if (!jacobi_active(S, mode)) return;  // uniform over the cluster
     const SplitJob& J = jobs[j];
     const SlotBuffers Bf = slots[J.slot];
-    const double2* src;
-    int sr, sc, ld, rows_of_src;
-    jacobi_task(J, S, Bf, mode, src, sr, sc, ld, rows_of_src);
-    const int M = rows_of_src ? sc : sr;
-    const int N = rows_of_src ? sr : sc;
+    JacobiMatrix X = jacobi_matrix(J, S, Bf, mode);
+    const bool pre = jacobi_preconditioned(S, mode);
+    if (phase == kPhaseFinish) {  // from X V, in the slot's W buffer
+        X.p = Bf.w;
+        X.ld = X.M;
+        X.by_rows = 0;
+        X.by_cols = 1;
+    }
+    const bool dusted = pre || phase == kPhaseFinish;  // entries already dust-zeroed
+    const int M = X.M, N = X.N;
     const int K = (N + 2 * b - 1) / (2 * b);
     const int nblk = 2 * K;
     const int Np = nblk * b;
@@ -642,15 +651,10 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int nthreads = blockDim.x;
     const int nwarps = nthreads / 32;
-    const double2* wsrc = Bf.w;
-    auto src_at = [&](int i, int col) -> double2 {
-        if (phase == kPhaseFinish) return wsrc[size_t(col) * M + i];
-        return rows_of_src ? cconj(src[size_t(col) * ld + i]) : src[size_t(i) * ld + col];
-    };
     // Frobenius norm: CTA r reads columns r, r+C, ...
     double part = 0;
     for (int col = rank; col < N; col += C)
-        for (int i = tid; i < M; i += nthreads) part += cnorm2(src_at(i, col));
+        for (int i = tid; i < M; i += nthreads) part += cnorm2(X.at(i, col));
     for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
     if (lane == 0) red[wid] = part;
     __syncthreads();
@@ -669,8 +673,8 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
     for (int col = rank; col < Np; col += C) {
         T* x = G + size_t(col) * len;
         for (int i = tid; i < M; i += nthreads) {
-            double2 v = col < N ? src_at(i, col) : cmake(0, 0);
-            if (phase != kPhaseFinish && cnorm2(v) < dust2) v = cmake(0, 0);
+            double2 v = col < N ? X.at(i, col) : cmake(0, 0);
+            if (!dusted && cnorm2(v) < dust2) v = cmake(0, 0);
             chk_in += cnorm2(v);
             x[i] = to_store<T>(v);
         }
@@ -794,7 +798,7 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
         }
         for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
         if (lane == 0) {
-            Bf.sigma[col] = sqrt(s2);
+            Bf.sigma[col] = jacobi_sigma(s2, fro2, mode);
             chk_out += s2;
         }
     }
@@ -814,6 +818,7 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
                 tin += rc->chk_in;
                 tout += rc->chk_out;
             }
+            if (pre) tin = S.pre_fro2;  // the matrix before its QR
             const double tol = kF64 ? kSvdCheckTol : kSvdCheckTolFp32;
             if (fabs(tout - tin) > tol * tin + 1e-28) atomicOr(status, kStatusSvdCheck);
         }
@@ -828,7 +833,9 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
 // p 0.56984029), to 1e-9 ||X||_F ||x|| + 1e-14.  The Jacobi keeps W = X V =
 // U Sigma and no V, and U Sigma V^H x = U U^H X x over the columns with
 // sigma > 0, so with y = X x the rebuilt vector is W diag(1/sigma^2) W^H y:
-// it equals y only when W's columns are orthogonal and span X's range.
+// it equals y only when W's columns are orthogonal and span X's range.  A
+// Jacobi on R^H (jacobi_qr.cu) leaves X's right vectors in W: the same check
+// on X^H, which covers the QR too.
 // Columns at the storage's rounding level (the Jacobi's noise floor) are
 // left out: their direction is noise and they carry less than the tolerance.
 // One CTA per (job, probe); a failure sets the same status as the Frobenius
@@ -836,8 +843,46 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
 // ---------------------------------------------------------------------------
 constexpr int kProbeMax = 512;
 
-__global__ void __launch_bounds__(256) svd_probe_kernel(const SplitJob* jobs, const SplitState* st,
-                                                        const SlotBuffers* slots, int mode, int fp32, int* status) {
+// out[i] = sum_c A(i, c) x[c] for i < M, c < N.  With `down` A(i, c) runs
+// fastest in memory over i: a thread per row, the columns dealt to
+// kProbeThreads / (M rounded up to a warp) groups of threads whose parts are
+// added in order; else a warp per row, lanes along it.  Ends with a barrier.
+template <typename At>
+__device__ __forceinline__ void probe_matvec(int M, int N, bool down, At at, const double2* x, double2* out,
+                                             double2* parts) {
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    if (down) {
+        const int span = (M + 31) & ~31, groups = kProbeThreads / span;  // span <= 512
+        const int g = tid / span, i = tid % span;
+        double2 acc = cmake(0, 0);
+        if (g < groups && i < M)
+#pragma unroll 8
+            for (int c = g; c < N; c += groups) cfma(acc, at(i, c), x[c]);
+        if (g < groups) parts[tid] = acc;
+        __syncthreads();
+        for (int r = tid; r < M; r += kProbeThreads) {
+            double2 t = parts[r];
+            for (int q = 1; q < groups; ++q) t = cadd(t, parts[q * span + r]);
+            out[r] = t;
+        }
+    } else {
+        for (int i = wid; i < M; i += kProbeThreads / 32) {
+            double2 acc = cmake(0, 0);
+#pragma unroll 4
+            for (int c = lane; c < N; c += 32) cfma(acc, at(i, c), x[c]);
+            for (int o = 16; o > 0; o >>= 1) {
+                acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+                acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+            }
+            if (lane == 0) out[i] = acc;
+        }
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kProbeThreads) svd_probe_kernel(const SplitJob* jobs, const SplitState* st,
+                                                                  const SlotBuffers* slots, int mode, int fp32,
+                                                                  int* status) {
     const int j = blockIdx.x;
     const int probe = blockIdx.y;
     const SplitState S = st[j];
@@ -847,74 +892,50 @@ __global__ void __launch_bounds__(256) svd_probe_kernel(const SplitJob* jobs, co
     const double2* src;
     int sr, sc, ld, rows_of_src;
     jacobi_task(J, S, Bf, mode, src, sr, sc, ld, rows_of_src);
+    // W's columns are left vectors of X, or with a preconditioned Jacobi left
+    // vectors of X^H: the check is made on that matrix, M x N with K columns of W.
+    const int K = rows_of_src ? sr : sc;
+    if (jacobi_preconditioned(S, mode)) rows_of_src = !rows_of_src;
     const int M = rows_of_src ? sc : sr;
     const int N = rows_of_src ? sr : sc;
     if (M > kProbeMax || N > kProbeMax) {
         if (threadIdx.x == 0) atomicOr(status, kStatusBadShape);
         return;
     }
-    __shared__ double2 xs[kProbeMax], ys[kProbeMax], zs[kProbeMax];
-    __shared__ double red[8];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+    __shared__ double2 xs[kProbeMax], ys[kProbeMax], zs[kProbeMax], parts[kProbeThreads];
+    __shared__ double red[kProbeThreads / 32];
+    const int tid = threadIdx.x;
     const double step = 0.754877666 + double(probe) * 0.56984029;
     double fro2_part = 0;
-    for (int c = tid; c < N; c += blockDim.x) {
+    for (int c = tid; c < N; c += kProbeThreads) {
         double sn, cs;
         sincos(double(c + 1) * step, &sn, &cs);
         xs[c] = cmake(sn, cs);
+    }
+    for (int c = tid; c < K; c += kProbeThreads) {
         const double sg = Bf.sigma[c];
         fro2_part += sg * sg;
     }
-    for (int o = 16; o > 0; o >>= 1) fro2_part += __shfl_xor_sync(0xffffffffu, fro2_part, o);
-    if (lane == 0) red[wid] = fro2_part;
-    __syncthreads();
-    double fro2 = 0;
-    for (int w = 0; w < nw; ++w) fro2 += red[w];
+    const double fro2 = block_total(fro2_part, red);  // its barriers also publish xs
     const double floor2 = (fp32 ? 1e-12 : 1e-30) * fro2;
-    // y = X x, one warp per row.
-    for (int i = wid; i < M; i += nw) {
-        double2 acc = cmake(0, 0);
-        for (int c = lane; c < N; c += 32) {
-            const double2 a = rows_of_src ? cconj(src[size_t(c) * ld + i]) : src[size_t(i) * ld + c];
-            cfma(acc, a, xs[c]);
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
-            acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
-        }
-        if (lane == 0) ys[i] = acc;
-    }
-    __syncthreads();
-    // z = diag(1/sigma^2) W^H y, one warp per column.
-    for (int c = wid; c < N; c += nw) {
+    // y = X x.
+    if (rows_of_src)
+        probe_matvec(M, N, true, [&](int i, int c) { return cconj(src[size_t(c) * ld + i]); }, xs, ys, parts);
+    else
+        probe_matvec(M, N, false, [&](int i, int c) { return src[size_t(i) * ld + c]; }, xs, ys, parts);
+    // z = diag(1/sigma^2) W^H y.
+    probe_matvec(K, M, false, [&](int c, int i) { return cconj(Bf.w[size_t(c) * M + i]); }, ys, zs, parts);
+    for (int c = tid; c < K; c += kProbeThreads) {
         const double sg = Bf.sigma[c];
-        double2 acc = cmake(0, 0);
-        if (sg * sg > floor2) {
-            const double2* wc = Bf.w + size_t(c) * M;
-            for (int i = lane; i < M; i += 32) cfma_conj(acc, wc[i], ys[i]);
-            for (int o = 16; o > 0; o >>= 1) {
-                acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
-                acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
-            }
-            acc = cscale(acc, 1.0 / (sg * sg));
-        }
-        if (lane == 0) zs[c] = acc;
+        zs[c] = sg * sg > floor2 ? cscale(zs[c], 1.0 / (sg * sg)) : cmake(0, 0);
     }
     __syncthreads();
-    // |y - W z|^2, one thread per row.
+    // |y - W z|^2.
+    probe_matvec(M, K, true, [&](int i, int c) { return Bf.w[size_t(c) * M + i]; }, zs, xs, parts);
     double err2 = 0;
-    for (int i = tid; i < M; i += blockDim.x) {
-        double2 r = cmake(0, 0);
-        for (int c = 0; c < N; ++c) cfma(r, Bf.w[size_t(c) * M + i], zs[c]);
-        err2 += cnorm2(csub(ys[i], r));
-    }
-    for (int o = 16; o > 0; o >>= 1) err2 += __shfl_xor_sync(0xffffffffu, err2, o);
-    __syncthreads();
-    if (lane == 0) red[wid] = err2;
-    __syncthreads();
+    for (int i = tid; i < M; i += kProbeThreads) err2 += cnorm2(csub(ys[i], xs[i]));
+    const double e2 = block_total(err2, red);
     if (tid == 0) {
-        double e2 = 0;
-        for (int w = 0; w < nw; ++w) e2 += red[w];
         const double tol = fp32 ? 1e-4 : 1e-9;  // the Frobenius check's tolerance of each form
         if (!(sqrt(e2) <= tol * sqrt(fro2) * sqrt(double(N)) + 1e-14)) atomicOr(status, kStatusSvdCheck);
     }
@@ -934,10 +955,8 @@ __global__ void __launch_bounds__(256) precond_gemm_kernel(const SplitJob* jobs,
     if (!jacobi_active(S, mode)) return;
     const SplitJob& J = jobs[j];
     const SlotBuffers B = slots[J.slot];
-    const double2* src;
-    int sr, sc, ld, rows_of_src;
-    jacobi_task(J, S, B, mode, src, sr, sc, ld, rows_of_src);
-    const int M = rows_of_src ? sc : sr, N = rows_of_src ? sr : sc;
+    const JacobiMatrix X = jacobi_matrix(J, S, B, mode);
+    const int M = X.M, N = X.N;
     const bool last = stage == kPrecondXV;
     const int m = last ? M : N, n = N, k = N;
     const int i0 = blockIdx.y * kGemmT, n0 = blockIdx.x * kGemmT;
@@ -948,11 +967,11 @@ __global__ void __launch_bounds__(256) precond_gemm_kernel(const SplitJob* jobs,
     double2* G = B.omega;
     double2* Vout = second ? B.z : B.zr;
     const bool gram = stage == kPrecondGram1 || stage == kPrecondGram2;
-    const double dust2 = kDustRel * kDustRel * S.fro2;
+    const double dust2 = jacobi_preconditioned(S, mode) ? 0.0 : kDustRel * kDustRel * S.fro2;
     auto a_at = [&](int i, int kk) -> double2 {
         if (gram) return cconj(V[size_t(i) * N + kk]);  // V^H
         if (!last) return V[size_t(kk) * N + i];
-        const double2 x = rows_of_src ? cconj(src[size_t(kk) * ld + i]) : src[size_t(i) * ld + kk];
+        const double2 x = X.at(i, kk);
         return cnorm2(x) < dust2 ? cmake(0, 0) : x;  // X, dust-zeroed as the first phase loaded it
     };
     auto b_at = [&](int kk, int jj) -> double2 {
@@ -1088,8 +1107,11 @@ __global__ void finalize_kernel(const SplitJob* jobs, SplitState* st, const Slot
 // or B^H, so (kept columns, sigma > 0):
 //   kRecoverBW:   T = B W_k                  (ell x chi, into the slot's z, column pc)
 //   kRecoverQT:   L = Q T s^-3/2             (range finder, rows x chi, into site p)
-//   kRecoverExact: R = s^-3/2 W_k^H theta    (theta, rows >= cols, into site p+1)
-//                  L = theta W_k s^-3/2      (theta^H, rows < cols, into site p)
+//   kRecoverExact: R = s^-3/2 W_k^H theta    (W left vectors, into site p+1)
+//                  L = theta W_k s^-3/2      (W right vectors, into site p)
+// A range finder's Jacobi on R^H (jacobi_qr.cu) leaves B's left vectors in W:
+//   kRecoverBW:   R = s^-3/2 W_k^H B         (chi x cols, into site p+1)
+//   kRecoverQT:   L = Q W_k s^-1/2           (rows x chi, into site p)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) recover_gemm_kernel(const SplitJob* jobs, const SplitState* st,
                                                            const SlotBuffers* slots, DeviceMps mps, int stage) {
@@ -1106,8 +1128,9 @@ __global__ void __launch_bounds__(256) recover_gemm_kernel(const SplitJob* jobs,
     int m, n, k, kind;
     if (stage == kRecoverBW) {
         m = ell; n = chi; k = cols; kind = 0;
+        if (S.pre_rsvd) { m = chi; n = cols; k = ell; kind = 4; }
     } else if (stage == kRecoverQT) {
-        m = rows; n = chi; k = ell; kind = 1;
+        m = rows; n = chi; k = ell; kind = S.pre_rsvd ? 5 : 1;
     } else if (!S.w_rows_of_src) {
         m = chi; n = cols; k = rows; kind = 2;
     } else {
@@ -1120,6 +1143,8 @@ __global__ void __launch_bounds__(256) recover_gemm_kernel(const SplitJob* jobs,
             case 0: return B.b[size_t(i) * cols + kk];                          // B[j][c]
             case 1: return B.q[size_t(kk) * rows + i];                          // Q[r][t]
             case 2: return cconj(B.w[size_t(B.perm[i]) * rows + kk]);          // conj W[r][pc(m)]
+            case 4: return cconj(B.w[size_t(B.perm[i]) * ell + kk]);           // conj W[t][pc(m)]
+            case 5: return B.q[size_t(kk) * rows + i];                          // Q[r][t]
             default: return B.theta[size_t(i) * cols + kk];                     // theta[r][c]
         }
     };
@@ -1128,6 +1153,8 @@ __global__ void __launch_bounds__(256) recover_gemm_kernel(const SplitJob* jobs,
             case 0: return B.w[size_t(B.perm[nn]) * cols + kk];                 // W[c][pc(m)]
             case 1: return B.z[size_t(B.perm[nn]) * ell + kk];                  // T[t][pc(m)]
             case 2: return B.theta[size_t(kk) * cols + nn];                     // theta[r][c]
+            case 4: return B.b[size_t(kk) * cols + nn];                         // B[t][c]
+            case 5: return B.w[size_t(B.perm[nn]) * ell + kk];                  // W[t][pc(m)]
             default: return B.w[size_t(B.perm[nn]) * cols + kk];                // W[c][pc(m)]
         }
     };
@@ -1161,6 +1188,10 @@ __global__ void __launch_bounds__(256) recover_gemm_kernel(const SplitJob* jobs,
         const double sg = B.sigma[B.perm[mm]];
         return sg > 0.0 ? 1.0 / (sg * sqrt(sg)) : 0.0;
     };
+    auto inv_s12 = [&](int mm) {
+        const double sg = B.sigma[B.perm[mm]];
+        return sg > 0.0 ? 1.0 / sqrt(sg) : 0.0;
+    };
     for (int x = 0; x < 2; ++x)
         for (int y = 0; y < 2; ++y) {
             const int i = i0 + tr + 16 * x, nn = n0 + tc + 16 * y;
@@ -1169,15 +1200,17 @@ __global__ void __launch_bounds__(256) recover_gemm_kernel(const SplitJob* jobs,
             switch (kind) {
                 case 0: B.z[size_t(B.perm[nn]) * ell + i] = v; break;
                 case 1: mps.site[J.p][size_t(i) * chi + nn] = cscale(v, inv_s32(nn)); break;
-                case 2: mps.site[J.p + 1][size_t(i) * cols + nn] = cscale(v, inv_s32(i)); break;
+                case 2:
+                case 4: mps.site[J.p + 1][size_t(i) * cols + nn] = cscale(v, inv_s32(i)); break;
+                case 5: mps.site[J.p][size_t(i) * chi + nn] = cscale(v, inv_s12(nn)); break;
                 default: mps.site[J.p][size_t(i) * chi + nn] = cscale(v, inv_s32(nn)); break;
             }
         }
 }
 
 // ---------------------------------------------------------------------------
-// absorb: the sides that are plain copies of W (L = W / sqrt(s) for theta,
-// R = W^H / sqrt(s) for theta^H and B^H), and the new bond dims
+// absorb: the sides that are plain copies of W (L = W / sqrt(s) where W holds
+// left vectors, R = W^H / sqrt(s) where it holds right ones), and the new bond dims
 // (mps.rs:1156-1168, 1039-1051).  The other side comes from
 // recover_gemm_kernel.
 // ---------------------------------------------------------------------------
@@ -1191,7 +1224,9 @@ __global__ void __launch_bounds__(256) absorb_kernel(const SplitJob* jobs, const
     const int chi = S.chi, rows = S.rows, cols = S.cols;
     const long stride = long(gridDim.x) * blockDim.x;
     const long t0 = long(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (S.final_kind == 0 && !S.w_rows_of_src) {
+    if (S.final_kind == 1 && S.pre_rsvd) {
+        // Both sides come from recover_gemm_kernel.
+    } else if (S.final_kind == 0 && !S.w_rows_of_src) {
         // L = W / sqrt(s), W rows x cols; R comes from recover_gemm_kernel.
         double2* Ls = mps.site[J.p];
         for (long e = t0; e < long(rows) * chi; e += stride) {

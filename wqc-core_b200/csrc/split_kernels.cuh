@@ -26,6 +26,19 @@ constexpr int jacobi_ring_warps(int kr, int elem) {
     const int regs = 2 * kr * elem / 4 + 62;
     return regs <= 80 ? 24 : regs <= 128 ? 16 : 12;
 }
+// QR before the Jacobi (jacobi_qr.cu): instances by row groups, columns a CTA
+// holds at a time, and the tasks it takes -- from 16 columns (one SVD of 8 columns took 43 us
+// without and 56 with it, of 16 columns 125 and 101, of 32 385 and 220) to the
+// rows an instance holds.
+constexpr int kJacobiQrMin = 16, kJacobiQrMax = 512, kJacobiQrPerCta = 16;
+constexpr int jacobi_qr_kr(int M) {
+    const int need = (M + 31) / 32;
+    return need <= 2 ? (need < 1 ? 1 : need) : need <= 4 ? 4 : need <= 6 ? 6 : need <= 8 ? 8 : need <= 12 ? 12 : 16;
+}
+inline bool jacobi_qr_takes(int M, int N) { return N >= kJacobiQrMin && M <= kJacobiQrMax; }
+cudaError_t jacobi_qr_attributes();  // of every instance, once per process
+cudaError_t launch_jacobi_qr(int kr, int C, int tasks, cudaStream_t stream, const SplitJob* jobs, SplitState* st,
+                             const SlotBuffers* slots, const int* idx, int mode, int* status);
 constexpr int kJacobiRingMaxCluster = 16;
 // Entry of a launch's task list: the job in the wave and log2 of the number
 // of CTAs it runs on.
@@ -105,6 +118,7 @@ inline int jacobi_staged_b(int M, int N, size_t elem, size_t smem_limit, size_t*
 // Elements (double2) of the `gs` workspace for two-site matrices up to R x R.
 inline size_t jacobi_staged_elems(int R) { return size_t(R + 32) * size_t(R); }
 // Probe-vector factorisation check of every active Jacobi task (grid: jobs x 2).
+constexpr int kProbeThreads = 1024;
 __global__ void svd_probe_kernel(const SplitJob* jobs, const SplitState* st, const SlotBuffers* slots, int mode,
                                  int fp32, int* status);
 // noise_rel: singular values below noise_rel * (largest) count as zero (0 in
