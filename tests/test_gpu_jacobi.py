@@ -109,3 +109,33 @@ def test_tasks_of_unlike_shapes_in_one_wave(cuda_ctx):
         assert np.linalg.norm(a - b) <= 12 * 180 * np.finfo(float).eps * np.linalg.norm(a)
         alone.close()
     together.close()
+
+
+@pytest.mark.parametrize("dl,k,dr", [(8, 16, 4), (16, 32, 16), (32, 50, 30), (64, 128, 64)])
+@pytest.mark.parametrize("multiplicity", [2, 5])
+def test_clusters_of_equal_singular_values(cuda_ctx, dl, k, dr, multiplicity):
+    """Any small inner product turns a pair of equal columns by a large angle,
+    so the iteration may not stop on the size of the inner products alone."""
+    rng = np.random.default_rng(k + multiplicity)
+    k = min(k, 2 * dl, 2 * dr)
+    s = np.repeat(np.exp(-np.arange(-(-k // multiplicity)) / 3.0), multiplicity)[:k]
+    u = np.linalg.qr(cplx(rng, 2 * dl, k))[0]
+    v = np.linalg.qr(cplx(rng, 2 * dr, k))[0]
+    theta = (u * s) @ v.conj().T
+    m = W.CudaMps(4, 256, ctx=cuda_ctx)  # launch shapes of the upper bounds, far above the bonds
+    m.set_split_rule(W.SPLIT_RULE_EXACT)
+    for q, shape in enumerate([(1, 2, 100), (100, 2, 256), (256, 2, 100), (100, 2, 1)]):
+        m.set_site(q, cplx(rng, *shape))
+    sites = [cplx(rng, 1, 2, dl), (u * np.sqrt(s)).reshape(dl, 2, k), (np.sqrt(s)[:, None] * v.conj().T).reshape(k, 2, dr),
+             cplx(rng, dr, 2, 1)]
+    for q, t in enumerate(sites):
+        m.set_site(q, t)
+    m.apply_two_qubit_at_positions(1, 2, np.eye(4), True)
+    kept = int(m.bond_dims()[1])
+    assert kept == int((s > 1e-12).sum())
+    left, right = m.site(1).reshape(2 * dl, kept), m.site(2).reshape(kept, 2 * dr)
+    assert np.linalg.norm(left @ right - theta) <= 6 * 2 * max(dl, dr) * np.finfo(float).eps * np.linalg.norm(theta)
+    # Both sides are U sqrt(S) and sqrt(S) V^H: their Gram matrices are S.
+    for gram in (left.conj().T @ left, right @ right.conj().T):
+        assert np.linalg.norm(gram - np.diag(np.diag(gram))) <= 6 * 2 * max(dl, dr) * np.finfo(float).eps * s[0] / s[kept - 1]
+    m.close()

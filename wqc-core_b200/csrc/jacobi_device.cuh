@@ -9,7 +9,7 @@ namespace wqc {
 
 struct JacobiCtl {
     int rot;                         // rotations of this sweep
-    int coarse;                      // a pair entered this sweep less orthogonal than the stop bound
+    int ecos, esin;                  // binary exponents of this sweep's largest cos^2 and sin^2 (JacobiSweep)
     unsigned long long relmax_bits;  // last allowed sweep: largest squared |gamma|^2 / (alpha beta) (double bits)
     double fro_part;
     double chk_in, chk_out;  // this CTA's share of ||X||_F^2 (after dust zeroing) and of sum sigma^2
@@ -26,11 +26,32 @@ constexpr double kSvdCheckTolFp32 = 1e-4;
 // Pairs count as orthogonal at |gamma| <= tol sqrt(alpha beta), just above
 // the rounding of an M <= 512 dot product (sqrt(M) eps: 5e-15 in FP64, 3e-6
 // in FP32), so the sweeps stop and the singular values are exact to second
-// order.  A sweep that every pair entered orthogonal to the stop bound (1e-8;
-// 2e-3) ends the iteration: one-sided Jacobi converges quadratically, so that
-// sweep leaves them at about its square, below tol.  All squared.
+// order.  Squared.
 constexpr double kJacobiTol2 = 1e-28, kJacobiTol2Fp32 = 1.6e-11;
-constexpr double kJacobiStop2 = 1e-16, kJacobiStop2Fp32 = 4e-6;
+
+// What a sweep learns from its pairs: rotations, and of the rotated pairs the
+// largest cos^2 = |gamma|^2 / (alpha beta) they entered with and the largest
+// sin^2 of a rotation, as binary exponents (integer compares off the
+// rotation's chain, in place of a division on it).  The ratio itself is taken
+// on the last allowed sweep, where the error message reports it.
+struct JacobiSweep {
+    int rot = 0;
+    int ecos = -8192, esin = -8192;
+    double relmax = 0.0;
+};
+
+// A sweep ends the iteration when it leaves every pair orthogonal: a pair it
+// made orthogonal is spoiled by later rotations of its columns, by at most
+// about (largest sin) x (largest cos of what is mixed in).  With separated
+// singular values sin is of cos's size and a cos below 1e-8 leaves 1e-16; but
+// in a cluster of equal ones any small gamma turns the pair by a large angle,
+// and the sweep would leave what it entered with (1e-9 was seen on the
+// doubly degenerate theta of Clifford-like circuits).  FP64: cos < 2^-26.5 and
+// sin cos < 2^-50.  The complex64 phase only prepares the FP64 one: cos < 2e-3.
+__device__ __forceinline__ bool jacobi_done(bool f64, int rot, int ecos, int esin) {
+    if (rot == 0) return true;
+    return f64 ? ecos < -53 && ecos + esin < -100 : ecos < -18;
+}
 
 // Singular values of an exact SVD at or below 18 eps ||X||_F are reported as
 // zero: rounding leaves such values where X has none, their W columns are not
@@ -119,21 +140,12 @@ __device__ __forceinline__ void warp_sum4(R& a, R& b, R& g, R& h, int lane) {
     h = __shfl_sync(0xffffffffu, v, 24);
 }
 
-// What a sweep learns from its pairs.  The convergence test needs only
-// whether some pair entered above the stop bound; the ratio itself (an FP64
-// division on every rotation's chain) is taken on the last allowed sweep,
-// where the error message reports it.
-struct JacobiSweep {
-    int rot = 0;
-    bool coarse = false;
-    double relmax = 0.0;
-};
-
 // A warp's findings into its CTA's control block.
 __device__ __forceinline__ void jacobi_report(JacobiCtl& ctl, const JacobiSweep& sw, int lane) {
     if (lane != 0) return;
     if (sw.rot) atomicAdd(&ctl.rot, sw.rot);
-    if (sw.coarse) atomicOr(&ctl.coarse, 1);
+    atomicMax(&ctl.ecos, sw.ecos);
+    atomicMax(&ctl.esin, sw.esin);
     if (sw.relmax > 0.0) atomicMax(&ctl.relmax_bits, (unsigned long long)__double_as_longlong(sw.relmax));
 }
 
@@ -146,13 +158,12 @@ __device__ __forceinline__ void jacobi_report(JacobiCtl& ctl, const JacobiSweep&
 // form is c^2 = (1 + |d| / r) / 2 and w = sign(d) gamma / (2 r c): two
 // dependent reciprocal square roots (85 cycles each on B200) and no
 // division, where the tangent form took three and its phase a fourth.
-__device__ __forceinline__ bool jacobi_params(double a, double bb, double gr, double gi, double tol2, double stop_rel2,
+__device__ __forceinline__ bool jacobi_params(double a, double bb, double gr, double gi, double tol2,
                                               double noise_floor, bool want_ratio, JacobiSweep& sw, double& c,
                                               double& wr, double& wi) {
     const double g2 = fma(gr, gr, gi * gi);
     const double ab = a * bb;
     if (fmin(a, bb) <= noise_floor) return false;  // the smaller column is at the storage's rounding level
-    sw.coarse |= g2 > stop_rel2 * ab;
     if (want_ratio) sw.relmax = fmax(sw.relmax, g2 / ab);
     if (g2 == 0.0 || g2 <= tol2 * ab) return false;
     const double d = 0.5 * (bb - a);
@@ -173,6 +184,9 @@ __device__ __forceinline__ bool jacobi_params(double a, double bb, double gr, do
         wi = (gi / r) * f;
     }
     ++sw.rot;
+    auto exponent = [](double x) { return __double2hiint(x) >> 20; };
+    sw.ecos = max(sw.ecos, exponent(g2) - exponent(ab));
+    sw.esin = max(sw.esin, exponent(fma(wr, wr, wi * wi)) - 1023);
     return true;
 }
 

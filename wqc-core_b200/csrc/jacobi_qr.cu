@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(NW * 32) jacobi_qr_kernel(const SplitJob* jobs
         else
             __syncthreads();
     };
+    sync();  // every CTA has started: its shared memory may be stored into
     // Squared column norms, on every CTA; the order of the columns.
     for (int col = rank * NW + wid; col < N; col += C * NW) {
         double s = 0;

@@ -17,8 +17,8 @@ namespace {
 // dot products: the rest hold the accumulated V of the precision form's first
 // phase and are rotated along.  Returns false when the pair is left alone.
 template <typename T, int KR, bool kV>
-__device__ __forceinline__ bool rotate_reg(T (&u)[KR], T (&v)[KR], int km, double tol2, double stop_rel2,
-                                           double noise_floor, bool want_ratio, int lane, JacobiSweep& sw) {
+__device__ __forceinline__ bool rotate_reg(T (&u)[KR], T (&v)[KR], int km, double tol2, double noise_floor,
+                                           bool want_ratio, int lane, JacobiSweep& sw) {
     using R = typename JacobiReal<T>::R;
     R a0 = 0, b0 = 0, gr0 = 0, gi0 = 0, a1 = 0, b1 = 0, gr1 = 0, gi1 = 0;
 #pragma unroll
@@ -41,7 +41,7 @@ __device__ __forceinline__ bool rotate_reg(T (&u)[KR], T (&v)[KR], int km, doubl
     gi0 += gi1;
     warp_sum4(a0, b0, gr0, gi0, lane);
     double c64, wr64, wi64;
-    if (!jacobi_params(a0, b0, gr0, gi0, tol2, stop_rel2, noise_floor, want_ratio, sw, c64, wr64, wi64)) return false;
+    if (!jacobi_params(a0, b0, gr0, gi0, tol2, noise_floor, want_ratio, sw, c64, wr64, wi64)) return false;
     const R wr = R(wr64), wi = R(wi64), c = R(c64);
 #pragma unroll
     for (int k = 0; k < KR; ++k) {
@@ -174,7 +174,6 @@ __global__ void __launch_bounds__(jacobi_ring_warps(KR, sizeof(T)) * 32) jacobi_
         }
     }
     const double tol2 = kF64 ? kJacobiTol2 : kJacobiTol2Fp32;
-    const double stop_rel2 = kF64 ? kJacobiStop2 : kJacobiStop2Fp32;
     const double noise_floor = (kF64 ? 1e-30 : 1e-12) * fro2;  // squared column norm: 1e-15 (1e-6) of ||W||_F
     const bool mine = wid < b;
     T u[KR], v[KR];
@@ -195,7 +194,7 @@ __global__ void __launch_bounds__(jacobi_ring_warps(KR, sizeof(T)) * 32) jacobi_
     for (; sweep < max_sweeps; ++sweep) {
         if (tid == 0) {
             ctl.rot = 0;
-            ctl.coarse = 0;
+            ctl.ecos = ctl.esin = -8192;
             ctl.relmax_bits = 0ull;
         }
         JacobiSweep my;
@@ -216,7 +215,7 @@ __global__ void __launch_bounds__(jacobi_ring_warps(KR, sizeof(T)) * 32) jacobi_
                     T* q = column(pq < be / 2 ? 1 : 0, e2);
                     load(u, p);
                     load(v, q);
-                    if (rotate_reg<T, KR, kV>(u, v, km, tol2, stop_rel2, noise_floor, want_ratio, lane, my)) {
+                    if (rotate_reg<T, KR, kV>(u, v, km, tol2, noise_floor, want_ratio, lane, my)) {
                         store(p, u);
                         store(q, v);
                     }
@@ -241,7 +240,7 @@ __global__ void __launch_bounds__(jacobi_ring_warps(KR, sizeof(T)) * 32) jacobi_
                     bool rotated = false;
                     if (mine) {
                         load(v, q);
-                        rotated = rotate_reg<T, KR, kV>(u, v, km, tol2, stop_rel2, noise_floor, want_ratio, lane, my);
+                        rotated = rotate_reg<T, KR, kV>(u, v, km, tol2, noise_floor, want_ratio, lane, my);
                     }
                     if (k < b - 1) {
                         if (rotated) store(q, v);
@@ -288,22 +287,22 @@ __global__ void __launch_bounds__(jacobi_ring_warps(KR, sizeof(T)) * 32) jacobi_
                 }
             }
         }
-        // Cluster-wide findings decide convergence: nothing rotated, or every
-        // pair entered this sweep orthogonal to the stop bound.
+        // Cluster-wide findings decide convergence.
         jacobi_report(ctl, my, lane);
-        int total = 0, coarse = 0;
+        int total = 0, ecos = -8192, esin = -8192;
         unsigned long long relmax_bits = 0;
         cluster.sync();
         for (int r = 0; r < C; ++r) {
             const JacobiCtl* rc = cluster.map_shared_rank(&ctl, r);
             total += rc->rot;
-            coarse |= rc->coarse;
+            ecos = max(ecos, rc->ecos);
+            esin = max(esin, rc->esin);
             relmax_bits = max(relmax_bits, rc->relmax_bits);
         }
         cluster.sync();
         last_rot = total;
         last_relmax_bits = relmax_bits;
-        if (total == 0 || !coarse) {
+        if (jacobi_done(kF64, total, ecos, esin)) {
             converged = true;
             break;
         }

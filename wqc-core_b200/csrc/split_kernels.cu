@@ -527,8 +527,7 @@ __global__ void __launch_bounds__(kQrClusterThreads, 1) qr_cluster_kernel(const 
 
 template <typename T>
 __device__ __forceinline__ void jacobi_rotate(T* __restrict__ xp, T* __restrict__ xq, int M, int len, double tol2,
-                                              double stop_rel2, double noise_floor, bool want_ratio, int lane,
-                                              JacobiSweep& sw) {
+                                              double noise_floor, bool want_ratio, int lane, JacobiSweep& sw) {
     using R = typename JacobiReal<T>::R;
     // Two rows per lane per iteration into two accumulator sets: the loads
     // of the second row overlap the first's FMAs and the dependent chains
@@ -559,7 +558,7 @@ __device__ __forceinline__ void jacobi_rotate(T* __restrict__ xp, T* __restrict_
     gi_ += gi1;
     warp_sum4(a_, b_, gr_, gi_, lane);
     double c64, wr64, wi64;
-    if (!jacobi_params(a_, b_, gr_, gi_, tol2, stop_rel2, noise_floor, want_ratio, sw, c64, wr64, wi64)) return;
+    if (!jacobi_params(a_, b_, gr_, gi_, tol2, noise_floor, want_ratio, sw, c64, wr64, wi64)) return;
     const R wr = R(wr64), wi = R(wi64), cr = R(c64);
     auto rot = [&](const T u, const T v, T& p, T& q) {
         p.x = fma(cr, u.x, -fma(wr, v.x, wi * v.y));
@@ -683,7 +682,6 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
     __threadfence();
     cluster.sync();
     const double tol2 = kF64 ? kJacobiTol2 : kJacobiTol2Fp32;
-    const double stop_rel2 = kF64 ? kJacobiStop2 : kJacobiStop2Fp32;
     const double noise_floor = (kF64 ? 1e-30 : 1e-12) * fro2;  // squared column norm: 1e-15 (1e-6) of ||W||_F
     int sweep = 0;
     bool converged = false;
@@ -692,7 +690,7 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
     for (; sweep < max_sweeps; ++sweep) {
         if (tid == 0) {
             ctl.rot = 0;
-            ctl.coarse = 0;
+            ctl.ecos = ctl.esin = -8192;
             ctl.relmax_bits = 0ull;
         }
         __syncthreads();
@@ -721,7 +719,7 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
                             const int e1 = circle_at(i, s2, bb), e2 = circle_at(bb - 1 - i, s2, bb);
                             if (e1 < b && e2 < b)
                                 jacobi_rotate(base + size_t(e1) * len, base + size_t(e2) * len, M, len, tol2,
-                                              stop_rel2, noise_floor, want_ratio, lane, my);
+                                              noise_floor, want_ratio, lane, my);
                         }
                         __syncthreads();
                     }
@@ -729,7 +727,7 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
                 for (int k = 0; k < b; ++k) {
                     for (int i = wid; i < b; i += nwarps) {
                         const int e2 = (i + k) % b;
-                        jacobi_rotate(sA + size_t(i) * len, sB + size_t(e2) * len, M, len, tol2, stop_rel2,
+                        jacobi_rotate(sA + size_t(i) * len, sB + size_t(e2) * len, M, len, tol2,
                                       noise_floor, want_ratio, lane, my);
                     }
                     __syncthreads();
@@ -747,19 +745,20 @@ __global__ void __launch_bounds__(kJacobiStagedThreads) jacobi_staged_kernel(con
         }
         jacobi_report(ctl, my, lane);
         __syncthreads();
-        int total = 0, coarse = 0;
+        int total = 0, ecos = -8192, esin = -8192;
         unsigned long long relmax_bits = 0;
         cluster.sync();
         for (int r = 0; r < C; ++r) {
             const JacobiCtl* rc = cluster.map_shared_rank(&ctl, r);
             total += rc->rot;
-            coarse |= rc->coarse;
+            ecos = max(ecos, rc->ecos);
+            esin = max(esin, rc->esin);
             relmax_bits = max(relmax_bits, rc->relmax_bits);
         }
         cluster.sync();
         ctl_rot_last = total;
         ctl_relmax_bits_last = relmax_bits;
-        if (total == 0 || !coarse) {
+        if (jacobi_done(kF64, total, ecos, esin)) {
             converged = true;
             break;
         }
