@@ -1,0 +1,94 @@
+"""Pauli expectations from shared environments against the terms' dense
+contraction, around the tile edges and on both sides of the rule that sends
+small bonds to the walk over all sites; batches; shot marginals.
+
+Bound: an expectation of a unit state is a chain of products of backward
+stable factors of norm at most 1, 2 n contractions of up to 2 chi terms, so
+its error is below 4 n chi eps; half a dozen such factors are allowed."""
+import numpy as np
+import pytest
+
+import wqc_cuda as W
+from wqc_cuda import circuits as C
+
+pytestmark = pytest.mark.gpu
+
+PAULI = {"I": np.eye(2), "X": np.array([[0, 1], [1, 0]]), "Y": np.array([[0, -1j], [1j, 0]]), "Z": np.diag([1, -1])}
+
+
+def sites(n, chi, seed):
+    rng = np.random.default_rng(seed)
+    b = [min(2 ** min(i, n - i, 20), chi) for i in range(n + 1)]
+    out = []
+    for q in range(n):
+        a = rng.standard_normal((2 * b[q + 1], b[q])) + 1j * rng.standard_normal((2 * b[q + 1], b[q]))
+        out.append(np.linalg.qr(a)[0].conj().T.reshape(b[q], 2, b[q + 1]))
+    return out
+
+
+def value(tensors, label):
+    n = len(tensors)
+    env = np.ones((1, 1), dtype=complex)
+    for q, t in enumerate(tensors):
+        op = np.einsum("st,atb->asb", PAULI[label[n - 1 - q]], t)
+        env = np.tensordot(np.tensordot(env, op, (0, 0)), t.conj(), ((0, 1), (0, 1)))
+    return env[0, 0].real
+
+
+def labels_of(n, seed):
+    rng = np.random.default_rng(seed)
+    out = ["I" * n, "X" * n, "Z" + "I" * (n - 1), "I" * (n - 1) + "Y"]
+    for _ in range(6):
+        lo = int(rng.integers(0, n))
+        hi = int(rng.integers(lo, n)) + 1
+        out.append("I" * lo + "".join(rng.choice(list("IXYZ"), hi - lo)) + "I" * (n - hi))
+    return out
+
+
+@pytest.mark.parametrize("n,chi", [(1, 1), (2, 2), (6, 3), (9, 15), (9, 16), (10, 17), (11, 24), (11, 25), (12, 33),
+                                   (13, 48), (14, 64), (15, 127), (18, 200)])
+def test_expectation_matches_dense_contraction(cuda_ctx, n, chi):
+    tensors = sites(n, chi, 7 * n + chi)
+    m = W.CudaMps(n, chi, ctx=cuda_ctx)
+    for q, t in enumerate(tensors):
+        m.set_site(q, t)
+    labels = labels_of(n, n)
+    tol = 24 * n * chi * np.finfo(float).eps
+    for lab in labels:
+        assert abs(m.expectation([lab], [1.0]) - value(tensors, lab)) <= tol
+    coeffs = np.arange(1, len(labels) + 1) * (0.5 + 0.25j)
+    want = sum(c * value(tensors, lab) for c, lab in zip(coeffs, labels))
+    assert abs(m.expectation(labels, coeffs) - want) <= tol * np.abs(coeffs).sum()
+    m.close()
+
+
+@pytest.mark.parametrize("n,chis", [(6, [2, 3, 8]), (12, [40, 33, 7])])
+def test_batch_expectation_matches_single_states(cuda_ctx, n, chis):
+    gates = [C.gates_array(C.ry_rz_brickwork(n, 9, s)) for s in range(len(chis))]
+    labels, coeffs = labels_of(n, 3), np.linspace(0.1, 1.0, 10)
+    b = W.CudaBatch([n] * len(chis), chis, ctx=cuda_ctx)
+    b.apply_slices(gates)
+    got = b.expectations(labels, coeffs)
+    for s, chi in enumerate(chis):
+        m = W.run(n, chi, gates[s], ctx=cuda_ctx)
+        tensors = [m.site(q) for q in range(n)]
+        want = sum(c * value(tensors, lab) for c, lab in zip(coeffs, labels))
+        # The slices' own splits differ from a single state's by rounding, 1e-10 at most.
+        assert abs(got[s] - want) <= 1e-10 * np.abs(coeffs).sum()
+        m.close()
+    b.close()
+
+
+@pytest.mark.parametrize("n,chi", [(5, 4), (10, 17), (12, 40)])
+def test_first_qubit_of_the_shots_follows_its_marginal(cuda_ctx, n, chi):
+    tensors = sites(n, chi, n)
+    m = W.CudaMps(n, chi, ctx=cuda_ctx)
+    for q, t in enumerate(tensors):
+        m.set_site(q, t)
+    shots = 20000
+    draws = m.sample(range(n), shots, 11)
+    for q in (0, n // 2, n - 1):
+        p1 = 0.5 * (1.0 - value(tensors, "I" * (n - 1 - q) + "Z" + "I" * q))
+        ones = int(((draws >> np.uint64(q)) & np.uint64(1)).sum())
+        assert abs(ones - shots * p1) <= 6 * np.sqrt(shots * max(p1 * (1 - p1), 1e-3))
+    m.close()

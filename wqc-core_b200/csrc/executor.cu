@@ -270,6 +270,7 @@ struct wqc_mps {
     size_t h_stage_cap = 0;
     cudaEvent_t stage_done = nullptr;
     Arena d_stage;
+    Arena scratch;  // of the reads (environments, dense state), grown as they need it
     wqc_split_info* d_records = nullptr;
     size_t rec_cap = 0;
     uint32_t rec_count = 0;
@@ -364,6 +365,32 @@ void dfree(wqc_mps* m, void* p, size_t bytes) {
     if (!p) return;
     cudaFree(p);
     m->bytes_now -= bytes;
+}
+
+// Device memory for one read, kept with the state for the next one (a
+// cudaMalloc and cudaFree a call cost more than most reads).  The reads of a
+// state follow one another on its stream, and each ends with a
+// synchronisation, so there is one arena.
+constexpr size_t kScratchKeep = size_t(512) << 20;  // larger arenas are given back after the call
+wqc_status get_scratch(wqc_mps* m, size_t bytes, void** p) {
+    if (bytes > m->scratch.cap) {
+        if (m->scratch.d) {
+            CUDA_TRY(cudaStreamSynchronize(m->stream));
+            dfree(m, m->scratch.d, m->scratch.cap);
+        }
+        m->scratch.d = nullptr;
+        m->scratch.cap = 0;
+        if (wqc_status s = dmalloc(m, &m->scratch.d, bytes)) return s;
+        m->scratch.cap = bytes;
+    }
+    *p = m->scratch.d;
+    return WQC_OK;
+}
+void trim_scratch(wqc_mps* m) {
+    if (m->scratch.cap <= kScratchKeep) return;
+    dfree(m, m->scratch.d, m->scratch.cap);
+    m->scratch.d = nullptr;
+    m->scratch.cap = 0;
 }
 
 std::once_flag g_attr_once;
@@ -1248,6 +1275,105 @@ wqc_status sync_status(wqc_mps* m) {
     return WQC_OK;
 }
 
+// <psi|P_t|psi> of every term on every segment of `width` sites, vals[seg *
+// nterms + t]; ends with the state's synchronisation.  Terms are cut to the
+// sites between their first and last non-identity ones and share the identity
+// environments on both sides, so a local observable costs one chain and a few
+// products a term: 99 local terms on 50 sites took 141 ms as walks over all
+// sites and 2.0 ms so at bond 128, 1.8 and 0.59 at 32, 1.28 and 0.59 at 24.  At
+// small bonds, where a site's products are shorter than a launch, one launch
+// walks every term over all sites: bond 16, 20 sites 0.12 ms against 0.27; and
+// bond 24 where the terms span the register (20 such terms on 20 sites 0.22 ms
+// against 0.48, at bond 32 0.98 against 0.50).
+constexpr int kPauliWalkBond = 16, kPauliWalkBondLong = 24;
+wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, const char* labels, uint32_t nterms,
+                        std::vector<double2>& vals) {
+    const int nseg = int(firsts.size());
+    vals.resize(size_t(nseg) * nterms);
+    const size_t E = size_t(m->chi) * m->chi;
+    int bond = 1;
+    for (int b : m->ub) bond = std::max(bond, b);
+    auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
+    const size_t lab_b = al(size_t(nterms) * width + 16), int_b = al(size_t(nterms) * sizeof(int));
+    const size_t out_b = al(size_t(nseg) * nterms * sizeof(double2)), first_b = al(nseg * sizeof(int));
+    std::vector<int> start(nterms), span(nterms);
+    int longest_all = 1;
+    for (uint32_t t = 0; t < nterms; ++t) {
+        int lo = width, hi = -1;
+        for (int q = 0; q < width; ++q)
+            if (labels[size_t(t) * width + (width - 1 - q)] != 'I') {
+                lo = std::min(lo, q);
+                hi = q;
+            }
+        start[t] = hi < 0 ? 0 : lo;
+        span[t] = hi < 0 ? 1 : hi - lo + 1;
+        longest_all = std::max(longest_all, span[t]);
+    }
+    const bool walk = bond <= kPauliWalkBond || (bond <= kPauliWalkBondLong && 2 * longest_all > width);
+    // Segments and terms at a time, within the memory a state keeps.
+    const size_t seg_b = (size_t(3) * width + 4) * E * sizeof(double2);
+    const int segs = walk ? 1 : int(std::max<size_t>(1, std::min<size_t>(size_t(std::min(nseg, 16384)), (kScratchKeep / 2) / seg_b)));
+    const size_t term_b = 4 * E * sizeof(double2);
+    const uint32_t terms = walk ? nterms
+                                : uint32_t(std::max<size_t>(1, std::min<size_t>(std::min<size_t>(nterms, 65535 / segs),
+                                                                                (kScratchKeep / 4) / (term_b * segs))));
+    void* base = nullptr;
+    const size_t work_b = al(walk ? size_t(nterms) * term_b : size_t(segs) * (seg_b + size_t(terms) * term_b));
+    if (wqc_status s = get_scratch(m, work_b + lab_b + 2 * int_b + out_b + first_b, &base)) return s;
+    char* p = static_cast<char*>(base);
+    double2* work = reinterpret_cast<double2*>(p);
+    char* d_lab = p + work_b;
+    int* d_start = reinterpret_cast<int*>(d_lab + lab_b);
+    int* d_span = reinterpret_cast<int*>(reinterpret_cast<char*>(d_start) + int_b);
+    double2* d_out = reinterpret_cast<double2*>(reinterpret_cast<char*>(d_span) + int_b);
+    int* d_first = reinterpret_cast<int*>(reinterpret_cast<char*>(d_out) + out_b);
+    CUDA_TRY(cudaMemcpyAsync(d_lab, labels, size_t(nterms) * width, cudaMemcpyHostToDevice, m->stream));
+    if (walk) {
+        // One launch per segment on a view of its sites; launches share the scratch in stream order.
+        for (int s = 0; s < nseg; ++s) {
+            DeviceMps view = m->dev;
+            view.site += firsts[s];
+            view.dl += firsts[s];
+            view.dr += firsts[s];
+            view.n = width;
+            pauli_expectation_kernel<<<nterms, 256, 0, m->stream>>>(view, d_lab, int(nterms), work, m->chi,
+                                                                    d_out + size_t(s) * nterms);
+            count_launch(m, -1);
+        }
+    } else {
+        CUDA_TRY(cudaMemcpyAsync(d_start, start.data(), nterms * sizeof(int), cudaMemcpyHostToDevice, m->stream));
+        CUDA_TRY(cudaMemcpyAsync(d_span, span.data(), nterms * sizeof(int), cudaMemcpyHostToDevice, m->stream));
+        CUDA_TRY(cudaMemcpyAsync(d_first, firsts.data(), nseg * sizeof(int), cudaMemcpyHostToDevice, m->stream));
+        for (int s0 = 0; s0 < nseg; s0 += segs) {
+            EnvChains ch{};
+            ch.base = work;
+            ch.seg_stride = (size_t(3) * width + 4) * E;
+            ch.t_off = 0;
+            ch.l_off = size_t(2) * width * E;
+            ch.r_off = ch.l_off + 2 * E;
+            ch.h_off = ch.r_off + size_t(width) * E;
+            ch.firsts = d_first + s0;
+            ch.nseg = std::min(segs, nseg - s0);
+            ch.width = width;
+            ch.cap = m->chi;
+            ch.left = true;
+            const EnvTerms tm{d_lab, d_start, d_span, work + size_t(segs) * ch.seg_stride};
+            m->stats.total_launches += launch_env_chains(m->dev, ch, true, bond, m->stream);
+            for (uint32_t t0 = 0; t0 < nterms; t0 += terms) {
+                const int count = int(std::min<uint32_t>(terms, nterms - t0));
+                const int longest = *std::max_element(span.begin() + t0, span.begin() + t0 + count);
+                m->stats.total_launches += launch_env_terms(m->dev, ch, tm, int(t0), count, int(nterms), longest, bond,
+                                                            d_out + size_t(s0) * nterms, m->stream);
+            }
+        }
+    }
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(cudaMemcpyAsync(vals.data(), d_out, vals.size() * sizeof(double2), cudaMemcpyDeviceToHost, m->stream));
+    const wqc_status rc = sync_status(m);
+    trim_scratch(m);
+    return rc;
+}
+
 }  // namespace
 
 // Lets entry points defined in other files of the library set the message
@@ -1612,6 +1738,7 @@ void wqc_mps_destroy(wqc_mps* m) {
     for (auto e : m->wave_done) cudaEventDestroy(e);
     if (m->call_start) cudaEventDestroy(m->call_start);
     dfree(m, m->d_stage.d, 0);
+    dfree(m, m->scratch.d, 0);
     if (m->h_stage) cudaFreeHost(m->h_stage);
     if (m->h_cancel) cudaFreeHost(const_cast<int*>(m->h_cancel));
     for (auto& e : m->events) {
@@ -1713,48 +1840,9 @@ wqc_status wqc_batch_expectation_pauli(wqc_mps* m, const char* labels, const dou
         for (int s = 0; s < 2 * nseg; ++s) out[s] = 0;
         return WQC_OK;
     }
-    const size_t E = size_t(m->chi) * m->chi;
-    const size_t scratch = size_t(nterms) * 4 * E * sizeof(double2);
-    const size_t lab_bytes = size_t(nterms) * width + 16;
-    const size_t out_bytes = size_t(nterms) * nseg * sizeof(double2);
-    void* d_lab = nullptr;
-    void* d_scr = nullptr;
-    void* d_out = nullptr;
-    if (wqc_status s = dmalloc(m, &d_lab, lab_bytes)) return s;
-    if (wqc_status s = dmalloc(m, &d_scr, scratch)) {
-        dfree(m, d_lab, lab_bytes);
-        return s;
-    }
-    if (wqc_status s = dmalloc(m, &d_out, out_bytes)) {
-        dfree(m, d_lab, lab_bytes);
-        dfree(m, d_scr, scratch);
-        return s;
-    }
-    wqc_status rc = WQC_OK;
-    std::vector<double2> vals(size_t(nterms) * nseg);
-    cudaError_t e = cudaMemcpyAsync(d_lab, labels, size_t(nterms) * width, cudaMemcpyHostToDevice, m->stream);
-    // One launch per slice on a view of its sites; launches share the scratch
-    // in stream order.
-    for (int s = 0; s < nseg && e == cudaSuccess; ++s) {
-        DeviceMps view = m->dev;
-        const int first = m->seg_first[s];
-        view.site += first;
-        view.dl += first;
-        view.dr += first;
-        view.n = width;
-        pauli_expectation_kernel<<<nterms, 256, 0, m->stream>>>(view, static_cast<const char*>(d_lab), int(nterms),
-                                                                  static_cast<double2*>(d_scr), m->chi,
-                                                                  static_cast<double2*>(d_out) + size_t(s) * nterms);
-        count_launch(m, -1);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(vals.data(), d_out, out_bytes, cudaMemcpyDeviceToHost, m->stream);
-    if (e != cudaSuccess) rc = fail(WQC_ERR_CUDA, cudaGetErrorString(e));
-    if (rc == WQC_OK) rc = sync_status(m);
-    dfree(m, d_lab, lab_bytes);
-    dfree(m, d_scr, scratch);
-    dfree(m, d_out, out_bytes);
-    if (rc != WQC_OK) return rc;
+    std::vector<int> firsts(m->seg_first.begin(), m->seg_first.end());
+    std::vector<double2> vals;
+    if (wqc_status st = pauli_values(m, firsts, width, labels, nterms, vals)) return st;
     for (int s = 0; s < nseg; ++s) {
         double re = 0, im = 0;
         for (uint32_t t = 0; t < nterms; ++t) {  // coeff * Re<P> (expectation.rs:177-185), term order
@@ -2098,68 +2186,38 @@ wqc_status wqc_mps_sample(wqc_mps* m, const uint32_t* qubits, uint32_t count, ui
     if (wqc_status s = check_uploaded_chain(m)) return s;
     if (wqc_status s = sync_status(m)) return s;
     const int n = m->n;
-    std::vector<int> dl(n), dr(n);
-    CUDA_TRY(cudaMemcpy(dl.data(), m->d_dl, n * sizeof(int), cudaMemcpyDeviceToHost));
-    CUDA_TRY(cudaMemcpy(dr.data(), m->d_dr, n * sizeof(int), cudaMemcpyDeviceToHost));
-    // E_q (dl[q] x dl[q]) at env_off[q]; E_n = 1 at env_off[n].
-    std::vector<unsigned long long> env_off(n + 1);
-    unsigned long long total = 0;
-    for (int q = 0; q < n; ++q) {
-        env_off[q] = total;
-        total += (unsigned long long)dl[q] * dl[q];
-    }
-    env_off[n] = total;
-    total += 1;
-    const size_t env_bytes = total * sizeof(double2);
-    const size_t tmp_bytes = size_t(2) * m->chi * m->chi * sizeof(double2);
-    const size_t aux_bytes = (n + 1) * sizeof(unsigned long long) + n * sizeof(int) + 64;
+    const size_t E = size_t(m->chi) * m->chi;
+    const size_t env_bytes = (size_t(n) + 2) * E * sizeof(double2);  // R of every site, H
+    const size_t aux_bytes = ((n + 1) * sizeof(int) + 255) & ~size_t(255);
     const size_t out_bytes = size_t(shots) * sizeof(uint64_t);
-    void *d_env = nullptr, *d_tmp = nullptr, *d_aux = nullptr, *d_out = nullptr;
-    auto release = [&]() {
-        if (d_env) dfree(m, d_env, env_bytes);
-        if (d_tmp) dfree(m, d_tmp, tmp_bytes);
-        if (d_aux) dfree(m, d_aux, aux_bytes);
-        if (d_out) dfree(m, d_out, out_bytes);
-    };
-    for (auto& pr : {std::make_pair(&d_env, env_bytes), std::make_pair(&d_tmp, tmp_bytes),
-                     std::make_pair(&d_aux, aux_bytes), std::make_pair(&d_out, out_bytes)})
-        if (wqc_status st = dmalloc(m, pr.first, pr.second)) {
-            release();
-            return st;
-        }
-    double2* env = static_cast<double2*>(d_env);
-    double2* tmp = static_cast<double2*>(d_tmp);
-    unsigned long long* d_off = static_cast<unsigned long long*>(d_aux);
-    int* d_bitpos = reinterpret_cast<int*>(d_off + n + 1);
-    const double2 one = cmake(1.0, 0.0);
-    cudaError_t e = cudaMemcpyAsync(env + env_off[n], &one, sizeof(double2), cudaMemcpyHostToDevice, m->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_off, env_off.data(), (n + 1) * sizeof(unsigned long long), cudaMemcpyHostToDevice,
-                            m->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_bitpos, bitpos.data(), n * sizeof(int), cudaMemcpyHostToDevice, m->stream);
-    // Right environments, from the last site down to site 1 (E_0 is not drawn from).
-    for (int q = n - 1; q >= 1 && e == cudaSuccess; --q) {
-        const int l = dl[q], r = dr[q];
-        const int g1 = int(std::min<long>((2L * l * r + 255) / 256, 4L * m->ctx->sm_count));
-        const int g2 = int(std::min<long>((long(l) * l + 255) / 256, 4L * m->ctx->sm_count));
-        sample_env_half_kernel<<<g1, 256, 0, m->stream>>>(m->site_ptr[q], l, r, env + env_off[q + 1], tmp);
-        sample_env_kernel<<<g2, 256, 0, m->stream>>>(m->site_ptr[q], l, r, tmp, env + env_off[q]);
-        count_launch(m, -1);
-        count_launch(m, -1);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) {
-        const int grid = int(std::min<long>(long(shots), 8L * m->ctx->sm_count));
-        sample_shots_kernel<<<grid, 256, 3 * m->chi * sizeof(double2), m->stream>>>(
-            m->dev, env, d_off, d_bitpos, (unsigned long long)seed, int(shots), static_cast<unsigned long long*>(d_out));
-        count_launch(m, -1);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, m->stream);
+    void* base = nullptr;
+    if (wqc_status st = get_scratch(m, env_bytes + aux_bytes + out_bytes, &base)) return st;
+    double2* env = static_cast<double2*>(base);
+    int* d_bitpos = reinterpret_cast<int*>(static_cast<char*>(base) + env_bytes);
+    auto* d_out = reinterpret_cast<unsigned long long*>(static_cast<char*>(base) + env_bytes + aux_bytes);
+    bitpos.push_back(0);  // the chain's first site, after the bit positions
+    CUDA_TRY(cudaMemcpyAsync(d_bitpos, bitpos.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice, m->stream));
+    EnvChains ch{};
+    ch.base = env;
+    ch.r_off = 0;
+    ch.h_off = size_t(n) * E;
+    ch.firsts = d_bitpos + n;
+    ch.nseg = 1;
+    ch.width = n;
+    ch.cap = m->chi;
+    ch.left = false;
+    int bond = 1;
+    for (int b : m->ub) bond = std::max(bond, b);
+    m->stats.total_launches += launch_env_chains(m->dev, ch, true, bond, m->stream);
+    const int grid = int(std::min<long>(long(shots), 8L * m->ctx->sm_count));
+    sample_shots_kernel<<<grid, 256, 3 * m->chi * sizeof(double2), m->stream>>>(m->dev, env, d_bitpos,
+                                                                                (unsigned long long)seed, int(shots), d_out);
+    count_launch(m, -1);
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, m->stream));
     m->stats.d2h_bytes += out_bytes;
-    wqc_status rc = e == cudaSuccess ? sync_status(m) : fail(WQC_ERR_CUDA, cudaGetErrorString(e));
-    release();
+    const wqc_status rc = sync_status(m);
+    trim_scratch(m);
     return rc;
 }
 
@@ -2176,39 +2234,8 @@ wqc_status wqc_mps_expectation_pauli(wqc_mps* m, const char* labels, const doubl
         return WQC_OK;
     }
     if (wqc_status st = check_uploaded_chain(m)) return st;
-    const size_t E = size_t(m->chi) * m->chi;
-    const size_t scratch = size_t(nterms) * 4 * E * sizeof(double2);
-    void* d_lab = nullptr;
-    void* d_scr = nullptr;
-    void* d_out = nullptr;
-    if (wqc_status s = dmalloc(m, &d_lab, size_t(nterms) * m->n + 16)) return s;
-    if (wqc_status s = dmalloc(m, &d_scr, scratch)) {
-        dfree(m, d_lab, size_t(nterms) * m->n + 16);
-        return s;
-    }
-    if (wqc_status s = dmalloc(m, &d_out, nterms * sizeof(double2))) {
-        dfree(m, d_lab, size_t(nterms) * m->n + 16);
-        dfree(m, d_scr, scratch);
-        return s;
-    }
-    wqc_status rc = WQC_OK;
-    std::vector<double2> vals(nterms);
-    cudaError_t e = cudaMemcpyAsync(d_lab, labels, size_t(nterms) * m->n, cudaMemcpyHostToDevice, m->stream);
-    if (e == cudaSuccess) {
-        pauli_expectation_kernel<<<nterms, 256, 0, m->stream>>>(m->dev, static_cast<const char*>(d_lab), int(nterms),
-                                                                  static_cast<double2*>(d_scr), m->chi,
-                                                                  static_cast<double2*>(d_out));
-        count_launch(m, -1);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(vals.data(), d_out, nterms * sizeof(double2), cudaMemcpyDeviceToHost, m->stream);
-    if (e != cudaSuccess) rc = fail(WQC_ERR_CUDA, cudaGetErrorString(e));
-    if (rc == WQC_OK) rc = sync_status(m);
-    dfree(m, d_lab, size_t(nterms) * m->n + 16);
-    dfree(m, d_scr, scratch);
-    dfree(m, d_out, nterms * sizeof(double2));
-    if (rc != WQC_OK) return rc;
+    std::vector<double2> vals;
+    if (wqc_status st = pauli_values(m, {0}, m->n, labels, nterms, vals)) return st;
     double re = 0, im = 0;
     for (uint32_t t = 0; t < nterms; ++t) {  // coeff * Re<P> (expectation.rs:177-185)
         const double v = vals[t].x;

@@ -286,32 +286,6 @@ __global__ void __launch_bounds__(256) overlap_next_kernel(const double2* tmp, i
 // their marginal distribution.
 // ---------------------------------------------------------------------------
 
-// tmp[a][s][c'] = sum_c A[a][s][c] E[c][c'] for one site (l x 2 x r).
-__global__ void __launch_bounds__(256) sample_env_half_kernel(const double2* site, int l, int r,
-                                                              const double2* env_next, double2* tmp) {
-    const long total = 2L * l * r;
-    for (long e = long(blockIdx.x) * blockDim.x + threadIdx.x; e < total; e += long(gridDim.x) * blockDim.x) {
-        const int cp = int(e % r);
-        const double2* arow = site + (e / r) * r;
-        double2 acc = cmake(0, 0);
-        for (int c = 0; c < r; ++c) cfma(acc, arow[c], env_next[size_t(c) * r + cp]);
-        tmp[e] = acc;
-    }
-}
-
-// env[a][a'] = sum_{s, c'} tmp[a][s][c'] conj(A[a'][s][c'])  (l x l).
-__global__ void __launch_bounds__(256) sample_env_kernel(const double2* site, int l, int r, const double2* tmp,
-                                                         double2* env) {
-    const long total = long(l) * l;
-    for (long e = long(blockIdx.x) * blockDim.x + threadIdx.x; e < total; e += long(gridDim.x) * blockDim.x) {
-        const double2* t = tmp + (e / l) * 2 * r;
-        const double2* k = site + (e % l) * 2 * r;
-        double2 acc = cmake(0, 0);
-        for (int x = 0; x < 2 * r; ++x) cfma_conj(acc, k[x], t[x]);
-        env[e] = acc;
-    }
-}
-
 // SplitMix64 (Steele, Lea and Flood, OOPSLA 2014): the uniform draw of shot
 // `shot` at site q is the top 53 bits of mix(mix(seed ^ mix(shot)) + q).
 __device__ __forceinline__ unsigned long long splitmix64(unsigned long long z) {
@@ -326,11 +300,11 @@ __device__ __forceinline__ double sample_uniform(unsigned long long seed, unsign
     return double(splitmix64(key + (unsigned long long)q) >> 11) * 0x1.0p-53;
 }
 
-// One CTA per shot (grid-stride over shots).  envs + env_off[q] holds E_q
-// (dl[q] x dl[q]; E_n is 1 x 1); bitpos[q] is the output bit of qubit q, or
+// One CTA per shot (grid-stride over shots).  envs + q cap^2 holds E_{q+1}
+// (dr[q] x dr[q], the right environment of site q); bitpos[q] is the output bit of qubit q, or
 // -1 when q is not measured.  Dynamic shared memory: 3 * chi_max complex.
 __global__ void __launch_bounds__(256) sample_shots_kernel(DeviceMps mps, const double2* envs,
-                                                           const unsigned long long* env_off, const int* bitpos,
+                                                           const int* bitpos,
                                                            unsigned long long seed, int shots,
                                                            unsigned long long* out) {
     extern __shared__ __align__(16) double2 sv[];
@@ -346,7 +320,7 @@ __global__ void __launch_bounds__(256) sample_shots_kernel(DeviceMps mps, const 
         for (int q = 0; q < mps.n; ++q) {
             const int l = mps.dl[q], r = mps.dr[q];
             const double2* A = mps.site[q];
-            const double2* E = envs + env_off[q + 1];  // r x r
+            const double2* E = envs + size_t(q) * mps.chi_max * mps.chi_max;  // r x r
             for (int c = tid; c < r; c += blockDim.x) {
                 double2 a0 = cmake(0, 0), a1 = cmake(0, 0);
                 for (int a = 0; a < l; ++a) {

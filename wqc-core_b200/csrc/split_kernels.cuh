@@ -1,6 +1,7 @@
 // Kernel entry points of the two-site split pipeline and the site kernels.
 #pragma once
 
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -148,10 +149,31 @@ __global__ void pauli_expectation_kernel(DeviceMps mps, const char* labels, int 
                                          int env_cap, double2* out);
 __global__ void overlap_half_kernel(const double2* env, int kl, int bl, const double2* ket, int kr, double2* tmp);
 __global__ void overlap_next_kernel(const double2* tmp, int bl, int kr, const double2* bra, int br, double2* next);
-__global__ void sample_env_half_kernel(const double2* site, int l, int r, const double2* env_next, double2* tmp);
-__global__ void sample_env_kernel(const double2* site, int l, int r, const double2* tmp, double2* env);
-__global__ void sample_shots_kernel(DeviceMps mps, const double2* envs, const unsigned long long* env_off,
-                                    const int* bitpos, unsigned long long seed, int shots, unsigned long long* out);
+// Environments (env_kernels.cu).  The identity chains of `nseg` runs of
+// `width` sites (firsts[seg] ..), each with its buffers seg_stride entries
+// apart: T (2 cap^2 a site), L (two of cap^2), R (cap^2 a site; R_q contracts
+// the sites right of q) and H (2 cap^2).  `left` false: the right chain only.
+struct EnvChains {
+    double2* base;
+    size_t seg_stride, t_off, l_off, r_off, h_off;
+    const int* firsts;
+    int nseg, width, cap;
+    bool left;
+};
+// Pauli terms: labels (term t's character width-1-q acts on site q), the first
+// site that is not the identity and the number of sites from it to the last
+// such one; `work`: 4 cap^2 entries per segment and term of a launch.
+struct EnvTerms {
+    const char* labels;
+    const int* start;
+    const int* span;
+    double2* work;
+};
+// Both return the number of kernels launched; `bond` bounds every bond.
+int launch_env_chains(const DeviceMps& mps, const EnvChains& ch, bool right, int bond, cudaStream_t stream);
+int launch_env_terms(const DeviceMps& mps, const EnvChains& ch, const EnvTerms& tm, int t0, int count, int nterms,
+                     int longest, int bond, double2* out, cudaStream_t stream);
+__global__ void sample_shots_kernel(DeviceMps mps, const double2* envs, const int* bitpos, unsigned long long seed, int shots, unsigned long long* out);
 
 // Adjoint kernels (adjoint_kernels.cu).
 struct Adj1q {
