@@ -3,67 +3,11 @@
 // environments of shot sampling.
 #include "common.cuh"
 #include "split_kernels.cuh"
+#include "tile_gemm.cuh"
 
 namespace wqc {
 
 namespace {
-
-constexpr int kEnvTile = 16, kEnvK = 32, kEnvThreads = kEnvTile * kEnvTile;
-
-struct EnvSmem {
-    double2 a[kEnvK][kEnvTile + 1], b[kEnvK][kEnvTile + 1];
-};
-
-// One 16 x 16 tile of C = A B, one output per thread.  at_a(m, k) and
-// at_b(k, n) give zero outside the operands; `a_along_k` (`b_along_k`) says
-// which index runs fastest in memory, and the threads of a load follow it.
-// The next K block is fetched while this one is multiplied.  A K block is
-// bound by its FP64 work (128 DFMA a thread); one output per thread keeps a
-// chain's single 128 x 256 product on 128 CTAs.
-template <class FA, class FB, class FS>
-__device__ __forceinline__ void env_tile(EnvSmem& sm, int m0, int n0, int m, int n, int k, bool a_along_k, bool b_along_k, FA at_a,
-                                         FB at_b, FS store) {
-    constexpr int kLoads = kEnvK * kEnvTile / kEnvThreads;
-    const int tid = threadIdx.x, tm = tid / kEnvTile, tn = tid % kEnvTile;
-    double2 fa[kLoads], fb[kLoads];
-    auto place = [&](int e, bool along_k, int& i, int& kk) {
-        if (along_k) {
-            i = e / kEnvK;
-            kk = e % kEnvK;
-        } else {
-            i = e % kEnvTile;
-            kk = e / kEnvTile;
-        }
-    };
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int u = 0; u < kLoads; ++u) {
-            int i, kk;
-            place(tid + u * kEnvThreads, a_along_k, i, kk);
-            fa[u] = m0 + i < m && k0 + kk < k ? at_a(m0 + i, k0 + kk) : cmake(0, 0);
-            place(tid + u * kEnvThreads, b_along_k, i, kk);
-            fb[u] = n0 + i < n && k0 + kk < k ? at_b(k0 + kk, n0 + i) : cmake(0, 0);
-        }
-    };
-    double2 acc = cmake(0, 0);
-    fetch(0);
-    for (int k0 = 0; k0 < k; k0 += kEnvK) {
-#pragma unroll
-        for (int u = 0; u < kLoads; ++u) {
-            int i, kk;
-            place(tid + u * kEnvThreads, a_along_k, i, kk);
-            sm.a[kk][i] = fa[u];
-            place(tid + u * kEnvThreads, b_along_k, i, kk);
-            sm.b[kk][i] = fb[u];
-        }
-        __syncthreads();
-        if (k0 + kEnvK < k) fetch(k0 + kEnvK);
-#pragma unroll
-        for (int kk = 0; kk < kEnvK; ++kk) cfma(acc, sm.a[kk][tm], sm.b[kk][tn]);
-        __syncthreads();
-    }
-    if (m0 + tm < m && n0 + tn < n) store(m0 + tm, n0 + tn, acc);
-}
 
 // (P t)[so] for the row t = (t0, t1) over the physical index.
 __device__ __forceinline__ double2 pauli_row(char ch, int so, double2 t0, double2 t1) {
@@ -76,12 +20,12 @@ __device__ __forceinline__ double2 pauli_row(char ch, int so, double2 t0, double
 }
 
 // T[a'][s][b] = sum_a E[a][a'] A[a][s][b]; E is [1] at the left end.
-__device__ __forceinline__ void left_half(EnvSmem& sm, const DeviceMps& mps, int q, const double2* env, bool first, double2* T,
+__device__ __forceinline__ void left_half(TileSmem& sm, const DeviceMps& mps, int q, const double2* env, bool first, double2* T,
                                           int m0, int n0) {
     const int l = mps.dl[q], r = mps.dr[q];
     if (m0 >= l || n0 >= 2 * r) return;
     const double2* s = mps.site[q];
-    env_tile(
+    tile_gemm(
         sm, m0, n0, l, 2 * r, l, false, false,
         [&](int ap, int a) { return first ? cmake(1.0, 0.0) : env[size_t(a) * l + ap]; },
         [&](int a, int x) { return s[size_t(a) * 2 * r + x]; },
@@ -89,12 +33,12 @@ __device__ __forceinline__ void left_half(EnvSmem& sm, const DeviceMps& mps, int
 }
 
 // E'[b][b'] = sum_{a', s} (P T)[a'][s][b] conj(A[a'][s][b']).
-__device__ __forceinline__ void left_next(EnvSmem& sm, const DeviceMps& mps, int q, const double2* T, char ch, double2* out, int m0,
+__device__ __forceinline__ void left_next(TileSmem& sm, const DeviceMps& mps, int q, const double2* T, char ch, double2* out, int m0,
                                           int n0) {
     const int l = mps.dl[q], r = mps.dr[q];
     if (m0 >= r || n0 >= r) return;
     const double2* s = mps.site[q];
-    env_tile(
+    tile_gemm(
         sm, m0, n0, r, r, 2 * l, false, false,
         [&](int b, int x) {
             const double2* t = T + size_t(x >> 1) * 2 * r + b;
@@ -110,14 +54,14 @@ __device__ __forceinline__ void left_next(EnvSmem& sm, const DeviceMps& mps, int
 // below nseg takes the left chain at site `step` from the left, the rest the
 // right chain at the mirrored site.  phase 0 multiplies the environment into
 // the site, phase 1 closes it with the conjugate site.
-__global__ void __launch_bounds__(kEnvThreads) env_chain_kernel(DeviceMps mps, EnvChains ch, int step, int phase) {
-    __shared__ EnvSmem sm;
+__global__ void __launch_bounds__(kTileThreads) env_chain_kernel(DeviceMps mps, EnvChains ch, int step, int phase) {
+    __shared__ TileSmem sm;
     const int seg = blockIdx.z % ch.nseg;
     const bool right = int(blockIdx.z) / ch.nseg + (ch.left ? 0 : 1) == 1;
     const int first = ch.firsts[seg];
     const size_t E = size_t(ch.cap) * ch.cap;
     double2* base = ch.base + size_t(seg) * ch.seg_stride;
-    const int m0 = blockIdx.y * kEnvTile, n0 = blockIdx.x * kEnvTile;
+    const int m0 = blockIdx.y * kTile, n0 = blockIdx.x * kTile;
     if (!right) {
         const int q = first + step;
         double2* T = base + ch.t_off + size_t(step) * 2 * E;
@@ -137,14 +81,14 @@ __global__ void __launch_bounds__(kEnvThreads) env_chain_kernel(DeviceMps mps, E
     if (phase == 0) {
         if (step == 0 && m0 == 0 && n0 == 0 && threadIdx.x == 0) R[0] = cmake(1.0, 0.0);
         if (at == 0 || m0 >= 2 * l || n0 >= r) return;
-        env_tile(  // H[a, s][b'] = sum_b A[a, s][b] R[b][b']
+        tile_gemm(  // H[a, s][b'] = sum_b A[a, s][b] R[b][b']
             sm, m0, n0, 2 * l, r, r, true, false, [&](int x, int b) { return s[size_t(x) * r + b]; },
             [&](int b, int bp) { return step == 0 ? cmake(1.0, 0.0) : R[size_t(b) * r + bp]; },
             [&](int x, int bp, double2 v) { H[size_t(x) * r + bp] = v; });
     } else {
         if (at == 0 || m0 >= l || n0 >= l) return;
         double2* out = R - E;
-        env_tile(  // R[a][a'] = sum_{s, b'} H[a][s, b'] conj(A[a'][s, b'])
+        tile_gemm(  // R[a][a'] = sum_{s, b'} H[a][s, b'] conj(A[a'][s, b'])
             sm, m0, n0, l, l, 2 * r, true, true, [&](int a, int x) { return H[size_t(a) * 2 * r + x]; },
             [&](int x, int ap) { return cconj(s[size_t(ap) * 2 * r + x]); },
             [&](int a, int ap, double2 v) { out[size_t(a) * l + ap] = v; });
@@ -154,16 +98,16 @@ __global__ void __launch_bounds__(kEnvThreads) env_chain_kernel(DeviceMps mps, E
 // One half of step `step` of the terms t0 .. t0 + count - 1 of every segment:
 // a term starts from the left chain's T at its first non-identity site, so
 // its first step has no half of phase 0.
-__global__ void __launch_bounds__(kEnvThreads) env_term_kernel(DeviceMps mps, EnvChains ch, EnvTerms tm, int t0,
+__global__ void __launch_bounds__(kTileThreads) env_term_kernel(DeviceMps mps, EnvChains ch, EnvTerms tm, int t0,
                                                                int count, int step, int phase) {
-    __shared__ EnvSmem sm;
+    __shared__ TileSmem sm;
     const int local = blockIdx.z % count, seg = blockIdx.z / count, t = t0 + local;
     if (step >= tm.span[t]) return;
     const size_t E = size_t(ch.cap) * ch.cap;
     const double2* base = ch.base + size_t(seg) * ch.seg_stride;
     double2* mine = tm.work + (size_t(seg) * count + local) * 4 * E;  // two environments, then T
     const int at = tm.start[t] + step, q = ch.firsts[seg] + at;
-    const int m0 = blockIdx.y * kEnvTile, n0 = blockIdx.x * kEnvTile;
+    const int m0 = blockIdx.y * kTile, n0 = blockIdx.x * kTile;
     if (phase == 0) {
         left_half(sm, mps, q, mine + (step & 1) * E, false, mine + 2 * E, m0, n0);
     } else {
@@ -201,12 +145,12 @@ __global__ void __launch_bounds__(256) env_dot_kernel(DeviceMps mps, EnvChains c
 // one CTA per Pauli term (50 sites, chi 128, 99 terms: 142 ms).
 int launch_env_chains(const DeviceMps& mps, const EnvChains& ch, bool right, int bond, cudaStream_t stream) {
     const unsigned z = unsigned(ch.nseg) * ((ch.left ? 1 : 0) + (right ? 1 : 0));
-    const unsigned b1 = unsigned(bond + kEnvTile - 1) / kEnvTile, b2 = unsigned(2 * bond + kEnvTile - 1) / kEnvTile;
+    const unsigned b1 = unsigned(bond + kTile - 1) / kTile, b2 = unsigned(2 * bond + kTile - 1) / kTile;
     const unsigned both = ch.left && right ? b2 : 0;  // the chains' halves are b1 x b2 and b2 x b1 tiles
     for (int step = 0; step < ch.width; ++step) {
-        env_chain_kernel<<<dim3(std::max(ch.left ? b2 : b1, both), std::max(right ? b2 : b1, both), z), kEnvThreads, 0,
+        env_chain_kernel<<<dim3(std::max(ch.left ? b2 : b1, both), std::max(right ? b2 : b1, both), z), kTileThreads, 0,
                            stream>>>(mps, ch, step, 0);
-        env_chain_kernel<<<dim3(b1, b1, z), kEnvThreads, 0, stream>>>(mps, ch, step, 1);
+        env_chain_kernel<<<dim3(b1, b1, z), kTileThreads, 0, stream>>>(mps, ch, step, 1);
     }
     return 2 * ch.width;
 }
@@ -214,14 +158,14 @@ int launch_env_chains(const DeviceMps& mps, const EnvChains& ch, bool right, int
 int launch_env_terms(const DeviceMps& mps, const EnvChains& ch, const EnvTerms& tm, int t0, int count, int nterms,
                      int longest, int bond, double2* out, cudaStream_t stream) {
     const unsigned z = unsigned(ch.nseg) * unsigned(count);
-    const unsigned b1 = unsigned(bond + kEnvTile - 1) / kEnvTile, b2 = unsigned(2 * bond + kEnvTile - 1) / kEnvTile;
+    const unsigned b1 = unsigned(bond + kTile - 1) / kTile, b2 = unsigned(2 * bond + kTile - 1) / kTile;
     int launches = 1;
     for (int step = 0; step < longest; ++step) {
         if (step > 0) {
-            env_term_kernel<<<dim3(b2, b1, z), kEnvThreads, 0, stream>>>(mps, ch, tm, t0, count, step, 0);
+            env_term_kernel<<<dim3(b2, b1, z), kTileThreads, 0, stream>>>(mps, ch, tm, t0, count, step, 0);
             ++launches;
         }
-        env_term_kernel<<<dim3(b1, b1, z), kEnvThreads, 0, stream>>>(mps, ch, tm, t0, count, step, 1);
+        env_term_kernel<<<dim3(b1, b1, z), kTileThreads, 0, stream>>>(mps, ch, tm, t0, count, step, 1);
         ++launches;
     }
     env_dot_kernel<<<dim3(count, ch.nseg), 256, 0, stream>>>(mps, ch, tm, t0, count, nterms, out);

@@ -54,6 +54,7 @@ wqc_status fail_oom(uint64_t required, uint64_t available) {
     } while (0)
 
 constexpr int kMaxSweeps = 60;
+constexpr int kOzAutoBond = 192;  // default merges take int8 digit slices above this bond
 constexpr int kDenseMaxQubits = 28;  // 2^28 complex128 = 4 GiB on the host
 constexpr size_t kSlotBudget = size_t(1) << 30;  // split workspace per chi_max bucket
 constexpr size_t kSmemLimit = 232448 - 1024;  // 227 KB opt-in per block, minus static shared memory
@@ -232,6 +233,7 @@ struct wqc_mps {
     // WQC_MERGE_TC_INT8 (wqc_mps_set_merge): merges from int8 digit slices
     // on the tensor cores (tc_ozaki.cu), staged per wave job
     bool oz = false;
+    bool oz_auto = false;  // the default: by size, until wqc_mps_set_merge says which
     void* oz_pool = nullptr;
     size_t oz_bytes = 0;
     OzPlanes oz_planes;
@@ -1005,9 +1007,15 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
         const double noise_rel = m->tc ? 1e-6 : 0.0;
         {
             Timed t(m, 1);
-            prepare_kernel<<<(nj + 127) / 128, 128, 0, m->stream>>>(d_jobs, m->d_state, nj, m->dev);
-            count_launch(m, 1);
-            if (m->oz) {
+            // A state that was not told which merge to use takes the FMA tiles
+            // where they are faster (one merge at bond 32 15 us against 27, at
+            // 128 37 against 49, at 192 58 against 58, at 256 73 against 64).
+            const bool oz = m->oz && (!m->oz_auto || std::min(w.max_dl, w.max_dr) > kOzAutoBond);
+            if (oz || m->tc) {
+                prepare_kernel<<<(nj + 127) / 128, 128, 0, m->stream>>>(d_jobs, m->d_state, nj, m->dev);
+                count_launch(m, 1);
+            }
+            if (oz) {
                 // rows of L by warps, N tiles of R (8 values of b) by blocks
                 const int a_blocks = std::max(1, (w.max_rows + 7) / 8);
                 const int ntiles = (w.max_dr + 7) / 8;
@@ -1092,11 +1100,20 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
             for (const Group& gr : w.groups)
                 if (gr.mode == mode && gr.nph == 2)
                     if (wqc_status s = launch_phase(gr, gr.ph[1], mode, kPhaseFinish, false, on)) return s;
+            // The check only reads the SVD: beside the cut where the side
+            // stream is free; the next wave waits for it.
+            const bool aside = !w.any_rsvd;
+            if (aside) {
+                CUDA_TRY(cudaEventRecord(m->fork_ev, on));
+                CUDA_TRY(cudaStreamWaitEvent(m->side, m->fork_ev, 0));
+            }
+            cudaStream_t ps = aside ? m->side : on;
             {
-                Timed t(m, 4, on);
-                svd_probe_kernel<<<dim3(nj, 2), kProbeThreads, 0, on>>>(d_jobs, m->d_state, m->d_slots, mode, 0, m->d_status);
+                Timed t(m, 4, ps);
+                svd_probe_kernel<<<dim3(nj, 2), kProbeThreads, 0, ps>>>(d_jobs, m->d_state, m->d_slots, mode, 0, m->d_status);
                 count_launch(m, 4);
             }
+            if (aside) CUDA_TRY(cudaEventRecord(m->join_ev, m->side));
             return WQC_OK;
         };
         // Exact-path SVDs on the side stream, concurrently with the range
@@ -1108,6 +1125,19 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
             CUDA_TRY(cudaStreamWaitEvent(m->side, m->fork_ev, 0));
         }
         if (wqc_status s = jacobi(kJacobiExact, xs)) return s;
+        auto tiles = [](int x) { return (x + 15) / 16; };
+        if (!w.any_rsvd) {
+            Timed t(m, 4);
+            const int kmax = std::min(m->chi, std::min(w.max_rows, w.max_cols));
+            const int tn = tiles(std::max(w.max_cols, kmax)), tm = tiles(std::max(w.max_rows, kmax));
+            const int copies = std::max(1, std::min(64, std::max(w.max_rows, w.max_cols) * kmax / 1024));
+            cut_kernel<<<dim3(tm * tn + copies, nj), 256, 0, m->stream>>>(d_jobs, m->d_state, m->d_slots, m->dev, tm * tn,
+                                                                        tn, m->chi, noise_rel, m->d_records, m->d_status);
+            count_launch(m, 4);
+            CUDA_TRY(cudaStreamWaitEvent(m->stream, m->join_ev, 0));
+            if (track) CUDA_TRY(cudaEventRecord(m->wave_done[wi], m->stream));
+            continue;
+        }
         {
             Timed t(m, 4, xs);
             finalize_kernel<<<nj, 256, 0, xs>>>(d_jobs, m->d_state, m->d_slots, kJacobiExact, m->chi, noise_rel,
@@ -1119,7 +1149,7 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
             {
                 Timed t(m, 2);
                 omega_kernel<<<dim3(32, nj), 256, 0, m->stream>>>(d_jobs, m->d_state, m->d_slots);
-                const int tr = (w.max_rows + 31) / 32, tc = (w.max_cols + 31) / 32, te = (w.max_ell + 31) / 32;
+                const int tr = tiles(w.max_rows), tc = tiles(w.max_cols), te = tiles(w.max_ell);
                 rsvd_gemm_kernel<<<dim3(te, tr, nj), 256, 0, m->stream>>>(d_jobs, m->d_state, m->d_slots, kStageY0);
                 rsvd_gemm_kernel<<<dim3(te, tc, nj), 256, 0, m->stream>>>(d_jobs, m->d_state, m->d_slots, kStageZ);
                 rsvd_gemm_kernel<<<dim3(te, tr, nj), 256, 0, m->stream>>>(d_jobs, m->d_state, m->d_slots, kStageY);
@@ -1180,16 +1210,13 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
             // The side the Jacobi does not accumulate, as tiled GEMMs over the
             // kept columns (chi <= min(chi_max, rows, cols)).
             const int kmax = std::min(m->chi, std::min(w.max_rows, w.max_cols));
-            auto tiles = [](int x) { return (x + 31) / 32; };
-            if (w.any_rsvd) {
-                recover_gemm_kernel<<<dim3(tiles(std::max(w.max_cols, kmax)), tiles(std::max(w.max_ell, kmax)), nj), 256, 0,
-                                      m->stream>>>(
-                    d_jobs, m->d_state, m->d_slots, m->dev, kRecoverBW);
-                recover_gemm_kernel<<<dim3(tiles(kmax), tiles(w.max_rows), nj), 256, 0, m->stream>>>(
-                    d_jobs, m->d_state, m->d_slots, m->dev, kRecoverQT);
-                count_launch(m, 4);
-                count_launch(m, 4);
-            }
+            recover_gemm_kernel<<<dim3(tiles(std::max(w.max_cols, kmax)), tiles(std::max(w.max_ell, kmax)), nj), 256, 0,
+                              m->stream>>>(
+                d_jobs, m->d_state, m->d_slots, m->dev, kRecoverBW);
+            recover_gemm_kernel<<<dim3(tiles(kmax), tiles(w.max_rows), nj), 256, 0, m->stream>>>(
+                d_jobs, m->d_state, m->d_slots, m->dev, kRecoverQT);
+            count_launch(m, 4);
+            count_launch(m, 4);
             recover_gemm_kernel<<<dim3(tiles(std::max(w.max_cols, kmax)), tiles(std::max(w.max_rows, kmax)), nj), 256,
                                   0, m->stream>>>(d_jobs, m->d_state, m->d_slots, m->dev, kRecoverExact);
             count_launch(m, 4);
@@ -1611,6 +1638,7 @@ static wqc_status create_state(wqc_cuda_ctx* ctx, const std::vector<int>& ns, co
     m->d_small = static_cast<double2*>(p);
     m->d_counters = reinterpret_cast<unsigned long long*>(m->d_small + small - 4);
     if (cudaMemset(m->d_small, 0, small * sizeof(double2)) != cudaSuccess) return bail(fail(WQC_ERR_CUDA, "memset"));
+    m->oz_auto = oz_default;
     if (oz_default)
         if (wqc_status st = oz_enable(m)) return bail(st);
     if (ns.size() == 1) {  // the trace feeders' environment cache (single states)
@@ -1934,6 +1962,7 @@ wqc_status wqc_mps_set_merge(wqc_mps* m, int32_t merge) {
     if (m->tc) return fail(WQC_ERR_INVALID, "the tensor-core form merges on its own TF32 path");
     CUDA_TRY(cudaSetDevice(m->ctx->device));
     CUDA_TRY(cudaStreamSynchronize(m->stream));  // no enqueued merge still reads the planes
+    m->oz_auto = false;
     if (merge == WQC_MERGE_TC_INT8) return oz_enable(m);
     m->oz = false;
     return WQC_OK;

@@ -14,6 +14,7 @@
 #include "common.cuh"
 #include "jacobi_device.cuh"
 #include "split_kernels.cuh"
+#include "tile_gemm.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -22,17 +23,8 @@ namespace wqc {
 // ---------------------------------------------------------------------------
 // prepare: bond dims and the exact / range-finder decision (mps.rs:937-954).
 // ---------------------------------------------------------------------------
-__global__ void prepare_kernel(const SplitJob* jobs, SplitState* st, int njobs, DeviceMps mps) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= njobs) return;
-    const SplitJob& J = jobs[j];
+__device__ __forceinline__ SplitState split_state(const SplitJob& J, const DeviceMps& mps) {
     SplitState s{};
-    if (*mps.cancel) {  // cancelled: every later kernel of this wave skips the job
-        s.skip = 1;
-        st[j] = s;
-        if (j == 0) atomicOr(mps.status, kStatusCancelled);
-        return;
-    }
     s.dl = mps.dl[J.p];
     s.dr = mps.dr[J.p + 1];
     s.k = min(mps.dr[J.p], mps.dl[J.p + 1]);
@@ -50,7 +42,25 @@ __global__ void prepare_kernel(const SplitJob* jobs, SplitState* st, int njobs, 
     // W of X = theta (rows >= cols) holds left vectors, of theta^H right ones;
     // a Jacobi on R^H gives the other side.
     s.w_rows_of_src = (s.rows < s.cols) != (s.pre_exact != 0) ? 1 : 0;
+    return s;
+}
+
+// The state of a job as the wave's later kernels read it; a cancelled job is
+// skipped by all of them.
+__device__ __forceinline__ void publish_state(const SplitJob* jobs, SplitState* st, int j, const DeviceMps& mps) {
+    SplitState s{};
+    if (*mps.cancel) {
+        s.skip = 1;
+        if (j == 0) atomicOr(mps.status, kStatusCancelled);
+    } else {
+        s = split_state(jobs[j], mps);
+    }
     st[j] = s;
+}
+
+__global__ void prepare_kernel(const SplitJob* jobs, SplitState* st, int njobs, DeviceMps mps) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < njobs) publish_state(jobs, st, j, mps);
 }
 
 // ---------------------------------------------------------------------------
@@ -60,13 +70,17 @@ __global__ void prepare_kernel(const SplitJob* jobs, SplitState* st, int njobs, 
 // ---------------------------------------------------------------------------
 constexpr int kMergeTA = 16, kMergeTB = 16, kMergeTK = 16;
 
-__global__ void __launch_bounds__(256) merge_gate_kernel(const SplitJob* jobs, const SplitState* st,
+__global__ void __launch_bounds__(256) merge_gate_kernel(const SplitJob* jobs, SplitState* st,
                                                          const SlotBuffers* slots, DeviceMps mps) {
     const int j = blockIdx.z;
     const SplitJob& J = jobs[j];
-    const SplitState S = st[j];
+    // Every CTA derives the job's state from the bonds, and one stores it: no
+    // kernel of its own before the merge.  The others merge even if that one
+    // finds the job cancelled; nothing reads their theta then.
+    const SplitState S = split_state(J, mps);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) publish_state(jobs, st, j, mps);
     const int a0 = blockIdx.y * kMergeTA, b0 = blockIdx.x * kMergeTB;
-    if (S.skip || a0 >= S.dl || b0 >= S.dr) return;
+    if (a0 >= S.dl || b0 >= S.dr) return;
     const double2* L = mps.site[J.p];      // [dl][2][k']  with k' = dr of site p
     const double2* R = mps.site[J.p + 1];  // [k''][2][dr] with k'' = dl of site p+1
     const int ldl = mps.dr[J.p];           // row stride of L's (a,s) rows
@@ -151,88 +165,45 @@ __global__ void omega_kernel(const SplitJob* jobs, const SplitState* st, const S
 }
 
 // ---------------------------------------------------------------------------
-// Batched complex FP64 GEMM for the range finder.  C(m x n) = A(m x k) B(k x n)
-// with strided / conjugated operand views derived per job from its state.
+// Batched complex FP64 GEMMs of the range finder, dimensions from the job's state.
 // ---------------------------------------------------------------------------
-struct MatView {
-    const double2* p;
-    long rs, cs;
-    int conj;
-};
-
-__device__ __forceinline__ double2 view_at(const MatView& v, int i, int kk) {
-    const double2 x = v.p[i * v.rs + kk * v.cs];
-    return v.conj ? cconj(x) : x;
-}
-
 constexpr int kGemmT = 32, kGemmK = 16;
 
-__global__ void __launch_bounds__(256) rsvd_gemm_kernel(const SplitJob* jobs, const SplitState* st,
-                                                        const SlotBuffers* slots, int stage) {
+__global__ void __launch_bounds__(kTileThreads) rsvd_gemm_kernel(const SplitJob* jobs, const SplitState* st,
+                                                                 const SlotBuffers* slots, int stage) {
     const int j = blockIdx.z;
     const SplitState S = st[j];
     if (!S.use_rsvd) return;
     const SlotBuffers B = slots[jobs[j].slot];
     const int rows = S.rows, cols = S.cols, ell = S.ell;
-    MatView A, Bv;
-    double2* Cp;
-    long c_rs, c_cs;
-    int m, n, k;
+    const int m0 = blockIdx.y * kTile, n0 = blockIdx.x * kTile;
+    const int m = stage == kStageZ ? cols : stage == kStageB ? ell : rows, n = stage == kStageB ? cols : ell;
+    if (m0 >= m || n0 >= n) return;
+    __shared__ TileSmem sm;
+    auto theta = [&](int i, int k) { return B.theta[size_t(i) * cols + k]; };
     switch (stage) {
         case kStageY0:  // Y0 = theta * Omega   (rows x ell)
-            A = {B.theta, cols, 1, 0};
-            Bv = {B.omega, ell, 1, 0};
-            Cp = B.y0; c_rs = ell; c_cs = 1; m = rows; n = ell; k = cols;
+            tile_gemm(sm, m0, n0, m, n, cols, true, false, theta,
+                      [&](int k, int c) { return B.omega[size_t(k) * ell + c]; },
+                      [&](int i, int c, double2 v) { B.y0[size_t(i) * ell + c] = v; });
             break;
         case kStageZ:  // Z = theta^H * Y0    (cols x ell)
-            A = {B.theta, 1, cols, 1};
-            Bv = {B.y0, ell, 1, 0};
-            Cp = B.zr; c_rs = ell; c_cs = 1; m = cols; n = ell; k = rows;
+            tile_gemm(sm, m0, n0, m, n, rows, false, false,
+                      [&](int i, int k) { return cconj(B.theta[size_t(k) * cols + i]); },
+                      [&](int k, int c) { return B.y0[size_t(k) * ell + c]; },
+                      [&](int i, int c, double2 v) { B.zr[size_t(i) * ell + c] = v; });
             break;
         case kStageY:  // Y = theta * Z, stored column-major for the QR
-            A = {B.theta, cols, 1, 0};
-            Bv = {B.zr, ell, 1, 0};
-            Cp = B.y; c_rs = 1; c_cs = rows; m = rows; n = ell; k = cols;
+            tile_gemm(sm, m0, n0, m, n, cols, true, false, theta,
+                      [&](int k, int c) { return B.zr[size_t(k) * ell + c]; },
+                      [&](int i, int c, double2 v) { B.y[size_t(c) * rows + i] = v; });
             break;
         default:  // kStageB: B = Q^H * theta  (ell x cols), Q column-major rows x ell
-            A = {B.q, rows, 1, 1};
-            Bv = {B.theta, cols, 1, 0};
-            Cp = B.b; c_rs = cols; c_cs = 1; m = ell; n = cols; k = rows;
+            tile_gemm(sm, m0, n0, m, n, rows, true, false,
+                      [&](int i, int k) { return cconj(B.q[size_t(i) * rows + k]); }, theta,
+                      [&](int i, int c, double2 v) { B.b[size_t(i) * cols + c] = v; });
             break;
     }
-    const int i0 = blockIdx.y * kGemmT, n0 = blockIdx.x * kGemmT;
-    if (i0 >= m || n0 >= n) return;
-    __shared__ double2 As[kGemmT][kGemmK + 1];
-    __shared__ double2 Bs[kGemmK][kGemmT + 1];
-    const int tid = threadIdx.x;
-    const int tr = tid / 16, tc = tid % 16;  // 2x2 outputs per thread
-    double2 acc[2][2] = {{cmake(0, 0), cmake(0, 0)}, {cmake(0, 0), cmake(0, 0)}};
-    for (int k0 = 0; k0 < k; k0 += kGemmK) {
-        for (int e = tid; e < kGemmT * kGemmK; e += 256) {
-            const int r = e / kGemmK, c = e % kGemmK;
-            As[r][c] = (i0 + r < m && k0 + c < k) ? view_at(A, i0 + r, k0 + c) : cmake(0, 0);
-        }
-        for (int e = tid; e < kGemmK * kGemmT; e += 256) {
-            const int r = e / kGemmT, c = e % kGemmT;
-            Bs[r][c] = (k0 + r < k && n0 + c < n) ? view_at(Bv, k0 + r, n0 + c) : cmake(0, 0);
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int c = 0; c < kGemmK; ++c) {
-            const double2 a0 = As[tr][c], a1 = As[tr + 16][c];
-            const double2 b0 = Bs[c][tc], b1 = Bs[c][tc + 16];
-            cfma(acc[0][0], a0, b0);
-            cfma(acc[0][1], a0, b1);
-            cfma(acc[1][0], a1, b0);
-            cfma(acc[1][1], a1, b1);
-        }
-        __syncthreads();
-    }
-    for (int x = 0; x < 2; ++x)
-        for (int y = 0; y < 2; ++y) {
-            const int i = i0 + tr + 16 * x, jj = n0 + tc + 16 * y;
-            if (i < m && jj < n) Cp[i * c_rs + jj * c_cs] = acc[x][y];
-        }
 }
 
 // ---------------------------------------------------------------------------
@@ -1016,68 +987,61 @@ __global__ void __launch_bounds__(256) precond_gemm_kernel(const SplitJob* jobs,
 }
 
 // ---------------------------------------------------------------------------
-// finalize: stable descending sort, truncation rule, ambiguity test,
-// discarded weight and the split record.
+// The cut: stable descending sort, truncation rule, discarded weight and the
+// split record, then both sides into the sites.
 // ---------------------------------------------------------------------------
-__global__ void finalize_kernel(const SplitJob* jobs, SplitState* st, const SlotBuffers* slots, int mode,
-                                int chi_max, double noise_rel, wqc_split_info* records, int* status) {
-    const int j = blockIdx.x;
-    SplitState& S = st[j];
-    if (!jacobi_active(S, mode)) return;
-    const SplitJob& J = jobs[j];
-    const SlotBuffers B = slots[J.slot];
-    const int N = mode == kJacobiRsvd ? S.ell : min(S.rows, S.cols);
-    __shared__ double vals[1024];
-    const int tid = threadIdx.x;
-    // rank_j = #{i : s_i > s_j or (s_i == s_j and i < j)}
-    for (int c = tid; c < N; c += blockDim.x) {
-        const double sj = B.sigma[c];
+struct CutSmem {
+    double vals[1024];  // singular values, descending, noise at zero
+    int perm[1024];     // sorted position -> column of W
+};
+
+// rank_j = #{i : s_i > s_j or (s_i == s_j and i < j)}; every thread of the CTA.
+__device__ __forceinline__ void sort_values(CutSmem& sm, const double* sigma, int N, int mode, double noise_rel) {
+    const int tid = threadIdx.x, nt = blockDim.x;
+    for (int c = tid; c < N; c += nt) sm.perm[c] = c;  // a NaN among the values leaves places unwritten below
+    __shared__ double raw[1024];
+    for (int c = tid; c < N; c += nt) raw[c] = sigma[c];
+    __syncthreads();
+    for (int c = tid; c < N; c += nt) {
+        const double sj = raw[c];
         int r = 0;
         for (int i = 0; i < N; ++i) {
-            const double si = B.sigma[i];
+            const double si = raw[i];
             r += (si > sj || (si == sj && i < c)) ? 1 : 0;
         }
-        B.perm[r] = c;
+        sm.perm[r] = c;
     }
     __syncthreads();
-    const double floor_abs = N > 0 ? noise_rel * B.sigma[B.perm[0]] : 0.0;
-    for (int c = tid; c < N; c += blockDim.x) {
-        double v = B.sigma[B.perm[c]];
+    const double floor_abs = N > 0 ? noise_rel * raw[sm.perm[0]] : 0.0;
+    for (int c = tid; c < N; c += nt) {
+        double v = raw[sm.perm[c]];
         if (mode == kJacobiRsvd && v < kRsvdZero) v = 0.0;
         if (v < floor_abs) v = 0.0;
-        vals[c] = v;
+        sm.vals[c] = v;
     }
     __syncthreads();
-    if (tid != 0) return;
-    // retained_chi (svd_guard.rs:25-35)
+}
+
+// retained_chi (svd_guard.rs:25-35); every thread of the CTA.
+__device__ __forceinline__ int kept_bond(const CutSmem& sm, int N, const SplitJob& J, const SplitState& S, int chi_max) {
     int rank = 0;
-    bool bad = false;
-    for (int i = 0; i < N; ++i) {
-        if (vals[i] > kSingularCutoff) ++rank;
-        if (!isfinite(vals[i]) || vals[i] < 0.0) bad = true;
+    for (int base = 0; base < N; base += blockDim.x) {
+        const int c = base + int(threadIdx.x);
+        rank += __syncthreads_count(c < N && sm.vals[c] > kSingularCutoff);
     }
-    int chi = N == 0 ? 0 : min(min(max(rank, 1), J.chi_max > 0 ? J.chi_max : chi_max), min(S.rows, S.cols));
-    if (mode == kJacobiRsvd) {
-        // needs_f64_fallback (svd_guard.rs:58-76)
-        bool fb = bad || chi == 0;
-        for (int i = 0; i < N && !fb; ++i)
-            if (vals[i] > 0.0 && fabs(vals[i] - kSingularCutoff) <= kCutoffAbsBand) fb = true;
-        if (!fb && chi > 0 && chi < N) {
-            const double kept = vals[chi - 1], dropped = vals[chi];
-            const double scale = fmax(fmax(kept, dropped), 1e-30);
-            if (fabs(kept - dropped) / scale < kChiRelGap) fb = true;
-        }
-        if (fb) {
-            S.need_exact = 1;
-            S.path = WQC_SPLIT_RSVD_FALLBACK;
-            return;
-        }
-        S.final_kind = 1;
-    } else {
-        S.final_kind = 0;
+    return N == 0 ? 0 : min(min(max(rank, 1), J.chi_max > 0 ? J.chi_max : chi_max), min(S.rows, S.cols));
+}
+
+// The outcome of an exact SVD, or of a range finder that is accepted; one thread.
+__device__ __forceinline__ void record_cut(const CutSmem& sm, int N, int chi, int final_kind, const SplitJob& J,
+                                           SplitState& S, wqc_split_info* records, int* status) {
+    bool bad = false;
+    for (int i = 0; i < N; ++i)
+        if (!isfinite(sm.vals[i]) || sm.vals[i] < 0.0) bad = true;
+    if (final_kind == 0) {
         if (J.reject) {
             for (int i = chi; i < N; ++i)
-                if (vals[i] > kSingularCutoff) {
+                if (sm.vals[i] > kSingularCutoff) {
                     atomicOr(status, kStatusTruncationRejected);
                     break;
                 }
@@ -1085,7 +1049,8 @@ __global__ void finalize_kernel(const SplitJob* jobs, SplitState* st, const Slot
         if (bad) atomicOr(status, kStatusNonFinite);
     }
     double disc = 0;
-    for (int i = chi; i < N; ++i) disc += vals[i] * vals[i];
+    for (int i = chi; i < N; ++i) disc += sm.vals[i] * sm.vals[i];
+    S.final_kind = final_kind;
     S.chi = chi;
     S.discarded = disc;
     wqc_split_info info;
@@ -1097,6 +1062,42 @@ __global__ void finalize_kernel(const SplitJob* jobs, SplitState* st, const Slot
     info.chi = chi;
     info.discarded_weight = disc;
     records[J.seq] = info;
+}
+
+// finalize: the cut of a wave in which range finders take part, with the
+// ambiguity test that sends one back to the exact path.
+__global__ void finalize_kernel(const SplitJob* jobs, SplitState* st, const SlotBuffers* slots, int mode,
+                                int chi_max, double noise_rel, wqc_split_info* records, int* status) {
+    const int j = blockIdx.x;
+    SplitState& S = st[j];
+    if (!jacobi_active(S, mode)) return;
+    const SplitJob& J = jobs[j];
+    const SlotBuffers B = slots[J.slot];
+    const int N = mode == kJacobiRsvd ? S.ell : min(S.rows, S.cols);
+    __shared__ CutSmem sm;
+    sort_values(sm, B.sigma, N, mode, noise_rel);
+    for (int c = threadIdx.x; c < N; c += blockDim.x) B.perm[c] = sm.perm[c];
+    const int chi = kept_bond(sm, N, J, S, chi_max);
+    if (threadIdx.x != 0) return;
+    if (mode == kJacobiRsvd) {
+        // needs_f64_fallback (svd_guard.rs:58-76)
+        bool fb = chi == 0;
+        for (int i = 0; i < N && !fb; ++i) {
+            if (!isfinite(sm.vals[i]) || sm.vals[i] < 0.0) fb = true;
+            if (sm.vals[i] > 0.0 && fabs(sm.vals[i] - kSingularCutoff) <= kCutoffAbsBand) fb = true;
+        }
+        if (!fb && chi > 0 && chi < N) {
+            const double kept = sm.vals[chi - 1], dropped = sm.vals[chi];
+            const double scale = fmax(fmax(kept, dropped), 1e-30);
+            if (fabs(kept - dropped) / scale < kChiRelGap) fb = true;
+        }
+        if (fb) {
+            S.need_exact = 1;
+            S.path = WQC_SPLIT_RSVD_FALLBACK;
+            return;
+        }
+    }
+    record_cut(sm, N, chi, mode == kJacobiRsvd ? 1 : 0, J, S, records, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -1112,8 +1113,34 @@ __global__ void finalize_kernel(const SplitJob* jobs, SplitState* st, const Slot
 //   kRecoverBW:   R = s^-3/2 W_k^H B         (chi x cols, into site p+1)
 //   kRecoverQT:   L = Q W_k s^-1/2           (rows x chi, into site p)
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) recover_gemm_kernel(const SplitJob* jobs, const SplitState* st,
-                                                           const SlotBuffers* slots, DeviceMps mps, int stage) {
+__device__ __forceinline__ double inv_s32(double sg) { return sg > 0.0 ? 1.0 / (sg * sqrt(sg)) : 0.0; }
+__device__ __forceinline__ double inv_s12(double sg) { return sg > 0.0 ? 1.0 / sqrt(sg) : 0.0; }
+
+// The recovered side of an exact SVD, one tile.
+__device__ __forceinline__ void recover_exact(TileSmem& sm, int m0, int n0, const SplitJob& J, const SplitState& S,
+                                              const SlotBuffers& B, const int* perm, int chi, const DeviceMps& mps) {
+    const int rows = S.rows, cols = S.cols;
+    if (!S.w_rows_of_src) {
+        if (m0 >= chi || n0 >= cols) return;
+        double2* R = mps.site[J.p + 1];
+        tile_gemm(
+            sm, m0, n0, chi, cols, rows, true, false,
+            [&](int i, int k) { return cconj(B.w[size_t(perm[i]) * rows + k]); },
+            [&](int k, int c) { return B.theta[size_t(k) * cols + c]; },
+            [&](int i, int c, double2 v) { R[size_t(i) * cols + c] = cscale(v, inv_s32(B.sigma[perm[i]])); });
+    } else {
+        if (m0 >= rows || n0 >= chi) return;
+        double2* L = mps.site[J.p];
+        tile_gemm(
+            sm, m0, n0, rows, chi, cols, true, true, [&](int i, int k) { return B.theta[size_t(i) * cols + k]; },
+            [&](int k, int c) { return B.w[size_t(perm[c]) * cols + k]; },
+            [&](int i, int c, double2 v) { L[size_t(i) * chi + c] = cscale(v, inv_s32(B.sigma[perm[c]])); });
+    }
+}
+
+__global__ void __launch_bounds__(kTileThreads) recover_gemm_kernel(const SplitJob* jobs, const SplitState* st,
+                                                                    const SlotBuffers* slots, DeviceMps mps,
+                                                                    int stage) {
     const int j = blockIdx.z;
     const SplitJob& J = jobs[j];
     const SplitState S = st[j];
@@ -1122,97 +1149,63 @@ __global__ void __launch_bounds__(256) recover_gemm_kernel(const SplitJob* jobs,
     if ((stage == kRecoverExact) == rf) return;
     const SlotBuffers B = slots[J.slot];
     const int rows = S.rows, cols = S.cols, ell = S.ell, chi = S.chi;
-    // C[i][n] = sum_k A(i, k) Bm(k, n); which operand is gathered by perm
-    // depends on the stage.
-    int m, n, k, kind;
-    if (stage == kRecoverBW) {
-        m = ell; n = chi; k = cols; kind = 0;
-        if (S.pre_rsvd) { m = chi; n = cols; k = ell; kind = 4; }
-    } else if (stage == kRecoverQT) {
-        m = rows; n = chi; k = ell; kind = S.pre_rsvd ? 5 : 1;
-    } else if (!S.w_rows_of_src) {
-        m = chi; n = cols; k = rows; kind = 2;
+    const int m0 = blockIdx.y * kTile, n0 = blockIdx.x * kTile;
+    __shared__ TileSmem sm;
+    if (stage == kRecoverExact) {
+        recover_exact(sm, m0, n0, J, S, B, B.perm, chi, mps);
+        return;
+    }
+    auto q_at = [&](int i, int k) { return B.q[size_t(k) * rows + i]; };
+    if (stage == kRecoverBW && !S.pre_rsvd) {
+        if (m0 >= ell || n0 >= chi) return;
+        tile_gemm(
+            sm, m0, n0, ell, chi, cols, true, true, [&](int i, int k) { return B.b[size_t(i) * cols + k]; },
+            [&](int k, int c) { return B.w[size_t(B.perm[c]) * cols + k]; },
+            [&](int i, int c, double2 v) { B.z[size_t(B.perm[c]) * ell + i] = v; });
+    } else if (stage == kRecoverBW) {
+        if (m0 >= chi || n0 >= cols) return;
+        double2* R = mps.site[J.p + 1];
+        tile_gemm(
+            sm, m0, n0, chi, cols, ell, true, false,
+            [&](int i, int k) { return cconj(B.w[size_t(B.perm[i]) * ell + k]); },
+            [&](int k, int c) { return B.b[size_t(k) * cols + c]; },
+            [&](int i, int c, double2 v) { R[size_t(i) * cols + c] = cscale(v, inv_s32(B.sigma[B.perm[i]])); });
     } else {
-        m = rows; n = chi; k = cols; kind = 3;
+        if (m0 >= rows || n0 >= chi) return;
+        double2* L = mps.site[J.p];
+        const double2* T = S.pre_rsvd ? B.w : B.z;
+        tile_gemm(
+            sm, m0, n0, rows, chi, ell, false, true, q_at,
+            [&](int k, int c) { return T[size_t(B.perm[c]) * ell + k]; },
+            [&](int i, int c, double2 v) {
+                const double sg = B.sigma[B.perm[c]];
+                L[size_t(i) * chi + c] = cscale(v, S.pre_rsvd ? inv_s12(sg) : inv_s32(sg));
+            });
     }
-    const int i0 = blockIdx.y * kGemmT, n0 = blockIdx.x * kGemmT;
-    if (i0 >= m || n0 >= n) return;
-    auto a_at = [&](int i, int kk) -> double2 {
-        switch (kind) {
-            case 0: return B.b[size_t(i) * cols + kk];                          // B[j][c]
-            case 1: return B.q[size_t(kk) * rows + i];                          // Q[r][t]
-            case 2: return cconj(B.w[size_t(B.perm[i]) * rows + kk]);          // conj W[r][pc(m)]
-            case 4: return cconj(B.w[size_t(B.perm[i]) * ell + kk]);           // conj W[t][pc(m)]
-            case 5: return B.q[size_t(kk) * rows + i];                          // Q[r][t]
-            default: return B.theta[size_t(i) * cols + kk];                     // theta[r][c]
-        }
-    };
-    auto b_at = [&](int kk, int nn) -> double2 {
-        switch (kind) {
-            case 0: return B.w[size_t(B.perm[nn]) * cols + kk];                 // W[c][pc(m)]
-            case 1: return B.z[size_t(B.perm[nn]) * ell + kk];                  // T[t][pc(m)]
-            case 2: return B.theta[size_t(kk) * cols + nn];                     // theta[r][c]
-            case 4: return B.b[size_t(kk) * cols + nn];                         // B[t][c]
-            case 5: return B.w[size_t(B.perm[nn]) * ell + kk];                  // W[t][pc(m)]
-            default: return B.w[size_t(B.perm[nn]) * cols + kk];                // W[c][pc(m)]
-        }
-    };
-    __shared__ double2 As[kGemmT][kGemmK + 1];
-    __shared__ double2 Bs[kGemmK][kGemmT + 1];
-    const int tid = threadIdx.x;
-    const int tr = tid / 16, tc = tid % 16;
-    double2 acc[2][2] = {{cmake(0, 0), cmake(0, 0)}, {cmake(0, 0), cmake(0, 0)}};
-    for (int k0 = 0; k0 < k; k0 += kGemmK) {
-        for (int e = tid; e < kGemmT * kGemmK; e += 256) {
-            const int r = e / kGemmK, c = e % kGemmK;
-            As[r][c] = (i0 + r < m && k0 + c < k) ? a_at(i0 + r, k0 + c) : cmake(0, 0);
-        }
-        for (int e = tid; e < kGemmK * kGemmT; e += 256) {
-            const int r = e / kGemmT, c = e % kGemmT;
-            Bs[r][c] = (k0 + r < k && n0 + c < n) ? b_at(k0 + r, n0 + c) : cmake(0, 0);
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int c = 0; c < kGemmK; ++c) {
-            const double2 a0 = As[tr][c], a1 = As[tr + 16][c];
-            const double2 b0 = Bs[c][tc], b1 = Bs[c][tc + 16];
-            cfma(acc[0][0], a0, b0);
-            cfma(acc[0][1], a0, b1);
-            cfma(acc[1][0], a1, b0);
-            cfma(acc[1][1], a1, b1);
-        }
-        __syncthreads();
-    }
-    auto inv_s32 = [&](int mm) {
-        const double sg = B.sigma[B.perm[mm]];
-        return sg > 0.0 ? 1.0 / (sg * sqrt(sg)) : 0.0;
-    };
-    auto inv_s12 = [&](int mm) {
-        const double sg = B.sigma[B.perm[mm]];
-        return sg > 0.0 ? 1.0 / sqrt(sg) : 0.0;
-    };
-    for (int x = 0; x < 2; ++x)
-        for (int y = 0; y < 2; ++y) {
-            const int i = i0 + tr + 16 * x, nn = n0 + tc + 16 * y;
-            if (i >= m || nn >= n) continue;
-            const double2 v = acc[x][y];
-            switch (kind) {
-                case 0: B.z[size_t(B.perm[nn]) * ell + i] = v; break;
-                case 1: mps.site[J.p][size_t(i) * chi + nn] = cscale(v, inv_s32(nn)); break;
-                case 2:
-                case 4: mps.site[J.p + 1][size_t(i) * cols + nn] = cscale(v, inv_s32(i)); break;
-                case 5: mps.site[J.p][size_t(i) * chi + nn] = cscale(v, inv_s12(nn)); break;
-                default: mps.site[J.p][size_t(i) * chi + nn] = cscale(v, inv_s32(nn)); break;
-            }
-        }
 }
 
-// ---------------------------------------------------------------------------
-// absorb: the sides that are plain copies of W (L = W / sqrt(s) where W holds
-// left vectors, R = W^H / sqrt(s) where it holds right ones), and the new bond dims
-// (mps.rs:1156-1168, 1039-1051).  The other side comes from
-// recover_gemm_kernel.
-// ---------------------------------------------------------------------------
+// The side that is a plain copy of W (L = W / sqrt(s) where W holds left
+// vectors, R = W^H / sqrt(s) where it holds right ones; mps.rs:1156-1168,
+// 1039-1051), entries t0, t0 + stride, ...
+__device__ __forceinline__ void copy_side(const SplitJob& J, const SplitState& S, const SlotBuffers& B, bool left,
+                                          const int* perm, int chi, const DeviceMps& mps, long t0, long stride) {
+    const int rows = S.rows, cols = S.cols;
+    if (left) {
+        double2* Ls = mps.site[J.p];
+        for (long e = t0; e < long(rows) * chi; e += stride) {
+            const int r = int(e / chi), pc = perm[e % chi];
+            Ls[e] = cscale(B.w[size_t(pc) * rows + r], inv_s12(B.sigma[pc]));  // L[(r/2)][r%2][m] at r*chi + m
+        }
+    } else {
+        double2* Rs = mps.site[J.p + 1];
+        for (long e = t0; e < long(chi) * cols; e += stride) {
+            const int c = int(e % cols), pc = perm[e / cols];
+            Rs[e] = cscale(cconj(B.w[size_t(pc) * cols + c]), inv_s12(B.sigma[pc]));  // R[m][c/dr][c%dr]
+        }
+    }
+}
+
+// absorb: the copied sides of a wave with range finders, and the new bonds.
 __global__ void __launch_bounds__(256) absorb_kernel(const SplitJob* jobs, const SplitState* st,
                                                      const SlotBuffers* slots, DeviceMps mps) {
     const int j = blockIdx.y;
@@ -1220,35 +1213,53 @@ __global__ void __launch_bounds__(256) absorb_kernel(const SplitJob* jobs, const
     const SplitState S = st[j];
     if (S.skip) return;
     const SlotBuffers B = slots[J.slot];
-    const int chi = S.chi, rows = S.rows, cols = S.cols;
-    const long stride = long(gridDim.x) * blockDim.x;
-    const long t0 = long(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (S.final_kind == 1 && S.pre_rsvd) {
-        // Both sides come from recover_gemm_kernel.
-    } else if (S.final_kind == 0 && !S.w_rows_of_src) {
-        // L = W / sqrt(s), W rows x cols; R comes from recover_gemm_kernel.
-        double2* Ls = mps.site[J.p];
-        for (long e = t0; e < long(rows) * chi; e += stride) {
-            const int r = int(e / chi), m = int(e % chi);
-            const int pc = B.perm[m];
-            const double sg = B.sigma[pc];
-            const double2 w = B.w[size_t(pc) * rows + r];
-            Ls[e] = sg > 0.0 ? cscale(w, 1.0 / sqrt(sg)) : cmake(0, 0);  // L[(r/2)][r%2][m] at r*chi + m
-        }
-    } else {
-        // R = W^H / sqrt(s), W cols x (ell or rows); L comes from recover_gemm_kernel.
-        double2* Rs = mps.site[J.p + 1];
-        for (long e = t0; e < long(chi) * cols; e += stride) {
-            const int m = int(e / cols), c = int(e % cols);
-            const int pc = B.perm[m];
-            const double sg = B.sigma[pc];
-            const double2 w = B.w[size_t(pc) * cols + c];
-            Rs[e] = sg > 0.0 ? cscale(cconj(w), 1.0 / sqrt(sg)) : cmake(0, 0);  // R[m][c/dr][c%dr]
-        }
-    }
+    if (!(S.final_kind == 1 && S.pre_rsvd))  // both sides come from recover_gemm_kernel
+        copy_side(J, S, B, S.final_kind == 0 && !S.w_rows_of_src, B.perm, S.chi, mps,
+                  long(blockIdx.x) * blockDim.x + threadIdx.x, long(gridDim.x) * blockDim.x);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        mps.dr[J.p] = chi;
-        mps.dl[J.p + 1] = chi;
+        mps.dr[J.p] = S.chi;
+        mps.dl[J.p + 1] = S.chi;
+    }
+}
+
+// The whole cut of a wave without range finders in one launch: every CTA sorts
+// the values for itself (N^2 / 256 compares a thread, ~2 us at N = 256) and
+// then computes a tile of the recovered side (blocks below `tiles`, tiles_n to
+// a row) or copies a part of the other; block 0 records.  Three launches, two
+// of them a few microseconds of work behind a launch each, took 27 us at 64
+// columns and 87 us at 256.
+__global__ void __launch_bounds__(kTileThreads) cut_kernel(const SplitJob* jobs, SplitState* st,
+                                                           const SlotBuffers* slots, DeviceMps mps, int tiles,
+                                                           int tiles_n, int chi_max, double noise_rel,
+                                                           wqc_split_info* records, int* status) {
+    const int j = blockIdx.y;
+    const SplitJob& J = jobs[j];
+    const SplitState S = st[j];
+    if (!jacobi_active(S, kJacobiExact)) return;
+    const SlotBuffers B = slots[J.slot];
+    const int N = min(S.rows, S.cols);
+    const int bx = blockIdx.x, m0 = (bx / tiles_n) * kTile, n0 = (bx % tiles_n) * kTile;
+    // Tiles past what the largest kept bond can need leave before the sort.
+    if (bx > 0 && bx < tiles &&
+        (S.w_rows_of_src ? m0 >= S.rows || n0 >= min(N, J.chi_max) : m0 >= min(N, J.chi_max) || n0 >= S.cols))
+        return;
+    __shared__ CutSmem cut;
+    sort_values(cut, B.sigma, N, kJacobiExact, noise_rel);
+    const int chi = kept_bond(cut, N, J, S, chi_max);
+    if (bx < tiles) {
+        __shared__ TileSmem sm;
+        recover_exact(sm, m0, n0, J, S, B, cut.perm, chi, mps);
+    } else {
+        copy_side(J, S, B, !S.w_rows_of_src, cut.perm, chi, mps, long(bx - tiles) * blockDim.x + threadIdx.x,
+                  long(gridDim.x - tiles) * blockDim.x);
+    }
+    if (bx == 0) {
+        for (int c = threadIdx.x; c < N; c += blockDim.x) B.perm[c] = cut.perm[c];
+        if (threadIdx.x == 0) {
+            record_cut(cut, N, chi, 0, J, st[j], records, status);
+            mps.dr[J.p] = chi;
+            mps.dl[J.p + 1] = chi;
+        }
     }
 }
 

@@ -50,7 +50,7 @@ __host__ __device__ inline int jacobi_entry_cluster(int e) { return 1 << (e >> k
 constexpr int kJacobiStagedThreads = 512;
 
 __global__ void prepare_kernel(const SplitJob* jobs, SplitState* st, int njobs, DeviceMps mps);
-__global__ void merge_gate_kernel(const SplitJob* jobs, const SplitState* st, const SlotBuffers* slots,
+__global__ void merge_gate_kernel(const SplitJob* jobs, SplitState* st, const SlotBuffers* slots,
                                   DeviceMps mps);
 __global__ void omega_kernel(const SplitJob* jobs, const SplitState* st, const SlotBuffers* slots);
 __global__ void rsvd_gemm_kernel(const SplitJob* jobs, const SplitState* st, const SlotBuffers* slots, int stage);
@@ -129,6 +129,8 @@ __global__ void finalize_kernel(const SplitJob* jobs, SplitState* st, const Slot
 enum { kRecoverBW = 0, kRecoverQT = 1, kRecoverExact = 2 };
 __global__ void recover_gemm_kernel(const SplitJob* jobs, const SplitState* st, const SlotBuffers* slots,
                                     DeviceMps mps, int stage);
+__global__ void cut_kernel(const SplitJob* jobs, SplitState* st, const SlotBuffers* slots, DeviceMps mps, int tiles,
+                           int tiles_n, int chi_max, double noise_rel, wqc_split_info* records, int* status);
 __global__ void absorb_kernel(const SplitJob* jobs, const SplitState* st, const SlotBuffers* slots,
                               DeviceMps mps);
 
