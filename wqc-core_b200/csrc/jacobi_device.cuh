@@ -75,12 +75,11 @@ __device__ __forceinline__ double block_total(double v, double* red) {
     return t;
 }
 
+// Position pos of the circle method on b items after `step` < b - 1 turns.
 __device__ __forceinline__ int circle_at(int pos, int step, int b) {
     if (pos == 0) return 0;
-    const int m = b - 1;
-    int v = (pos - 1 - step) % m;
-    if (v < 0) v += m;
-    return v + 1;
+    const int v = pos - 1 - step;
+    return (v < 0 ? v + b - 1 : v) + 1;
 }
 
 // Rotates columns xp, xq (each W then Z, `len` entries, W part `M`).  All
@@ -163,9 +162,10 @@ __device__ __forceinline__ bool jacobi_params(double a, double bb, double gr, do
                                               double& wr, double& wi) {
     const double g2 = fma(gr, gr, gi * gi);
     const double ab = a * bb;
-    if (fmin(a, bb) <= noise_floor) return false;  // the smaller column is at the storage's rounding level
+    // Left alone: the smaller column is at the storage's rounding level, or
+    // the pair is orthogonal to tol.  (A NaN is rotated, and rejected later.)
+    if (fmin(a, bb) <= noise_floor || g2 <= tol2 * ab) return false;
     if (want_ratio) sw.relmax = fmax(sw.relmax, g2 / ab);
-    if (g2 == 0.0 || g2 <= tol2 * ab) return false;
     const double d = 0.5 * (bb - a);
     const double r2 = fma(d, d, g2);
     if (g2 > 1e-290) {

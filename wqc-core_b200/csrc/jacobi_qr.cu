@@ -221,6 +221,9 @@ __global__ void __launch_bounds__(NW * 32) jacobi_qr_kernel(const SplitJob* jobs
                 double2* pub = panel + local * LD;
                 if (wid == local % NW) publish<0>(a, local / NW, pub, lane);
                 __syncthreads();
+                // Warps whose columns are all finished leave the FP64 pipe to
+                // the others (the step is bound by it while all take part).
+                if (first + (NC - 1) * NW + wid < c || first + wid >= N) continue;
                 const int ck = c >> 5, cl = c & 31;
                 double2 x[KR];
                 double sums[kSums];
@@ -334,18 +337,19 @@ namespace {
 
 using QrKernel = void (*)(const SplitJob*, SplitState*, const SlotBuffers*, const int*, int, int*);
 
-// Instances by row groups, kJacobiQrPerCta columns a CTA.  One column per warp where the
-// cluster holds the matrix that way: a step's instructions are issued by every
-// warp at about five cycles each, so columns are better spread over warps and
-// CTAs than stacked in a warp (256 x 256: 0.81 ms with 4 columns in each of 4
-// warps).
+// Instances by row groups, kJacobiQrPerCta columns a CTA.  A step's
+// instructions are issued by every warp at about five cycles each, so columns
+// are better spread over warps and CTAs than stacked in a warp (256 x 256:
+// 0.81 ms with 4 columns in each of 4 warps), as long as two columns' rows fit
+// the registers (0.62 ms with one column in each of 16 warps, which spill;
+// 0.55 with two in each of 8).
 QrKernel qr_kernel(int kr) {
     switch (kr) {
         case 1: return jacobi_qr_kernel<1, 1, 16>;
         case 2: return jacobi_qr_kernel<2, 1, 16>;
         case 4: return jacobi_qr_kernel<4, 1, 16>;
-        case 6: return jacobi_qr_kernel<6, 1, 16>;
-        case 8: return jacobi_qr_kernel<8, 1, 16>;
+        case 6: return jacobi_qr_kernel<6, 2, 8>;
+        case 8: return jacobi_qr_kernel<8, 2, 8>;
         case 12: return jacobi_qr_kernel<12, 2, 8>;
         default: return jacobi_qr_kernel<16, 2, 8>;
     }
@@ -370,7 +374,7 @@ cudaError_t launch_jacobi_qr(int kr, int C, int tasks, cudaStream_t stream, cons
                              const SlotBuffers* slots, const int* idx, int mode, int* status) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tasks * C);
-    cfg.blockDim = dim3(kr > 8 ? 256 : 512);
+    cfg.blockDim = dim3(kr > 4 ? 256 : 512);
     cfg.dynamicSmemBytes = qr_smem(kr);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];

@@ -22,11 +22,8 @@ constexpr int jacobi_ring_kr(bool fp32, int M, int vrows) {
     return need <= 4 ? (need < 1 ? 1 : need) : need <= 6 ? 6 : need <= 8 ? 8 : need <= 12 ? 12 : 0;
 }
 // Warps of its largest CTA, one per column of a block: what 64 Ki registers
-// hold of two columns' rows per lane and about 60 registers besides.
-constexpr int jacobi_ring_warps(int kr, int elem) {
-    const int regs = 2 * kr * elem / 4 + 62;
-    return regs <= 80 ? 24 : regs <= 128 ? 16 : 12;
-}
+// hold of two columns' rows per lane and about 70 registers besides.
+constexpr int jacobi_ring_warps(int kr, int elem) { return 2 * kr * elem / 4 + 70 <= 128 ? 16 : 12; }
 // QR before the Jacobi (jacobi_qr.cu): instances by row groups, columns a CTA
 // holds at a time, and the tasks it takes -- from 16 columns (one SVD of 8 columns took 43 us
 // without and 56 with it, of 16 columns 125 and 101, of 32 385 and 220) to the
