@@ -27,6 +27,7 @@
 // side); the other side is recovered as theta^H U S^-1 or theta V S^-1.
 #include "common.cuh"
 #include "split_kernels.cuh"
+#include "tile_gemm.cuh"
 
 namespace wqc {
 
@@ -44,112 +45,108 @@ __device__ __forceinline__ double2 pauli_conj_row(char ch, const double2* a, int
     }
 }
 
-// Left and right environments of every site for each Pauli term (one CTA
-// per term).  EL_q[a][a'] (ket a, bra a') contracts sites 0..q-1 of
-// <psi| P |psi>; ER_q[b][b'] contracts sites q+1..n-1.  With
+// Left and right environments of every site for each Pauli term.  EL_q[a][a']
+// (ket a, bra a') contracts sites 0..q-1 of <psi| P |psi>; ER_q[b][b']
+// contracts sites q+1..n-1.  With
 // At[a', s, b'] = sum_{s'} P[s'][s] conj(A[a', s', b']):
 //   EL_{q+1}[b][b'] = sum_{a, a', s} EL_q[a][a'] A[a, s, b] At[a', s, b'],
 //   ER_{q-1}[a][a'] = sum_{b, b', s} A[a, s, b] ER_q[b][b'] At[a', s, b'].
 // envs: (n + 1) cap^2 entries per term for EL, then n cap^2 for ER;
-// tmp: cap * 2 * cap per term.  vals[t] = <psi|P_t|psi> = EL_n[0][0].
-__global__ void __launch_bounds__(256) adj_pauli_envs_kernel(DeviceMps mps, const char* labels, int nterms, int cap,
-                                                             double2* envs, double2* tmp_all, double2* vals) {
-    const int t = blockIdx.x;
-    if (t >= nterms) return;
-    const int n = mps.n;
+// tmp: cap * 2 * cap per term and direction.  <psi|P_t|psi> = EL_n[0][0].
+//
+// One half of one step for every term and both directions: blockIdx.x = 2 t +
+// direction, the left environments at site `step`, the right ones at the
+// mirrored site.  phase 0 multiplies the environment into the site, phase 1
+// closes it.  (As one CTA per term that walked all sites, 63 terms on 32 sites
+// at chi 64 took 25.6 ms, which was the walk's latency.)
+__global__ void __launch_bounds__(kTileThreads) adj_pauli_envs_kernel(DeviceMps mps, const char* labels, int cap,
+                                                                      int step, int phase, double2* envs,
+                                                                      double2* tmp_all) {
+    __shared__ TileSmem sm;
+    const int t = blockIdx.x >> 1;
+    const bool right = blockIdx.x & 1;
+    const int n = mps.n, q = right ? n - 1 - step : step;
     const size_t E = size_t(cap) * cap;
     double2* EL = envs + size_t(t) * (2 * n + 1) * E;
     double2* ER = EL + size_t(n + 1) * E;
-    double2* tmp = tmp_all + size_t(t) * 2 * E;
-    const char* lab = labels + size_t(t) * n;
-    if (threadIdx.x == 0) {
-        EL[0] = cmake(1.0, 0.0);
-        ER[size_t(n - 1) * E] = cmake(1.0, 0.0);
-    }
-    __syncthreads();
-    for (int q = 0; q < n; ++q) {
-        const int l = mps.dl[q], r = mps.dr[q];
-        const double2* A = mps.site[q];
+    double2* tmp = tmp_all + size_t(blockIdx.x) * 2 * E;
+    const char ch = labels[size_t(t) * n + (n - 1 - q)];
+    const int l = mps.dl[q], r = mps.dr[q], m0 = blockIdx.y * kTile, n0 = blockIdx.z * kTile;
+    const double2* A = mps.site[q];
+    const bool first = step == 0;  // the environment is [1]
+    if (first && phase == 0 && m0 == 0 && n0 == 0 && threadIdx.x == 0) (right ? ER + size_t(n - 1) * E : EL)[0] = cmake(1.0, 0.0);
+    if (!right) {
         const double2* cur = EL + size_t(q) * E;  // l x l
         double2* nxt = EL + size_t(q + 1) * E;    // r x r
-        const char ch = lab[n - 1 - q];
-        // tmp[a'][s][b] = sum_a cur[a][a'] A[a, s, b]
-        for (long e = threadIdx.x; e < long(l) * 2 * r; e += blockDim.x) {
-            const int ap = int(e / (2 * r)), rem = int(e % (2 * r));
-            double2 acc = cmake(0, 0);
-            for (int a = 0; a < l; ++a) cfma(acc, cur[size_t(a) * l + ap], A[size_t(a) * 2 * r + rem]);
-            tmp[e] = acc;
+        if (phase == 0) {  // tmp[a'][s][b] = sum_a cur[a][a'] A[a, s, b]
+            if (m0 >= l || n0 >= 2 * r) return;
+            tile_gemm(
+                sm, m0, n0, l, 2 * r, l, false, false,
+                [&](int ap, int a) { return first ? cmake(1.0, 0.0) : cur[size_t(a) * l + ap]; },
+                [&](int a, int x) { return A[size_t(a) * 2 * r + x]; },
+                [&](int ap, int x, double2 v) { tmp[size_t(ap) * 2 * r + x] = v; });
+        } else {
+            if (m0 >= r || n0 >= r) return;
+            tile_gemm(
+                sm, m0, n0, r, r, 2 * l, false, false, [&](int b, int x) { return tmp[size_t(x) * r + b]; },
+                [&](int x, int bp) { return pauli_conj_row(ch, A + size_t(x >> 1) * 2 * r + bp, x & 1, size_t(r)); },
+                [&](int b, int bp, double2 v) { nxt[size_t(b) * r + bp] = v; });
         }
-        __syncthreads();
-        for (long e = threadIdx.x; e < long(r) * r; e += blockDim.x) {
-            const int b = int(e / r), bp = int(e % r);
-            double2 acc = cmake(0, 0);
-            for (int ap = 0; ap < l; ++ap)
-                for (int s = 0; s < 2; ++s)
-                    cfma(acc, tmp[(size_t(ap) * 2 + s) * r + b],
-                         pauli_conj_row(ch, A + size_t(ap) * 2 * r + bp, s, size_t(r)));
-            nxt[e] = acc;
-        }
-        __syncthreads();
+        return;
     }
-    if (threadIdx.x == 0) vals[t] = EL[size_t(n) * E];
-    for (int q = n - 1; q > 0; --q) {
-        const int l = mps.dl[q], r = mps.dr[q];
-        const double2* A = mps.site[q];
-        const double2* cur = ER + size_t(q) * E;  // r x r
-        double2* nxt = ER + size_t(q - 1) * E;    // l x l
-        const char ch = lab[n - 1 - q];
-        // tmp[a][s][b'] = sum_b A[a, s, b] cur[b][b']
-        for (long e = threadIdx.x; e < long(l) * 2 * r; e += blockDim.x) {
-            const int as = int(e / r), bp = int(e % r);
-            double2 acc = cmake(0, 0);
-            for (int b = 0; b < r; ++b) cfma(acc, A[size_t(as) * r + b], cur[size_t(b) * r + bp]);
-            tmp[e] = acc;
-        }
-        __syncthreads();
-        for (long e = threadIdx.x; e < long(l) * l; e += blockDim.x) {
-            const int a = int(e / l), ap = int(e % l);
-            double2 acc = cmake(0, 0);
-            for (int s = 0; s < 2; ++s)
-                for (int bp = 0; bp < r; ++bp)
-                    cfma(acc, tmp[(size_t(a) * 2 + s) * r + bp],
-                         pauli_conj_row(ch, A + size_t(ap) * 2 * r + bp, s, size_t(r)));
-            nxt[e] = acc;
-        }
-        __syncthreads();
+    if (q == 0) return;
+    const double2* cur = ER + size_t(q) * E;  // r x r
+    double2* nxt = ER + size_t(q - 1) * E;    // l x l
+    if (phase == 0) {  // tmp[a][s][b'] = sum_b A[a, s, b] cur[b][b']
+        if (m0 >= 2 * l || n0 >= r) return;
+        tile_gemm(
+            sm, m0, n0, 2 * l, r, r, true, false, [&](int x, int b) { return A[size_t(x) * r + b]; },
+            [&](int b, int bp) { return first ? cmake(1.0, 0.0) : cur[size_t(b) * r + bp]; },
+            [&](int x, int bp, double2 v) { tmp[size_t(x) * r + bp] = v; });
+    } else {
+        if (m0 >= l || n0 >= l) return;
+        tile_gemm(
+            sm, m0, n0, l, l, 2 * r, true, true, [&](int a, int x) { return tmp[size_t(a) * 2 * r + x]; },
+            [&](int x, int ap) {
+                const int s = x / r, bp = x - s * r;
+                return pauli_conj_row(ch, A + size_t(ap) * 2 * r + bp, s, size_t(r));
+            },
+            [&](int a, int ap, double2 v) { nxt[size_t(a) * l + ap] = v; });
     }
 }
 
-// Holes of site q for the terms of one chunk (grid: sites x terms):
+// Holes of every site for the terms of one chunk (blockIdx.x = term n + site):
 // H[a, s, b] = sum_{a', b'} EL_q[a][a'] At[a', s, b'] ER_q[b][b'], written to
-// holes[(t * n + q) * cap * 2 * cap]; half-products in tmp (same layout).
-__global__ void __launch_bounds__(256) adj_pauli_holes_kernel(DeviceMps mps, const char* labels, int t0, int cap,
-                                                              const double2* envs, double2* tmp_all,
-                                                              double2* holes) {
-    const int q = blockIdx.x, tl = blockIdx.y, t = t0 + tl;
-    const int n = mps.n;
+// holes[(t * n + q) * cap * 2 * cap]; half-products (phase 0) in tmp (same
+// layout).
+__global__ void __launch_bounds__(kTileThreads) adj_pauli_holes_kernel(DeviceMps mps, const char* labels, int t0,
+                                                                       int cap, int phase, const double2* envs,
+                                                                       double2* tmp_all, double2* holes) {
+    __shared__ TileSmem sm;
+    const int n = mps.n, q = blockIdx.x % n, tl = blockIdx.x / n, t = t0 + tl;
     const size_t E = size_t(cap) * cap, S = size_t(cap) * 2 * cap;
     const double2* EL = envs + size_t(t) * (2 * n + 1) * E + size_t(q) * E;
     const double2* ER = envs + size_t(t) * (2 * n + 1) * E + size_t(n + 1 + q) * E;
     double2* tmp = tmp_all + (size_t(tl) * n + q) * S;
     double2* H = holes + (size_t(tl) * n + q) * S;
-    const int l = mps.dl[q], r = mps.dr[q];
+    const int l = mps.dl[q], r = mps.dr[q], m0 = blockIdx.y * kTile, n0 = blockIdx.z * kTile;
     const double2* A = mps.site[q];
     const char ch = labels[size_t(t) * n + (n - 1 - q)];
-    for (long e = threadIdx.x; e < long(l) * 2 * r; e += blockDim.x) {
-        const int a = int(e / (2 * r)), s = int((e / r) % 2), bp = int(e % r);
-        double2 acc = cmake(0, 0);
-        for (int ap = 0; ap < l; ++ap)
-            cfma(acc, EL[size_t(a) * l + ap], pauli_conj_row(ch, A + size_t(ap) * 2 * r + bp, s, size_t(r)));
-        tmp[e] = acc;
-    }
-    __syncthreads();
-    for (long e = threadIdx.x; e < long(l) * 2 * r; e += blockDim.x) {
-        const long as = e / r;
-        const int b = int(e % r);
-        double2 acc = cmake(0, 0);
-        for (int bp = 0; bp < r; ++bp) cfma(acc, tmp[as * r + bp], ER[size_t(b) * r + bp]);
-        H[e] = acc;
+    if (phase == 0) {
+        if (m0 >= l || n0 >= 2 * r) return;
+        tile_gemm(
+            sm, m0, n0, l, 2 * r, l, true, false, [&](int a, int ap) { return EL[size_t(a) * l + ap]; },
+            [&](int ap, int x) {
+                const int s = x / r, bp = x - s * r;
+                return pauli_conj_row(ch, A + size_t(ap) * 2 * r + bp, s, size_t(r));
+            },
+            [&](int a, int x, double2 v) { tmp[size_t(a) * 2 * r + x] = v; });
+    } else {
+        if (m0 >= 2 * l || n0 >= r) return;
+        tile_gemm(
+            sm, m0, n0, 2 * l, r, r, true, true, [&](int x, int bp) { return tmp[size_t(x) * r + bp]; },
+            [&](int bp, int b) { return ER[size_t(b) * r + bp]; },
+            [&](int x, int b, double2 v) { H[size_t(x) * r + b] = v; });
     }
 }
 
@@ -265,7 +262,7 @@ __device__ __forceinline__ double2 zat(const ZView& v, int i, int k) {
 
 constexpr int kAdjT = 32, kAdjK = 16;
 
-__global__ void __launch_bounds__(256) adj_split_gemm_kernel(AdjSplit A, int stage) {
+__global__ void __launch_bounds__(kTileThreads) adj_split_gemm_kernel(AdjSplit A, int stage) {
     const SplitState S = *A.st;
     const int m = S.rows, n = S.cols, N = min(m, n), R = A.R, kin = S.k;
     ZView a, b;
@@ -309,42 +306,17 @@ __global__ void __launch_bounds__(256) adj_split_gemm_kernel(AdjSplit A, int sta
             a = {A.site_l, 1, kin, 1}; b = {A.tb0, 1, R, 0}; c = A.bar_r; crs = n; ccs = 1; M_ = kin; N_ = n; K_ = m;
             break;
     }
-    const int i0 = blockIdx.y * kAdjT, j0 = blockIdx.x * kAdjT;
+    const int i0 = blockIdx.y * kTile, j0 = blockIdx.x * kTile;
     if (i0 >= M_ || j0 >= N_) return;
-    __shared__ double2 As[kAdjT][kAdjK + 1];
-    __shared__ double2 Bs[kAdjK][kAdjT + 1];
-    const int tid = threadIdx.x, tr = tid / 16, tc = tid % 16;
-    double2 accv[2][2] = {{cmake(0, 0), cmake(0, 0)}, {cmake(0, 0), cmake(0, 0)}};
-    for (int k0 = 0; k0 < K_; k0 += kAdjK) {
-        for (int e = tid; e < kAdjT * kAdjK; e += 256) {
-            const int r = e / kAdjK, cc = e % kAdjK;
-            As[r][cc] = (i0 + r < M_ && k0 + cc < K_) ? zat(a, i0 + r, k0 + cc) : cmake(0, 0);
-        }
-        for (int e = tid; e < kAdjK * kAdjT; e += 256) {
-            const int r = e / kAdjT, cc = e % kAdjT;
-            Bs[r][cc] = (k0 + r < K_ && j0 + cc < N_) ? zat(b, k0 + r, j0 + cc) : cmake(0, 0);
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int cc = 0; cc < kAdjK; ++cc) {
-            const double2 a0 = As[tr][cc], a1 = As[tr + 16][cc];
-            const double2 b0 = Bs[cc][tc], b1 = Bs[cc][tc + 16];
-            cfma(accv[0][0], a0, b0);
-            cfma(accv[0][1], a0, b1);
-            cfma(accv[1][0], a1, b0);
-            cfma(accv[1][1], a1, b1);
-        }
-        __syncthreads();
-    }
-    for (int x = 0; x < 2; ++x)
-        for (int y = 0; y < 2; ++y) {
-            const int i = i0 + tr + 16 * x, j = j0 + tc + 16 * y;
-            if (i >= M_ || j >= N_) continue;
-            double2 v = accv[x][y];
+    __shared__ TileSmem sm;
+    tile_gemm(
+        sm, i0, j0, M_, N_, K_, a.cs == 1, b.rs == 1, [&](int i, int k) { return zat(a, i, k); },
+        [&](int k, int j) { return zat(b, k, j); },
+        [&](int i, int j, double2 v) {
             if (cscale_by) v = cscale(v, cscale_by[j]);
             double2* dst = c + i * crs + j * ccs;
             *dst = acc ? cadd(*dst, v) : v;
-        }
+        });
 }
 
 // Stage 3 (grid-stride over R x R): s_bar, then Z, T1 = U_bar s^-1 (= Q1)

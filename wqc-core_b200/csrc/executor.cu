@@ -25,6 +25,7 @@
 #include "common.cuh"
 #include "split_kernels.cuh"
 #include "tc_gemm.cuh"
+#include "tile_gemm.cuh"
 
 using namespace wqc;
 
@@ -2575,18 +2576,25 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
         const size_t E = size_t(chi) * chi;
         char* d_lab = nullptr;
         double* d_cre = nullptr;
-        double2 *envs = nullptr, *tmp = nullptr, *vals = nullptr;
+        double2 *envs = nullptr, *tmp = nullptr;
         if (wqc_status st = buf.get(&d_lab, size_t(nterms) * n + 16)) return st;
         if (wqc_status st = buf.get(&d_cre, nterms)) return st;
         if (wqc_status st = buf.get(&envs, size_t(nterms) * (2 * n + 1) * E)) return st;
-        if (wqc_status st = buf.get(&tmp, size_t(nterms) * 2 * E)) return st;
-        if (wqc_status st = buf.get(&vals, nterms)) return st;
+        if (wqc_status st = buf.get(&tmp, size_t(nterms) * 4 * E)) return st;
         std::vector<double> cre(nterms);
         for (uint32_t t = 0; t < nterms; ++t) cre[t] = coeffs[2 * t];
         CUDA_TRY(cudaMemcpyAsync(d_lab, labels, size_t(nterms) * n, cudaMemcpyHostToDevice, m->stream));
         CUDA_TRY(cudaMemcpyAsync(d_cre, cre.data(), nterms * sizeof(double), cudaMemcpyHostToDevice, m->stream));
-        adj_pauli_envs_kernel<<<nterms, 256, 0, m->stream>>>(m->dev, d_lab, int(nterms), chi, envs, tmp, vals);
-        count_launch(m, -1);
+        int bond = 1;
+        for (int b : m->ub) bond = std::max(bond, b);
+        const unsigned b1 = unsigned(bond + kTile - 1) / kTile, b2 = unsigned(2 * bond + kTile - 1) / kTile;
+        for (int step = 0; step < n; ++step)
+            for (int phase = 0; phase < 2; ++phase) {
+                const unsigned t = phase == 0 ? b2 : b1;
+                adj_pauli_envs_kernel<<<dim3(2 * nterms, t, t), kTileThreads, 0, m->stream>>>(m->dev, d_lab, chi, step,
+                                                                                              phase, envs, tmp);
+                count_launch(m, -1);
+            }
         // Holes in chunks of terms, accumulated in term order.
         const size_t per_term = 2 * size_t(n) * site_cap * sizeof(double2);
         const int chunk = int(std::max<size_t>(1, std::min<size_t>(16, (size_t(1) << 30) / per_term)));
@@ -2596,7 +2604,11 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
         const int agrid = int(std::max<size_t>(1, std::min<size_t>((site_cap + 255) / 256, 64)));
         for (uint32_t t0 = 0; t0 < nterms; t0 += uint32_t(chunk)) {
             const int cnt = int(std::min<uint32_t>(uint32_t(chunk), nterms - t0));
-            adj_pauli_holes_kernel<<<dim3(n, cnt), 256, 0, m->stream>>>(m->dev, d_lab, int(t0), chi, envs, htmp, holes);
+            adj_pauli_holes_kernel<<<dim3(n * cnt, b1, b2), kTileThreads, 0, m->stream>>>(m->dev, d_lab, int(t0), chi, 0,
+                                                                                          envs, htmp, holes);
+            adj_pauli_holes_kernel<<<dim3(n * cnt, b2, b1), kTileThreads, 0, m->stream>>>(m->dev, d_lab, int(t0), chi, 1,
+                                                                                          envs, htmp, holes);
+            count_launch(m, -1);
             adj_pauli_accumulate_kernel<<<dim3(agrid, n), 256, 0, m->stream>>>(m->dev, d_bars, holes, d_cre, int(t0),
                                                                              cnt, chi, t0 == 0 ? 1 : 0);
             count_launch(m, -1);
@@ -2604,7 +2616,9 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
         }
         CUDA_TRY(cudaGetLastError());
         std::vector<double2> hv(nterms);
-        CUDA_TRY(cudaMemcpyAsync(hv.data(), vals, nterms * sizeof(double2), cudaMemcpyDeviceToHost, m->stream));
+        // <psi|P_t|psi>: the first entry of every term's last left environment.
+        CUDA_TRY(cudaMemcpy2DAsync(hv.data(), sizeof(double2), envs + size_t(n) * E, (2 * size_t(n) + 1) * E * sizeof(double2),
+                                   sizeof(double2), nterms, cudaMemcpyDeviceToHost, m->stream));
         CUDA_TRY(cudaStreamSynchronize(m->stream));
         double re = 0, im = 0;
         for (uint32_t t = 0; t < nterms; ++t) {  // coeff * Re<P> (expectation.rs:177-185), term order
@@ -2656,7 +2670,7 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
             if (!o.two) slot_gate.push_back(o.gate);
     }
     const int eg = int(std::min<long>((long(R) * R + 255) / 256, 4L * m->ctx->sm_count));
-    const dim3 gg((R + 31) / 32, (R + 31) / 32);
+    const dim3 gg((R + kTile - 1) / kTile, (R + kTile - 1) / kTile);
     for (size_t sgi = a->starts.size(); sgi-- > 0;) {
         const uint32_t g0 = a->starts[sgi];
         const uint32_t g1 = sgi + 1 < a->starts.size() ? a->starts[sgi + 1] : uint32_t(a->gates.size());
@@ -2755,16 +2769,16 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
             A.sq = wsd + R;
             A.R = R;
             adj_split_prep_kernel<<<eg, 256, 0, m->stream>>>(A);
-            adj_split_gemm_kernel<<<gg, 256, 0, m->stream>>>(A, kAdjStageOther);
-            adj_split_gemm_kernel<<<gg, 256, 0, m->stream>>>(A, kAdjStageM);
-            adj_split_gemm_kernel<<<gg, 256, 0, m->stream>>>(A, kAdjStageN);
+            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageOther);
+            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageM);
+            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageN);
             adj_split_assemble_kernel<<<eg, 256, 0, m->stream>>>(A);
-            adj_split_gemm_kernel<<<gg, 256, 0, m->stream>>>(A, kAdjStageT1);
-            adj_split_gemm_kernel<<<gg, 256, 0, m->stream>>>(A, kAdjStageTb);
-            adj_split_gemm_kernel<<<gg, 256, 0, m->stream>>>(A, kAdjStageTb2);
+            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageT1);
+            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageTb);
+            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageTb2);
             adj_split_gate_kernel<<<eg, 256, 0, m->stream>>>(A);
-            adj_split_gemm_kernel<<<gg, 256, 0, m->stream>>>(A, kAdjStageBarL);
-            adj_split_gemm_kernel<<<gg, 256, 0, m->stream>>>(A, kAdjStageBarR);
+            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageBarL);
+            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageBarR);
             for (int c = 0; c < 11; ++c) count_launch(m, -1);
         }
         CUDA_TRY(cudaGetLastError());

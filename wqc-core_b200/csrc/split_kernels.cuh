@@ -201,10 +201,10 @@ struct AdjSplit {
 };
 enum { kAdjStageOther = 0, kAdjStageM, kAdjStageN, kAdjStageT1, kAdjStageTb, kAdjStageTb2, kAdjStageBarL,
        kAdjStageBarR };
-__global__ void adj_pauli_envs_kernel(DeviceMps mps, const char* labels, int nterms, int cap, double2* envs,
-                                      double2* tmp_all, double2* vals);
-__global__ void adj_pauli_holes_kernel(DeviceMps mps, const char* labels, int t0, int cap, const double2* envs,
-                                       double2* tmp_all, double2* holes);
+__global__ void adj_pauli_envs_kernel(DeviceMps mps, const char* labels, int cap, int step, int phase, double2* envs,
+                                      double2* tmp_all);
+__global__ void adj_pauli_holes_kernel(DeviceMps mps, const char* labels, int t0, int cap, int phase,
+                                       const double2* envs, double2* tmp_all, double2* holes);
 __global__ void adj_pauli_accumulate_kernel(DeviceMps mps, double2* const* bars, const double2* holes,
                                             const double* coef_re, int t0, int count, int cap, int first);
 __global__ void adj_one_qubit_kernel(double2* bar, const double2* before, const int* dims, Adj1q g, double* grad);
