@@ -115,3 +115,36 @@ def test_config3_adjoint_against_differences_and_shift(cuda_ctx):
     # the shift rule applied to truncated evaluations is not the truncated
     # map's derivative; at chi 64 they differ by the truncation's effect
     assert np.abs(grad[params] - fx["shift_grad"]).max() <= 1e-3
+
+
+@pytest.mark.parametrize("n,every", [(16, 0), (17, 1)])
+def test_adjoint_of_wide_steps_at_two_capacities(cuda_ctx, n, every):
+    """Layers of n // 2 disjoint splits: at chi 256 a step's reverse runs in
+    several parts (six workspaces fit), at chi 32 in one.  Nothing is truncated,
+    so both are the derivative of the same map, to the bar of the comparison
+    with the numpy sweep; and so is the parameter-shift value of one angle."""
+    rng = np.random.default_rng(n)
+    g = []
+    for layer in range(4):
+        for q in range(n):
+            g.append(C.g1((C.RX, C.RY)[(q + layer) % 2], q, rng.uniform(0.3, 2.8)))
+        for q in range(layer % 2, n - 1, 2):
+            g.append(C.g2(C.CNOT if (q + layer) % 3 else C.CZ, q, q + 1))
+    gates = C.gates_array(g)
+    labels, coeffs = C.zz_x_observable(n)
+    cps = [len(g) // 2] if every else []
+    got = []
+    for chi in (32, 256):
+        m = W.CudaMps(n, chi, ctx=cuda_ctx)
+        got.append(W.Adjoint(m, gates, cps).backward(labels, coeffs))
+        m.close()
+    (f0, g0), (f1, g1) = got
+    assert abs(f0 - f1) <= 1e-11 * max(1.0, abs(f0))
+    assert np.abs(g0 - g1).max() <= 1e-9 * max(1.0, np.abs(g0).max())
+    i = n // 2
+    shift = []
+    for d in (np.pi / 2, -np.pi / 2):
+        gp = gates.copy()
+        gp["angle"][i] += d
+        shift.append(device_value(n, 32, gp, labels, coeffs, cuda_ctx))
+    assert abs(g1[i] - 0.5 * (shift[0] - shift[1])) <= 1e-9 * max(1.0, np.abs(g0).max())

@@ -57,8 +57,9 @@ __device__ __forceinline__ double2 pauli_conj_row(char ch, const double2* a, int
 // One half of one step for every term and both directions: blockIdx.x = 2 t +
 // direction, the left environments at site `step`, the right ones at the
 // mirrored site.  phase 0 multiplies the environment into the site, phase 1
-// closes it.  (As one CTA per term that walked all sites, 63 terms on 32 sites
-// at chi 64 took 25.6 ms, which was the walk's latency.)
+// closes it.  The walk is a chain of n steps, so what bounds it is the latency of
+// a step: 63 terms on 32 sites at chi 64 took 25.6 ms with one CTA per term, and
+// take 2 ms with one CTA per tile of a step's products.
 __global__ void __launch_bounds__(kTileThreads) adj_pauli_envs_kernel(DeviceMps mps, const char* labels, int cap,
                                                                       int step, int phase, double2* envs,
                                                                       double2* tmp_all) {
@@ -170,12 +171,14 @@ __global__ void __launch_bounds__(256) adj_pauli_accumulate_kernel(DeviceMps mps
     }
 }
 
-// Reverse of a one-qubit gate A' = u A at a site of shape dims[0] x 2 x
-// dims[1] (one CTA): grad[slot] = Re <bar, du A_before> when du is given
-// (a rotation angle), then bar <- u^H bar.
-__global__ void __launch_bounds__(256) adj_one_qubit_kernel(double2* bar, const double2* before, const int* dims,
-                                                            Adj1q g, double* grad) {
-    const int l = dims[0], r = dims[1];
+// Reverse of one-qubit gates A' = u A at sites of shape dims[0] x 2 x dims[1],
+// one CTA a gate: grad[slot] = Re <bar, du A_before> when du is given (a
+// rotation angle), then bar <- u^H bar.
+__global__ void __launch_bounds__(256) adj_one_qubit_kernel(const Adj1q* gates, double* grad) {
+    const Adj1q g = gates[blockIdx.x];
+    double2* bar = g.bar;
+    const double2* before = g.before;
+    const int l = g.dims[0], r = g.dims[1];
     __shared__ double red[8];
     double part = 0;
     for (long e = threadIdx.x; e < long(l) * r; e += blockDim.x) {
@@ -204,8 +207,57 @@ __global__ void __launch_bounds__(256) adj_one_qubit_kernel(double2* bar, const 
     }
 }
 
+// ----- the tape -----------------------------------------------------------
+// A step's operations touch disjoint sites and are taped together: blockIdx.x
+// is the operation, blockIdx.y a part of its data.  Only the entries that the
+// shapes on the device call for are copied (copying every site and matrix at
+// its capacity, one copy a part, took 15 copies a split).
+__device__ __forceinline__ void adj_copy(double2* dst, const double2* src, long count) {
+    for (long e = long(blockIdx.y) * blockDim.x + threadIdx.x; e < count; e += long(gridDim.y) * blockDim.x)
+        dst[e] = src[e];
+}
+
+// Before the step: the site (two: both sites) of every operation; a one-qubit
+// gate's bonds.
+__global__ void __launch_bounds__(256) adj_tape_before_kernel(DeviceMps mps, const AdjTape* ops, AdjTapeLayout L,
+                                                              int two) {
+    const AdjTape t = ops[blockIdx.x];
+    for (int h = 0; h < 1 + two; ++h) {
+        const int q = t.site + h;
+        adj_copy(reinterpret_cast<double2*>(t.base + h * L.site_b), mps.site[q], 2L * mps.dl[q] * mps.dr[q]);
+    }
+    if (!two && blockIdx.y == 0 && threadIdx.x == 0) {
+        int* dims = reinterpret_cast<int*>(t.base + L.site_b);
+        dims[0] = mps.dl[t.site];
+        dims[1] = mps.dr[t.site];
+    }
+}
+
+// After it: what the split in slot blockIdx.x leaves there.  A split that was
+// cancelled leaves an empty state, which the reverse passes over.
+__global__ void __launch_bounds__(256) adj_tape_after_kernel(const SplitState* states, const SlotBuffers* slots,
+                                                             const AdjTape* ops, AdjTapeLayout L) {
+    const AdjTape t = ops[blockIdx.x];
+    const SlotBuffers B = slots[blockIdx.x];
+    SplitState S = states[blockIdx.x];
+    if (S.skip) S.dl = S.dr = S.k = S.rows = S.cols = S.chi = 0;
+    const long N = min(S.rows, S.cols), M = S.w_rows_of_src ? S.cols : S.rows;
+    adj_copy(reinterpret_cast<double2*>(t.base + L.theta_off), B.theta, long(S.rows) * S.cols);
+    adj_copy(reinterpret_cast<double2*>(t.base + L.w_off), B.w, M * N);
+    if (blockIdx.y != 0) return;
+    double* sigma = reinterpret_cast<double*>(t.base + L.sigma_off);
+    int* perm = reinterpret_cast<int*>(t.base + L.perm_off);
+    for (int i = threadIdx.x; i < N; i += blockDim.x) {
+        sigma[i] = B.sigma[i];
+        perm[i] = B.perm[i];
+    }
+    if (threadIdx.x == 0) *reinterpret_cast<SplitState*>(t.base + L.state_off) = S;
+}
+
 // ----- reverse of a split -------------------------------------------------
 // Workspace matrices are column-major with leading dimension R (= 2 chi_max).
+// The last grid dimension is the split: a step's splits go through each stage
+// together.
 __device__ __forceinline__ int adj_active(const AdjSplit& A, int i, double smax) {
     return A.sigma[A.perm[i]] > kAdjNullRel * smax;
 }
@@ -214,7 +266,8 @@ __device__ __forceinline__ int adj_active(const AdjSplit& A, int i, double smax)
 // theta, V for theta^H), scaled to unit columns and sorted by descending
 // singular value; s^-1 and sqrt(s); U_bar = L_bar sqrt(s) and V_bar =
 // R_bar^H sqrt(s) over the kept columns (zero elsewhere).
-__global__ void __launch_bounds__(256) adj_split_prep_kernel(AdjSplit A) {
+__global__ void __launch_bounds__(256) adj_split_prep_kernel(const AdjSplit* splits) {
+    const AdjSplit A = splits[blockIdx.y];
     const SplitState S = *A.st;
     const int m = S.rows, n = S.cols, N = min(m, n), k = S.chi, R = A.R;
     const int M = S.w_rows_of_src ? n : m;  // entries of a column of W
@@ -242,8 +295,8 @@ __global__ void __launch_bounds__(256) adj_split_prep_kernel(AdjSplit A) {
     }
 }
 
-// The split's GEMMs as 32 x 32 FP64 tiles over strided, optionally
-// conjugated views, with the dimensions read from the tape's SplitState.
+// The split's GEMMs as FP64 tiles (tile_gemm.cuh; 32 x 32 tiles put a 128 x 128
+// product on 16 CTAs and took 8.8 us) over strided, optionally conjugated views, with the dimensions read from the tape's SplitState.
 // Stages (kAdjStage*): Other, the side W does not hold (V = theta^H U s^-1,
 // or U = theta V s^-1); M = U^H U_bar; N = V^H V_bar; T1 += U Z;
 // theta_bar = T1 V^H; theta_bar += U Q2^H; the cotangent of site p,
@@ -260,9 +313,8 @@ __device__ __forceinline__ double2 zat(const ZView& v, int i, int k) {
     return v.conj ? cconj(x) : x;
 }
 
-constexpr int kAdjT = 32, kAdjK = 16;
-
-__global__ void __launch_bounds__(kTileThreads) adj_split_gemm_kernel(AdjSplit A, int stage) {
+__global__ void __launch_bounds__(kTileThreads) adj_split_gemm_kernel(const AdjSplit* splits, int stage) {
+    const AdjSplit A = splits[blockIdx.z];
     const SplitState S = *A.st;
     const int m = S.rows, n = S.cols, N = min(m, n), R = A.R, kin = S.k;
     ZView a, b;
@@ -323,7 +375,8 @@ __global__ void __launch_bounds__(kTileThreads) adj_split_gemm_kernel(AdjSplit A
 // and V_bar <- V_bar s^-1 (= Q2).  s_bar_i = (Re(U_i^H L_bar_i) +
 // Re(R_bar_i V_i)) / (2 sqrt(s_i)) = Re(M_ii + N_ii) / (2 s_i) since
 // U_bar_i = L_bar_i sqrt(s_i) and V_bar_i = R_bar_i^H sqrt(s_i).
-__global__ void __launch_bounds__(256) adj_split_assemble_kernel(AdjSplit A) {
+__global__ void __launch_bounds__(256) adj_split_assemble_kernel(const AdjSplit* splits) {
+    const AdjSplit A = splits[blockIdx.y];
     const SplitState S = *A.st;
     const int m = S.rows, n = S.cols, N = min(m, n), k = S.chi, R = A.R;
     const double smax = N > 0 ? A.sigma[A.perm[0]] : 0.0;
@@ -365,7 +418,8 @@ __global__ void __launch_bounds__(256) adj_split_assemble_kernel(AdjSplit A) {
 
 // Stage 5: the gate's reverse, theta_bar0[(a, si, ti, b)] = sum_{so, to}
 // conj(u[(so, to), (si, ti)]) theta_bar[(a, so, to, b)].
-__global__ void __launch_bounds__(256) adj_split_gate_kernel(AdjSplit A) {
+__global__ void __launch_bounds__(256) adj_split_gate_kernel(const AdjSplit* splits) {
+    const AdjSplit A = splits[blockIdx.y];
     const SplitState S = *A.st;
     const int dl = S.dl, dr = S.dr, R = A.R;
     const long stride = long(gridDim.x) * blockDim.x;

@@ -2478,14 +2478,39 @@ struct AdjBuffers {
     }
 };
 
-// One recomputed operation on the tape.
-struct TapeEntry {
+// Operations of a segment that touch disjoint sites and are of one kind: they
+// are recomputed, taped and reversed together.  A segment is a chain of steps
+// and each is bound by the latency of one split, so what counts is how many
+// there are: the 32-qubit ansatz, 6 layers at chi 64 with a checkpoint every 2
+// (ladders, so two splits a step at most), took 52 ms one operation at a time
+// and takes 31.
+struct AdjStep {
     bool two;
-    int site;
-    int gate;
-    double2 u[16];
-    size_t off;  // byte offset of its data in the tape arena
+    std::vector<size_t> ops;  // indices into the segment's operations
 };
+
+// An operation goes into the first step of its kind after the last one on its
+// sites; at most `most` splits a step (each has a slot of its own).
+std::vector<AdjStep> adj_steps(int n, const std::vector<Op>& ops, size_t most) {
+    std::vector<AdjStep> steps, out;
+    std::vector<size_t> next(n, 0);  // first step that a site is free in; odd steps hold splits
+    for (size_t i = 0; i < ops.size(); ++i) {
+        const Op& o = ops[i];
+        size_t t = o.two ? std::max(next[o.site], next[o.site + 1]) : next[o.site];
+        if ((t & 1) != size_t(o.two)) ++t;
+        while (steps.size() <= t) steps.push_back({(steps.size() & 1) != 0, {}});
+        steps[t].ops.push_back(i);
+        next[o.site] = t + 1;
+        if (o.two) next[o.site + 1] = t + 1;
+    }
+    for (const AdjStep& s : steps)
+        for (size_t i = 0; i < s.ops.size();) {
+            const size_t cnt = std::min(s.ops.size() - i, s.two ? most : s.ops.size());
+            out.push_back({s.two, std::vector<size_t>(s.ops.begin() + long(i), s.ops.begin() + long(i + cnt))});
+            i += cnt;
+        }
+    return out;
+}
 
 }  // namespace
 
@@ -2641,19 +2666,29 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
     if (wqc_status st = buf.get(&d_grad, n1q + 1)) return st;
     CUDA_TRY(cudaMemsetAsync(d_grad, 0, (n1q + 1) * sizeof(double), m->stream));
     std::vector<int> slot_gate;  // gate of each gradient slot
-    // Split workspace (column-major R x R matrices) and the slot-0 buffers.
-    double2* ws = nullptr;
-    double* wsd = nullptr;
-    if (wqc_status st = buf.get(&ws, 10 * size_t(R) * R)) return st;
-    if (wqc_status st = buf.get(&wsd, 2 * size_t(R))) return st;
-    SlotBuffers slot0;
-    CUDA_TRY(cudaMemcpy(&slot0, m->d_slots, sizeof(slot0), cudaMemcpyDeviceToHost));
+    // Split workspaces (ten column-major R x R matrices each), for as many
+    // splits of a step at a time as fit 256 MiB, or else the device: a circuit
+    // of ladders has about half a segment's layers in a step.
+    const size_t RR = size_t(R) * R, ws_b = (10 * RR) * sizeof(double2) + 2 * size_t(R) * sizeof(double);
+    const size_t most = size_t(std::min(m->bucket_cap[0], 32768));
+    char* ws = nullptr;
+    size_t width = std::max<size_t>(1, std::min(most, (size_t(256) << 20) / ws_b));
+    for (;; width /= 2) {
+        const wqc_status st = buf.get(&ws, width * ws_b);
+        if (st == WQC_OK) break;
+        if (width == 1) return st;
+    }
     // Tape layout of one operation (bytes, 256-aligned parts).
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t site_b = al(site_cap * sizeof(double2));
-    const size_t mat_b = al(size_t(R) * R * sizeof(double2));
-    const size_t one_b = site_b + al(2 * sizeof(int));
-    const size_t two_b = 2 * site_b + 2 * mat_b + al(R * sizeof(double)) + al(R * sizeof(int)) + al(sizeof(SplitState));
+    AdjTapeLayout L{};
+    L.site_b = al(site_cap * sizeof(double2));
+    L.theta_off = 2 * L.site_b;
+    L.w_off = L.theta_off + al(RR * sizeof(double2));
+    L.sigma_off = L.w_off + al(RR * sizeof(double2));
+    L.perm_off = L.sigma_off + al(R * sizeof(double));
+    L.state_off = L.perm_off + al(R * sizeof(int));
+    const size_t one_b = L.site_b + al(2 * sizeof(int));
+    const size_t two_b = L.state_off + al(sizeof(SplitState));
     char* tape = nullptr;
     size_t tape_cap = 0;
     // First gradient slot of each segment (one-qubit operations in program order).
@@ -2670,116 +2705,132 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
             if (!o.two) slot_gate.push_back(o.gate);
     }
     const int eg = int(std::min<long>((long(R) * R + 255) / 256, 4L * m->ctx->sm_count));
-    const dim3 gg((R + kTile - 1) / kTile, (R + kTile - 1) / kTile);
     for (size_t sgi = a->starts.size(); sgi-- > 0;) {
         const uint32_t g0 = a->starts[sgi];
         const uint32_t g1 = sgi + 1 < a->starts.size() ? a->starts[sgi + 1] : uint32_t(a->gates.size());
         if (g1 <= g0) continue;
         Expander ex;
         if (wqc_status st = expand(n, a->gates.data() + g0, g1 - g0, false, ex)) return st;
-        std::vector<TapeEntry> ents;
-        size_t need = 0;
+        // The tape: every operation's data, then the steps' descriptors.
+        const std::vector<AdjStep> steps = adj_steps(n, ex.ops, most);
+        size_t nops[2] = {0, 0}, data_b = 0;
         for (const Op& o : ex.ops) {
-            TapeEntry t{};
-            t.two = o.two;
-            t.site = o.site;
-            t.gate = o.gate + int(g0);
-            if (o.two)
-                std::memcpy(t.u, o.ueff, sizeof(t.u));
-            else
-                std::memcpy(t.u, o.m2.u, sizeof(o.m2.u));
-            t.off = need;
-            need += o.two ? two_b : one_b;
-            ents.push_back(t);
+            ++nops[o.two];
+            data_b += o.two ? two_b : one_b;
         }
+        const size_t tape_off = data_b, split_off = tape_off + al(ex.ops.size() * sizeof(AdjTape));
+        const size_t one_off = split_off + al(nops[1] * sizeof(AdjSplit));
+        const size_t need = one_off + al(nops[0] * sizeof(Adj1q));
         if (need > tape_cap) {
             if (tape) buf.release(tape);
             tape = nullptr;
             if (wqc_status st = buf.get(&tape, need)) return st;
             tape_cap = need;
         }
-        // Recompute the segment one operation at a time, taping each one's inputs.
+        std::vector<size_t> slot_of(ex.ops.size());
+        for (size_t i = 0, sl = seg_slot0[sgi]; i < ex.ops.size(); ++i) slot_of[i] = ex.ops[i].two ? 0 : sl++;
+        std::vector<AdjTape> tapes;
+        std::vector<AdjSplit> splits;
+        std::vector<Adj1q> ones;
+        char* base = tape;
+        for (const AdjStep& s : steps)
+            for (size_t i = 0; i < s.ops.size(); ++i) {
+                const Op& o = ex.ops[s.ops[i]];
+                tapes.push_back({base, o.site});
+                if (!o.two) {
+                    Adj1q g{};
+                    std::memcpy(g.u, o.m2.u, sizeof(g.u));
+                    g.has_du = rotation_derivative(a->gates[o.gate + int(g0)], g.du) ? 1 : 0;
+                    g.slot = int(slot_of[s.ops[i]]);
+                    g.bar = bars[o.site];
+                    g.before = reinterpret_cast<const double2*>(base);
+                    g.dims = reinterpret_cast<const int*>(base + L.site_b);
+                    ones.push_back(g);
+                    base += one_b;
+                    continue;
+                }
+                AdjSplit A{};
+                A.site_l = reinterpret_cast<const double2*>(base);
+                A.site_r = reinterpret_cast<const double2*>(base + L.site_b);
+                A.theta = reinterpret_cast<const double2*>(base + L.theta_off);
+                A.w = reinterpret_cast<const double2*>(base + L.w_off);
+                A.sigma = reinterpret_cast<const double*>(base + L.sigma_off);
+                A.perm = reinterpret_cast<const int*>(base + L.perm_off);
+                A.st = reinterpret_cast<const SplitState*>(base + L.state_off);
+                A.bar_l = bars[o.site];
+                A.bar_r = bars[o.site + 1];
+                std::memcpy(A.u, o.ueff, sizeof(A.u));
+                double2* w = reinterpret_cast<double2*>(ws + (i % width) * ws_b);
+                A.U = w; A.V = w + RR; A.Ub = w + 2 * RR; A.Vb = w + 3 * RR; A.M = w + 4 * RR; A.Nm = w + 5 * RR;
+                A.Z = w + 6 * RR; A.T1 = w + 7 * RR; A.tb = w + 8 * RR; A.tb0 = w + 9 * RR;
+                A.inv = reinterpret_cast<double*>(w + 10 * RR);
+                A.sq = A.inv + R;
+                A.R = R;
+                splits.push_back(A);
+                base += two_b;
+            }
+        const AdjTape* d_tapes = reinterpret_cast<const AdjTape*>(tape + tape_off);
+        const AdjSplit* d_splits = reinterpret_cast<const AdjSplit*>(tape + split_off);
+        const Adj1q* d_ones = reinterpret_cast<const Adj1q*>(tape + one_off);
+        CUDA_TRY(cudaMemcpyAsync(tape + tape_off, tapes.data(), tapes.size() * sizeof(AdjTape), cudaMemcpyHostToDevice,
+                                 m->stream));
+        CUDA_TRY(cudaMemcpyAsync(tape + split_off, splits.data(), splits.size() * sizeof(AdjSplit),
+                                 cudaMemcpyHostToDevice, m->stream));
+        CUDA_TRY(cudaMemcpyAsync(tape + one_off, ones.data(), ones.size() * sizeof(Adj1q), cudaMemcpyHostToDevice,
+                                 m->stream));
+        // Recompute the segment step by step, taping each one's inputs.
         if (wqc_status st = adj_restore(a, sgi)) return st;
-        for (size_t k = 0; k < ex.ops.size(); ++k) {
-            const Op& o = ex.ops[k];
-            char* base = tape + ents[k].off;
-            if (!o.two) {
-                CUDA_TRY(cudaMemcpyAsync(base, m->site_ptr[o.site], site_cap * sizeof(double2),
-                                         cudaMemcpyDeviceToDevice, m->stream));
-                CUDA_TRY(cudaMemcpyAsync(base + site_b, m->d_dl + o.site, sizeof(int), cudaMemcpyDeviceToDevice,
-                                         m->stream));
-                CUDA_TRY(cudaMemcpyAsync(base + site_b + sizeof(int), m->d_dr + o.site, sizeof(int),
-                                         cudaMemcpyDeviceToDevice, m->stream));
-            } else {
-                CUDA_TRY(cudaMemcpyAsync(base, m->site_ptr[o.site], site_cap * sizeof(double2),
-                                         cudaMemcpyDeviceToDevice, m->stream));
-                CUDA_TRY(cudaMemcpyAsync(base + site_b, m->site_ptr[o.site + 1], site_cap * sizeof(double2),
-                                         cudaMemcpyDeviceToDevice, m->stream));
+        std::vector<Op> step_ops;
+        size_t first = 0;
+        for (const AdjStep& s : steps) {
+            step_ops.clear();
+            int bond = 1;
+            for (size_t i : s.ops) {
+                const Op& o = ex.ops[i];
+                step_ops.push_back(o);
+                bond = std::max(std::max(bond, m->left_bond(o.site)), m->right_bond(o.site));
+                if (o.two) bond = std::max(bond, m->right_bond(o.site + 1));
             }
-            std::vector<Op> one{o};
-            if (wqc_status st = run_ops(m, one)) return st;
-            if (o.two) {
-                char* p = base + 2 * site_b;
-                CUDA_TRY(cudaMemcpyAsync(p, slot0.theta, size_t(R) * R * sizeof(double2), cudaMemcpyDeviceToDevice,
-                                         m->stream));
-                CUDA_TRY(cudaMemcpyAsync(p + mat_b, slot0.w, size_t(R) * R * sizeof(double2),
-                                         cudaMemcpyDeviceToDevice, m->stream));
-                CUDA_TRY(cudaMemcpyAsync(p + 2 * mat_b, slot0.sigma, R * sizeof(double), cudaMemcpyDeviceToDevice,
-                                         m->stream));
-                CUDA_TRY(cudaMemcpyAsync(p + 2 * mat_b + al(R * sizeof(double)), slot0.perm, R * sizeof(int),
-                                         cudaMemcpyDeviceToDevice, m->stream));
-                CUDA_TRY(cudaMemcpyAsync(p + 2 * mat_b + al(R * sizeof(double)) + al(R * sizeof(int)), m->d_state,
-                                         sizeof(SplitState), cudaMemcpyDeviceToDevice, m->stream));
+            const unsigned cnt = unsigned(s.ops.size());
+            auto parts = [&](long entries) { return unsigned(std::max(1L, std::min(16L, entries / 1024))); };
+            adj_tape_before_kernel<<<dim3(cnt, parts(2L * bond * bond)), 256, 0, m->stream>>>(m->dev, d_tapes + first, L,
+                                                                                            s.two ? 1 : 0);
+            count_launch(m, -1);
+            if (wqc_status st = run_ops(m, step_ops)) return st;
+            if (s.two) {
+                adj_tape_after_kernel<<<dim3(cnt, parts(4L * bond * bond)), 256, 0, m->stream>>>(m->d_state, m->d_slots,
+                                                                                               d_tapes + first, L);
+                count_launch(m, -1);
             }
+            first += s.ops.size();
         }
         // Reverse sweep over the segment.
-        size_t slot = seg_slot0[sgi];
-        for (const TapeEntry& t : ents) slot += t.two ? 0 : 1;
-        for (size_t k = ents.size(); k-- > 0;) {
-            const TapeEntry& t = ents[k];
-            const char* base = tape + t.off;
-            if (!t.two) {
-                --slot;
-                Adj1q g{};
-                std::memcpy(g.u, t.u, sizeof(g.u));
-                g.has_du = rotation_derivative(a->gates[t.gate], g.du) ? 1 : 0;
-                g.slot = int(slot);
-                adj_one_qubit_kernel<<<1, 256, 0, m->stream>>>(bars[t.site], reinterpret_cast<const double2*>(base),
-                                                               reinterpret_cast<const int*>(base + site_b), g, d_grad);
+        size_t at[2] = {nops[0], nops[1]};
+        for (size_t k = steps.size(); k-- > 0;) {
+            const unsigned all_of = unsigned(steps[k].ops.size());
+            at[steps[k].two] -= all_of;
+            if (!steps[k].two) {
+                adj_one_qubit_kernel<<<all_of, 256, 0, m->stream>>>(d_ones + at[0], d_grad);
                 count_launch(m, -1);
                 continue;
             }
-            AdjSplit A{};
-            const char* p = base + 2 * site_b;
-            A.site_l = reinterpret_cast<const double2*>(base);
-            A.site_r = reinterpret_cast<const double2*>(base + site_b);
-            A.theta = reinterpret_cast<const double2*>(p);
-            A.w = reinterpret_cast<const double2*>(p + mat_b);
-            A.sigma = reinterpret_cast<const double*>(p + 2 * mat_b);
-            A.perm = reinterpret_cast<const int*>(p + 2 * mat_b + al(R * sizeof(double)));
-            A.st = reinterpret_cast<const SplitState*>(p + 2 * mat_b + al(R * sizeof(double)) + al(R * sizeof(int)));
-            A.bar_l = bars[t.site];
-            A.bar_r = bars[t.site + 1];
-            std::memcpy(A.u, t.u, sizeof(A.u));
-            double2* w = ws;
-            const size_t RR = size_t(R) * R;
-            A.U = w; A.V = w + RR; A.Ub = w + 2 * RR; A.Vb = w + 3 * RR; A.M = w + 4 * RR; A.Nm = w + 5 * RR;
-            A.Z = w + 6 * RR; A.T1 = w + 7 * RR; A.tb = w + 8 * RR; A.tb0 = w + 9 * RR;
-            A.inv = wsd;
-            A.sq = wsd + R;
-            A.R = R;
-            adj_split_prep_kernel<<<eg, 256, 0, m->stream>>>(A);
-            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageOther);
-            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageM);
-            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageN);
-            adj_split_assemble_kernel<<<eg, 256, 0, m->stream>>>(A);
-            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageT1);
-            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageTb);
-            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageTb2);
-            adj_split_gate_kernel<<<eg, 256, 0, m->stream>>>(A);
-            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageBarL);
-            adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageBarR);
-            for (int c = 0; c < 11; ++c) count_launch(m, -1);
+            for (unsigned i = 0; i < all_of; i += unsigned(width)) {
+                const unsigned cnt = std::min(unsigned(width), all_of - i);
+                const AdjSplit* A = d_splits + at[1] + i;
+                const dim3 ge(eg, cnt), gg((R + kTile - 1) / kTile, (R + kTile - 1) / kTile, cnt);
+                adj_split_prep_kernel<<<ge, 256, 0, m->stream>>>(A);
+                adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageOther);
+                adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageM);
+                adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageN);
+                adj_split_assemble_kernel<<<ge, 256, 0, m->stream>>>(A);
+                adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageT1);
+                adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageTb);
+                adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageTb2);
+                adj_split_gate_kernel<<<ge, 256, 0, m->stream>>>(A);
+                adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageBarL);
+                adj_split_gemm_kernel<<<gg, kTileThreads, 0, m->stream>>>(A, kAdjStageBarR);
+                for (int c = 0; c < 11; ++c) count_launch(m, -1);
+            }
         }
         CUDA_TRY(cudaGetLastError());
     }

@@ -180,6 +180,19 @@ struct Adj1q {
     double2 du[4];  // d u / d angle (rotations)
     int has_du;
     int slot;       // gradient slot of this gate instance
+    double2* bar;   // cotangent of its site
+    const double2* before;  // the site before the gate, from the tape
+    const int* dims;        // its bonds
+};
+// One recomputed operation on the tape, and where the parts of a two-site one
+// lie from its base: both sites before it, then theta, W, sigma, perm and the
+// split's state after it.  A one-qubit gate has its site and its bonds.
+struct AdjTape {
+    char* base;
+    int site;
+};
+struct AdjTapeLayout {
+    size_t site_b, theta_off, w_off, sigma_off, perm_off, state_off;
 };
 // One split of the reverse sweep: the tape's copies of its forward inputs
 // and outputs, the cotangent sites it updates, and the workspace matrices
@@ -207,11 +220,14 @@ __global__ void adj_pauli_holes_kernel(DeviceMps mps, const char* labels, int t0
                                        const double2* envs, double2* tmp_all, double2* holes);
 __global__ void adj_pauli_accumulate_kernel(DeviceMps mps, double2* const* bars, const double2* holes,
                                             const double* coef_re, int t0, int count, int cap, int first);
-__global__ void adj_one_qubit_kernel(double2* bar, const double2* before, const int* dims, Adj1q g, double* grad);
-__global__ void adj_split_prep_kernel(AdjSplit A);
-__global__ void adj_split_gemm_kernel(AdjSplit A, int stage);
-__global__ void adj_split_assemble_kernel(AdjSplit A);
-__global__ void adj_split_gate_kernel(AdjSplit A);
+__global__ void adj_one_qubit_kernel(const Adj1q* gates, double* grad);
+__global__ void adj_tape_before_kernel(DeviceMps mps, const AdjTape* ops, AdjTapeLayout L, int two);
+__global__ void adj_tape_after_kernel(const SplitState* states, const SlotBuffers* slots, const AdjTape* ops,
+                                      AdjTapeLayout L);
+__global__ void adj_split_prep_kernel(const AdjSplit* splits);
+__global__ void adj_split_gemm_kernel(const AdjSplit* splits, int stage);
+__global__ void adj_split_assemble_kernel(const AdjSplit* splits);
+__global__ void adj_split_gate_kernel(const AdjSplit* splits);
 
 // Shared memory of a CTA of the cluster Jacobi: two blocks of b columns.
 inline size_t jacobi_ring_smem(int b, int kr, size_t elem) { return size_t(2) * b * 32 * kr * elem; }
