@@ -1092,9 +1092,9 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
                 // V orthonormalised (two Newton-Schulz steps), X V for every job of the mode, then the FP64 finish.
                 Timed t(m, 0, on);
                 const int side = std::max(w.max_rows, w.max_cols);
-                const dim3 g((side + 31) / 32, (side + 31) / 32, nj);
+                const dim3 g((side + kTile - 1) / kTile, (side + kTile - 1) / kTile, nj);
                 for (int stage = 0; stage < kPrecondStages; ++stage) {
-                    precond_gemm_kernel<<<g, 256, 0, on>>>(d_jobs, m->d_state, m->d_slots, mode, stage);
+                    precond_gemm_kernel<<<g, kTileThreads, 0, on>>>(d_jobs, m->d_state, m->d_slots, mode, stage);
                     count_launch(m, 0);
                 }
             }

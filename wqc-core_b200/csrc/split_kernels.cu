@@ -167,7 +167,6 @@ __global__ void omega_kernel(const SplitJob* jobs, const SplitState* st, const S
 // ---------------------------------------------------------------------------
 // Batched complex FP64 GEMMs of the range finder, dimensions from the job's state.
 // ---------------------------------------------------------------------------
-constexpr int kGemmT = 32, kGemmK = 16;
 
 __global__ void __launch_bounds__(kTileThreads) rsvd_gemm_kernel(const SplitJob* jobs, const SplitState* st,
                                                                  const SlotBuffers* slots, int stage) {
@@ -913,12 +912,13 @@ __global__ void __launch_bounds__(kProbeThreads) svd_probe_kernel(const SplitJob
 
 // ---------------------------------------------------------------------------
 // The precision form's FP64 products between its Jacobi phases (see
-// split_kernels.cuh): 32 x 32 tiles, batched over the wave's jobs.  G lives
+// split_kernels.cuh): 16 x 16 tiles (96 x 96 matrices: 14 us a product with
+// 32 x 32 tiles, on 9 CTAs a job; 7 with these), batched over the wave's jobs.  G lives
 // in the slot's omega and y0 buffers and V' in zr and y (each pair holds
 // 2 R ell >= R^2 entries); none of them is in use while an SVD of the job
 // runs.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) precond_gemm_kernel(const SplitJob* jobs, const SplitState* st,
+__global__ void __launch_bounds__(kTileThreads) precond_gemm_kernel(const SplitJob* jobs, const SplitState* st,
                                                            const SlotBuffers* slots, int mode, int stage) {
     const int j = blockIdx.z;
     const SplitState S = st[j];
@@ -929,7 +929,7 @@ __global__ void __launch_bounds__(256) precond_gemm_kernel(const SplitJob* jobs,
     const int M = X.M, N = X.N;
     const bool last = stage == kPrecondXV;
     const int m = last ? M : N, n = N, k = N;
-    const int i0 = blockIdx.y * kGemmT, n0 = blockIdx.x * kGemmT;
+    const int i0 = blockIdx.y * kTile, n0 = blockIdx.x * kTile;
     if (i0 >= m || n0 >= n) return;
     // Two Newton-Schulz steps: V (z) -> zr -> z; then X V from z.
     const bool second = stage >= kPrecondGram2;
@@ -952,38 +952,14 @@ __global__ void __launch_bounds__(256) precond_gemm_kernel(const SplitJob* jobs,
         }
         return V[size_t(jj) * N + kk];
     };
-    __shared__ double2 As[kGemmT][kGemmK + 1];
-    __shared__ double2 Bs[kGemmK][kGemmT + 1];
-    const int tid = threadIdx.x, tr = tid / 16, tc = tid % 16;
-    double2 acc[2][2] = {{cmake(0, 0), cmake(0, 0)}, {cmake(0, 0), cmake(0, 0)}};
-    for (int k0 = 0; k0 < k; k0 += kGemmK) {
-        for (int e = tid; e < kGemmT * kGemmK; e += 256) {
-            const int r = e / kGemmK, c = e % kGemmK;
-            As[r][c] = (i0 + r < m && k0 + c < k) ? a_at(i0 + r, k0 + c) : cmake(0, 0);
-        }
-        for (int e = tid; e < kGemmK * kGemmT; e += 256) {
-            const int r = e / kGemmT, c = e % kGemmT;
-            Bs[r][c] = (k0 + r < k && n0 + c < n) ? b_at(k0 + r, n0 + c) : cmake(0, 0);
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int c = 0; c < kGemmK; ++c) {
-            const double2 a0 = As[tr][c], a1 = As[tr + 16][c];
-            const double2 b0 = Bs[c][tc], b1 = Bs[c][tc + 16];
-            cfma(acc[0][0], a0, b0);
-            cfma(acc[0][1], a0, b1);
-            cfma(acc[1][0], a1, b0);
-            cfma(acc[1][1], a1, b1);
-        }
-        __syncthreads();
-    }
     double2* C = gram ? G : last ? B.w : Vout;
     const int ldc = last ? M : N;
-    for (int x = 0; x < 2; ++x)
-        for (int y = 0; y < 2; ++y) {
-            const int i = i0 + tr + 16 * x, jj = n0 + tc + 16 * y;
-            if (i < m && jj < n) C[size_t(jj) * ldc + i] = acc[x][y];
-        }
+    __shared__ TileSmem sm;
+    // C is column-major, so the transposed product is what stores in runs.
+    tile_gemm(
+        sm, n0, i0, n, m, k, true, gram, [&](int jj, int kk) { return b_at(kk, jj); },
+        [&](int kk, int i) { return a_at(i, kk); },
+        [&](int jj, int i, double2 v) { C[size_t(jj) * ldc + i] = v; });
 }
 
 // ---------------------------------------------------------------------------
