@@ -357,7 +357,7 @@ def tensor_core_leg(W, torch, ctx, w, rule, flush, gemm_only: bool = False) -> d
                                                    merge=W.MERGE_TC_INT8)
     out["int8_merge"] = {
         "form": "plain FP64 form with every merge from int8 digit slices on the tensor cores (WQC_MERGE_TC_INT8, "
-                "the single-state default)",
+                "a single state's default above bond 192)",
         "value": i8_splits / (i8_ms * 1e-3),
         "ffma_value": fp64_splits / (fp64_ms * 1e-3),
         "unit": UNIT,
@@ -1220,7 +1220,8 @@ def run_cuda(args) -> None:
             "dtype": "f64",
             "data": "synthetic (seeded generator, same circuit every run)",
             "config": dict(workload_config(w, args.split_rule, g0, windows),
-                           merge="int8 digit slices on the tcgen05 tensor cores, FP64-level (the state default)"),
+                           merge="the state default: FP64 FMA tiles up to bond 192, int8 digit slices on the tcgen05 tensor "
+                                 "cores (FP64-level) above"),
             "e2e": {
                 "value": e2e,
                 "unit": UNIT,
@@ -1231,7 +1232,7 @@ def run_cuda(args) -> None:
             },
             "roofline": {
                 "bound": "fp64",
-                "kernel": "jacobi_cluster_kernel (FP64 one-sided Jacobi SVD)",
+                "kernel": "jacobi_qr_kernel + jacobi_ring_kernel (FP64 one-sided Jacobi SVD)",
                 "achieved": achieved,
                 "peak": peak,
                 "unit": "TFLOP/s",

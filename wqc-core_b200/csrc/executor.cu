@@ -1599,7 +1599,7 @@ static wqc_status create_state(wqc_cuda_ctx* ctx, const std::vector<int>& ns, co
         tc_b_bytes = size_t(2) * m->nslots * m->tc_npad * m->tc_kpad * sizeof(float);
     }
     // States from wqc_mps_create merge from int8 digit slices on the tensor
-    // cores by default (FP64-level, wqc_mps_set_merge); batches (a batch of
+    // cores where that is faster (FP64-level, kOzAutoBond); batches (a batch of
     // one included) keep FMA merges, whose many slots would each need digit
     // planes.
     const bool oz_default = single_state && !m->tc;
