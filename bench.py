@@ -1237,9 +1237,10 @@ def run_cuda(args) -> None:
                 "peak": peak,
                 "unit": "TFLOP/s",
                 "frac": (achieved / peak) if (achieved and peak) else None,
-                "traffic": 767232,
-                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one saturated launch "
-                                  "(five exact 256 x 256 splits on 16-CTA clusters); W stays in shared memory",
+                "traffic": 10713344,
+                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one saturated QR launch and its "
+                                  "Jacobi launch (five exact 256 x 256 splits on 16-CTA clusters, caches flushed "
+                                  "before each): the input once each; the columns stay on the SMs",
                 "peak_source": "FP64 cuBLAS DGEMM 8192^3 measured in this run (the FP64 pipe: no tensor-core "
                                "instruction is issued; MEASURED_PEAKS.json has no FP64 figure)",
                 "flops_per_step": flops / steps,
