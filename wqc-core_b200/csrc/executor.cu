@@ -1092,9 +1092,20 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
                 // V orthonormalised (two Newton-Schulz steps), X V for every job of the mode, then the FP64 finish.
                 Timed t(m, 0, on);
                 const int side = std::max(w.max_rows, w.max_cols);
-                const dim3 g((side + kTile - 1) / kTile, (side + kTile - 1) / kTile, nj);
+                // Small tiles while large ones would leave SMs idle.  A batch
+                // takes large ones whatever it holds: the two round
+                // differently, and a slice's results do not depend on the
+                // other slices.
+                const int large = (side + kPrecondTile - 1) / kPrecondTile;
+                const bool small = !m->batch && long(large) * large * nj < 2L * m->ctx->sm_count;
+                const unsigned side_t = unsigned(small ? (side + kTile - 1) / kTile : large);
                 for (int stage = 0; stage < kPrecondStages; ++stage) {
-                    precond_gemm_kernel<<<g, kTileThreads, 0, on>>>(d_jobs, m->d_state, m->d_slots, mode, stage);
+                    if (small)
+                        precond_gemm_kernel<true><<<dim3(side_t, side_t, nj), 256, 0, on>>>(d_jobs, m->d_state, m->d_slots,
+                                                                                             mode, stage);
+                    else
+                        precond_gemm_kernel<false><<<dim3(side_t, side_t, nj), 256, 0, on>>>(d_jobs, m->d_state, m->d_slots,
+                                                                                             mode, stage);
                     count_launch(m, 0);
                 }
             }

@@ -912,14 +912,19 @@ __global__ void __launch_bounds__(kProbeThreads) svd_probe_kernel(const SplitJob
 
 // ---------------------------------------------------------------------------
 // The precision form's FP64 products between its Jacobi phases (see
-// split_kernels.cuh): 16 x 16 tiles (96 x 96 matrices: 14 us a product with
-// 32 x 32 tiles, on 9 CTAs a job; 7 with these), batched over the wave's jobs.  G lives
+// split_kernels.cuh), batched over the wave's jobs.  Waves of few jobs take
+// 16 x 16 tiles (96 x 96 matrices: 7 us a product, against 14 with 32 x 32 tiles
+// on 9 CTAs a job); waves that fill the device 32 x 32, four outputs a thread,
+// which read shared memory half as often (a batch of 128 slices of bonds up to
+// 128: 1.53 s, against 1.66 with the small tiles).  G lives
 // in the slot's omega and y0 buffers and V' in zr and y (each pair holds
 // 2 R ell >= R^2 entries); none of them is in use while an SVD of the job
 // runs.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kTileThreads) precond_gemm_kernel(const SplitJob* jobs, const SplitState* st,
+template <bool kSmall>
+__global__ void __launch_bounds__(256) precond_gemm_kernel(const SplitJob* jobs, const SplitState* st,
                                                            const SlotBuffers* slots, int mode, int stage) {
+    constexpr int kT = kSmall ? kTile : kPrecondTile;
     const int j = blockIdx.z;
     const SplitState S = st[j];
     if (!jacobi_active(S, mode)) return;
@@ -929,7 +934,7 @@ __global__ void __launch_bounds__(kTileThreads) precond_gemm_kernel(const SplitJ
     const int M = X.M, N = X.N;
     const bool last = stage == kPrecondXV;
     const int m = last ? M : N, n = N, k = N;
-    const int i0 = blockIdx.y * kTile, n0 = blockIdx.x * kTile;
+    const int i0 = blockIdx.y * kT, n0 = blockIdx.x * kT;
     if (i0 >= m || n0 >= n) return;
     // Two Newton-Schulz steps: V (z) -> zr -> z; then X V from z.
     const bool second = stage >= kPrecondGram2;
@@ -954,13 +959,49 @@ __global__ void __launch_bounds__(kTileThreads) precond_gemm_kernel(const SplitJ
     };
     double2* C = gram ? G : last ? B.w : Vout;
     const int ldc = last ? M : N;
-    __shared__ TileSmem sm;
-    // C is column-major, so the transposed product is what stores in runs.
-    tile_gemm(
-        sm, n0, i0, n, m, k, true, gram, [&](int jj, int kk) { return b_at(kk, jj); },
-        [&](int kk, int i) { return a_at(i, kk); },
-        [&](int jj, int i, double2 v) { C[size_t(jj) * ldc + i] = v; });
+    if constexpr (kSmall) {
+        __shared__ TileSmem sm;
+        // C is column-major, so the transposed product is what stores in runs.
+        tile_gemm(
+            sm, n0, i0, n, m, k, true, gram, [&](int jj, int kk) { return b_at(kk, jj); },
+            [&](int kk, int i) { return a_at(i, kk); },
+            [&](int jj, int i, double2 v) { C[size_t(jj) * ldc + i] = v; });
+    } else {
+        constexpr int kK = 16;
+        __shared__ double2 As[kT][kK + 1];
+        __shared__ double2 Bs[kK][kT + 1];
+        const int tid = threadIdx.x, tr = tid / 16, tc = tid % 16;
+        double2 acc[2][2] = {{cmake(0, 0), cmake(0, 0)}, {cmake(0, 0), cmake(0, 0)}};
+        for (int k0 = 0; k0 < k; k0 += kK) {
+            for (int e = tid; e < kT * kK; e += 256) {
+                const int r = e / kK, c = e % kK;
+                As[r][c] = (i0 + r < m && k0 + c < k) ? a_at(i0 + r, k0 + c) : cmake(0, 0);
+            }
+            for (int e = tid; e < kK * kT; e += 256) {
+                const int r = e / kT, c = e % kT;
+                Bs[r][c] = (k0 + r < k && n0 + c < n) ? b_at(k0 + r, n0 + c) : cmake(0, 0);
+            }
+            __syncthreads();
+#pragma unroll 4
+            for (int c = 0; c < kK; ++c) {
+                const double2 a0 = As[tr][c], a1 = As[tr + 16][c];
+                const double2 b0 = Bs[c][tc], b1 = Bs[c][tc + 16];
+                cfma(acc[0][0], a0, b0);
+                cfma(acc[0][1], a0, b1);
+                cfma(acc[1][0], a1, b0);
+                cfma(acc[1][1], a1, b1);
+            }
+            __syncthreads();
+        }
+        for (int x = 0; x < 2; ++x)
+            for (int y = 0; y < 2; ++y) {
+                const int i = i0 + tr + 16 * x, jj = n0 + tc + 16 * y;
+                if (i < m && jj < n) C[size_t(jj) * ldc + i] = acc[x][y];
+            }
+    }
 }
+template __global__ void precond_gemm_kernel<true>(const SplitJob*, const SplitState*, const SlotBuffers*, int, int);
+template __global__ void precond_gemm_kernel<false>(const SplitJob*, const SplitState*, const SlotBuffers*, int, int);
 
 // ---------------------------------------------------------------------------
 // The cut: stable descending sort, truncation rule, discarded weight and the

@@ -87,6 +87,8 @@ cudaError_t launch_jacobi_staged(bool fp32, const cudaLaunchConfig_t& cfg, const
 // rotations to ~1e-12, then to FP64 rounding), then X V into the slot's W
 // buffer, X dust-zeroed as the first phase loaded it.
 enum { kPrecondGram1 = 0, kPrecondStep1, kPrecondGram2, kPrecondStep2, kPrecondXV, kPrecondStages };
+constexpr int kPrecondTile = 32;  // of waves that fill the device (kSmall: kTile)
+template <bool kSmall>
 __global__ void precond_gemm_kernel(const SplitJob* jobs, const SplitState* st, const SlotBuffers* slots, int mode,
                                     int stage);
 // Shape of the staged Jacobi for an M x N working matrix on a cluster of C
