@@ -224,6 +224,20 @@ WQC_API wqc_status wqc_mps_set_merge(wqc_mps* mps, int32_t merge);
 WQC_API wqc_status wqc_schedule_gates(uint32_t n, const wqc_gate* gates, uint32_t count, int32_t* split_site,
                                       int32_t* split_level, uint32_t max, uint32_t* nsplits, uint32_t* nlevels);
 
+/* Host-only: the Jacobi launches that wqc_mps_apply_gates would make for
+ * `gates` on a fresh state of n sites and bond chi (slices > 0: on a batch of
+ * that many) on a device of sm_count SMs and clusters of up to max_cluster
+ * CTAs, without a device; for tests of the planner.  rule is a
+ * wqc_split_rule, or -1 for the direct SVDs of an adjoint; force_cluster > 0
+ * gives every task that cluster size where it fits (an autotuned context).
+ * Eight numbers a launch: wave, kernel (0 cluster, 1 staged), tasks, CTAs a
+ * cluster, threads a CTA, the kernel's limit of them, shared memory, its
+ * limit; at most `max` launches are written, *launches receives the total. */
+WQC_API wqc_status wqc_debug_svd_launches(uint32_t n, uint32_t chi, uint32_t slices, int32_t precision, int32_t rule,
+                                          int32_t sm_count, int32_t max_cluster, int32_t force_cluster,
+                                          const wqc_gate* gates, uint32_t count, int32_t* out, uint32_t max,
+                                          uint32_t* launches);
+
 /* Wait for the enqueued work; reports device-side failures. */
 WQC_API wqc_status wqc_mps_synchronize(wqc_mps* mps);
 

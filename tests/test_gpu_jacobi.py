@@ -139,3 +139,56 @@ def test_clusters_of_equal_singular_values(cuda_ctx, dl, k, dr, multiplicity):
     for gram in (left.conj().T @ left, right @ right.conj().T):
         assert np.linalg.norm(gram - np.diag(np.diag(gram))) <= 6 * 2 * max(dl, dr) * np.finfo(float).eps * s[0] / s[kept - 1]
     m.close()
+
+
+@pytest.mark.parametrize("precision", [W.PRECISION_FP64, W.PRECISION_FP32])
+def test_wide_register_shares_launches_between_long_and_short_columns(cuda_ctx, precision):
+    """64 qubits at chi 128: a saturated wave's 128-column tasks would like
+    blocks of 16 columns beside the 256-column tasks' instance, which is compiled
+    for 12 warps.  CZs commute, so the bonds stay 2 while their bounds, which
+    the launches are shaped by, grow to 128.  Against the oracle: a split of the
+    unit state errs by 6 N eps, N = 4, and there are fewer than layers n of them."""
+    import oracle as O
+
+    n, chi, layers = 64, 128, 18
+    g = [C.g1(C.RY, q, 0.1 + 0.6 * np.sin(q) ** 2) for q in range(n)]
+    for k in range(layers):
+        g += [C.g2(C.CZ, q, q + 1) for q in range(k % 2, n - 1, 2)]
+    gates = C.gates_array(g)
+    m = W.CudaMps(n, chi, ctx=cuda_ctx, precision=precision)
+    m.apply_gates(gates)
+    ref = O.run(n, chi, gates)
+    assert m.split_records()["chi"].tolist() == ref.records()["chi"].tolist()
+    amp, want = m.amplitude_zero(), ref.amplitude_zero()
+    assert abs(amp - want) <= layers * n * 24 * np.finfo(float).eps
+    m.close()
+
+
+@pytest.mark.parametrize("precision", [W.PRECISION_FP64, W.PRECISION_FP32])
+def test_short_columns_beside_the_longest(cuda_ctx, precision):
+    """Two splits of one wave, 26 columns and 256, and each on its own."""
+    rng = np.random.default_rng(9)
+    bonds = [1, 2, 13, 20, 13, 2, 4, 128, 128, 128, 4, 2, 1]
+    n = len(bonds) - 1
+    sites = [cplx(rng, bonds[q], 2, bonds[q + 1]) for q in range(n)]
+    pairs = [2, 7]  # 26 x 26 and 256 x 256
+
+    def state(gates):
+        m = W.CudaMps(n, 128, ctx=cuda_ctx, precision=precision)
+        m.set_split_rule(W.SPLIT_RULE_EXACT)
+        for q, t in enumerate(sites):
+            m.set_site(q, t)
+        m.apply_gates(C.gates_array([C.g2(C.CNOT, p, p + 1) for p in gates]))
+        return m
+
+    together = state(pairs)
+    for p in pairs:
+        alone = state([p])
+        a = np.einsum("asg,gtb->astb", alone.site(p), alone.site(p + 1))
+        b = np.einsum("asg,gtb->astb", together.site(p), together.site(p + 1))
+        assert a.shape == b.shape
+        # A random 256 x 256 theta is cut to 128 values; neighbours of the cut
+        # lie about sigma_1 / 256 apart, which amplifies each side's 6 N eps.
+        assert np.linalg.norm(a - b) <= 12 * 256 * 256 * np.finfo(float).eps * np.linalg.norm(a)
+        alone.close()
+    together.close()

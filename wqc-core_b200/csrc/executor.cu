@@ -456,12 +456,15 @@ bool ring_shape(int M, int N, int vrows, size_t elem, int C, RingShape* out) {
 // counts.  A batch fills the GPU, so SM time decides, with as many CTAs on an
 // SM as fit it, but never less than the FP64 work; that choice depends on the
 // shape alone, so a slice's results do not depend on the other slices of its
-// batch.  0: no cluster size fits.
+// batch.  `most_warps` bounds the CTA of a task that shares a launch with
+// longer columns, whose instance is compiled for fewer warps.  0: no cluster
+// size fits.
 int choose_cluster(const wqc_cuda_ctx* ctx, int M, int N, int max_c, int njobs, int sm_count, size_t elem,
-                   bool throughput, int vrows = 0) {
+                   bool throughput, int vrows = 0, int most_warps = 32) {
     RingShape s;
+    auto shaped = [&](int Cc) { return ring_shape(M, N, vrows, elem, Cc, &s) && s.warps <= most_warps; };
     if (ctx) {
-        auto fits = [&](int Cc) { return Cc >= 1 && Cc <= max_c && !(Cc & (Cc - 1)) && ring_shape(M, N, vrows, elem, Cc, &s); };
+        auto fits = [&](int Cc) { return Cc >= 1 && Cc <= max_c && !(Cc & (Cc - 1)) && shaped(Cc); };
         if (ctx->force_C > 0 && fits(ctx->force_C)) return ctx->force_C;
         for (const auto& t : ctx->tuned)
             if (t.M == M && t.N == N && t.len == M + vrows && t.elem == int(elem) &&
@@ -471,7 +474,7 @@ int choose_cluster(const wqc_cuda_ctx* ctx, int M, int N, int max_c, int njobs, 
     int best = 0;
     double best_cost = 1e300;
     for (int Cc = 1; Cc <= std::min(max_c, kJacobiRingMaxCluster); Cc *= 2) {
-        if (!ring_shape(M, N, vrows, elem, Cc, &s)) continue;
+        if (!shaped(Cc)) continue;
         const double kr = s.kr * double(elem) / sizeof(double2);
         const double work = s.b * (25.0 + 10.0 * kr);  // FP64 pipe cycles of a round
         const double round = 850.0 + work + 0.6 * kr * kr * s.b;
@@ -747,9 +750,12 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
             // Jacobi groups: the tasks of a mode that run in one launch (one
             // per phase).  Launches of a stream follow one another, so a
             // latency-bound wave puts all of a mode's cluster tasks into one
-            // launch, whatever their shapes: it lasts as long as its longest
-            // task.  A batch keeps tasks of unlike column length apart, whose
-            // registers and shared memory would be those of the longest.
+            // launch: it lasts as long as its longest task.  The launch runs
+            // the instance of its longest columns, so the wave's other tasks
+            // take cluster sizes whose CTAs that instance allows
+            // (`most_warps`); one with none gets a launch with its like.  A
+            // batch keeps tasks of unlike column length apart, whose registers
+            // and shared memory would be those of the longest.
             struct GKey {
                 int mode, k1, k2;
             };
@@ -806,24 +812,25 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                 remaining -= sel.size();
             }
             const int nj_wave = int(sel.size());
+            auto cluster_of = [&](int M, int N, size_t elem, int vrows, int most_warps) {
+                return choose_cluster(m->ctx, M, N, m->ctx->max_cluster, nj_wave, m->ctx->sm_count, elem, m->batch,
+                                      vrows, most_warps);
+            };
             // A shape beyond every cluster goes to the staged kernel: its key
             // is -b, the width of its blocks (0: no kernel takes it).
-            auto key_of = [&](int M, int N, size_t elem, int vrows, int& c) {
-                c = choose_cluster(m->ctx, M, N, m->ctx->max_cluster, nj_wave, m->ctx->sm_count, elem, m->batch, vrows);
-                if (c < 1) return -jacobi_staged_b(M + vrows, N, elem, kSmemLimit, nullptr);
-                return m->batch ? jacobi_ring_kr(elem == sizeof(float2), M, vrows) : 1;
+            auto key_of = [&](int M, int N, size_t elem, int vrows, int most_warps, int& c) {
+                const int kr = jacobi_ring_kr(elem == sizeof(float2), M, vrows);
+                c = cluster_of(M, N, elem, vrows, most_warps);
+                if (c >= 1) return m->batch ? kr : 1;
+                c = cluster_of(M, N, elem, vrows, 32);
+                if (c >= 1) return 1 + kr;
+                return -jacobi_staged_b(M + vrows, N, elem, kSmemLimit, nullptr);
             };
-            auto add_task = [&](int mode, int M, int N, int local) {
-                Task t{local, 0, 0};
-                int k1, k2 = 0;
-                if (m->fp32) {
-                    k1 = key_of(M, N, sizeof(float2), N, t.c1);
-                    k2 = key_of(M, N, sizeof(double2), 0, t.c2);
-                } else {
-                    k1 = key_of(M, N, sizeof(double2), 0, t.c1);
-                }
-                add(mode, k1, k2, t);
+            struct WaveTask {
+                int mode, M, N, local;
             };
+            std::vector<WaveTask> wave_tasks;
+            auto add_task = [&](int mode, int M, int N, int local) { wave_tasks.push_back({mode, M, N, local}); };
             w.jobs_off = int(plan.jobs.size());
             w.njobs = nj_wave;
             for (int local = 0; local < nj_wave; ++local) {
@@ -852,6 +859,24 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                     jacobi_dims(k, kJacobiRsvd, M, N);
                     add_task(kJacobiRsvd, M, N, local);
                 }
+            }
+            // Warps of the instance that the cluster tasks of a mode share, per phase.
+            int most_warps[3][2] = {{32, 32}, {32, 32}, {32, 32}};
+            const size_t elem1 = m->fp32 ? sizeof(float2) : sizeof(double2);
+            if (!m->batch)
+                for (const WaveTask& t : wave_tasks)
+                    for (int ph = 0; ph < (m->fp32 ? 2 : 1); ++ph) {
+                        const size_t elem = ph == 0 ? elem1 : sizeof(double2);
+                        const int vrows = m->fp32 && ph == 0 ? t.N : 0;
+                        if (cluster_of(t.M, t.N, elem, vrows, 32) < 1) continue;
+                        const int kr = jacobi_ring_kr(elem == sizeof(float2), t.M, vrows);
+                        most_warps[t.mode][ph] = std::min(most_warps[t.mode][ph], jacobi_ring_warps(kr, int(elem)));
+                    }
+            for (const WaveTask& t : wave_tasks) {
+                Task out{t.local, 0, 0};
+                const int k1 = key_of(t.M, t.N, elem1, m->fp32 ? t.N : 0, most_warps[t.mode][0], out.c1);
+                const int k2 = m->fp32 ? key_of(t.M, t.N, sizeof(double2), 0, most_warps[t.mode][1], out.c2) : 0;
+                add(t.mode, k1, k2, out);
             }
             // Launch shape of one phase for the tasks of a group.
             auto fill = [&](PhaseCfg& pc, int key, bool first, int mode, const std::vector<Task>& tasks, size_t elem,
@@ -937,8 +962,31 @@ wqc_status ensure_records(wqc_mps* m, size_t need) {
     return WQC_OK;
 }
 
+// Threads a CTA of the phase's kernel may have.
+int phase_thread_limit(const PhaseCfg& pc, bool fp32) {
+    return pc.staged ? kJacobiStagedThreads
+                     : 32 * jacobi_ring_warps(pc.kr, int(fp32 ? sizeof(float2) : sizeof(double2)));
+}
+
+// Every SVD launch of a plan against the limits of its kernel, before any of
+// the plan is enqueued.
+wqc_status check_plan(const Plan& plan) {
+    for (const Wave& w : plan.waves)
+        for (const Group& g : w.groups)
+            for (int ph = 0; ph < g.nph; ++ph) {
+                const PhaseCfg& pc = g.ph[ph];
+                if (pc.C < 1 || (pc.staged && pc.b < 1))
+                    return fail(WQC_ERR_INVALID, "two-site matrix too large for the cluster-resident Jacobi SVD");
+                if (pc.threads > phase_thread_limit(pc, g.nph == 2 && ph == 0) || pc.smem > kSmemLimit)
+                    return fail(WQC_ERR_INVALID, "a Jacobi launch of " + std::to_string(pc.threads) + " threads and " +
+                                                     std::to_string(pc.smem) + " bytes does not fit its kernel");
+            }
+    return WQC_OK;
+}
+
 wqc_status launch_plan(wqc_mps* m, Plan& plan) {
     if (plan.waves.empty()) return WQC_OK;
+    if (wqc_status s = check_plan(plan)) return s;
     if (wqc_status s = ensure_records(m, size_t(plan.first_seq) + plan.nsplits)) return s;
     size_t off = 0;
     const size_t o_oq = stage_section(off, plan.oq);
@@ -1047,7 +1095,6 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
         }
         auto launch_phase = [&](const Group& gr, const PhaseCfg& pc, int mode, int phase, bool fp32,
                                 cudaStream_t on) -> wqc_status {
-            if (pc.C < 1 || (pc.staged && pc.b < 1)) return fail(WQC_ERR_INVALID, "two-site matrix too large for the cluster-resident Jacobi SVD");
             Timed t(m, 0, on);
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(gr.count * pc.C);
@@ -1503,37 +1550,24 @@ uint64_t wqc_mps_workspace_bytes(uint32_t n, uint32_t chi) {
     return v > ~uint64_t(0) ? ~uint64_t(0) : uint64_t(v);
 }
 
-static wqc_status create_state(wqc_cuda_ctx* ctx, const std::vector<int>& ns, const std::vector<int>& chis,
-                               int32_t precision, bool reject, int nslots_req, wqc_mps** out,
-                               bool single_state = false) {
-    if (!ctx || !out) return fail(WQC_ERR_INVALID, "null argument");
-    if (ns.empty()) return fail(WQC_ERR_INVALID, "no slices");
-    long total_n = 0;
-    int chi_cap = 0;
-    for (size_t i = 0; i < ns.size(); ++i) {
-        if (ns[i] <= 0)
-            return fail(WQC_ERR_INVALID_QUBIT_COUNT, "Invalid qubit count: " + std::to_string(ns[i]) + ". Max limit is 40.");
-        if (chis[i] <= 0) return fail(WQC_ERR_INVALID, "MPS max bond dimension must be > 0");
-        if (chis[i] > 256) return fail(WQC_ERR_INVALID, "the cuda backend supports max_bond_dim <= 256");
-        total_n += ns[i];
-        chi_cap = std::max(chi_cap, chis[i]);
+// The host side of a state: its slices, the capacity of every site (offsets
+// into the site pool) and the buckets of split slots.  No device work.
+static void lay_out(wqc_mps* m, wqc_cuda_ctx* ctx, const std::vector<int>& ns, const std::vector<int>& chis,
+                    int32_t precision, int nslots_req, std::vector<size_t>& site_off,
+                    std::vector<size_t>& bucket_bytes, std::vector<size_t>& bucket_gs) {
+    int n = 0;
+    for (size_t sl = 0; sl < ns.size(); ++sl) {
+        n += ns[sl];
+        m->chi = std::max(m->chi, chis[sl]);
     }
-    if (precision != WQC_PRECISION_FP64 && precision != WQC_PRECISION_FP32 && precision != WQC_PRECISION_TF32X3)
-        return fail(WQC_ERR_INVALID, "unsupported precision form");
-    if (total_n > (1L << 24)) return fail(WQC_ERR_INVALID, "too many sites");
-    CUDA_TRY(cudaSetDevice(ctx->device));
-    auto* m = new wqc_mps();
-    const int n = int(total_n);
     m->ctx = ctx;
     m->n = n;
-    m->chi = chi_cap;
-    m->reject = reject;
     m->fp32 = precision != WQC_PRECISION_FP64;
     m->tc = precision == WQC_PRECISION_TF32X3;
     m->ub.assign(n > 0 ? n - 1 : 0, 1);
     m->site_chi.resize(n);
     m->site_slice.resize(n);
-    std::vector<size_t> site_off(n + 1, 0);
+    site_off.assign(n + 1, 0);
     for (size_t sl = 0, g = 0; sl < ns.size(); ++sl) {
         m->seg_first.push_back(int(g));
         m->seg_n.push_back(ns[sl]);
@@ -1544,17 +1578,6 @@ static wqc_status create_state(wqc_cuda_ctx* ctx, const std::vector<int>& ns, co
             site_off[g + 1] = site_off[g] + size_t(chis[sl]) * 2 * chis[sl];
         }
     }
-    auto bail = [&](wqc_status st) {
-        wqc_mps_destroy(m);
-        return st;
-    };
-    if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(fail(WQC_ERR_CUDA, "stream"));
-    if (cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking) != cudaSuccess) return bail(fail(WQC_ERR_CUDA, "stream"));
-    if (cudaEventCreateWithFlags(&m->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&m->join_ev, cudaEventDisableTiming) != cudaSuccess)
-        return bail(fail(WQC_ERR_CUDA, "event"));
-    if (cudaEventCreateWithFlags(&m->stage_done, cudaEventDisableTiming) != cudaSuccess) return bail(fail(WQC_ERR_CUDA, "event"));
-    cudaEventRecord(m->stage_done, m->stream);
     // Split workspace: one bucket of slots per distinct chi_max, each slot
     // holding theta, w, z, the range finder's buffers and tau for two-site
     // matrices up to R x R, R = 2 chi_max (plus the staged Jacobi's workspace
@@ -1570,7 +1593,6 @@ static wqc_status create_state(wqc_cuda_ctx* ctx, const std::vector<int>& ns, co
                (fp32 &&
                 choose_cluster(nullptr, M, N, ctx->max_cluster, 1, ctx->sm_count, sizeof(float2), false, N) < 1);
     };
-    std::vector<size_t> bucket_bytes, bucket_gs;
     {
         std::vector<int> cs(chis);
         std::sort(cs.begin(), cs.end());
@@ -1595,6 +1617,43 @@ static wqc_status create_state(wqc_cuda_ctx* ctx, const std::vector<int>& ns, co
             m->nslots += int(cap);
         }
     }
+}
+
+static wqc_status create_state(wqc_cuda_ctx* ctx, const std::vector<int>& ns, const std::vector<int>& chis,
+                               int32_t precision, bool reject, int nslots_req, wqc_mps** out,
+                               bool single_state = false) {
+    if (!ctx || !out) return fail(WQC_ERR_INVALID, "null argument");
+    if (ns.empty()) return fail(WQC_ERR_INVALID, "no slices");
+    long total_n = 0;
+    int chi_cap = 0;
+    for (size_t i = 0; i < ns.size(); ++i) {
+        if (ns[i] <= 0)
+            return fail(WQC_ERR_INVALID_QUBIT_COUNT, "Invalid qubit count: " + std::to_string(ns[i]) + ". Max limit is 40.");
+        if (chis[i] <= 0) return fail(WQC_ERR_INVALID, "MPS max bond dimension must be > 0");
+        if (chis[i] > 256) return fail(WQC_ERR_INVALID, "the cuda backend supports max_bond_dim <= 256");
+        total_n += ns[i];
+        chi_cap = std::max(chi_cap, chis[i]);
+    }
+    if (precision != WQC_PRECISION_FP64 && precision != WQC_PRECISION_FP32 && precision != WQC_PRECISION_TF32X3)
+        return fail(WQC_ERR_INVALID, "unsupported precision form");
+    if (total_n > (1L << 24)) return fail(WQC_ERR_INVALID, "too many sites");
+    CUDA_TRY(cudaSetDevice(ctx->device));
+    auto* m = new wqc_mps();
+    const int n = int(total_n);
+    m->reject = reject;
+    std::vector<size_t> site_off, bucket_bytes, bucket_gs;
+    lay_out(m, ctx, ns, chis, precision, nslots_req, site_off, bucket_bytes, bucket_gs);
+    auto bail = [&](wqc_status st) {
+        wqc_mps_destroy(m);
+        return st;
+    };
+    if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(fail(WQC_ERR_CUDA, "stream"));
+    if (cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking) != cudaSuccess) return bail(fail(WQC_ERR_CUDA, "stream"));
+    if (cudaEventCreateWithFlags(&m->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&m->join_ev, cudaEventDisableTiming) != cudaSuccess)
+        return bail(fail(WQC_ERR_CUDA, "event"));
+    if (cudaEventCreateWithFlags(&m->stage_done, cudaEventDisableTiming) != cudaSuccess) return bail(fail(WQC_ERR_CUDA, "event"));
+    cudaEventRecord(m->stage_done, m->stream);
     size_t slot_pool_bytes = 0;
     for (size_t b = 0; b < m->bucket_chi.size(); ++b) slot_pool_bytes += bucket_bytes[b] * size_t(m->bucket_cap[b]);
     const size_t site_bytes = site_off[n] * sizeof(double2);
@@ -1814,6 +1873,51 @@ wqc_status wqc_schedule_gates(uint32_t n, const wqc_gate* gates, uint32_t count,
     }
     *nsplits = k;
     *nlevels = uint32_t(top + 1);
+    return WQC_OK;
+}
+
+wqc_status wqc_debug_svd_launches(uint32_t n, uint32_t chi, uint32_t slices, int32_t precision, int32_t rule,
+                                  int32_t sm_count, int32_t max_cluster, int32_t force_cluster, const wqc_gate* gates,
+                                  uint32_t count, int32_t* out, uint32_t max, uint32_t* launches) {
+    if (n == 0 || chi == 0 || chi > 256 || (!gates && count) || !launches || (!out && max))
+        return fail(WQC_ERR_INVALID, "null argument");
+    Expander ex;
+    if (wqc_status s = expand(int(n), gates, count, false, ex)) return s;
+    wqc_cuda_ctx ctx;
+    ctx.sm_count = sm_count;
+    ctx.max_cluster = max_cluster;
+    ctx.force_C = force_cluster;
+    wqc_mps m;
+    std::vector<size_t> site_off, bucket_bytes, bucket_gs;
+    const size_t nseg = std::max(1u, slices);
+    lay_out(&m, &ctx, std::vector<int>(nseg, int(n)), std::vector<int>(nseg, int(chi)), precision, 0, site_off,
+            bucket_bytes, bucket_gs);
+    m.batch = slices > 0;
+    m.exact_only = rule != WQC_SPLIT_RULE_REFERENCE;
+    m.direct_svd = rule < 0;
+    std::vector<Op> ops;
+    for (size_t sl = 0; sl < nseg; ++sl)
+        for (Op o : ex.ops) {
+            o.site += int(sl * n);
+            o.slice = int(sl);
+            ops.push_back(o);
+        }
+    Plan plan;
+    build_plan(&m, ops, plan);
+    uint32_t k = 0;
+    auto put = [&](int wave, int kind, int tasks, int C, int threads, int limit, size_t smem) {
+        const int32_t row[8] = {wave, kind, tasks, C, threads, limit, int32_t(smem), int32_t(kSmemLimit)};
+        if (k < max) std::copy(row, row + 8, out + size_t(k) * 8);
+        ++k;
+    };
+    for (size_t wi = 0; wi < plan.waves.size(); ++wi)
+        for (const Group& g : plan.waves[wi].groups)
+            for (int ph = 0; ph < g.nph; ++ph) {
+                const PhaseCfg& pc = g.ph[ph];
+                put(int(wi), pc.staged ? 1 : 0, g.count, pc.C, pc.threads,
+                    phase_thread_limit(pc, g.nph == 2 && ph == 0), pc.smem);
+            }
+    *launches = k;
     return WQC_OK;
 }
 

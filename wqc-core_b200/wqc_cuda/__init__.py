@@ -49,7 +49,7 @@ EXPORTS = (
     "wqc_mps_amplitude_zero", "wqc_mps_site_amplitudes", "wqc_mps_bond_dims", "wqc_mps_download_site",
     "wqc_mps_upload_site", "wqc_mps_expectation_pauli", "wqc_mps_set_split_rule", "wqc_mps_split_count", "wqc_mps_split_records",
     "wqc_mps_peak_vram_bytes", "wqc_mps_backend_label", "wqc_mps_set_profiling", "wqc_mps_kernel_stats",
-    "wqc_mps_reset_stats", "wqc_mps_stream", "wqc_schedule_gates", "wqc_mps_reset", "wqc_mps_debug_workspace",
+    "wqc_mps_reset_stats", "wqc_mps_stream", "wqc_schedule_gates", "wqc_mps_reset", "wqc_mps_debug_workspace", "wqc_debug_svd_launches",
     "wqc_batch_create", "wqc_batch_apply_gates", "wqc_batch_amplitudes", "wqc_batch_slice_times",
     "wqc_expectation_pauli_noalloc", "wqc_batch_expectation_pauli", "wqc_mps_sample",
     "wqc_mps_overlap", "wqc_cuda_last_oom", "wqc_mps_site_amplitudes_many", "wqc_mps_to_dense",
@@ -156,6 +156,8 @@ def lib():
         L.wqc_schedule_gates.argtypes = [U32, P, U32, ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(ctypes.c_int32),
                                          U32, ctypes.POINTER(U32), ctypes.POINTER(U32)]
         L.wqc_mps_debug_workspace.argtypes = [P, U32, ctypes.c_int32, P, ctypes.c_uint64]
+        L.wqc_debug_svd_launches.argtypes = [U32, U32, U32] + [ctypes.c_int32] * 5 + [
+            P, U32, ctypes.POINTER(ctypes.c_int32), U32, ctypes.POINTER(U32)]
         L.wqc_batch_create.argtypes = [P, U32, ctypes.POINTER(U32), ctypes.POINTER(U32), ctypes.c_int32, U32,
                                        ctypes.POINTER(P)]
         L.wqc_batch_apply_gates.argtypes = [P, P, ctypes.POINTER(U32)]
