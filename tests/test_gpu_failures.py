@@ -47,6 +47,31 @@ def test_nan_site_gives_an_error_not_a_result(cuda_ctx):
     assert abs(m.amplitude_zero()) < 1e-15
 
 
+@pytest.mark.parametrize("bond", [32, 128])  # theta 64 x 64 and 256 x 256: the QR comes first
+@pytest.mark.parametrize("where", [(0, 0, 0), (-1, 1, 5)])
+def test_nan_before_the_qr_gives_the_same_error_every_time(cuda_ctx, bond, where):
+    """The columns of a theta that holds a NaN have no ranks by norm; whatever
+    their order, each is factored once, so the outcome does not depend on timing."""
+    rng = np.random.default_rng(bond)
+    dims = [1, bond, bond, bond, 1]
+    sites = [rng.standard_normal((dims[q], 2, dims[q + 1])) + 0j for q in range(4)]
+    sites[1][where] = np.nan
+    seen = set()
+    for _ in range(8):
+        m = W.CudaMps(4, bond, ctx=cuda_ctx)
+        m.set_split_rule(W.SPLIT_RULE_EXACT)
+        for q, t in enumerate(sites):
+            m.set_site(q, t)
+        m.apply_gates(C.gates_array([C.g2(C.CNOT, 1, 2)]))
+        with pytest.raises(W.WqcCudaError) as e:
+            m.synchronize()
+        seen.add((e.value.code, str(e.value)))
+        m.close()
+    assert len(seen) == 1, seen
+    code, text = seen.pop()
+    assert code == W.ERR_SVD_FAILED and "non-finite" in text
+
+
 def test_state_beyond_device_memory_is_refused(cuda_ctx):
     n = 100_000  # 100000 * 256^2 * 32 B = 210 GB of sites alone
     with pytest.raises(W.WqcCudaError) as e:

@@ -131,14 +131,16 @@ __global__ void __launch_bounds__(NW * 32) jacobi_qr_kernel(const SplitJob* jobs
     double fro2 = 0;
     for (int c = lane; c < N; c += 32) fro2 += norms[c];
     for (int o = 16; o > 0; o >>= 1) fro2 += __shfl_xor_sync(0xffffffffu, fro2, o);
+    // Every place of `order` is written once: a NaN among the norms (and so in
+    // their sum) leaves no ranks, and the columns stay where they are; the
+    // result is rejected later.
+    const bool ranked = fro2 == fro2;
     for (int c = tid; c < N; c += NW * 32) {
         const double nc = norms[c];
         int r = 0;
         for (int i = 0; i < N; ++i) r += (norms[i] > nc || (norms[i] == nc && i < c)) ? 1 : 0;
-        if (nc == nc) order[r] = c;
+        order[ranked ? r : c] = c;
     }
-    if (!(fro2 == fro2))  // NaN: any order, the result is rejected later
-        for (int c = tid; c < N; c += NW * 32) order[c] = c;
     __syncthreads();
     const double dust = sqrt(fro2) * kDustRel;
     const double dust2 = dust * dust;
