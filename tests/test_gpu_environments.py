@@ -79,6 +79,25 @@ def test_batch_expectation_matches_single_states(cuda_ctx, n, chis):
     b.close()
 
 
+@pytest.mark.parametrize("n,chis", [(12, [40, 8, 33, 24, 8]), (10, [3, 32, 16, 20])])
+def test_a_slice_has_the_same_expectation_in_any_batch(cuda_ctx, n, chis):
+    """Bit for bit: whether a slice's terms walk its sites or share chains is
+    decided by its own bonds."""
+    gates = [C.gates_array(C.ry_rz_brickwork(n, 9, s)) for s in range(len(chis))]
+    labels, coeffs = labels_of(n, 3), np.linspace(0.1, 1.0, 10)
+
+    def values(which):
+        b = W.CudaBatch([n] * len(which), [chis[s] for s in which], ctx=cuda_ctx)
+        b.apply_slices([gates[s] for s in which])
+        out = [complex(x) for x in b.expectations(labels, coeffs)]
+        b.close()
+        return out
+
+    together = values(range(len(chis)))
+    assert together == [values([s])[0] for s in range(len(chis))]
+    assert together[::-1] == values(range(len(chis))[::-1])
+
+
 @pytest.mark.parametrize("n,chi", [(5, 4), (10, 17), (12, 40)])
 def test_first_qubit_of_the_shots_follows_its_marginal(cuda_ctx, n, chi):
     tensors = sites(n, chi, n)

@@ -1370,15 +1370,14 @@ wqc_status sync_status(wqc_mps* m) {
 // small bonds, where a site's products are shorter than a launch, one launch
 // walks every term over all sites: bond 16, 20 sites 0.12 ms against 0.27; and
 // bond 24 where the terms span the register (20 such terms on 20 sites 0.22 ms
-// against 0.48, at bond 32 0.98 against 0.50).
+// against 0.48, at bond 32 0.98 against 0.50).  The rule looks at a segment's
+// own bonds: a slice's values do not depend on the other slices of its batch.
 constexpr int kPauliWalkBond = 16, kPauliWalkBondLong = 24;
 wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, const char* labels, uint32_t nterms,
                         std::vector<double2>& vals) {
     const int nseg = int(firsts.size());
     vals.resize(size_t(nseg) * nterms);
     const size_t E = size_t(m->chi) * m->chi;
-    int bond = 1;
-    for (int b : m->ub) bond = std::max(bond, b);
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
     const size_t lab_b = al(size_t(nterms) * width + 16), int_b = al(size_t(nterms) * sizeof(int));
     const size_t out_b = al(size_t(nseg) * nterms * sizeof(double2)), first_b = al(nseg * sizeof(int));
@@ -1395,16 +1394,35 @@ wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, c
         span[t] = hi < 0 ? 1 : hi - lo + 1;
         longest_all = std::max(longest_all, span[t]);
     }
-    const bool walk = bond <= kPauliWalkBond || (bond <= kPauliWalkBondLong && 2 * longest_all > width);
+    // The walked segments first, then those that take chains.
+    std::vector<int> order, chained;
+    int bond = 1;  // bound of the chained segments' bonds
+    for (int sl = 0; sl < nseg; ++sl) {
+        int own = 1;
+        for (int q = firsts[sl]; q + 1 < firsts[sl] + width; ++q) own = std::max(own, m->ub[q]);
+        if (own <= kPauliWalkBond || (own <= kPauliWalkBondLong && 2 * longest_all > width)) {
+            order.push_back(sl);
+        } else {
+            chained.push_back(sl);
+            bond = std::max(bond, own);
+        }
+    }
+    const int nwalk = int(order.size()), nchain = int(chained.size());
+    std::vector<int> chain_firsts;
+    for (int sl : chained) {
+        order.push_back(sl);
+        chain_firsts.push_back(firsts[sl]);
+    }
     // Segments and terms at a time, within the memory a state keeps.
     const size_t seg_b = (size_t(3) * width + 4) * E * sizeof(double2);
-    const int segs = walk ? 1 : int(std::max<size_t>(1, std::min<size_t>(size_t(std::min(nseg, 16384)), (kScratchKeep / 2) / seg_b)));
+    const int segs =
+        int(std::max<size_t>(1, std::min<size_t>(size_t(std::min(nchain, 16384)), (kScratchKeep / 2) / seg_b)));
     const size_t term_b = 4 * E * sizeof(double2);
-    const uint32_t terms = walk ? nterms
-                                : uint32_t(std::max<size_t>(1, std::min<size_t>(std::min<size_t>(nterms, 65535 / segs),
-                                                                                (kScratchKeep / 4) / (term_b * segs))));
+    const uint32_t terms = uint32_t(std::max<size_t>(
+        1, std::min<size_t>(std::min<size_t>(nterms, 65535 / segs), (kScratchKeep / 4) / (term_b * segs))));
     void* base = nullptr;
-    const size_t work_b = al(walk ? size_t(nterms) * term_b : size_t(segs) * (seg_b + size_t(terms) * term_b));
+    const size_t work_b = al(std::max(nwalk ? size_t(nterms) * term_b : 0,
+                                      nchain ? size_t(segs) * (seg_b + size_t(terms) * term_b) : 0));
     if (wqc_status s = get_scratch(m, work_b + lab_b + 2 * int_b + out_b + first_b, &base)) return s;
     char* p = static_cast<char*>(base);
     double2* work = reinterpret_cast<double2*>(p);
@@ -1414,23 +1432,23 @@ wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, c
     double2* d_out = reinterpret_cast<double2*>(reinterpret_cast<char*>(d_span) + int_b);
     int* d_first = reinterpret_cast<int*>(reinterpret_cast<char*>(d_out) + out_b);
     CUDA_TRY(cudaMemcpyAsync(d_lab, labels, size_t(nterms) * width, cudaMemcpyHostToDevice, m->stream));
-    if (walk) {
-        // One launch per segment on a view of its sites; launches share the scratch in stream order.
-        for (int s = 0; s < nseg; ++s) {
-            DeviceMps view = m->dev;
-            view.site += firsts[s];
-            view.dl += firsts[s];
-            view.dr += firsts[s];
-            view.n = width;
-            pauli_expectation_kernel<<<nterms, 256, 0, m->stream>>>(view, d_lab, int(nterms), work, m->chi,
-                                                                    d_out + size_t(s) * nterms);
-            count_launch(m, -1);
-        }
-    } else {
+    // One launch per walked segment on a view of its sites; launches share the scratch in stream order.
+    for (int s = 0; s < nwalk; ++s) {
+        const int first = firsts[order[s]];
+        DeviceMps view = m->dev;
+        view.site += first;
+        view.dl += first;
+        view.dr += first;
+        view.n = width;
+        pauli_expectation_kernel<<<nterms, 256, 0, m->stream>>>(view, d_lab, int(nterms), work, m->chi,
+                                                                d_out + size_t(s) * nterms);
+        count_launch(m, -1);
+    }
+    if (nchain) {
         CUDA_TRY(cudaMemcpyAsync(d_start, start.data(), nterms * sizeof(int), cudaMemcpyHostToDevice, m->stream));
         CUDA_TRY(cudaMemcpyAsync(d_span, span.data(), nterms * sizeof(int), cudaMemcpyHostToDevice, m->stream));
-        CUDA_TRY(cudaMemcpyAsync(d_first, firsts.data(), nseg * sizeof(int), cudaMemcpyHostToDevice, m->stream));
-        for (int s0 = 0; s0 < nseg; s0 += segs) {
+        CUDA_TRY(cudaMemcpyAsync(d_first, chain_firsts.data(), nchain * sizeof(int), cudaMemcpyHostToDevice, m->stream));
+        for (int s0 = 0; s0 < nchain; s0 += segs) {
             EnvChains ch{};
             ch.base = work;
             ch.seg_stride = (size_t(3) * width + 4) * E;
@@ -1439,7 +1457,7 @@ wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, c
             ch.r_off = ch.l_off + 2 * E;
             ch.h_off = ch.r_off + size_t(width) * E;
             ch.firsts = d_first + s0;
-            ch.nseg = std::min(segs, nseg - s0);
+            ch.nseg = std::min(segs, nchain - s0);
             ch.width = width;
             ch.cap = m->chi;
             ch.left = true;
@@ -1449,14 +1467,17 @@ wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, c
                 const int count = int(std::min<uint32_t>(terms, nterms - t0));
                 const int longest = *std::max_element(span.begin() + t0, span.begin() + t0 + count);
                 m->stats.total_launches += launch_env_terms(m->dev, ch, tm, int(t0), count, int(nterms), longest, bond,
-                                                            d_out + size_t(s0) * nterms, m->stream);
+                                                            d_out + size_t(nwalk + s0) * nterms, m->stream);
             }
         }
     }
     CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaMemcpyAsync(vals.data(), d_out, vals.size() * sizeof(double2), cudaMemcpyDeviceToHost, m->stream));
+    std::vector<double2> got(vals.size());
+    CUDA_TRY(cudaMemcpyAsync(got.data(), d_out, got.size() * sizeof(double2), cudaMemcpyDeviceToHost, m->stream));
     const wqc_status rc = sync_status(m);
     trim_scratch(m);
+    for (int s = 0; s < nseg; ++s)
+        std::copy_n(got.begin() + size_t(s) * nterms, nterms, vals.begin() + size_t(order[s]) * nterms);
     return rc;
 }
 
