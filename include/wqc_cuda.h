@@ -224,6 +224,11 @@ WQC_API wqc_status wqc_mps_set_merge(wqc_mps* mps, int32_t merge);
 WQC_API wqc_status wqc_schedule_gates(uint32_t n, const wqc_gate* gates, uint32_t count, int32_t* split_site,
                                       int32_t* split_level, uint32_t max, uint32_t* nsplits, uint32_t* nlevels);
 
+/* The state may allocate at most `bytes` more device memory than it holds now
+ * (0: no limit again): an allocation beyond that fails as on a full device.
+ * For tests of the calls that make do with less. */
+WQC_API wqc_status wqc_mps_debug_limit_bytes(wqc_mps* mps, uint64_t bytes);
+
 /* Host-only: the Jacobi launches that wqc_mps_apply_gates would make for
  * `gates` on a fresh state of n sites and bond chi (slices > 0: on a batch of
  * that many) on a device of sm_count SMs and clusters of up to max_cluster

@@ -111,3 +111,71 @@ def test_first_qubit_of_the_shots_follows_its_marginal(cuda_ctx, n, chi):
         ones = int(((draws >> np.uint64(q)) & np.uint64(1)).sum())
         assert abs(ones - shots * p1) <= 6 * np.sqrt(shots * max(p1 * (1 - p1), 1e-3))
     m.close()
+
+
+@pytest.mark.parametrize("n,chi,cap", [(14, 64, 64), (12, 33, 256)])
+@pytest.mark.parametrize("kib", [6000, 3600, 1200, 330])
+def test_expectation_makes_do_with_less_memory(cuda_ctx, n, chi, cap, kib):
+    """A device without room for the chains: fewer terms at a time (3600 KiB at
+    bond 64), then the walk over all sites, at last of one term (256 KiB and the
+    labels at bond 64).  No trace of the refused allocations is left."""
+    tensors = sites(n, chi, 7 * n + chi)
+    labels = labels_of(n, n)
+    coeffs = np.linspace(1.0, 2.0, len(labels))
+    want = sum(c * value(tensors, lab) for c, lab in zip(coeffs, labels))
+    m = W.CudaMps(n, cap, ctx=cuda_ctx)
+    for q, t in enumerate(tensors):
+        m.set_site(q, t)
+    before = W.last_oom()
+    m.debug_limit_bytes(kib << 10)
+    tol = 24 * n * chi * np.finfo(float).eps * coeffs.sum()
+    assert abs(m.expectation(labels, coeffs) - want) <= tol
+    assert W.last_oom() == before
+    m.debug_limit_bytes(0)
+    assert abs(m.expectation(labels, coeffs) - want) <= tol
+    m.close()
+
+
+def test_batch_expectation_makes_do_with_less_memory(cuda_ctx):
+    """Slices on both sides of the walking rule, all walking one term at a time."""
+    n, chis = 12, [40, 33, 7]
+    b = W.CudaBatch([n] * len(chis), chis, ctx=cuda_ctx)
+    b.apply_slices([C.gates_array(C.ry_rz_brickwork(n, 9, s)) for s in range(len(chis))])
+    labels, coeffs = labels_of(n, 3), np.linspace(0.1, 1.0, 10)
+    b.debug_limit_bytes(200 << 10)
+    little = b.expectations(labels, coeffs)
+    b.debug_limit_bytes(0)
+    tol = 24 * n * 40 * np.finfo(float).eps * np.abs(coeffs).sum() * 2  # either value's bound; states of norm near 1
+    assert np.abs(little - b.expectations(labels, coeffs)).max() <= tol
+    b.close()
+
+
+def test_a_read_that_finds_no_memory_is_refused_and_the_next_one_works(cuda_ctx):
+    n, chi = 14, 64
+    m = W.CudaMps(n, chi, ctx=cuda_ctx)
+    for q, t in enumerate(sites(n, chi, 1)):
+        m.set_site(q, t)
+    m.debug_limit_bytes(64 << 10)
+    for read in (lambda: m.expectation(["Z" * n], [1.0]), lambda: m.sample(range(n), 10, 1)):
+        with pytest.raises(W.WqcCudaError) as e:
+            read()
+        assert e.value.code == W.ERR_OOM and e.value.required > e.value.available
+    m.debug_limit_bytes(0)
+    assert np.isfinite(m.expectation(["Z" * n], [1.0])) and len(m.sample(range(n), 10, 1)) == 10
+    m.close()
+
+
+def test_shots_need_room_for_the_bonds_not_for_the_capacity(cuda_ctx):
+    """Right environments of bonds up to 32 take 60 KiB and their product's half
+    32 KiB; at the capacity of 256 they would take 14 MiB."""
+    n = 12
+    tensors = sites(n, 32, 5)
+    draws = []
+    for cap, kib in ((256, 400), (256, 0), (64, 0)):
+        m = W.CudaMps(n, cap, ctx=cuda_ctx)
+        for q, t in enumerate(tensors):
+            m.set_site(q, t)
+        m.debug_limit_bytes(kib << 10)
+        draws.append(m.sample(range(n), 500, 3).tolist())
+        m.close()
+    assert draws[0] == draws[1] == draws[2]

@@ -74,7 +74,8 @@ __global__ void __launch_bounds__(kTileThreads) env_chain_kernel(DeviceMps mps, 
     }
     // R_q[b][b'] contracts the sites right of q; R of the last site is [1].
     const int at = ch.width - 1 - step, q = first + at;
-    double2* R = base + ch.r_off + size_t(at) * E;
+    auto right_of = [&](int x) { return base + (ch.r_at ? size_t(ch.r_at[x]) : ch.r_off + size_t(x) * E); };
+    double2* R = right_of(at);
     double2* H = base + ch.h_off;
     const int l = mps.dl[q], r = mps.dr[q];
     const double2* s = mps.site[q];
@@ -87,7 +88,7 @@ __global__ void __launch_bounds__(kTileThreads) env_chain_kernel(DeviceMps mps, 
             [&](int x, int bp, double2 v) { H[size_t(x) * r + bp] = v; });
     } else {
         if (at == 0 || m0 >= l || n0 >= l) return;
-        double2* out = R - E;
+        double2* out = right_of(at - 1);
         tile_gemm(  // R[a][a'] = sum_{s, b'} H[a][s, b'] conj(A[a'][s, b'])
             sm, m0, n0, l, l, 2 * r, true, true, [&](int a, int x) { return H[size_t(a) * 2 * r + x]; },
             [&](int x, int ap) { return cconj(s[size_t(ap) * 2 * r + x]); },

@@ -48,6 +48,18 @@ wqc_status fail_oom(uint64_t required, uint64_t available) {
                                  std::to_string(available) + " bytes free on the device");
 }
 
+// The error state of the thread, put back by a call that made do without what
+// it was refused.
+struct ErrorState {
+    std::string err = g_err;
+    uint64_t required = g_oom_required, available = g_oom_available;
+    void restore() const {
+        g_err = err;
+        g_oom_required = required;
+        g_oom_available = available;
+    }
+};
+
 #define CUDA_TRY(expr)                                                                                    \
     do {                                                                                                  \
         cudaError_t e_ = (expr);                                                                          \
@@ -307,6 +319,7 @@ struct wqc_mps {
     bool uploaded = false;
     // accounting
     uint64_t bytes_now = 0, bytes_peak = 0;
+    uint64_t bytes_limit = ~uint64_t(0);  // wqc_mps_debug_limit_bytes
     bool profiling = false;
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> events;
     std::vector<cudaEvent_t> event_pool;
@@ -353,6 +366,8 @@ static wqc_status oz_enable(wqc_mps* m) {
 namespace {
 
 wqc_status dmalloc(wqc_mps* m, void** p, size_t bytes) {
+    if (m->bytes_now + bytes > m->bytes_limit)
+        return fail_oom(bytes, m->bytes_limit > m->bytes_now ? m->bytes_limit - m->bytes_now : 0);
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -1361,6 +1376,15 @@ wqc_status sync_status(wqc_mps* m) {
     return WQC_OK;
 }
 
+// The bonds left of every site, then right of every site, as they are on the
+// device; waits for the stream.
+wqc_status read_bonds(wqc_mps* m, std::vector<int>& dl_dr) {
+    dl_dr.resize(2 * size_t(m->n));
+    CUDA_TRY(cudaStreamSynchronize(m->stream));
+    CUDA_TRY(cudaMemcpy(dl_dr.data(), m->d_dl, dl_dr.size() * sizeof(int), cudaMemcpyDeviceToHost));
+    return WQC_OK;
+}
+
 // <psi|P_t|psi> of every term on every segment of `width` sites, vals[seg *
 // nterms + t]; ends with the state's synchronisation.  Terms are cut to the
 // sites between their first and last non-identity ones and share the identity
@@ -1372,12 +1396,16 @@ wqc_status sync_status(wqc_mps* m) {
 // bond 24 where the terms span the register (20 such terms on 20 sites 0.22 ms
 // against 0.48, at bond 32 0.98 against 0.50).  The rule looks at a segment's
 // own bonds: a slice's values do not depend on the other slices of its batch.
+// The chains hold 3 cap^2 entries a site, where cap is the state's chi_max; it
+// is the largest bond instead, which takes a synchronisation, where that
+// would be more than is kept between reads.  Where the device has no room for
+// the chains the terms go one at a time, and then all segments walk, with
+// four cap^2 entries for as many terms as fit.
 constexpr int kPauliWalkBond = 16, kPauliWalkBondLong = 24;
 wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, const char* labels, uint32_t nterms,
                         std::vector<double2>& vals) {
     const int nseg = int(firsts.size());
     vals.resize(size_t(nseg) * nterms);
-    const size_t E = size_t(m->chi) * m->chi;
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
     const size_t lab_b = al(size_t(nterms) * width + 16), int_b = al(size_t(nterms) * sizeof(int));
     const size_t out_b = al(size_t(nseg) * nterms * sizeof(double2)), first_b = al(nseg * sizeof(int));
@@ -1407,23 +1435,70 @@ wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, c
             bond = std::max(bond, own);
         }
     }
-    const int nwalk = int(order.size()), nchain = int(chained.size());
+    int nwalk = int(order.size()), nchain = int(chained.size());
     std::vector<int> chain_firsts;
     for (int sl : chained) {
         order.push_back(sl);
         chain_firsts.push_back(firsts[sl]);
     }
-    // Segments and terms at a time, within the memory a state keeps.
-    const size_t seg_b = (size_t(3) * width + 4) * E * sizeof(double2);
-    const int segs =
-        int(std::max<size_t>(1, std::min<size_t>(size_t(std::min(nchain, 16384)), (kScratchKeep / 2) / seg_b)));
-    const size_t term_b = 4 * E * sizeof(double2);
-    const uint32_t terms = uint32_t(std::max<size_t>(
-        1, std::min<size_t>(std::min<size_t>(nterms, 65535 / segs), (kScratchKeep / 4) / (term_b * segs))));
+    // Segments and terms at a time, within the memory that is kept between
+    // reads, or within what there is.
+    int segs = 1;
+    uint32_t terms = 1, walk_terms = nterms;
+    // Of an environment's side.  Not the host's bounds of the bonds: a split
+    // that a cancellation skips leaves a larger bond than they say.
+    int cap = m->chi;
+    size_t E = 1;
+    auto size_chains = [&](bool least) {
+        E = size_t(cap) * cap;
+        const size_t seg_b = (size_t(3) * width + 4) * E * sizeof(double2), term_b = 4 * E * sizeof(double2);
+        segs = least ? 1 : int(std::max<size_t>(1, std::min<size_t>(size_t(std::min(nchain, 16384)), (kScratchKeep / 2) / seg_b)));
+        terms = least ? 1
+                      : uint32_t(std::max<size_t>(1, std::min<size_t>(std::min<size_t>(nterms, 65535 / segs),
+                                                                      (kScratchKeep / 4) / (term_b * segs))));
+    };
+    auto work_bytes = [&]() {
+        const size_t walk_e = nwalk ? size_t(walk_terms) * 4 * E : 0;
+        const size_t chain_e = nchain ? size_t(segs) * ((size_t(3) * width + 4) * E + size_t(terms) * 4 * E) : 0;
+        return al(std::max(walk_e, chain_e) * sizeof(double2));
+    };
+    size_chains(false);
+    bool tight = false;
+    auto tighten = [&]() -> wqc_status {
+        std::vector<int> now;
+        if (wqc_status st = sync_status(m)) return st;
+        if (wqc_status st = read_bonds(m, now)) return st;
+        cap = *std::max_element(now.begin(), now.end());
+        bond = std::min(bond, cap);
+        tight = true;
+        size_chains(false);
+        return WQC_OK;
+    };
+    if (work_bytes() > kScratchKeep)
+        if (wqc_status st = tighten()) return st;
     void* base = nullptr;
-    const size_t work_b = al(std::max(nwalk ? size_t(nterms) * term_b : 0,
-                                      nchain ? size_t(segs) * (seg_b + size_t(terms) * term_b) : 0));
-    if (wqc_status s = get_scratch(m, work_b + lab_b + 2 * int_b + out_b + first_b, &base)) return s;
+    size_t work_b = 0;
+    for (const ErrorState before;;) {
+        work_b = work_bytes();
+        const wqc_status st = get_scratch(m, work_b + lab_b + 2 * int_b + out_b + first_b, &base);
+        if (st == WQC_OK) {
+            before.restore();
+            break;
+        }
+        if (st != WQC_ERR_OOM) return st;
+        if (!tight) {
+            if (wqc_status ts = tighten()) return ts;
+        } else if (nchain && (segs > 1 || terms > 1)) {
+            size_chains(true);
+        } else if (nchain) {
+            nwalk = nseg;
+            nchain = 0;
+        } else if (walk_terms > 1) {
+            walk_terms = (walk_terms + 1) / 2;
+        } else {
+            return st;
+        }
+    }
     char* p = static_cast<char*>(base);
     double2* work = reinterpret_cast<double2*>(p);
     char* d_lab = p + work_b;
@@ -1440,9 +1515,12 @@ wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, c
         view.dl += first;
         view.dr += first;
         view.n = width;
-        pauli_expectation_kernel<<<nterms, 256, 0, m->stream>>>(view, d_lab, int(nterms), work, m->chi,
-                                                                d_out + size_t(s) * nterms);
-        count_launch(m, -1);
+        for (uint32_t t0 = 0; t0 < nterms; t0 += walk_terms) {
+            const uint32_t count = std::min(walk_terms, nterms - t0);
+            pauli_expectation_kernel<<<count, 256, 0, m->stream>>>(view, d_lab + size_t(t0) * width, int(count), work,
+                                                                   cap, d_out + size_t(s) * nterms + t0);
+            count_launch(m, -1);
+        }
     }
     if (nchain) {
         CUDA_TRY(cudaMemcpyAsync(d_start, start.data(), nterms * sizeof(int), cudaMemcpyHostToDevice, m->stream));
@@ -1459,7 +1537,7 @@ wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, c
             ch.firsts = d_first + s0;
             ch.nseg = std::min(segs, nchain - s0);
             ch.width = width;
-            ch.cap = m->chi;
+            ch.cap = cap;
             ch.left = true;
             const EnvTerms tm{d_lab, d_start, d_span, work + size_t(segs) * ch.seg_stride};
             m->stats.total_launches += launch_env_chains(m->dev, ch, true, bond, m->stream);
@@ -1894,6 +1972,12 @@ wqc_status wqc_schedule_gates(uint32_t n, const wqc_gate* gates, uint32_t count,
     }
     *nsplits = k;
     *nlevels = uint32_t(top + 1);
+    return WQC_OK;
+}
+
+wqc_status wqc_mps_debug_limit_bytes(wqc_mps* m, uint64_t bytes) {
+    if (!m) return fail(WQC_ERR_INVALID, "null argument");
+    m->bytes_limit = bytes ? m->bytes_now + bytes : ~uint64_t(0);
     return WQC_OK;
 }
 
@@ -2352,31 +2436,41 @@ wqc_status wqc_mps_sample(wqc_mps* m, const uint32_t* qubits, uint32_t count, ui
     if (wqc_status s = check_uploaded_chain(m)) return s;
     if (wqc_status s = sync_status(m)) return s;
     const int n = m->n;
-    const size_t E = size_t(m->chi) * m->chi;
-    const size_t env_bytes = (size_t(n) + 2) * E * sizeof(double2);  // R of every site, H
-    const size_t aux_bytes = ((n + 1) * sizeof(int) + 255) & ~size_t(255);
+    // The right environment of site q (dr[q] x dr[q]) at env_at[q], then H.
+    std::vector<int> bonds;
+    if (wqc_status st = read_bonds(m, bonds)) return st;
+    const int bond = *std::max_element(bonds.begin(), bonds.end());
+    std::vector<unsigned long long> env_at(n);
+    size_t entries = 0;
+    for (int q = 0; q < n; ++q) {
+        env_at[q] = entries;
+        entries += size_t(bonds[n + q]) * bonds[n + q];
+    }
+    auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
+    const size_t env_bytes = al((entries + 2 * size_t(bond) * bond) * sizeof(double2));
+    const size_t at_bytes = al(n * sizeof(unsigned long long)), bit_bytes = al((n + 1) * sizeof(int));
     const size_t out_bytes = size_t(shots) * sizeof(uint64_t);
     void* base = nullptr;
-    if (wqc_status st = get_scratch(m, env_bytes + aux_bytes + out_bytes, &base)) return st;
+    if (wqc_status st = get_scratch(m, env_bytes + at_bytes + bit_bytes + out_bytes, &base)) return st;
     double2* env = static_cast<double2*>(base);
-    int* d_bitpos = reinterpret_cast<int*>(static_cast<char*>(base) + env_bytes);
-    auto* d_out = reinterpret_cast<unsigned long long*>(static_cast<char*>(base) + env_bytes + aux_bytes);
+    auto* d_at = reinterpret_cast<unsigned long long*>(static_cast<char*>(base) + env_bytes);
+    int* d_bitpos = reinterpret_cast<int*>(reinterpret_cast<char*>(d_at) + at_bytes);
+    auto* d_out = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(d_bitpos) + bit_bytes);
     bitpos.push_back(0);  // the chain's first site, after the bit positions
     CUDA_TRY(cudaMemcpyAsync(d_bitpos, bitpos.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice, m->stream));
+    CUDA_TRY(cudaMemcpyAsync(d_at, env_at.data(), n * sizeof(unsigned long long), cudaMemcpyHostToDevice, m->stream));
     EnvChains ch{};
     ch.base = env;
-    ch.r_off = 0;
-    ch.h_off = size_t(n) * E;
+    ch.r_at = d_at;
+    ch.h_off = entries;
     ch.firsts = d_bitpos + n;
     ch.nseg = 1;
     ch.width = n;
-    ch.cap = m->chi;
+    ch.cap = bond;
     ch.left = false;
-    int bond = 1;
-    for (int b : m->ub) bond = std::max(bond, b);
     m->stats.total_launches += launch_env_chains(m->dev, ch, true, bond, m->stream);
     const int grid = int(std::min<long>(long(shots), 8L * m->ctx->sm_count));
-    sample_shots_kernel<<<grid, 256, 3 * m->chi * sizeof(double2), m->stream>>>(m->dev, env, d_bitpos,
+    sample_shots_kernel<<<grid, 256, 3 * m->chi * sizeof(double2), m->stream>>>(m->dev, env, d_at, d_bitpos,
                                                                                 (unsigned long long)seed, int(shots), d_out);
     count_launch(m, -1);
     CUDA_TRY(cudaGetLastError());

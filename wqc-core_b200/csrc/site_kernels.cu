@@ -300,11 +300,11 @@ __device__ __forceinline__ double sample_uniform(unsigned long long seed, unsign
     return double(splitmix64(key + (unsigned long long)q) >> 11) * 0x1.0p-53;
 }
 
-// One CTA per shot (grid-stride over shots).  envs + q cap^2 holds E_{q+1}
-// (dr[q] x dr[q], the right environment of site q); bitpos[q] is the output bit of qubit q, or
-// -1 when q is not measured.  Dynamic shared memory: 3 * chi_max complex.
+// One CTA per shot (grid-stride over shots).  envs + env_at[q] holds E_{q+1}
+// (dr[q] x dr[q], the right environment of site q); bitpos[q] is the output
+// bit of qubit q, or -1 when q is not measured.  Dynamic shared memory: 3 * chi_max complex.
 __global__ void __launch_bounds__(256) sample_shots_kernel(DeviceMps mps, const double2* envs,
-                                                           const int* bitpos,
+                                                           const unsigned long long* env_at, const int* bitpos,
                                                            unsigned long long seed, int shots,
                                                            unsigned long long* out) {
     extern __shared__ __align__(16) double2 sv[];
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(256) sample_shots_kernel(DeviceMps mps, const 
         for (int q = 0; q < mps.n; ++q) {
             const int l = mps.dl[q], r = mps.dr[q];
             const double2* A = mps.site[q];
-            const double2* E = envs + size_t(q) * mps.chi_max * mps.chi_max;  // r x r
+            const double2* E = envs + env_at[q];  // r x r
             for (int c = tid; c < r; c += blockDim.x) {
                 double2 a0 = cmake(0, 0), a1 = cmake(0, 0);
                 for (int a = 0; a < l; ++a) {

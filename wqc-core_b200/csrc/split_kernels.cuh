@@ -153,10 +153,13 @@ __global__ void overlap_next_kernel(const double2* tmp, int bl, int kr, const do
 // Environments (env_kernels.cu).  The identity chains of `nseg` runs of
 // `width` sites (firsts[seg] ..), each with its buffers seg_stride entries
 // apart: T (2 cap^2 a site), L (two of cap^2), R (cap^2 a site; R_q contracts
-// the sites right of q) and H (2 cap^2).  `left` false: the right chain only.
+// the sites right of q) and H (2 cap^2).  `left` false: the right chain only;
+// then R may lie at offsets of its own, r_at[q], a site's no larger than its
+// bonds.
 struct EnvChains {
     double2* base;
     size_t seg_stride, t_off, l_off, r_off, h_off;
+    const unsigned long long* r_at;
     const int* firsts;
     int nseg, width, cap;
     bool left;
@@ -174,7 +177,8 @@ struct EnvTerms {
 int launch_env_chains(const DeviceMps& mps, const EnvChains& ch, bool right, int bond, cudaStream_t stream);
 int launch_env_terms(const DeviceMps& mps, const EnvChains& ch, const EnvTerms& tm, int t0, int count, int nterms,
                      int longest, int bond, double2* out, cudaStream_t stream);
-__global__ void sample_shots_kernel(DeviceMps mps, const double2* envs, const int* bitpos, unsigned long long seed, int shots, unsigned long long* out);
+__global__ void sample_shots_kernel(DeviceMps mps, const double2* envs, const unsigned long long* env_at,
+                                    const int* bitpos, unsigned long long seed, int shots, unsigned long long* out);
 
 // Adjoint kernels (adjoint_kernels.cu).
 struct Adj1q {

@@ -49,7 +49,8 @@ EXPORTS = (
     "wqc_mps_amplitude_zero", "wqc_mps_site_amplitudes", "wqc_mps_bond_dims", "wqc_mps_download_site",
     "wqc_mps_upload_site", "wqc_mps_expectation_pauli", "wqc_mps_set_split_rule", "wqc_mps_split_count", "wqc_mps_split_records",
     "wqc_mps_peak_vram_bytes", "wqc_mps_backend_label", "wqc_mps_set_profiling", "wqc_mps_kernel_stats",
-    "wqc_mps_reset_stats", "wqc_mps_stream", "wqc_schedule_gates", "wqc_mps_reset", "wqc_mps_debug_workspace", "wqc_debug_svd_launches",
+    "wqc_mps_reset_stats", "wqc_mps_stream", "wqc_schedule_gates", "wqc_mps_reset", "wqc_mps_debug_workspace",
+    "wqc_debug_svd_launches", "wqc_mps_debug_limit_bytes",
     "wqc_batch_create", "wqc_batch_apply_gates", "wqc_batch_amplitudes", "wqc_batch_slice_times",
     "wqc_expectation_pauli_noalloc", "wqc_batch_expectation_pauli", "wqc_mps_sample",
     "wqc_mps_overlap", "wqc_cuda_last_oom", "wqc_mps_site_amplitudes_many", "wqc_mps_to_dense",
@@ -156,6 +157,7 @@ def lib():
         L.wqc_schedule_gates.argtypes = [U32, P, U32, ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(ctypes.c_int32),
                                          U32, ctypes.POINTER(U32), ctypes.POINTER(U32)]
         L.wqc_mps_debug_workspace.argtypes = [P, U32, ctypes.c_int32, P, ctypes.c_uint64]
+        L.wqc_mps_debug_limit_bytes.argtypes = [P, ctypes.c_uint64]
         L.wqc_debug_svd_launches.argtypes = [U32, U32, U32] + [ctypes.c_int32] * 5 + [
             P, U32, ctypes.POINTER(ctypes.c_int32), U32, ctypes.POINTER(U32)]
         L.wqc_batch_create.argtypes = [P, U32, ctypes.POINTER(U32), ctypes.POINTER(U32), ctypes.c_int32, U32,
@@ -502,6 +504,10 @@ class CudaMps:
         out = np.zeros(count, dtype=dtype)
         _check(lib().wqc_mps_debug_workspace(self._h, slot, which, out.ctypes.data, out.nbytes))
         return out
+
+    def debug_limit_bytes(self, nbytes: int) -> None:
+        """At most `nbytes` more device memory from here on (see wqc_mps_debug_limit_bytes)."""
+        _check(lib().wqc_mps_debug_limit_bytes(self._h, nbytes))
 
     def stream(self) -> int:
         return int(lib().wqc_mps_stream(self._h) or 0)
