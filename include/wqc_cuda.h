@@ -10,6 +10,13 @@
  * thread at a time (the request's spawn_blocking thread, src/api.rs:342) and
  * owns one CUDA stream; calls enqueue device work and return, and the calls
  * that hand results to the host synchronise that stream.
+ *
+ * Memory: a state holds its sites and split workspace from its creation on.
+ * Pauli sums and shot sampling need more while they run; up to 512 MiB of that
+ * per device stays allocated for the next read of any state.  It is given back
+ * when an allocation of this library would fail without it, when the last
+ * state of the device is destroyed, and by wqc_cuda_device_info and
+ * wqc_cuda_close.
  */
 #ifndef WQC_CUDA_H
 #define WQC_CUDA_H
@@ -318,7 +325,11 @@ WQC_API wqc_status wqc_mps_sample(wqc_mps* mps, const uint32_t* qubits, uint32_t
 /* Sum_t coeff_t <psi|P_t|psi> for Pauli strings (labels: nterms strings of
  * qubit_count characters in IXYZ, character n-1-q acting on qubit q as in
  * src/expectation.rs:98-132; coeffs: re,im pairs).  Computed on the device
- * with transfer matrices, so it is not limited to 20 qubits. */
+ * with transfer matrices, so it is not limited to 20 qubits.  Above small
+ * bonds the terms share environments, (3 n + 4) chi^2 complex entries; where
+ * the device has no room for these, every term walks all sites, with four
+ * chi^2 entries for as many terms at a time as fit (WQC_ERR_OOM only when one
+ * does not). */
 WQC_API wqc_status wqc_mps_expectation_pauli(wqc_mps* mps, const char* labels, const double* coeffs, uint32_t nterms,
                                      double out[2]);
 

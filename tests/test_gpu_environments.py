@@ -179,3 +179,87 @@ def test_shots_need_room_for_the_bonds_not_for_the_capacity(cuda_ctx):
         draws.append(m.sample(range(n), 500, 3).tolist())
         m.close()
     assert draws[0] == draws[1] == draws[2]
+
+
+def free_bytes():
+    import torch
+
+    return torch.cuda.mem_get_info()[0]
+
+
+def read_state(ctx, n, chi, terms):
+    """A loaded state and a Pauli sum on it, with its value."""
+    tensors = sites(n, chi, n + chi)
+    m = W.CudaMps(n, chi, ctx=ctx)
+    for q, t in enumerate(tensors):
+        m.set_site(q, t)
+    labels = (labels_of(n, n) * (terms // 10 + 1))[:terms]
+    coeffs = np.full(terms, 1.0 / terms)
+    want = sum(c * value(tensors, lab) for c, lab in zip(coeffs[:10], labels[:10])) * (terms / 10)
+    return m, labels, coeffs, want
+
+
+def test_reads_of_many_states_keep_one_pool(cuda_ctx):
+    """What reads keep is bounded for the device, not for each state, and is
+    given back with the states or when the free memory is asked for."""
+    states = [read_state(cuda_ctx, 16, 128, 400) for _ in range(6)]
+    cuda_ctx.device_info()  # nothing idle
+    before = free_bytes()
+    for m, labels, coeffs, want in states:
+        assert abs(m.expectation(labels, coeffs) - want) <= 24 * 16 * 128 * np.finfo(float).eps
+        m.sample(range(16), 10, 1)
+    assert before - free_bytes() <= 512 << 20
+    cuda_ctx.device_info()
+    assert before - free_bytes() <= 4 << 20  # the allocator's granularity
+    for m, *_ in states:
+        m.close()
+
+
+def test_a_state_that_needs_what_reads_keep_gets_it(cuda_ctx):
+    import torch
+
+    cuda_ctx.device_info()
+    free0 = free_bytes()
+    m, labels, coeffs, want = read_state(cuda_ctx, 16, 128, 400)
+    cost = free0 - free_bytes()
+    m.expectation(labels, coeffs)
+    idle = free0 - cost - free_bytes()
+    assert 64 << 20 <= idle <= 512 << 20
+    ballast = torch.empty(free_bytes() - cost + idle // 2, dtype=torch.uint8, device="cuda")
+    try:
+        assert free_bytes() < cost
+        other = W.CudaMps(16, 128, ctx=cuda_ctx)
+        other.close()
+        assert abs(m.expectation(labels, coeffs) - want) <= 24 * 16 * 128 * np.finfo(float).eps
+    finally:
+        del ballast
+        torch.cuda.empty_cache()
+    m.close()
+
+
+def test_reads_of_several_threads_at_once(cuda_ctx):
+    """Threads with a state each share the pool, a block to one call at a time."""
+    import threading
+
+    shapes = [(12, 40, 30), (14, 64, 50), (13, 33, 10), (12, 90, 20)]
+    states = [read_state(cuda_ctx, *s) for s in shapes]
+    wrong = []
+
+    def work(k):
+        m, labels, coeffs, want = states[k]
+        n, chi, _ = shapes[k]
+        shots = m.sample(range(n), 50, k).tolist()
+        for _ in range(20):
+            if abs(m.expectation(labels, coeffs) - want) > 24 * n * chi * np.finfo(float).eps:
+                wrong.append(("value", k))
+            if m.sample(range(n), 50, k).tolist() != shots:
+                wrong.append(("shots", k))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(states))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    for m, *_ in states:
+        m.close()

@@ -955,7 +955,7 @@ wqc_status ensure_device(wqc_exact* ex, void** p, uint64_t* have, uint64_t need)
         *p = nullptr;
         *have = 0;
     }
-    if (cudaMalloc(p, need) != cudaSuccess) {
+    if (device_malloc(p, need) != cudaSuccess) {
         cudaGetLastError();
         *p = nullptr;
         size_t fr = 0, tot = 0;

@@ -23,6 +23,7 @@
 
 #include "../../include/wqc_cuda.h"
 #include "common.cuh"
+#include "scratch.h"
 #include "split_kernels.cuh"
 #include "tc_gemm.cuh"
 #include "tile_gemm.cuh"
@@ -285,7 +286,6 @@ struct wqc_mps {
     size_t h_stage_cap = 0;
     cudaEvent_t stage_done = nullptr;
     Arena d_stage;
-    Arena scratch;  // of the reads (environments, dense state), grown as they need it
     wqc_split_info* d_records = nullptr;
     size_t rec_cap = 0;
     uint32_t rec_count = 0;
@@ -320,6 +320,7 @@ struct wqc_mps {
     // accounting
     uint64_t bytes_now = 0, bytes_peak = 0;
     uint64_t bytes_limit = ~uint64_t(0);  // wqc_mps_debug_limit_bytes
+    int device = -1;                      // counted among its states (scratch.h); the context may close first
     bool profiling = false;
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> events;
     std::vector<cudaEvent_t> event_pool;
@@ -346,8 +347,8 @@ static wqc_status oz_enable(wqc_mps* m) {
     if (!m->oz_pool) {
         const int rpad = oz_rpad(2 * m->chi), npad = oz_npad(2 * m->chi), kpad = oz_kpad(m->chi);
         const size_t bytes = oz_state_bytes(m);
-        size_t fr = 0, tot = 0;
-        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return fail(WQC_ERR_CUDA, "cudaMemGetInfo");
+        size_t fr = 0;
+        if (device_room(bytes, &fr) != cudaSuccess) return fail(WQC_ERR_CUDA, "cudaMemGetInfo");
         if (bytes > fr) return fail_oom(bytes, fr);
         void* p = nullptr;
         if (wqc_status st = dmalloc(m, &p, bytes)) return st;
@@ -368,7 +369,7 @@ namespace {
 wqc_status dmalloc(wqc_mps* m, void** p, size_t bytes) {
     if (m->bytes_now + bytes > m->bytes_limit)
         return fail_oom(bytes, m->bytes_limit > m->bytes_now ? m->bytes_limit - m->bytes_now : 0);
-    cudaError_t e = cudaMalloc(p, bytes);
+    cudaError_t e = device_malloc(p, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
         size_t fr = 0, tot = 0;
@@ -385,31 +386,35 @@ void dfree(wqc_mps* m, void* p, size_t bytes) {
     m->bytes_now -= bytes;
 }
 
-// Device memory for one read, kept with the state for the next one (a
-// cudaMalloc and cudaFree a call cost more than most reads).  The reads of a
-// state follow one another on its stream, and each ends with a
-// synchronisation, so there is one arena.
-constexpr size_t kScratchKeep = size_t(512) << 20;  // larger arenas are given back after the call
-wqc_status get_scratch(wqc_mps* m, size_t bytes, void** p) {
-    if (bytes > m->scratch.cap) {
-        if (m->scratch.d) {
-            CUDA_TRY(cudaStreamSynchronize(m->stream));
-            dfree(m, m->scratch.d, m->scratch.cap);
-        }
-        m->scratch.d = nullptr;
-        m->scratch.cap = 0;
-        if (wqc_status s = dmalloc(m, &m->scratch.d, bytes)) return s;
-        m->scratch.cap = bytes;
+// Device memory of one read, from the device's pool; back there once the
+// state's stream has drained, whichever way the call ends.
+struct Scratch {
+    wqc_mps* m;
+    void* p = nullptr;
+    size_t cap = 0;
+    explicit Scratch(wqc_mps* mm) : m(mm) {}
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+    ~Scratch() {
+        if (!p) return;
+        cudaStreamSynchronize(m->stream);
+        m->bytes_now -= cap;
+        scratch_give(m->device, p, cap);
     }
-    *p = m->scratch.d;
-    return WQC_OK;
-}
-void trim_scratch(wqc_mps* m) {
-    if (m->scratch.cap <= kScratchKeep) return;
-    dfree(m, m->scratch.d, m->scratch.cap);
-    m->scratch.d = nullptr;
-    m->scratch.cap = 0;
-}
+    wqc_status get(size_t bytes) {
+        if (m->bytes_now + bytes <= m->bytes_limit) p = scratch_take(m->device, bytes, &cap);
+        if (!p) {
+            void* q = nullptr;
+            if (wqc_status s = dmalloc(m, &q, bytes)) return s;
+            p = q;
+            cap = bytes;
+            return WQC_OK;
+        }
+        m->bytes_now += cap;
+        m->bytes_peak = std::max(m->bytes_peak, m->bytes_now);
+        return WQC_OK;
+    }
+};
 
 std::once_flag g_attr_once;
 cudaError_t g_attr_err = cudaSuccess;
@@ -1476,11 +1481,11 @@ wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, c
     };
     if (work_bytes() > kScratchKeep)
         if (wqc_status st = tighten()) return st;
-    void* base = nullptr;
+    Scratch scratch(m);
     size_t work_b = 0;
     for (const ErrorState before;;) {
         work_b = work_bytes();
-        const wqc_status st = get_scratch(m, work_b + lab_b + 2 * int_b + out_b + first_b, &base);
+        const wqc_status st = scratch.get(work_b + lab_b + 2 * int_b + out_b + first_b);
         if (st == WQC_OK) {
             before.restore();
             break;
@@ -1499,7 +1504,7 @@ wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, c
             return st;
         }
     }
-    char* p = static_cast<char*>(base);
+    char* p = static_cast<char*>(scratch.p);
     double2* work = reinterpret_cast<double2*>(p);
     char* d_lab = p + work_b;
     int* d_start = reinterpret_cast<int*>(d_lab + lab_b);
@@ -1553,7 +1558,6 @@ wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, c
     std::vector<double2> got(vals.size());
     CUDA_TRY(cudaMemcpyAsync(got.data(), d_out, got.size() * sizeof(double2), cudaMemcpyDeviceToHost, m->stream));
     const wqc_status rc = sync_status(m);
-    trim_scratch(m);
     for (int s = 0; s < nseg; ++s)
         std::copy_n(got.begin() + size_t(s) * nterms, nterms, vals.begin() + size_t(order[s]) * nterms);
     return rc;
@@ -1631,11 +1635,15 @@ wqc_status wqc_cuda_open(int device, wqc_cuda_ctx** out) {
     return WQC_OK;
 }
 
-void wqc_cuda_close(wqc_cuda_ctx* ctx) { delete ctx; }
+void wqc_cuda_close(wqc_cuda_ctx* ctx) {
+    if (ctx) scratch_release(ctx->device);
+    delete ctx;
+}
 
 wqc_status wqc_cuda_device_info(wqc_cuda_ctx* ctx, uint64_t* total_bytes, uint64_t* free_bytes, int32_t* sm_count) {
     if (!ctx) return fail(WQC_ERR_INVALID, "null context");
     CUDA_TRY(cudaSetDevice(ctx->device));
+    scratch_release(ctx->device);
     size_t fr = 0, tot = 0;
     CUDA_TRY(cudaMemGetInfo(&fr, &tot));
     if (total_bytes) *total_bytes = tot;
@@ -1742,6 +1750,8 @@ static wqc_status create_state(wqc_cuda_ctx* ctx, const std::vector<int>& ns, co
     m->reject = reject;
     std::vector<size_t> site_off, bucket_bytes, bucket_gs;
     lay_out(m, ctx, ns, chis, precision, nslots_req, site_off, bucket_bytes, bucket_gs);
+    scratch_states(ctx->device, 1);
+    m->device = ctx->device;
     auto bail = [&](wqc_status st) {
         wqc_mps_destroy(m);
         return st;
@@ -1774,8 +1784,8 @@ static wqc_status create_state(wqc_cuda_ctx* ctx, const std::vector<int>& ns, co
     const bool oz_default = single_state && !m->tc;
     const uint64_t need = site_bytes + uint64_t(slot_pool_bytes) + tc_a_bytes + tc_b_bytes +
                           (oz_default ? oz_state_bytes(m) : 0);
-    size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return bail(fail(WQC_ERR_CUDA, "cudaMemGetInfo"));
+    size_t fr = 0;
+    if (device_room(need, &fr) != cudaSuccess) return bail(fail(WQC_ERR_CUDA, "cudaMemGetInfo"));
     if (need > fr) return bail(fail_oom(need, fr));
     void* p = nullptr;
     if (wqc_status st = dmalloc(m, &p, site_bytes)) return bail(st);
@@ -1936,7 +1946,6 @@ void wqc_mps_destroy(wqc_mps* m) {
     for (auto e : m->wave_done) cudaEventDestroy(e);
     if (m->call_start) cudaEventDestroy(m->call_start);
     dfree(m, m->d_stage.d, 0);
-    dfree(m, m->scratch.d, 0);
     if (m->h_stage) cudaFreeHost(m->h_stage);
     if (m->h_cancel) cudaFreeHost(const_cast<int*>(m->h_cancel));
     for (auto& e : m->events) {
@@ -1949,6 +1958,7 @@ void wqc_mps_destroy(wqc_mps* m) {
     if (m->join_ev) cudaEventDestroy(m->join_ev);
     if (m->side) cudaStreamDestroy(m->side);
     if (m->stream) cudaStreamDestroy(m->stream);
+    if (m->device >= 0) scratch_states(m->device, -1);
     delete m;
 }
 
@@ -2450,10 +2460,10 @@ wqc_status wqc_mps_sample(wqc_mps* m, const uint32_t* qubits, uint32_t count, ui
     const size_t env_bytes = al((entries + 2 * size_t(bond) * bond) * sizeof(double2));
     const size_t at_bytes = al(n * sizeof(unsigned long long)), bit_bytes = al((n + 1) * sizeof(int));
     const size_t out_bytes = size_t(shots) * sizeof(uint64_t);
-    void* base = nullptr;
-    if (wqc_status st = get_scratch(m, env_bytes + at_bytes + bit_bytes + out_bytes, &base)) return st;
-    double2* env = static_cast<double2*>(base);
-    auto* d_at = reinterpret_cast<unsigned long long*>(static_cast<char*>(base) + env_bytes);
+    Scratch scratch(m);
+    if (wqc_status st = scratch.get(env_bytes + at_bytes + bit_bytes + out_bytes)) return st;
+    double2* env = static_cast<double2*>(scratch.p);
+    auto* d_at = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch.p) + env_bytes);
     int* d_bitpos = reinterpret_cast<int*>(reinterpret_cast<char*>(d_at) + at_bytes);
     auto* d_out = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(d_bitpos) + bit_bytes);
     bitpos.push_back(0);  // the chain's first site, after the bit positions
@@ -2476,9 +2486,7 @@ wqc_status wqc_mps_sample(wqc_mps* m, const uint32_t* qubits, uint32_t count, ui
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, m->stream));
     m->stats.d2h_bytes += out_bytes;
-    const wqc_status rc = sync_status(m);
-    trim_scratch(m);
-    return rc;
+    return sync_status(m);
 }
 
 wqc_status wqc_mps_expectation_pauli(wqc_mps* m, const char* labels, const double* coeffs, uint32_t nterms,

@@ -731,7 +731,7 @@ wqc_status wqc_network_contract(wqc_network* net, uint32_t n, const wqc_gate* ga
         if (net->arena) cudaFree(net->arena);
         net->arena = nullptr;
         net->arena_bytes = 0;
-        if (cudaMalloc(reinterpret_cast<void**>(&net->arena), need) != cudaSuccess) {
+        if (device_malloc(reinterpret_cast<void**>(&net->arena), need) != cudaSuccess) {
             cudaGetLastError();
             size_t fr = 0, tot = 0;
             cudaMemGetInfo(&fr, &tot);
@@ -743,7 +743,7 @@ wqc_status wqc_network_contract(wqc_network* net, uint32_t n, const wqc_gate* ga
         if (net->table) cudaFree(net->table);
         net->table = nullptr;
         net->table_bytes = 0;
-        if (cudaMalloc(reinterpret_cast<void**>(&net->table), tab_bytes + jobs_bytes) != cudaSuccess) {
+        if (device_malloc(reinterpret_cast<void**>(&net->table), tab_bytes + jobs_bytes) != cudaSuccess) {
             cudaGetLastError();
             size_t fr = 0, tot = 0;
             cudaMemGetInfo(&fr, &tot);

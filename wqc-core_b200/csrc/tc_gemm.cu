@@ -13,6 +13,7 @@
 #include <string>
 
 #include "../../include/wqc_cuda.h"
+#include "scratch.h"
 #include "split_kernels.cuh"
 #include "tc_gemm.cuh"
 #include "tc_ptx.cuh"
@@ -432,8 +433,8 @@ WQC_API wqc_status wqc_tc_zgemm(wqc_cuda_ctx* ctx, uint32_t m, uint32_t n, uint3
                  bytes_c = size_t(m) * n * sizeof(double2);
     const size_t bytes_pa = size_t(2) * rpad * kpad * sizeof(float), bytes_pb = size_t(2) * npad * kpad * sizeof(float);
     const size_t need = bytes_a + bytes_b + bytes_c + bytes_pa + bytes_pb + 256;
-    size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return record_error(WQC_ERR_CUDA, "cudaMemGetInfo");
+    size_t fr = 0;
+    if (device_room(need, &fr) != cudaSuccess) return record_error(WQC_ERR_CUDA, "cudaMemGetInfo");
     if (need > fr) return record_oom(need, fr);
 
     void *dA = nullptr, *dB = nullptr, *dC = nullptr, *dPA = nullptr, *dPB = nullptr, *dSt = nullptr;

@@ -15,6 +15,7 @@
 #include <string>
 
 #include "../../include/wqc_cuda.h"
+#include "scratch.h"
 #include "split_kernels.cuh"
 #include "tc_gemm.cuh"
 #include "tc_ptx.cuh"
@@ -491,8 +492,8 @@ WQC_API wqc_status wqc_tc_zgemm_int8(wqc_cuda_ctx* ctx, uint32_t m, uint32_t n, 
     const size_t bytes_a = size_t(m) * k * sizeof(double2), bytes_b = size_t(k) * n * sizeof(double2),
                  bytes_c = size_t(m) * n * sizeof(double2), bytes_p = oz_planes_bytes(1, rpad, npad, kpad);
     const size_t need = bytes_a + bytes_b + bytes_c + bytes_p + 256;
-    size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return record_error(WQC_ERR_CUDA, "cudaMemGetInfo");
+    size_t fr = 0;
+    if (device_room(need, &fr) != cudaSuccess) return record_error(WQC_ERR_CUDA, "cudaMemGetInfo");
     if (need > fr) return record_oom(need, fr);
 
     void *dA = nullptr, *dB = nullptr, *dC = nullptr, *dP = nullptr, *dSt = nullptr;

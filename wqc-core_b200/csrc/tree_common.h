@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../include/wqc_cuda.h"
+#include "scratch.h"
 
 namespace wqc {
 wqc_status record_error(wqc_status code, const std::string& msg);  // executor.cu
