@@ -148,3 +148,50 @@ def test_adjoint_of_wide_steps_at_two_capacities(cuda_ctx, n, every):
         gp["angle"][i] += d
         shift.append(device_value(n, 32, gp, labels, coeffs, cuda_ctx))
     assert abs(g1[i] - 0.5 * (shift[0] - shift[1])) <= 1e-9 * max(1.0, np.abs(g0).max())
+
+
+def layers_of_splits(n, layers, seed):
+    rng = np.random.default_rng(seed)
+    g = []
+    for layer in range(layers):
+        g += [C.g1((C.RX, C.RY)[(q + layer) % 2], q, rng.uniform(0.3, 2.8)) for q in range(n)]
+        g += [C.g2(C.CNOT, q, q + 1) for q in range(layer % 2, n - 1, 2)]
+    return C.gates_array(g)
+
+
+@pytest.mark.parametrize("terms,layers,extra", [(31, 8, "one direction"), (1, 16, "one workspace")])
+def test_backward_makes_do_with_the_memory_of_one_split_at_a_time(cuda_ctx, terms, layers, extra):
+    """Where the device has no room for both directions' half-products, or for
+    more workspaces than one beside the tape, the reverse sweep does with
+    less; each product is the same, so the gradient is too."""
+    n, chi = 16, 64
+    gates = layers_of_splits(n, layers, 4)
+    labels, coeffs = C.zz_x_observable(n)
+    assert len(labels) == 31
+    labels, coeffs = labels[:terms], coeffs[:terms]
+    m = W.CudaMps(n, chi, ctx=cuda_ctx)
+    adj = W.Adjoint(m, gates)
+    want = adj.backward(labels, coeffs)
+    bars = n * 2 * chi * chi * 16
+    splits = sum(len(range(k % 2, n - 1, 2)) for k in range(layers))
+    if extra == "one direction":
+        env = chi * chi * 16
+        need = bars + terms * (2 * n + 1) * env + 2 * 16 * n * 2 * env + terms * 2 * env  # holes: 16 terms at a time
+    else:
+        site, square = 2 * chi * chi * 16, (2 * chi) ** 2 * 16
+        tape = splits * (2 * site + 2 * square + 2048) + layers * n * (site + 256) + splits * 1024
+        need = bars + tape + 10 * square
+    before = W.last_oom()
+    m.debug_limit_bytes(need + (1 << 20))  # less than another direction (4 MiB) or workspace (2.5 MiB)
+    got = adj.backward(labels, coeffs)
+    assert W.last_oom() == before
+    m.debug_limit_bytes(bars)
+    with pytest.raises(W.WqcCudaError) as e:
+        adj.backward(labels, coeffs)
+    assert e.value.code == W.ERR_OOM
+    m.debug_limit_bytes(0)
+    assert got[0] == want[0] and np.array_equal(got[1], want[1])
+    again = adj.backward(labels, coeffs)
+    assert again[0] == want[0] and np.array_equal(again[1], want[1])
+    adj.close()
+    m.close()

@@ -54,18 +54,18 @@ __device__ __forceinline__ double2 pauli_conj_row(char ch, const double2* a, int
 // envs: (n + 1) cap^2 entries per term for EL, then n cap^2 for ER;
 // tmp: cap * 2 * cap per term and direction.  <psi|P_t|psi> = EL_n[0][0].
 //
-// One half of one step for every term and both directions: blockIdx.x = 2 t +
-// direction, the left environments at site `step`, the right ones at the
-// mirrored site.  phase 0 multiplies the environment into the site, phase 1
+// One half of one step for every term and both directions (dirs = 2, blockIdx.x
+// = 2 t + direction) or one of them (dirs = 1: `dir`), the left environments
+// at site `step`, the right ones at the mirrored site.  phase 0 multiplies the environment into the site, phase 1
 // closes it.  The walk is a chain of n steps, so what bounds it is the latency of
 // a step: 63 terms on 32 sites at chi 64 took 25.6 ms with one CTA per term, and
 // take 2 ms with one CTA per tile of a step's products.
 __global__ void __launch_bounds__(kTileThreads) adj_pauli_envs_kernel(DeviceMps mps, const char* labels, int cap,
-                                                                      int step, int phase, double2* envs,
-                                                                      double2* tmp_all) {
+                                                                      int dirs, int dir, int step, int phase,
+                                                                      double2* envs, double2* tmp_all) {
     __shared__ TileSmem sm;
-    const int t = blockIdx.x >> 1;
-    const bool right = blockIdx.x & 1;
+    const int t = blockIdx.x / dirs;
+    const bool right = dir + int(blockIdx.x) % dirs == 1;
     const int n = mps.n, q = right ? n - 1 - step : step;
     const size_t E = size_t(cap) * cap;
     double2* EL = envs + size_t(t) * (2 * n + 1) * E;

@@ -2843,7 +2843,23 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
         if (wqc_status st = buf.get(&d_lab, size_t(nterms) * n + 16)) return st;
         if (wqc_status st = buf.get(&d_cre, nterms)) return st;
         if (wqc_status st = buf.get(&envs, size_t(nterms) * (2 * n + 1) * E)) return st;
-        if (wqc_status st = buf.get(&tmp, size_t(nterms) * 4 * E)) return st;
+        // Holes in chunks of terms, accumulated in term order.
+        const size_t per_term = 2 * size_t(n) * site_cap * sizeof(double2);
+        const int chunk = int(std::max<size_t>(1, std::min<size_t>(16, (size_t(1) << 30) / per_term)));
+        double2 *holes = nullptr, *htmp = nullptr;
+        if (wqc_status st = buf.get(&holes, size_t(chunk) * n * site_cap)) return st;
+        if (wqc_status st = buf.get(&htmp, size_t(chunk) * n * site_cap)) return st;
+        // Half-products of both directions, or of one after the other where
+        // the device has no room for both.
+        int dirs = 2;
+        for (const ErrorState before;; dirs = 1) {
+            const wqc_status st = buf.get(&tmp, size_t(nterms) * 2 * dirs * E);
+            if (st == WQC_OK) {
+                before.restore();
+                break;
+            }
+            if (st != WQC_ERR_OOM || dirs == 1) return st;
+        }
         std::vector<double> cre(nterms);
         for (uint32_t t = 0; t < nterms; ++t) cre[t] = coeffs[2 * t];
         CUDA_TRY(cudaMemcpyAsync(d_lab, labels, size_t(nterms) * n, cudaMemcpyHostToDevice, m->stream));
@@ -2851,19 +2867,14 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
         int bond = 1;
         for (int b : m->ub) bond = std::max(bond, b);
         const unsigned b1 = unsigned(bond + kTile - 1) / kTile, b2 = unsigned(2 * bond + kTile - 1) / kTile;
-        for (int step = 0; step < n; ++step)
-            for (int phase = 0; phase < 2; ++phase) {
-                const unsigned t = phase == 0 ? b2 : b1;
-                adj_pauli_envs_kernel<<<dim3(2 * nterms, t, t), kTileThreads, 0, m->stream>>>(m->dev, d_lab, chi, step,
-                                                                                              phase, envs, tmp);
-                count_launch(m, -1);
-            }
-        // Holes in chunks of terms, accumulated in term order.
-        const size_t per_term = 2 * size_t(n) * site_cap * sizeof(double2);
-        const int chunk = int(std::max<size_t>(1, std::min<size_t>(16, (size_t(1) << 30) / per_term)));
-        double2 *holes = nullptr, *htmp = nullptr;
-        if (wqc_status st = buf.get(&holes, size_t(chunk) * n * site_cap)) return st;
-        if (wqc_status st = buf.get(&htmp, size_t(chunk) * n * site_cap)) return st;
+        for (int dir = 0; dir < 2; dir += dirs)
+            for (int step = 0; step < n; ++step)
+                for (int phase = 0; phase < 2; ++phase) {
+                    const unsigned t = phase == 0 ? b2 : b1;
+                    adj_pauli_envs_kernel<<<dim3(dirs * nterms, t, t), kTileThreads, 0, m->stream>>>(
+                        m->dev, d_lab, chi, dirs, dir, step, phase, envs, tmp);
+                    count_launch(m, -1);
+                }
         const int agrid = int(std::max<size_t>(1, std::min<size_t>((site_cap + 255) / 256, 64)));
         for (uint32_t t0 = 0; t0 < nterms; t0 += uint32_t(chunk)) {
             const int cnt = int(std::min<uint32_t>(uint32_t(chunk), nterms - t0));
@@ -2905,17 +2916,24 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
     CUDA_TRY(cudaMemsetAsync(d_grad, 0, (n1q + 1) * sizeof(double), m->stream));
     std::vector<int> slot_gate;  // gate of each gradient slot
     // Split workspaces (ten column-major R x R matrices each), for as many
-    // splits of a step at a time as fit 256 MiB, or else the device: a circuit
-    // of ladders has about half a segment's layers in a step.
+    // splits of a step at a time as fit 256 MiB, or else what the tape leaves of
+    // the device: a circuit of ladders has about half a segment's layers in a step.
     const size_t RR = size_t(R) * R, ws_b = (10 * RR) * sizeof(double2) + 2 * size_t(R) * sizeof(double);
     const size_t most = size_t(std::min(m->bucket_cap[0], 32768));
     char* ws = nullptr;
     size_t width = std::max<size_t>(1, std::min(most, (size_t(256) << 20) / ws_b));
-    for (;; width /= 2) {
-        const wqc_status st = buf.get(&ws, width * ws_b);
-        if (st == WQC_OK) break;
-        if (width == 1) return st;
-    }
+    auto get_ws = [&]() -> wqc_status {
+        const ErrorState before;
+        for (;; width /= 2) {
+            const wqc_status st = buf.get(&ws, width * ws_b);
+            if (st == WQC_OK) {
+                before.restore();
+                return st;
+            }
+            if (st != WQC_ERR_OOM || width == 1) return st;
+        }
+    };
+    if (wqc_status st = get_ws()) return st;
     // Tape layout of one operation (bytes, 256-aligned parts).
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
     AdjTapeLayout L{};
@@ -2962,7 +2980,19 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
         if (need > tape_cap) {
             if (tape) buf.release(tape);
             tape = nullptr;
-            if (wqc_status st = buf.get(&tape, need)) return st;
+            tape_cap = 0;
+            // The tape comes before workspaces for more than one split.
+            for (const ErrorState before;;) {
+                const wqc_status st = buf.get(&tape, need);
+                if (st == WQC_OK) {
+                    before.restore();
+                    break;
+                }
+                if (st != WQC_ERR_OOM || width == 1) return st;
+                buf.release(ws);
+                width /= 2;
+                if (wqc_status ws_st = get_ws()) return ws_st;
+            }
             tape_cap = need;
         }
         std::vector<size_t> slot_of(ex.ops.size());

@@ -220,8 +220,8 @@ struct AdjSplit {
 };
 enum { kAdjStageOther = 0, kAdjStageM, kAdjStageN, kAdjStageT1, kAdjStageTb, kAdjStageTb2, kAdjStageBarL,
        kAdjStageBarR };
-__global__ void adj_pauli_envs_kernel(DeviceMps mps, const char* labels, int cap, int step, int phase, double2* envs,
-                                      double2* tmp_all);
+__global__ void adj_pauli_envs_kernel(DeviceMps mps, const char* labels, int cap, int dirs, int dir, int step, int phase,
+                                      double2* envs, double2* tmp_all);
 __global__ void adj_pauli_holes_kernel(DeviceMps mps, const char* labels, int t0, int cap, int phase,
                                        const double2* envs, double2* tmp_all, double2* holes);
 __global__ void adj_pauli_accumulate_kernel(DeviceMps mps, double2* const* bars, const double2* holes,
