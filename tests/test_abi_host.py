@@ -194,3 +194,21 @@ def test_pauli_labels_are_checked_before_the_c_abi():
         W.expectation_pauli_noalloc(0, 8, [2, 2, 1], ["ZZ"], [1.0])
     with pytest.raises(ValueError, match="coefficients"):
         W.expectation_pauli_noalloc(0, 8, [2, 2, 1], ["ZZZ"], [])
+
+
+def test_ptxas_report_reads_every_source_and_fails_with_the_compiler(tmp_path):
+    """A stand-in for nvcc that refuses several sources under -c -o, as nvcc
+    does, and prints what ptxas -v prints."""
+    import subprocess
+
+    nvcc = tmp_path / "nvcc"
+    nvcc.write_text('#!/bin/sh\nn=0\nfor a in "$@"; do case "$a" in *.cu) n=$((n + 1)); f=$a;; esac; done\n'
+                    '[ $n -eq 1 ] || { echo "a single input file is required"; exit 1; }\n'
+                    'echo "ptxas info : Compiling entry function of $f"\necho "ptxas info : Used 40 registers"\n')
+    nvcc.chmod(0o755)
+    make = ["make", "-s", "-C", os.path.join(ROOT, "wqc-core_b200"), "ptxas-report"]
+    got = subprocess.run(make + [f"NVCC={nvcc}"], capture_output=True, text=True)
+    assert got.returncode == 0, got.stderr
+    for src in ("split_kernels.cu", "jacobi_ring.cu", "jacobi_qr.cu"):
+        assert src in got.stdout
+    assert subprocess.run(make + ["NVCC=false"], capture_output=True).returncode != 0
