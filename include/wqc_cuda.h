@@ -169,7 +169,10 @@ WQC_API wqc_status wqc_mps_reset(wqc_mps* mps);
  * CNOT/CZ with SWAP routing and undo (mps.rs:353-375), CCNOT as the
  * reference's 15-gate decomposition (mps.rs:657-677); MEASURE/RESET/IF are
  * no-ops.  Splits on disjoint sites run concurrently; each site sees exactly
- * the reference's sequence of operations. */
+ * the reference's sequence of operations.  A split keeps the singular values
+ * above 1e-12 (svd_guard.rs:12); an exact SVD reports those at or below 4e-15
+ * of its matrix's Frobenius norm, where rounding alone leaves values, as zero,
+ * which comes before the absolute cutoff for norms above about 250. */
 WQC_API wqc_status wqc_mps_apply_gates(wqc_mps* mps, const wqc_gate* gates, uint32_t count);
 
 /* MpsState::apply_gate_adjoint (mps.rs:301-331) for each gate in order. */
@@ -380,8 +383,12 @@ WQC_API wqc_status wqc_expectation_pauli_noalloc(const double* sites, uint64_t s
  * a checkpoint of the sites at each gate index in `checkpoints` (for
  * instance the first gate of every second layer) and at the end; the state
  * then holds the circuit's output.  Every split takes the exact SVD (the
- * range finder's rank-48 test matrix has no meaningful derivative); single
- * states in the plain FP64 form only.
+ * range finder's rank-48 test matrix has no meaningful derivative), and runs
+ * the Jacobi on theta itself, where wqc_mps_apply_gates takes a QR first: the
+ * derivative needs the vectors of small singular values to more digits.  So
+ * the forward's state and that of the same gates through wqc_mps_apply_gates
+ * agree to rounding, not bit for bit.  Single states in the plain FP64 form
+ * only.
  *
  * wqc_adjoint_backward: value[0] = f, value[1] = sum_t Im(c_t) <P_t>;
  * grad[i] = d f / d angle of gate i (0 for gates without an angle).  The
