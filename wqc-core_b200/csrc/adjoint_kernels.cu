@@ -75,7 +75,8 @@ __global__ void __launch_bounds__(kTileThreads) adj_pauli_envs_kernel(DeviceMps 
     const int l = mps.dl[q], r = mps.dr[q], m0 = blockIdx.y * kTile, n0 = blockIdx.z * kTile;
     const double2* A = mps.site[q];
     const bool first = step == 0;  // the environment is [1]
-    if (first && phase == 0 && m0 == 0 && n0 == 0 && threadIdx.x == 0) (right ? ER + size_t(n - 1) * E : EL)[0] = cmake(1.0, 0.0);
+    if (first && phase == 0 && m0 == 0 && n0 == 0 && threadIdx.x == 0)
+        (right ? ER + size_t(n - 1) * E : EL)[0] = cmake(1.0, 0.0);
     if (!right) {
         const double2* cur = EL + size_t(q) * E;  // l x l
         double2* nxt = EL + size_t(q + 1) * E;    // r x r
@@ -296,7 +297,8 @@ __global__ void __launch_bounds__(256) adj_split_prep_kernel(const AdjSplit* spl
 }
 
 // The split's GEMMs as FP64 tiles (tile_gemm.cuh; 32 x 32 tiles put a 128 x 128
-// product on 16 CTAs and took 8.8 us) over strided, optionally conjugated views, with the dimensions read from the tape's SplitState.
+// product on 16 CTAs and took 8.8 us) over strided, optionally conjugated
+// views, with the dimensions read from the tape's SplitState.
 // Stages (kAdjStage*): Other, the side W does not hold (V = theta^H U s^-1,
 // or U = theta V s^-1); M = U^H U_bar; N = V^H V_bar; T1 += U Z;
 // theta_bar = T1 V^H; theta_bar += U Q2^H; the cotangent of site p,

@@ -111,20 +111,6 @@ struct SlotBuffers {
     void* gs;        // staged Jacobi workspace (padded W and Z columns), chi_max > 128 only
 };
 
-// One Jacobi SVD task: decompose X where column j of the tall working matrix
-// W (M x N, M >= N) is column j of src (rows_of_src = 0, M = src rows) or the
-// conjugate of row j of src (rows_of_src = 1, M = src cols).  src is
-// row-major with leading dimension ld.
-struct SvdTask {
-    const double2* src;
-    int src_rows, src_cols, ld;
-    int rows_of_src;
-    int active;
-    double2* w_out;  // M x N column-major
-    double2* z_out;  // N x N column-major
-    double* sigma;   // N
-};
-
 struct DeviceMps {
     double2** site;  // n pointers, each of capacity chi_cap * 2 * chi_cap
     int* dl;         // left bond of each site

@@ -20,8 +20,8 @@ __device__ __forceinline__ double2 pauli_row(char ch, int so, double2 t0, double
 }
 
 // T[a'][s][b] = sum_a E[a][a'] A[a][s][b]; E is [1] at the left end.
-__device__ __forceinline__ void left_half(TileSmem& sm, const DeviceMps& mps, int q, const double2* env, bool first, double2* T,
-                                          int m0, int n0) {
+__device__ __forceinline__ void left_half(TileSmem& sm, const DeviceMps& mps, int q, const double2* env, bool first,
+                                          double2* T, int m0, int n0) {
     const int l = mps.dl[q], r = mps.dr[q];
     if (m0 >= l || n0 >= 2 * r) return;
     const double2* s = mps.site[q];
@@ -33,8 +33,8 @@ __device__ __forceinline__ void left_half(TileSmem& sm, const DeviceMps& mps, in
 }
 
 // E'[b][b'] = sum_{a', s} (P T)[a'][s][b] conj(A[a'][s][b']).
-__device__ __forceinline__ void left_next(TileSmem& sm, const DeviceMps& mps, int q, const double2* T, char ch, double2* out, int m0,
-                                          int n0) {
+__device__ __forceinline__ void left_next(TileSmem& sm, const DeviceMps& mps, int q, const double2* T, char ch,
+                                          double2* out, int m0, int n0) {
     const int l = mps.dl[q], r = mps.dr[q];
     if (m0 >= r || n0 >= r) return;
     const double2* s = mps.site[q];
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256) env_dot_kernel(DeviceMps mps, EnvChains c
 
 // Every step of the identity chains; `bond` bounds the bonds.  Two launches a
 // site for both chains of every segment, instead of a walk over all sites on
-// one CTA per Pauli term (50 sites, chi 128, 99 terms: 142 ms).
+// one CTA per Pauli term (50 sites, chi 128, 99 terms: 141 ms).
 int launch_env_chains(const DeviceMps& mps, const EnvChains& ch, bool right, int bond, cudaStream_t stream) {
     const unsigned z = unsigned(ch.nseg) * ((ch.left ? 1 : 0) + (right ? 1 : 0));
     const unsigned b1 = unsigned(bond + kTile - 1) / kTile, b2 = unsigned(2 * bond + kTile - 1) / kTile;

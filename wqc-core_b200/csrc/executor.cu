@@ -1189,7 +1189,8 @@ wqc_status launch_plan(wqc_mps* m, Plan& plan) {
             cudaStream_t ps = aside ? m->side : on;
             {
                 Timed t(m, 4, ps);
-                svd_probe_kernel<<<dim3(nj, 2), kProbeThreads, 0, ps>>>(d_jobs, m->d_state, m->d_slots, mode, 0, m->d_status);
+                svd_probe_kernel<<<dim3(nj, 2), kProbeThreads, 0, ps>>>(d_jobs, m->d_state, m->d_slots, mode, 0,
+                                                                        m->d_status);
                 count_launch(m, 4);
             }
             if (aside) CUDA_TRY(cudaEventRecord(m->join_ev, m->side));
@@ -1457,7 +1458,9 @@ wqc_status pauli_values(wqc_mps* m, const std::vector<int>& firsts, int width, c
     auto size_chains = [&](bool least) {
         E = size_t(cap) * cap;
         const size_t seg_b = (size_t(3) * width + 4) * E * sizeof(double2), term_b = 4 * E * sizeof(double2);
-        segs = least ? 1 : int(std::max<size_t>(1, std::min<size_t>(size_t(std::min(nchain, 16384)), (kScratchKeep / 2) / seg_b)));
+        segs = least ? 1
+                     : int(std::max<size_t>(1, std::min<size_t>(size_t(std::min(nchain, 16384)),
+                                                                (kScratchKeep / 2) / seg_b)));
         terms = least ? 1
                       : uint32_t(std::max<size_t>(1, std::min<size_t>(std::min<size_t>(nterms, 65535 / segs),
                                                                       (kScratchKeep / 4) / (term_b * segs))));
