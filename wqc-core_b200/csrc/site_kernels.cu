@@ -300,9 +300,11 @@ __device__ __forceinline__ double sample_uniform(unsigned long long seed, unsign
     return double(splitmix64(key + (unsigned long long)q) >> 11) * 0x1.0p-53;
 }
 
-// One CTA per shot (grid-stride over shots).  envs + env_at[q] holds E_{q+1}
-// (dr[q] x dr[q], the right environment of site q); bitpos[q] is the output
-// bit of qubit q, or -1 when q is not measured.  Dynamic shared memory: 3 * chi_max complex.
+// One CTA per shot (grid-stride over shots).  envs + q chi_max^2, or with
+// kPacked envs + env_at[q], holds E_{q+1} (dr[q] x dr[q], the right environment
+// of site q); bitpos[q] is the output bit of qubit q, or -1 when q
+// is not measured.  Dynamic shared memory: 3 * chi_max complex.
+template <bool kPacked>
 __global__ void __launch_bounds__(256) sample_shots_kernel(DeviceMps mps, const double2* envs,
                                                            const unsigned long long* env_at, const int* bitpos,
                                                            unsigned long long seed, int shots,
@@ -320,7 +322,7 @@ __global__ void __launch_bounds__(256) sample_shots_kernel(DeviceMps mps, const 
         for (int q = 0; q < mps.n; ++q) {
             const int l = mps.dl[q], r = mps.dr[q];
             const double2* A = mps.site[q];
-            const double2* E = envs + env_at[q];  // r x r
+            const double2* E = envs + (kPacked ? size_t(env_at[q]) : size_t(q) * mps.chi_max * mps.chi_max);  // r x r
             for (int c = tid; c < r; c += blockDim.x) {
                 double2 a0 = cmake(0, 0), a1 = cmake(0, 0);
                 for (int a = 0; a < l; ++a) {
@@ -370,5 +372,9 @@ __global__ void __launch_bounds__(256) sample_shots_kernel(DeviceMps mps, const 
         if (tid == 0) out[shot] = bits;
     }
 }
+template __global__ void sample_shots_kernel<false>(DeviceMps, const double2*, const unsigned long long*, const int*,
+                                                    unsigned long long, int, unsigned long long*);
+template __global__ void sample_shots_kernel<true>(DeviceMps, const double2*, const unsigned long long*, const int*,
+                                                   unsigned long long, int, unsigned long long*);
 
 }  // namespace wqc

@@ -177,6 +177,7 @@ struct EnvTerms {
 int launch_env_chains(const DeviceMps& mps, const EnvChains& ch, bool right, int bond, cudaStream_t stream);
 int launch_env_terms(const DeviceMps& mps, const EnvChains& ch, const EnvTerms& tm, int t0, int count, int nterms,
                      int longest, int bond, double2* out, cudaStream_t stream);
+template <bool kPacked>
 __global__ void sample_shots_kernel(DeviceMps mps, const double2* envs, const unsigned long long* env_at,
                                     const int* bitpos, unsigned long long seed, int shots, unsigned long long* out);
 
