@@ -11,6 +11,7 @@
 #include <sys/stat.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -837,16 +838,6 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                 return choose_cluster(m->ctx, M, N, m->ctx->max_cluster, nj_wave, m->ctx->sm_count, elem, m->batch,
                                       vrows, most_warps);
             };
-            // A shape beyond every cluster goes to the staged kernel: its key
-            // is -b, the width of its blocks (0: no kernel takes it).
-            auto key_of = [&](int M, int N, size_t elem, int vrows, int most_warps, int& c) {
-                const int kr = jacobi_ring_kr(elem == sizeof(float2), M, vrows);
-                c = cluster_of(M, N, elem, vrows, most_warps);
-                if (c >= 1) return m->batch ? kr : 1;
-                c = cluster_of(M, N, elem, vrows, 32);
-                if (c >= 1) return 1 + kr;
-                return -jacobi_staged_b(M + vrows, N, elem, kSmemLimit, nullptr);
-            };
             struct WaveTask {
                 int mode, M, N, local;
             };
@@ -881,23 +872,42 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                     add_task(kJacobiRsvd, M, N, local);
                 }
             }
-            // Warps of the instance that the cluster tasks of a mode share, per phase.
+            // Cluster sizes, and the warps of the instance that the cluster
+            // tasks of a mode share, per phase.
+            const int phases = m->fp32 ? 2 : 1;
+            auto elem_of = [&](int ph) { return m->fp32 && ph == 0 ? sizeof(float2) : sizeof(double2); };
+            auto vrows_of = [&](const WaveTask& t, int ph) { return m->fp32 && ph == 0 ? t.N : 0; };
+            auto kr_of = [&](const WaveTask& t, int ph) {
+                return jacobi_ring_kr(m->fp32 && ph == 0, t.M, vrows_of(t, ph));
+            };
+            std::vector<std::array<int, 2>> sizes(wave_tasks.size());
             int most_warps[3][2] = {{32, 32}, {32, 32}, {32, 32}};
-            const size_t elem1 = m->fp32 ? sizeof(float2) : sizeof(double2);
-            if (!m->batch)
-                for (const WaveTask& t : wave_tasks)
-                    for (int ph = 0; ph < (m->fp32 ? 2 : 1); ++ph) {
-                        const size_t elem = ph == 0 ? elem1 : sizeof(double2);
-                        const int vrows = m->fp32 && ph == 0 ? t.N : 0;
-                        if (cluster_of(t.M, t.N, elem, vrows, 32) < 1) continue;
-                        const int kr = jacobi_ring_kr(elem == sizeof(float2), t.M, vrows);
-                        most_warps[t.mode][ph] = std::min(most_warps[t.mode][ph], jacobi_ring_warps(kr, int(elem)));
-                    }
-            for (const WaveTask& t : wave_tasks) {
-                Task out{t.local, 0, 0};
-                const int k1 = key_of(t.M, t.N, elem1, m->fp32 ? t.N : 0, most_warps[t.mode][0], out.c1);
-                const int k2 = m->fp32 ? key_of(t.M, t.N, sizeof(double2), 0, most_warps[t.mode][1], out.c2) : 0;
-                add(t.mode, k1, k2, out);
+            for (size_t i = 0; i < wave_tasks.size(); ++i)
+                for (int ph = 0; ph < phases; ++ph) {
+                    const WaveTask& t = wave_tasks[i];
+                    sizes[i][ph] = cluster_of(t.M, t.N, elem_of(ph), vrows_of(t, ph), 32);
+                    if (!m->batch && sizes[i][ph] >= 1)
+                        most_warps[t.mode][ph] =
+                            std::min(most_warps[t.mode][ph], jacobi_ring_warps(kr_of(t, ph), int(elem_of(ph))));
+                }
+            // A shape beyond every cluster goes to the staged kernel: its key
+            // is -b, the width of its blocks (0: no kernel takes it).
+            auto key_of = [&](const WaveTask& t, int ph, int& c) {
+                if (c < 1) return -jacobi_staged_b(t.M + vrows_of(t, ph), t.N, elem_of(ph), kSmemLimit, nullptr);
+                if (m->batch) return kr_of(t, ph);
+                RingShape s;
+                ring_shape(t.M, t.N, vrows_of(t, ph), elem_of(ph), c, &s);
+                if (s.warps <= most_warps[t.mode][ph]) return 1;
+                const int shared = cluster_of(t.M, t.N, elem_of(ph), vrows_of(t, ph), most_warps[t.mode][ph]);
+                if (shared < 1) return 1 + kr_of(t, ph);
+                c = shared;
+                return 1;
+            };
+            for (size_t i = 0; i < wave_tasks.size(); ++i) {
+                const WaveTask& t = wave_tasks[i];
+                Task out{t.local, sizes[i][0], sizes[i][1]};
+                const int k1 = key_of(t, 0, out.c1);
+                add(t.mode, k1, m->fp32 ? key_of(t, 1, out.c2) : 0, out);
             }
             // Launch shape of one phase for the tasks of a group.
             auto fill = [&](PhaseCfg& pc, int key, bool first, int mode, const std::vector<Task>& tasks, size_t elem,
