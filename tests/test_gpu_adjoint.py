@@ -195,3 +195,23 @@ def test_backward_makes_do_with_the_memory_of_one_split_at_a_time(cuda_ctx, term
     assert again[0] == want[0] and np.array_equal(again[1], want[1])
     adj.close()
     m.close()
+
+
+def test_backward_of_a_register_whose_environments_pass_2_gib_a_term(cuda_ctx):
+    """1024 sites at chi 256: (2 n + 1) chi^2 complex128 entries a term are
+    beyond the 2^31 - 1 bytes that a strided copy's pitch may have.  Rotations of a product
+    state: f = 0.5 cos a + 2 cos b - 3 cos a cos c in closed form."""
+    n, (a, b, c) = 1024, (0.7, 1.9, 2.6)
+    gates = C.gates_array([C.g1(C.RX, 0, a), C.g1(C.RY, n - 1, b), C.g1(C.RX, n // 2, c)])
+    coeffs = [0.5, 2.0, -3.0]
+    labels = ["".join("Z" if n - 1 - i in sites else "I" for i in range(n))
+              for sites in ((0,), (n - 1,), (0, n // 2))]
+    m = W.CudaMps(n, 256, ctx=cuda_ctx)
+    adj = W.Adjoint(m, gates)
+    f, g = adj.backward(labels, coeffs)
+    adj.close()
+    m.close()
+    # a few roundings of values up to 5.5
+    assert abs(f - (0.5 * np.cos(a) + 2 * np.cos(b) - 3 * np.cos(a) * np.cos(c))) <= 1e-13
+    want = np.array([-0.5 * np.sin(a) + 3 * np.sin(a) * np.cos(c), -2 * np.sin(b), 3 * np.cos(a) * np.sin(c)])
+    assert np.abs(g - want).max() <= 1e-13

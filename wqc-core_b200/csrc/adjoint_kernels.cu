@@ -152,6 +152,15 @@ __global__ void __launch_bounds__(kTileThreads) adj_pauli_holes_kernel(DeviceMps
     }
 }
 
+// <psi|P_t|psi> of every term side by side (a strided copy's pitch, the
+// environments of a term, ends at 2 GiB: 1024 sites at chi 256).
+__global__ void __launch_bounds__(256) adj_pauli_values_kernel(const double2* envs, int n, int cap, int nterms,
+                                                               double2* vals) {
+    const size_t E = size_t(cap) * cap;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nterms; t += gridDim.x * blockDim.x)
+        vals[t] = envs[(size_t(t) * (2 * n + 1) + n) * E];
+}
+
 // bar[q][e] (+)= sum over the chunk's terms, in term order, 2 Re(c_t) conj(H).
 __global__ void __launch_bounds__(256) adj_pauli_accumulate_kernel(DeviceMps mps, double2* const* bars,
                                                                    const double2* holes, const double* coef_re,

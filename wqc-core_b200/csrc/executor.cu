@@ -2649,10 +2649,10 @@ void* wqc_mps_stream(wqc_mps* m) { return m ? static_cast<void*>(m->stream) : nu
 // end, are copied to checkpoints.  Backward: the site cotangents of the end
 // state come from the observable's environments; then, segment by segment
 // from the last, the segment's state is restored from its checkpoint and its
-// operations are recomputed one at a time, the inputs each needs in reverse
-// (the site before a one-qubit gate; the sites, theta and the Jacobi's W,
-// singular values and order of a split) copied to a tape, and the tape is
-// swept in reverse (adjoint_kernels.cu).  The split rule is the exact one on
+// operations are recomputed by steps of disjoint ones, the inputs each needs
+// in reverse (the site before a one-qubit gate; the sites, theta and the
+// Jacobi's W, singular values and order of a split) copied to a tape, and the
+// tape is swept in reverse (adjoint_kernels.cu).  The split rule is the exact one on
 // every split (a range finder seeded by a rank-48 test matrix has no
 // meaningful derivative), and the plain FP64 form is required.
 // ===========================================================================
@@ -2879,9 +2879,10 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
         const size_t E = size_t(chi) * chi;
         char* d_lab = nullptr;
         double* d_cre = nullptr;
-        double2 *envs = nullptr, *tmp = nullptr;
+        double2 *envs = nullptr, *tmp = nullptr, *vals = nullptr;
         if (wqc_status st = buf.get(&d_lab, size_t(nterms) * n + 16)) return st;
         if (wqc_status st = buf.get(&d_cre, nterms)) return st;
+        if (wqc_status st = buf.get(&vals, nterms)) return st;
         if (wqc_status st = buf.get(&envs, size_t(nterms) * (2 * n + 1) * E)) return st;
         // Holes in chunks of terms, accumulated in term order.
         const size_t per_term = 2 * size_t(n) * site_cap * sizeof(double2);
@@ -2928,11 +2929,12 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
             count_launch(m, -1);
             count_launch(m, -1);
         }
+        const unsigned vgrid = std::min((nterms + 255) / 256, 1024u);
+        adj_pauli_values_kernel<<<vgrid, 256, 0, m->stream>>>(envs, n, chi, int(nterms), vals);
+        count_launch(m, -1);
         CUDA_TRY(cudaGetLastError());
         std::vector<double2> hv(nterms);
-        // <psi|P_t|psi>: the first entry of every term's last left environment.
-        CUDA_TRY(cudaMemcpy2DAsync(hv.data(), sizeof(double2), envs + size_t(n) * E, (2 * size_t(n) + 1) * E * sizeof(double2),
-                                   sizeof(double2), nterms, cudaMemcpyDeviceToHost, m->stream));
+        CUDA_TRY(cudaMemcpyAsync(hv.data(), vals, nterms * sizeof(double2), cudaMemcpyDeviceToHost, m->stream));
         CUDA_TRY(cudaStreamSynchronize(m->stream));
         double re = 0, im = 0;
         for (uint32_t t = 0; t < nterms; ++t) {  // coeff * Re<P> (expectation.rs:177-185), term order

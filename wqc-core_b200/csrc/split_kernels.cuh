@@ -225,6 +225,7 @@ __global__ void adj_pauli_envs_kernel(DeviceMps mps, const char* labels, int cap
                                       double2* envs, double2* tmp_all);
 __global__ void adj_pauli_holes_kernel(DeviceMps mps, const char* labels, int t0, int cap, int phase,
                                        const double2* envs, double2* tmp_all, double2* holes);
+__global__ void adj_pauli_values_kernel(const double2* envs, int n, int cap, int nterms, double2* vals);
 __global__ void adj_pauli_accumulate_kernel(DeviceMps mps, double2* const* bars, const double2* holes,
                                             const double* coef_re, int t0, int count, int cap, int first);
 __global__ void adj_one_qubit_kernel(const Adj1q* gates, double* grad);
