@@ -20,6 +20,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/wqc_cuda.h"
@@ -746,6 +747,7 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
     }
     plan.nsplits = seq - plan.first_seq;
     plan.slice_last_wave.assign(m->seg_first.size(), -1);
+    std::unordered_map<uint64_t, int> cluster_memo;
     for (LevelBuild& lb : levels) {
         // one-qubit ops run first, in one wave with no splits when needed
         std::vector<char> taken(lb.jobs.size(), 0);
@@ -834,9 +836,17 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                 remaining -= sel.size();
             }
             const int nj_wave = int(sel.size());
+            // A wave holds few shapes many times over: a shape's cluster size is
+            // worked out once (in a batch once for all waves, as it does not
+            // depend on their size).
+            if (!m->batch) cluster_memo.clear();
             auto cluster_of = [&](int M, int N, size_t elem, int vrows, int most_warps) {
-                return choose_cluster(m->ctx, M, N, m->ctx->max_cluster, nj_wave, m->ctx->sm_count, elem, m->batch,
-                                      vrows, most_warps);
+                const uint64_t key = (((uint64_t(M) * 1024 + N) * 1024 + vrows) * 64 + most_warps) * 2 + (elem == sizeof(float2));
+                const auto known = cluster_memo.emplace(key, 0);
+                if (known.second)
+                    known.first->second = choose_cluster(m->ctx, M, N, m->ctx->max_cluster, nj_wave, m->ctx->sm_count,
+                                                         elem, m->batch, vrows, most_warps);
+                return known.first->second;
             };
             struct WaveTask {
                 int mode, M, N, local;
