@@ -159,30 +159,34 @@ def layers_of_splits(n, layers, seed):
     return C.gates_array(g)
 
 
-@pytest.mark.parametrize("terms,layers,extra", [(31, 8, "one direction"), (1, 16, "one workspace")])
-def test_backward_makes_do_with_the_memory_of_one_split_at_a_time(cuda_ctx, terms, layers, extra):
-    """Where the device has no room for both directions' half-products, or for
-    more workspaces than one beside the tape, the reverse sweep does with
-    less; each product is the same, so the gradient is too."""
-    n, chi = 16, 64
+@pytest.mark.parametrize("n,terms,layers,extra", [(16, 31, 8, "holes in their place"), (4, 100, 8, "one direction"),
+                                                  (16, 1, 16, "one workspace")])
+def test_backward_makes_do_with_the_memory_of_one_split_at_a_time(cuda_ctx, n, terms, layers, extra):
+    """Where the device has no room for the half-products beside the holes, or
+    for those of both directions, or for more workspaces than one beside the
+    tape, the reverse sweep does with less; each product is the same, so the
+    gradient is too."""
+    chi = 64
     gates = layers_of_splits(n, layers, 4)
     labels, coeffs = C.zz_x_observable(n)
-    assert len(labels) == 31
-    labels, coeffs = labels[:terms], coeffs[:terms]
+    assert len(labels) == 2 * n - 1
+    labels, coeffs = (labels * 15)[:terms], np.tile(coeffs, 15)[:terms]
     m = W.CudaMps(n, chi, ctx=cuda_ctx)
     adj = W.Adjoint(m, gates)
     want = adj.backward(labels, coeffs)
     bars = n * 2 * chi * chi * 16
     splits = sum(len(range(k % 2, n - 1, 2)) for k in range(layers))
-    if extra == "one direction":
+    if extra != "one workspace":
         env = chi * chi * 16
-        need = bars + terms * (2 * n + 1) * env + 2 * 16 * n * 2 * env + terms * 2 * env  # holes: 16 terms at a time
+        holes, both = 2 * 16 * n * 2 * env, 4 * terms * env  # holes: 16 terms at a time
+        assert (both < holes) == (extra == "holes in their place") and both > 1 << 20
+        need = bars + terms * (2 * n + 1) * env + (holes if both < holes else (holes + both) // 2)
     else:
         site, square = 2 * chi * chi * 16, (2 * chi) ** 2 * 16
         tape = splits * (2 * site + 2 * square + 2048) + layers * n * (site + 256) + splits * 1024
         need = bars + tape + 10 * square
     before = W.last_oom()
-    m.debug_limit_bytes(need + (1 << 20))  # less than another direction (4 MiB) or workspace (2.5 MiB)
+    m.debug_limit_bytes(need + (1 << 20))  # less than a workspace (2.5 MiB)
     got = adj.backward(labels, coeffs)
     assert W.last_oom() == before
     m.debug_limit_bytes(bars)

@@ -2891,15 +2891,9 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
         double* d_cre = nullptr;
         double2 *envs = nullptr, *tmp = nullptr, *vals = nullptr;
         if (wqc_status st = buf.get(&d_lab, size_t(nterms) * n + 16)) return st;
-        if (wqc_status st = buf.get(&d_cre, nterms)) return st;
-        if (wqc_status st = buf.get(&vals, nterms)) return st;
+        if (wqc_status st = buf.get(&vals, nterms + (size_t(nterms) + 1) / 2)) return st;
+        d_cre = reinterpret_cast<double*>(vals + nterms);
         if (wqc_status st = buf.get(&envs, size_t(nterms) * (2 * n + 1) * E)) return st;
-        // Holes in chunks of terms, accumulated in term order.
-        const size_t per_term = 2 * size_t(n) * site_cap * sizeof(double2);
-        const int chunk = int(std::max<size_t>(1, std::min<size_t>(16, (size_t(1) << 30) / per_term)));
-        double2 *holes = nullptr, *htmp = nullptr;
-        if (wqc_status st = buf.get(&holes, size_t(chunk) * n * site_cap)) return st;
-        if (wqc_status st = buf.get(&htmp, size_t(chunk) * n * site_cap)) return st;
         // Half-products of both directions, or of one after the other where
         // the device has no room for both.
         int dirs = 2;
@@ -2926,6 +2920,23 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
                         m->dev, d_lab, chi, dirs, dir, step, phase, envs, tmp);
                     count_launch(m, -1);
                 }
+        // Holes in chunks of terms, accumulated in term order.  Allocated while
+        // the environments are worked out (0.6 ms), and in their half-products'
+        // place where the device has no room beside these.
+        const size_t per_term = 2 * size_t(n) * site_cap * sizeof(double2);
+        const int chunk = int(std::max<size_t>(1, std::min<size_t>(16, (size_t(1) << 30) / per_term)));
+        double2 *holes = nullptr, *htmp = nullptr;
+        for (double2** p : {&holes, &htmp}) {
+            const ErrorState before;
+            wqc_status st = buf.get(p, size_t(chunk) * n * site_cap);
+            if (st == WQC_ERR_OOM && tmp) {
+                buf.release(tmp);
+                tmp = nullptr;
+                st = buf.get(p, size_t(chunk) * n * site_cap);
+                if (st == WQC_OK) before.restore();
+            }
+            if (st != WQC_OK) return st;
+        }
         const int agrid = int(std::max<size_t>(1, std::min<size_t>((site_cap + 255) / 256, 64)));
         for (uint32_t t0 = 0; t0 < nterms; t0 += uint32_t(chunk)) {
             const int cnt = int(std::min<uint32_t>(uint32_t(chunk), nterms - t0));
@@ -2954,7 +2965,7 @@ wqc_status wqc_adjoint_backward(wqc_adjoint* a, const char* labels, const double
         value[0] = re;
         value[1] = im;
         buf.release(envs);
-        buf.release(tmp);
+        if (tmp) buf.release(tmp);
         buf.release(holes);
         buf.release(htmp);
     }
