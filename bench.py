@@ -1237,7 +1237,7 @@ def run_cuda(args) -> None:
                 "peak": peak,
                 "unit": "TFLOP/s",
                 "frac": (achieved / peak) if (achieved and peak) else None,
-                "traffic": 10713344,
+                "traffic": 10630912,
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one saturated QR launch and its "
                                   "Jacobi launch (five exact 256 x 256 splits on 16-CTA clusters, caches flushed "
                                   "before each): the input once each; the columns stay on the SMs",
