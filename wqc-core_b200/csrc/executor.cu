@@ -20,7 +20,6 @@
 #include <cstring>
 #include <mutex>
 #include <string>
-#include <unordered_map>
 #include <vector>
 
 #include "../../include/wqc_cuda.h"
@@ -747,7 +746,19 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
     }
     plan.nsplits = seq - plan.first_seq;
     plan.slice_last_wave.assign(m->seg_first.size(), -1);
-    std::unordered_map<uint64_t, int> cluster_memo;
+    struct WaveTask {
+        int mode, M, N, local;
+    };
+    std::vector<WaveTask> wave_tasks;
+    std::vector<std::array<int, 2>> sizes;
+    // A plan holds few shapes many times over: the cluster sizes last worked
+    // out, by shape and (outside batches, where it counts) the wave's splits.
+    // M, N and V's rows are at most 512, warps 32 and splits 2^24.
+    struct KnownCluster {
+        uint64_t key = 0;
+        int C = 0;
+    };
+    std::array<KnownCluster, 256> known_clusters;
     for (LevelBuild& lb : levels) {
         // one-qubit ops run first, in one wave with no splits when needed
         std::vector<char> taken(lb.jobs.size(), 0);
@@ -836,22 +847,17 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
                 remaining -= sel.size();
             }
             const int nj_wave = int(sel.size());
-            // A wave holds few shapes many times over: a shape's cluster size is
-            // worked out once (in a batch once for all waves, as it does not
-            // depend on their size).
-            if (!m->batch) cluster_memo.clear();
             auto cluster_of = [&](int M, int N, size_t elem, int vrows, int most_warps) {
-                const uint64_t key = (((uint64_t(M) * 1024 + N) * 1024 + vrows) * 64 + most_warps) * 2 + (elem == sizeof(float2));
-                const auto known = cluster_memo.emplace(key, 0);
-                if (known.second)
-                    known.first->second = choose_cluster(m->ctx, M, N, m->ctx->max_cluster, nj_wave, m->ctx->sm_count,
-                                                         elem, m->batch, vrows, most_warps);
-                return known.first->second;
+                const uint64_t shape_key = (uint64_t(M) << 20 | uint64_t(N) << 10 | uint64_t(vrows)) << 7 |
+                                           uint64_t(most_warps) << 1 | (elem == sizeof(float2) ? 1 : 0);
+                const uint64_t key = uint64_t(m->batch ? 0 : nj_wave) << 37 | shape_key;
+                KnownCluster& known = known_clusters[(key * 0x9E3779B97F4A7C15ull) >> 56];
+                if (known.key != key)
+                    known = {key, choose_cluster(m->ctx, M, N, m->ctx->max_cluster, nj_wave, m->ctx->sm_count, elem,
+                                                 m->batch, vrows, most_warps)};
+                return known.C;
             };
-            struct WaveTask {
-                int mode, M, N, local;
-            };
-            std::vector<WaveTask> wave_tasks;
+            wave_tasks.clear();
             auto add_task = [&](int mode, int M, int N, int local) { wave_tasks.push_back({mode, M, N, local}); };
             w.jobs_off = int(plan.jobs.size());
             w.njobs = nj_wave;
@@ -890,7 +896,7 @@ void build_plan(wqc_mps* m, const std::vector<Op>& ops, Plan& plan) {
             auto kr_of = [&](const WaveTask& t, int ph) {
                 return jacobi_ring_kr(m->fp32 && ph == 0, t.M, vrows_of(t, ph));
             };
-            std::vector<std::array<int, 2>> sizes(wave_tasks.size());
+            sizes.resize(wave_tasks.size());
             int most_warps[3][2] = {{32, 32}, {32, 32}, {32, 32}};
             for (size_t i = 0; i < wave_tasks.size(); ++i)
                 for (int ph = 0; ph < phases; ++ph) {
